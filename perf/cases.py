@@ -47,27 +47,27 @@ MLA_LAYERS = 4
 def listed():
     return [
         # a small model answering one user: nothing but latency
-        dict(name="dense small, 1 sequence", family="dense", size="small", kind="decode", rows=1, context=129),
+        dict(name="dense small 1 row", family="dense", size="small", kind="decode", rows=1, context=129),
         # the 2B model, one user with a conversation behind them
-        dict(name="dense 2b, 1 sequence", family="dense", size="2b", kind="decode", rows=1, context=2000),
+        dict(name="dense 2b 1 row", family="dense", size="2b", kind="decode", rows=1, context=2000),
         # a few users at once
-        dict(name="dense 2b, 8 sequences", family="dense", size="2b", kind="decode", rows=8, context=3000),
+        dict(name="dense 2b 8 rows", family="dense", size="2b", kind="decode", rows=8, context=3000),
         # a full server
-        dict(name="dense 2b, 64 sequences", family="dense", size="2b", kind="decode", rows=64, context=4096),
+        dict(name="dense 2b 64 rows", family="dense", size="2b", kind="decode", rows=64, context=4096),
         # an ordinary prompt, of no round length
-        dict(name="dense 2b, prompt 509", family="dense", size="2b", kind="prompt", rows=509, context=509),
+        dict(name="dense 2b prompt 509", family="dense", size="2b", kind="prompt", rows=509, context=509),
         # a long document
-        dict(name="dense 2b, prompt 4096", family="dense", size="2b", kind="prompt", rows=4096, context=4096),
-        dict(name="falinex 2b, 1 sequence", family="falinex", size="2b", kind="decode", rows=1, context=1500),
+        dict(name="dense 2b prompt 4096", family="dense", size="2b", kind="prompt", rows=4096, context=4096),
+        dict(name="falinex 2b 1 row", family="falinex", size="2b", kind="decode", rows=1, context=1500),
         # a server between quiet and full
-        dict(name="falinex 2b, 27 sequences", family="falinex", size="2b", kind="decode", rows=27, context=3000),
+        dict(name="falinex 2b 27 rows", family="falinex", size="2b", kind="decode", rows=27, context=3000),
         # continuous batching: a prompt's portion beside the decode rows of running sequences
-        dict(name="falinex 2b, prompt 1500 beside 5", family="falinex", size="2b", kind="prompt", rows=1500, others=5, context=1600),
+        dict(name="falinex 2b prompt 1500 beside 5", family="falinex", size="2b", kind="prompt", rows=1500, others=5, context=1600),
         # the headline benchmark's step and its prompt
-        dict(name="mla_moe, 1 sequence", family="mla_moe", kind="decode", rows=1, context=512, experts="bf16"),
+        dict(name="mla_moe 1 row", family="mla_moe", kind="decode", rows=1, context=512, experts="bf16"),
         # the serving configuration: a group of sequences over fp8 experts
-        dict(name="mla_moe fp8 experts, 8 sequences", family="mla_moe", kind="decode", rows=8, context=1024, experts="fp8"),
-        dict(name="mla_moe, prompt 512", family="mla_moe", kind="prompt", rows=512, context=512, experts="bf16"),
+        dict(name="mla_moe fp8 experts 8 rows", family="mla_moe", kind="decode", rows=8, context=1024, experts="fp8"),
+        dict(name="mla_moe prompt 512", family="mla_moe", kind="prompt", rows=512, context=512, experts="bf16"),
     ]
 
 
