@@ -3,8 +3,10 @@
 //   gqa_rope_kv_write_kernel  rotates q and k in place (half-rotation RoPE on the first rotary_dim
 //                             columns of every head, device-computed angles) and scatters k / v rows
 //                             into the paged caches [pages, page_tokens, kv_heads, head_dim]
-//   gqa_split_kernel          split-KV online-softmax attention: one CTA per (split, kv head, query
+//   gqa_split_mma_kernel      split-KV online-softmax attention: one CTA per (split, kv head, query
 //                             row) serves the G = Hq/Hkv query heads that share the kv head
+//   gqa_split_kernel          the same with products on the CUDA cores: heads of 256 columns, caches
+//                             that do not start on 16 bytes
 //   gqa_merge_kernel          log-sum-exp merge of the splits -> [T, Hq*head_dim] bf16
 //
 // Query rows carry their own position and sequence slot (continuous batching: rows of different
@@ -87,6 +89,8 @@ struct GqaParams {
   ScoreRule rule;
   AheadRule ahead;                                // entries that count as the first keys of a row
   float factor;                                   // of the result
+  // keys of a split of a row that sees n: an even share, at least kps, whole rounds of a CTA (64 keys)
+  __device__ __forceinline__ int per_split(int n) const { return (max(kps, (n + max_splits - 1) / max_splits) + 63) / 64 * 64; }
 };
 
 // what a row sees: entries ahead of its window, then the positions first .. pos
@@ -119,11 +123,9 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
   const int pos = p.positions[t];
   if (pos < 0) return;
   const Seen seen(p, pos);
-  const int n = seen.n;
-  const int k_begin = split * p.kps;
+  const int n = seen.n, per = p.per_split(n), k_begin = split * per;
   if (k_begin >= n) return;
-  // the last split also takes every key beyond max_splits * keys_per_split, so a long context is slower, never clipped
-  const int k_end = (split == p.max_splits - 1) ? n : min(n, k_begin + p.kps);
+  const int k_end = min(n, k_begin + per);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = p.slots[t];
   float qf[G][EPL];
@@ -219,142 +221,223 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
   }
 }
 
-// The same for groups of up to four query heads: HD / 8 lanes share a key (8 columns, one 16-byte load each), so a warp works on
-// 256 / HD keys at once and a score costs log2(HD / 8) shuffles for all of them; four keys per lane group are in flight, with one update of
-// the running maximum for the four. Every lane group keeps its own maximum, sum and output; they are merged within the warp at the
-// end, then across the warps as above.
-template <int HD, int G>
-__global__ void __launch_bounds__(256, 2) gqa_split_shared_kernel(GqaParams p) {
-  constexpr int C = 8, LP = HD / C, NG = 32 / LP, KB = 4;
+// The same on the tensor cores, for heads of 64 or 128 columns and groups of up to eight query heads. A CTA of four warps works on one split of
+// one (row, kv head); every warp streams 16 keys and values at a time through a ring of its own in shared memory (cp.async, 16 bytes, no barrier
+// among the warps) and keeps a running maximum, sum and output, merged at the end.
+//
+//   scores   m16n8k16: the group's query rows are rows 0-7 AND 8-15 of A (so both halves of C hold them), keys are columns
+//   values   the weights enter as two bf16 terms, value in rows 0-7 and remainder in rows 8-15 of A: one product carries 16 bits of a
+//            weight and the sum stays f32; the two halves of C are added at the end
+//
+// Bound by the stream of keys and values: a key costs a warp two instructions, where products on the CUDA cores (eight lanes to a key) cost 40 and
+// bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 87 us (3.8 TB/s); 8 rows of 1900 keys 46 -> 19 us, one row of
+// 2000 keys 14.8 -> 10.1 us, merge included. What is in flight per SM: two CTAs x
+// four warps x two stages of 8 KB, twice what the HBM's latency asks for.
+template <int HD>
+struct MmaSplit {
+  static constexpr int KEYS = 16, WARPS = 4, STAGES = 3, CH = HD / 8;      // CH: 16-byte chunks of a row
+  static constexpr int ROW = HD * 2, STAGE = 2 * KEYS * ROW;
+  static constexpr int SMEM = WARPS * STAGES * STAGE;
+};
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 16 bytes, or zeros where `live` is false
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// two weights as (values, remainders)
+__device__ __forceinline__ void two_terms(float a, float b, uint32_t* hi, uint32_t* lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  const float2 f = __bfloat1622float2(h);
+  *hi = *reinterpret_cast<const uint32_t*>(&h);
+  *lo = pack_bf16(a - f.x, b - f.y);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p) {
+  using S = MmaSplit<HD>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* sm_acc = reinterpret_cast<float*>(smem_raw);   // [8][G][HD]
-  float* sm_m = sm_acc + 8 * G * HD;
-  float* sm_l = sm_m + 8 * G;
   grid_dep_launch();
   grid_dep_wait();
   const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
   const int pos = p.positions[t];
   if (pos < 0) return;
   const Seen seen(p, pos);
-  const int n = seen.n;
-  const int k_begin = split * p.kps;
+  const int n = seen.n, per = p.per_split(n), k_begin = split * per;
   if (k_begin >= n) return;
-  const int k_end = (split == p.max_splits - 1) ? n : min(n, k_begin + p.kps);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / LP, sub = lane % LP;
+  const int k_end = min(n, k_begin + per);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2, G = p.Hq / p.Hkv;
   const int slot = p.slots[t];
-  float qf[G][C], acc[G][C], m[G], l[G], slope[G];
   const bool ruled = !p.rule.plain();
+  const float slope = p.rule.slopes && g < G ? p.rule.slopes[kvh * G + g] : 0.f;
+  // query row g: columns 16 i + c2 + {0, 1} and + 8
+  uint32_t q[HD / 16][2];
+  {
+    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + (g < G ? g : 0)) * HD + c2;
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + g) * HD + sub * C;
+    for (int i = 0; i < HD / 16; ++i)
 #pragma unroll
-    for (int i = 0; i < C; ++i) {
-      qf[g][i] = __bfloat162float(qh[i]) * p.scale;
-      acc[g][i] = 0.f;
-    }
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-    slope[g] = p.rule.slopes ? p.rule.slopes[kvh * G + g] : 0.f;
+      for (int j = 0; j < 2; ++j) {
+        const bf16 *e = qh + 16 * i + 8 * j;
+        q[i][j] = g < G ? (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16 : 0u;
+      }
   }
-  const long kv_elems = (long)p.Hkv * HD, head = (long)kvh * HD + sub * C;
-  // every lane takes the same number of rounds (the shuffles are warp-wide); a missing key scores -inf
-  for (int k0 = k_begin + warp * NG; k0 < k_end; k0 += 8 * NG * KB) {
-    uint4 kr[KB], vr[KB];
-    bool ok[KB];
+  float acc[HD / 8][4], m = -INFINITY, l = 0.f;
 #pragma unroll
-    for (int b = 0; b < KB; ++b) {
-      const int k = k0 + b * 8 * NG + grp;
-      ok[b] = k < k_end;
-      kr[b] = vr[b] = make_uint4(0, 0, 0, 0);
-      if (ok[b]) {
-        bool pooled;
-        const long r = key_row(p, seen, k, slot, &pooled);
-        if (r < 0) {
-          if (sub == 0 && p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
-          ok[b] = false;
-        } else {
-          kr[b] = *reinterpret_cast<const uint4*>((pooled ? (const bf16*)p.ahead.k : p.k_cache) + r * kv_elems + head);
-          vr[b] = *reinterpret_cast<const uint4*>((pooled ? (const bf16*)p.ahead.v : p.v_cache) + r * kv_elems + head);
-        }
-      }
+  for (int i = 0; i < HD / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+
+  const uint32_t ring = smem_addr(smem_raw) + warp * S::STAGES * S::STAGE;
+  const long kv_elems = (long)p.Hkv * HD;
+  const int first = k_begin + warp * S::KEYS, stride = S::WARPS * S::KEYS;
+  // where key `first + i * stride + (lane & 15)` lies: 2 * row + (1: among the blocks); -1: nowhere
+  auto locate = [&](int i) -> long {
+    const int k = first + i * stride + (lane & 15);
+    if (k >= k_end) return -1;
+    bool pooled;
+    const long r = key_row(p, seen, k, slot, &pooled);
+    if (r < 0) {
+      if (lane < 16 && p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
+      return -1;
     }
-    float s[KB][G];
+    return 2 * r + pooled;
+  };
+  auto load = [&](int stage, long where) {
+    const uint32_t base = ring + stage * S::STAGE;
+    const int ch = lane % S::CH;
 #pragma unroll
-    for (int b = 0; b < KB; ++b) {
-      float f[8];
-      unpack8(kr[b], f);
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        s[b][g] = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[b][g] = fmaf(qf[g][j], f[j], s[b][g]);
-#pragma unroll
-        for (int o = LP / 2; o > 0; o >>= 1) s[b][g] += __shfl_xor_sync(0xffffffffu, s[b][g], o);
-        if (ruled) s[b][g] = ruled_score<true>(s[b][g], p.rule, slope[g], n - 1 - (k0 + b * 8 * NG + grp));
-        if (!ok[b]) s[b][g] = -INFINITY;
-      }
+    for (int i = 0; i < S::KEYS * S::CH / 32; ++i) {
+      const int key = lane / S::CH + i * (32 / S::CH);
+      const long w = __shfl_sync(0xffffffffu, where, key);
+      const long at = w < 0 ? 0 : (w >> 1) * kv_elems + (long)kvh * HD + ch * 8;
+      const bf16* kb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.k : p.k_cache;
+      const bf16* vb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.v : p.v_cache;
+      const uint32_t dst = base + key * S::ROW + ((ch ^ (key & 7)) << 4);
+      copy16(dst, kb + at, w >= 0);
+      copy16(dst + S::KEYS * S::ROW, vb + at, w >= 0);
     }
+  };
+  const int tiles = first < k_end ? (k_end - first + stride - 1) / stride : 0;
+  long at[S::STAGES];          // of the tiles in the ring, by stage
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const float mn = fmaxf(fmaxf(m[g], fmaxf(s[0][g], s[1][g])), fmaxf(s[2][g], s[3][g]));
-      if (mn > m[g]) {
-        const float corr = __expf(m[g] - mn);
-        l[g] *= corr;
+  for (int i = 0; i < S::STAGES; ++i) at[i] = -1;
 #pragma unroll
-        for (int i = 0; i < C; ++i) acc[g][i] *= corr;
-        m[g] = mn;
-      }
-#pragma unroll
-      for (int b = 0; b < KB; ++b) {
-        s[b][g] = ok[b] ? __expf(s[b][g] - mn) : 0.f;
-        l[g] += s[b][g];
-      }
+  for (int i = 0; i < S::STAGES - 1; ++i) {
+    if (i < tiles) {
+      at[i] = locate(i);
+      load(i, at[i]);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  long next = S::STAGES - 1 < tiles ? locate(S::STAGES - 1) : -1;
+  for (int i0 = 0; i0 < tiles; i0 += S::STAGES) {
 #pragma unroll
-    for (int b = 0; b < KB; ++b) {
-      float f[8];
-      unpack8(vr[b], f);
+    for (int st = 0; st < S::STAGES; ++st) {
+      const int i = i0 + st;
+      if (i >= tiles) break;
+      constexpr int AHEAD = S::STAGES - 1;
+      const int to = (st + AHEAD) % S::STAGES;
+      if (i + AHEAD < tiles) {
+        at[to] = next;
+        load(to, next);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      next = i + AHEAD + 1 < tiles ? locate(i + AHEAD + 1) : -1;
+      asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+      __syncwarp();
+      const uint32_t kb = ring + st * S::STAGE, vb = kb + S::KEYS * S::ROW;
+      float s[2][4] = {};
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+      for (int kk = 0; kk < HD / 16; ++kk) {
+        uint32_t b[4];
+        const int key = (lane >> 4) * 8 + (lane & 7), ch = 2 * kk + ((lane >> 3) & 1);
+        ldsm4(kb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
+        mma16816(s[0], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[0], b[1]);
+        mma16816(s[1], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[2], b[3]);
+      }
+      // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against query row g
+      float w[4];
+      float mn = m;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[g][j] = fmaf(s[b][g], f[j], acc[g][j]);
+      for (int j = 0; j < 4; ++j) {
+        const int key = c2 + (j >> 1) * 8 + (j & 1);
+        w[j] = s[j >> 1][j & 1] * p.scale;
+        if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
+        if (__shfl_sync(0xffffffffu, at[st], key) < 0) w[j] = -INFINITY;
+        mn = fmaxf(mn, w[j]);
+      }
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+      mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+      if (__any_sync(0xffffffffu, mn > m)) {
+        const float corr = mn > m ? __expf(m - mn) : 1.f;
+        l *= corr;
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] *= corr;
+        m = mn;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        w[j] = w[j] == -INFINITY ? 0.f : __expf(w[j] - m);
+        l += w[j];
+      }
+      uint32_t a0, a1, a2, a3;
+      two_terms(w[0], w[1], &a0, &a1);
+      two_terms(w[2], w[3], &a2, &a3);
+#pragma unroll
+      for (int j = 0; j < HD / 16; ++j) {
+        uint32_t b[4];
+        const int key = ((lane >> 3) & 1) * 8 + (lane & 7), ch = 2 * j + (lane >> 4);
+        ldsm4t(vb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
+        mma16816(acc[2 * j], a0, a1, a2, a3, b[0], b[1]);
+        mma16816(acc[2 * j + 1], a0, a1, a2, a3, b[2], b[3]);
+      }
+      __syncwarp();            // the stage is read: a later round may overwrite it
     }
   }
-  __syncwarp();
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    float M = m[g];
-#pragma unroll
-    for (int o = LP; o < 32; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float w = m[g] == -INFINITY ? 0.f : __expf(m[g] - M);
-    float L = l[g] * w;
-#pragma unroll
-    for (int o = LP; o < 32; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-    if (lane == 0) {
-      sm_m[warp * G + g] = M;
-      sm_l[warp * G + g] = L;
-    }
-#pragma unroll
-    for (int i = 0; i < C; ++i) {
-      float a = acc[g][i] * w;
-#pragma unroll
-      for (int o = LP; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (grp == 0) sm_acc[((long)warp * G + g) * HD + sub * C + i] = a;
-    }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();             // the rings become the warps' results: [4][8][HD], maxima and sums
+  float* sm_acc = reinterpret_cast<float*>(smem_raw);
+  __shared__ float sm_m[S::WARPS * 8], sm_l[S::WARPS * 8];
+  if ((lane & 3) == 0) {
+    sm_m[warp * 8 + g] = m;
+    sm_l[warp * 8 + g] = l;
   }
+#pragma unroll
+  for (int j = 0; j < HD / 8; ++j)
+    *reinterpret_cast<float2*>(sm_acc + (warp * 8 + g) * HD + 8 * j + c2) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
   __syncthreads();
-  for (int g = 0; g < G; ++g) {
+  for (int h = 0; h < G; ++h) {
     float M = -INFINITY;
-    for (int w = 0; w < 8; ++w) M = fmaxf(M, sm_m[w * G + g]);
-    float wgt[8], L = 0.f;
-    for (int w = 0; w < 8; ++w) {
-      wgt[w] = (sm_m[w * G + g] == -INFINITY) ? 0.f : __expf(sm_m[w * G + g] - M);
-      L += wgt[w] * sm_l[w * G + g];
+#pragma unroll
+    for (int w = 0; w < S::WARPS; ++w) M = fmaxf(M, sm_m[w * 8 + h]);
+    float wgt[S::WARPS], L = 0.f;
+#pragma unroll
+    for (int w = 0; w < S::WARPS; ++w) {
+      wgt[w] = sm_m[w * 8 + h] == -INFINITY ? 0.f : __expf(sm_m[w * 8 + h] - M);
+      L += wgt[w] * sm_l[w * 8 + h];
     }
-    float* out = p.scratch + (((long)t * p.Hq + kvh * G + g) * p.max_splits + split) * (HD + 2);
-    for (int c = threadIdx.x; c < HD; c += blockDim.x) {
+    float* out = p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2);
+    for (int c = threadIdx.x; c < HD; c += 128) {
       float v = 0.f;
-      for (int w = 0; w < 8; ++w) v += wgt[w] * sm_acc[((long)w * G + g) * HD + c];
+#pragma unroll
+      for (int w = 0; w < S::WARPS; ++w) v += wgt[w] * sm_acc[(w * 8 + h) * HD + c];
       out[c] = v;
     }
     if (threadIdx.x == 0) {
@@ -375,8 +458,7 @@ __global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
   const int pos = p.positions[t];
   if (pos < 0) return;
   const int n = Seen(p, pos).n;
-  int ns = (n + p.kps - 1) / p.kps;
-  if (ns > p.max_splits) ns = p.max_splits;
+  const int per = p.per_split(n), ns = (n + per - 1) / per;
   const float* base = p.scratch + ((long)t * p.Hq + h) * p.max_splits * (HD + 2);
   if (threadIdx.x < 32) {      // up to 64 splits: two per lane
     const int s0 = threadIdx.x, s1 = threadIdx.x + 32;
@@ -401,25 +483,45 @@ __global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
   }
 }
 
+template <int HD>
+int launch_merge(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
+  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, out, ldo);
+}
 template <int HD, int G>
 int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   const size_t smem = (size_t)(8 * G * HD + 16 * G) * sizeof(float);
-  constexpr bool shared_keys = HD <= 128 && G <= 4;
-  auto k = shared_keys ? gqa_split_shared_kernel<shared_keys ? HD : 64, shared_keys ? G : 1> : gqa_split_kernel<HD, G>;
+  auto k = gqa_split_kernel<HD, G>;
   if (int rc = opt_in_smem(k, smem)) return rc;
   dim3 grid(p.max_splits, p.Hkv, p.T);
   if (int rc = launch_chain(k, grid, dim3(256), smem, s, p)) return rc;
-  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, out, ldo);
+  return launch_merge<HD>(p, out, ldo, s);
+}
+template <int HD>
+int launch_mma(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
+  constexpr int smem = MmaSplit<HD>::SMEM;
+  auto k = gqa_split_mma_kernel<HD>;
+  if (int rc = opt_in_smem(k, smem)) return rc;
+  if (int rc = launch_chain(k, dim3(p.max_splits, p.Hkv, p.T), dim3(128), smem, s, p)) return rc;
+  return launch_merge<HD>(p, out, ldo, s);
 }
 
 template <int HD>
-int dispatch_g(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
-  switch (p.Hq / p.Hkv) {
+int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
+  const int G = p.Hq / p.Hkv;
+  if (G != 1 && G != 2 && G != 4 && G != 8) return -1;
+  // Many rows fill the chip by themselves: then fewer splits, each longer, so that a CTA's start and end and the merge weigh less. Three waves of
+  // two CTAs per SM even out rows of unequal length.
+  const int rows = p.T > 0 ? p.T * p.Hkv : 1, want = (888 + rows - 1) / rows;
+  p.max_splits = p.max_splits < want ? p.max_splits : want;
+  if constexpr (HD <= 128) {
+    const uintptr_t bits = (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (p.ahead.pool > 0 ? (uintptr_t)p.ahead.k | (uintptr_t)p.ahead.v : 0);
+    if (bits % 16 == 0) return launch_mma<HD>(p, out, ldo, s);
+  }
+  switch (G) {
     case 1: return launch_gqa<HD, 1>(p, out, ldo, s);
     case 2: return launch_gqa<HD, 2>(p, out, ldo, s);
     case 4: return launch_gqa<HD, 4>(p, out, ldo, s);
-    case 8: return launch_gqa<HD, 8>(p, out, ldo, s);
-    default: return -1;
+    default: return launch_gqa<HD, 8>(p, out, ldo, s);
   }
 }
 
