@@ -9,10 +9,11 @@
 //               add the bias / residual, activation or soft limit, store bf16 or f32
 // Gated form: B holds gate rows [0, F) and up rows [F, 2 F); a tile's accumulator takes BN / 2 of each (two boxes per stage) and the
 // epilogue stores the gated unit's value (rope.cuh), so that a feed-forward's first half is one launch for any number of rows.
-// Split form: a product of one tile row with few columns spreads its K over blockIdx.z; its reader adds the parts in their order.
+// Split form: a product of one tile row with few columns spreads its K over blockIdx.z; its reader adds the parts in their order. Its box of A
+// holds the live rows only.
 // A and B are both K-major ("NT"), which is how activations [tokens, K] and weights [out, K] are
 // stored everywhere in this library, so no transposes are needed. M, N and K tails are handled by
-// TMA zero fill plus masked stores. Used for prefill chunks and batched decode (M >= 16); the
+// TMA zero fill plus masked stores. Used from 129 rows on (fewer: tc_gemm_rows.cu; 256 and up with as many columns: tc_gemm_2sm.cu); the
 // reference's counterpart is aclnnMatmul on [T<=4096, K] activations (token_executor.h:387-456).
 #include <cstdlib>
 
@@ -78,18 +79,17 @@ __device__ __forceinline__ void store_row32(const GemmParams& p, int row, int co
   }
 }
 
-// W (a divisor of 32) consecutive columns of a row of the gated result
-template <int W>
+// 32 consecutive columns of a row of the gated result
 __device__ __forceinline__ void store_gated(const GemmParams& p, int row, int col, const float* g, const float* u) {
   if (row >= p.M || col >= p.F) return;
-  float v[W];
+  float v[32];
 #pragma unroll
-  for (int i = 0; i < W; ++i) v[i] = gated_bf16(g[i], u[i], p.unit);
+  for (int i = 0; i < 32; ++i) v[i] = gated_bf16(g[i], u[i], p.unit);
   bf16* out = reinterpret_cast<bf16*>(p.c) + (long)row * p.ldc + col;
-  const int nvalid = min(W, p.F - col);
-  if (nvalid == W && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
+  const int nvalid = min(32, p.F - col);
+  if (nvalid == 32 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0)) {
 #pragma unroll
-    for (int i = 0; i < W / 8; ++i) reinterpret_cast<uint4*>(out)[i] = pack8(v + 8 * i);
+    for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(out)[i] = pack8(v + 8 * i);
   } else {
     for (int i = 0; i < nvalid; ++i) out[i] = __float2bfloat16_rn(v[i]);
   }
@@ -122,17 +122,14 @@ __global__ void __launch_bounds__(192) tc_gemm_kernel(const __grid_constant__ CU
       const int q = warp & 3;                       // TMEM lane quarter this warp may read
       const int row = m0 + q * 32 + lane;
 #pragma unroll 1
-      for (int c0 = 0; c0 < (GATED && BN > 32 ? NOUT : BN); c0 += 32) {
+      for (int c0 = 0; c0 < NOUT; c0 += 32) {
         float v[32];
         tmem_ld_32x32(pipe.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-        if (GATED && BN == 32) {
-          tmem_ld_wait();
-          store_gated<16>(p, row, n0, v, v + 16);
-        } else if (GATED) {
+        if (GATED) {
           float u[32];
           tmem_ld_32x32(pipe.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(NOUT + c0), u);
           tmem_ld_wait();
-          store_gated<32>(p, row, n0 + c0, v, u);
+          store_gated(p, row, n0 + c0, v, u);
         } else {
           tmem_ld_wait();
           store_row32(p, row, n0 + c0, v);
@@ -224,10 +221,13 @@ extern "C" int ifab_gemm_act_bf16(const void* a, long lda, const void* b, long l
   return ifab_gemm_epilogue_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, nullptr, act, 0.f, M, N, K, status, stream);
 }
 
-// The same with a bias [N] in f32 (or null) and, for cap > 0, a soft limit of the result (cap tanh(result / cap)) after the activation.
-extern "C" int ifab_gemm_epilogue_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
-                                       const float* bias, int act, float cap, int M, int N, int K, uint32_t* status, void* stream) {
+namespace {
+int gemm_epilogue(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias, int act,
+                  float cap, int fixed, int M, int N, int K, uint32_t* status, void* stream) {
   if (M < 1 || N < 1 || K < 8 || K % 8 || lda % 8 || ldb % 8 || cap < 0.f) return -1;
+  // a single tile row (decode steps, short prompts) is bound by the stream of B: tc_gemm_rows.cu
+  if (M <= BM)
+    return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, 0.f, 0.f, 0, fixed, M, N, K, status, stream);
   // from 256 x 256 up: CTA pairs (tcgen05.mma cta_group::2; same accumulation order, same bits) - persistent with two
   // accumulators when there is more than one tile per SM pair, one tile per pair otherwise
   if (M >= 256 && N >= 256 && N % 32 == 0 && two_sm_enabled()) {
@@ -235,41 +235,49 @@ extern "C" int ifab_gemm_epilogue_bf16(const void* a, long lda, const void* b, l
     return ifab_gemm_epilogue_bf16_2sm(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, tiles > 74, M, N, K, status, stream);
   }
   CUtensorMap ta, tb;
-  // A single tile row (batched decode) is bound by the stream of B: narrow tiles spread it over the SMs, two CTAs on each; the box of A
-  // holds the live rows only.
-  const bool one_row = M <= BM;
-  int BN = N > 128 ? 256 : 128;
-  if (one_row)
-    for (BN = 32; BN < 128 && (N + BN - 1) / BN > 296; BN *= 2) {}
-  const int a_rows = one_row ? (M + 7) / 8 * 8 : BM;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
+  const int BN = N > 128 ? 256 : 128;
+  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)BM)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN)) return rc;
-  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, a_rows, act, bias, cap, 0, {}, 0, 0};
+  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, BM, act, bias, cap, 0, {}, 0, 0};
   cudaStream_t s = (cudaStream_t)stream;
-  if (!one_row) return BN == 256 ? launch<256, 4>(ta, tb, p, s) : launch<128, 6>(ta, tb, p, s);
-  return BN == 128 ? launch<128, 3>(ta, tb, p, s) : BN == 64 ? launch<64, 4>(ta, tb, p, s) : launch<32, 5>(ta, tb, p, s);
+  return BN == 256 ? launch<256, 4>(ta, tb, p, s) : launch<128, 6>(ta, tb, p, s);
+}
+
+int gemm_gated(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int fixed, int M, int F, int K,
+               uint32_t* status, void* stream) {
+  const GatedUnit gu{unit, limit, alpha};
+  if (M < 1 || F < 8 || F % 8 || K < 8 || K % 8 || lda % 8 || ldb % 8 || !gated_ok(gu)) return -1;
+  if (M <= BM) return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, status, stream);
+  if (M >= 256 && F >= 128 && F % 32 == 0 && two_sm_enabled())
+    return ifab_gemm_gated_bf16_2sm(a, lda, b, ldb, c, ldc, unit, limit, alpha, M, F, K, status, stream);
+  CUtensorMap ta, tb;
+  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)BM)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, 128)) return rc;
+  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, BM, 0, nullptr, 0.f, F, gu, 0, 0};
+  return launch<256, 4, true>(ta, tb, p, (cudaStream_t)stream);
+}
+}  // namespace
+
+// The same with a bias [N] in f32 (or null) and, for cap > 0, a soft limit of the result (cap tanh(result / cap)) after the activation.
+extern "C" int ifab_gemm_epilogue_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
+                                       const float* bias, int act, float cap, int M, int N, int K, uint32_t* status, void* stream) {
+  return gemm_epilogue(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, M, N, K, status, stream);
+}
+// The same for a B that no kernel of the stream writes (weights): its first tiles may be read before the preceding kernel has ended.
+extern "C" int ifab_gemm_fixed_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
+                                    const float* bias, int act, float cap, int M, int N, int K, uint32_t* status, void* stream) {
+  return gemm_epilogue(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 1, M, N, K, status, stream);
 }
 
 // C[M, F] (bf16) = unit(A gate^T, A up^T) with B = [gate rows | up rows] ([2 F, K]) and the gated units of rope.cuh (0 SiLU, 1 ReLU, 2 limited). F % 8
 // == 0. Rows from 256 on go to the CTA pairs where F % 32 == 0.
 extern "C" int ifab_gemm_gated_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int M, int F,
                                     int K, uint32_t* status, void* stream) {
-  const GatedUnit gu{unit, limit, alpha};
-  if (M < 1 || F < 8 || F % 8 || K < 8 || K % 8 || lda % 8 || ldb % 8 || !gated_ok(gu)) return -1;
-  if (M >= 256 && F >= 128 && F % 32 == 0 && two_sm_enabled())
-    return ifab_gemm_gated_bf16_2sm(a, lda, b, ldb, c, ldc, unit, limit, alpha, M, F, K, status, stream);
-  const bool one_row = M <= BM;
-  int BN = 256;
-  if (one_row)
-    for (BN = 32; BN < 128 && (2 * F + BN - 1) / BN > 296; BN *= 2) {}
-  const int a_rows = one_row ? (M + 7) / 8 * 8 : BM;
-  CUtensorMap ta, tb;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, (uint32_t)(BN / 2))) return rc;
-  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, a_rows, 0, nullptr, 0.f, F, gu, 0, 0};
-  cudaStream_t s = (cudaStream_t)stream;
-  if (!one_row) return launch<256, 4, true>(ta, tb, p, s);
-  return BN == 128 ? launch<128, 3, true>(ta, tb, p, s) : BN == 64 ? launch<64, 4, true>(ta, tb, p, s) : launch<32, 5, true>(ta, tb, p, s);
+  return gemm_gated(a, lda, b, ldb, c, ldc, unit, limit, alpha, 0, M, F, K, status, stream);
+}
+extern "C" int ifab_gemm_gated_fixed_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int M, int F,
+                                          int K, uint32_t* status, void* stream) {
+  return gemm_gated(a, lda, b, ldb, c, ldc, unit, limit, alpha, 1, M, F, K, status, stream);
 }
 
 // Parts of C[M, N] (f32, M <= 128) = A B^T + bias along K: `parts` of them, part_stride elements apart; C is their sum. Every part gets K blocks of 64

@@ -2,8 +2,8 @@
 
 The decode kernels of ``DenseDecoder`` multiply at most 8 rows per pass on the CUDA cores; measured on a B200 a pass of
 8 rows costs about 5 ms for the 2B model, so a 2048-token prompt takes over a second. This path runs a chunk as
-matrix-matrix work: the four linears of a layer on the tcgen05 GEMM (gate/up through the grouped kernel's SwiGLU epilogue
-with a single "expert", the row-parallel o_proj and down projections through the fused GEMM + all-reduce kernel when the
+matrix-matrix work: the four linears of a layer on the tcgen05 GEMM (gate/up
+with the SwiGLU epilogue, the row-parallel o_proj and down projections through the fused GEMM + all-reduce kernel when the
 model is tensor parallel), rotary + cache append through the decode path's kernel, attention through its split-KV kernels
 with one query row per token (causality comes from the per-row positions), ``attn_rows`` query rows per launch.
 It shares weights, caches and the page table with the decoder, so decode continues from the state it leaves.
@@ -25,6 +25,7 @@ import torch
 from ..ops import decode as K
 from ..ops import gemm as G
 from ..ops import prefill as P
+from ..ops import stream_norm as N
 from .dense_gqa import BF16, DenseDecoder
 
 
@@ -37,24 +38,17 @@ class DensePrefill:
         self.dec, self.M, self.QC = dec, max_rows, attn_rows
         c, fab, dev = dec.cfg, dec.fabric, dec.fabric.device
         M = max_rows
-        Mpad = (M + 127) // 128 * 128          # whole 128-row tiles of the one-expert group are stored
         e = lambda *s, dt=BF16: torch.empty(*s, dtype=dt, device=dev)
         self.tokens = torch.zeros(M, dtype=torch.int32, device=dev)
         self.positions = torch.zeros(M, dtype=torch.int32, device=dev)
         self.slots = torch.zeros(M, dtype=torch.int32, device=dev)
         self.x_sym = fab.symmetric_empty((M, c.hidden)) if fab.world > 1 else None
         self.x = self.x_sym.tensor if self.x_sym is not None else e(M, c.hidden)
-        self.h = torch.zeros(Mpad, c.hidden, dtype=BF16, device=dev)
+        self.h = e(M, c.hidden)
         self.qkv = e(M, (dec.hq + 2 * dec.hk) * c.head_dim)
         self.attn = e(M, dec.hq * c.head_dim)
-        self.act = e(Mpad, c.ffn // fab.world)
+        self.act = e(M, c.ffn // fab.world)
         self.scratch = e(self.QC * dec.hq * dec.max_splits * (c.head_dim + 2), dt=torch.float32)
-        nt = (M + 127) // 128
-        st = torch.zeros(nt, 4, dtype=torch.int32)
-        for i in range(nt):
-            st[i, 1], st[i, 2] = i * 128, 128
-        self.tiles = st.to(dev)
-        self.ntiles = torch.zeros(1, dtype=torch.int32, device=dev)
         self.launches = 0
         # Prompt attention on the tensor cores for chunks of consecutive positions of one sequence (heads of 128 columns): keys and
         # values of the context are gathered out of their pages (values transposed) and attended by the tcgen05 attention kernel
@@ -125,7 +119,7 @@ class DensePrefill:
         xs = x.index_select(0, select)
         xn = K.rmsnorm(xs, d.w["final_norm"], c.eps)
         self.launches += 2
-        return G.gemm(xn, d.w["lm_head"], out_f32=True, status_ptr=d.fabric.desc.status)
+        return G.gemm(xn, d.w["lm_head"], out_f32=True, status_ptr=d.fabric.desc.status, fixed=True)
 
     def _layers_graphed(self, m: int) -> torch.Tensor:
         if m > self.graph_rows_max:
@@ -167,29 +161,28 @@ class DensePrefill:
         tok, pos, sl = self.tokens[:m], self.positions[:m], self.slots[:m]
         x, h = self.x[:m], self.h[:m]
         K.embedding(tok, w["embed"], out=x, status_ptr=st)
-        self.ntiles.fill_((m + 127) // 128)
         scale = 1.0 / math.sqrt(c.head_dim)
         for l in range(c.layers):
             p = f"layers.{l}."
             K.rmsnorm(x, w[p + "attn_norm"], c.eps, out=h)
-            qkv = G.gemm(h, w[p + "qkv"], out=self.qkv[:m], status_ptr=st)
+            qkv = G.gemm(h, w[p + "qkv"], out=self.qkv[:m], status_ptr=st, fixed=True)
             K.gqa_rope_kv_write(qkv, pos, sl, d.page_table, d.k_cache[l], d.v_cache[l], heads=d.hq, kv_heads=d.hk,
                                 head_dim=c.head_dim, theta=c.theta, status_ptr=st)
             self._attention(l, m, qkv, pos, sl, scale, st)
             if fab.world > 1:
                 G.gemm_allreduce(self.attn[:m], w[p + "o_proj"], fab, self._sym_rows(m), residual=x)
             else:
-                G.gemm(self.attn[:m], w[p + "o_proj"], residual=x, out=x, status_ptr=st)
+                G.gemm(self.attn[:m], w[p + "o_proj"], residual=x, out=x, status_ptr=st, fixed=True)
             K.rmsnorm(x, w[p + "ffn_norm"], c.eps, out=h)
             if m >= 256:
                 # whole 256-row tile pairs: the packed gate | up projection and its activation on CTA pairs, one persistent launch
                 G.gemm_swiglu(h, w[p + "gate_up"], out=self.act[:m], status_ptr=st)
             else:
-                P.grouped_gemm(self.h, w[p + "gate_up"].unsqueeze(0), self.tiles, self.ntiles, self.act[:m], swiglu=True, status_ptr=st)
+                N.gated_linear(h, w[p + "gate_up"], N.SILU, self.act[:m], status_ptr=st, fixed=True)
             if fab.world > 1:
                 G.gemm_allreduce(self.act[:m], w[p + "down"], fab, self._sym_rows(m), residual=x)
             else:
-                G.gemm(self.act[:m], w[p + "down"], residual=x, out=x, status_ptr=st)
+                G.gemm(self.act[:m], w[p + "down"], residual=x, out=x, status_ptr=st, fixed=True)
         self.launches = 1 + c.layers * (8 + 2 * ((m + self.QC - 1) // self.QC))
         return x
 

@@ -30,7 +30,7 @@ from .checkpoint import pad8
 from .stream_decoder import ATTN_ROWS, BF16, F32, StreamDecoder, StreamRows
 
 KERNEL_UNITS = ("misc", "post_norm", "linear_f32", "linear_attn", "linear_attn_tc", "window_attn", "decode_post_norm", "decode_gqa", "fa_prefill", "decode_moe", "sampling",
-                "tc_gemm", "tc_gemm_2sm")
+                "tc_gemm", "tc_gemm_rows", "tc_gemm_2sm")
 
 
 # ---------------------------------------------------------------------------------------------------------------------------
@@ -393,13 +393,13 @@ class FalinexDecoder(StreamDecoder):
             mx = L["m"]
             hv = mx.heads * mx.vdim
             last = i + 1 == len(self.layers) and final
-            N.linear(xa, L["in"], B.proj[:m, :L["cols"]], status_ptr=st)
+            N.linear(xa, L["in"], B.proj[:m, :L["cols"]], status_ptr=st, fixed=True)
             self._mix(B, L, m, pos, slot, plan)
-            N.linear(B.mixed[hv][:m], L["o"], y, status_ptr=st)
+            N.linear(B.mixed[hv][:m], L["o"], y, status_ptr=st, fixed=True)
             N.post_norm_add(y, L["norm1"], c.eps, x, xa, self.final_norm if last and not L["ff"] else None)
             if L["ff"]:
-                N.linear(xa, L["up"], B.act[L["ff"]][:m, :L["ff"]], "gelu_tanh", status_ptr=st)
-                N.linear(B.act[L["ff"]][:m], L["down"], y, status_ptr=st)
+                N.linear(xa, L["up"], B.act[L["ff"]][:m, :L["ff"]], "gelu_tanh", status_ptr=st, fixed=True)
+                N.linear(B.act[L["ff"]][:m], L["down"], y, status_ptr=st, fixed=True)
                 N.post_norm_add(y, L["norm2"], c.eps, x, xa, self.final_norm if last else None)
             if probe is not None:
                 probe.append(x.clone())

@@ -31,7 +31,7 @@ from .checkpoint import pad8
 from .stream_decoder import ATTN_ROWS, BF16, F32, StreamDecoder, StreamRows
 
 KERNEL_UNITS = ("misc", "post_norm", "hyper_streams", "gated_recurrence", "gated_delta", "gated_tiles", "linear_f32", "window_attn", "decode_gqa", "fa_prefill", "decode_post_norm",
-                "decode_hyper", "decode_moe", "sampling", "tc_gemm", "tc_gemm_2sm")
+                "decode_hyper", "decode_moe", "sampling", "tc_gemm", "tc_gemm_rows", "tc_gemm_2sm")
 MIXERS = ("parallel", "mamba2", "parallel_2")
 
 
@@ -360,7 +360,7 @@ class FubelornDecoder(StreamDecoder):
         width, k = w.shape
         n = 1 if B.parts is None else N.split_count(m, width, k)
         if n == 1:
-            N.linear(x, w, B.y[:m, :width], status_ptr=self.fabric.desc.status)
+            N.linear(x, w, B.y[:m, :width], status_ptr=self.fabric.desc.status, fixed=True)
             return B.y[:m]
         parts = B.parts[:n, :m]
         N.split_linear(x, w, parts[:, :, :width], status_ptr=self.fabric.desc.status)
@@ -389,12 +389,12 @@ class FubelornDecoder(StreamDecoder):
         for L in self.layers:
             l = L["c"]
             front(L["sub"][0])
-            N.linear(xa, L["in"], B.attn.proj[:m, :l.in_cols], status_ptr=st)
+            N.linear(xa, L["in"], B.attn.proj[:m, :l.in_cols], status_ptr=st, fixed=True)
             y, before = self._product(B, self._mix(B, L, m, pos, slot, plan), L["out"], m), L["sub"][0]
             if l.ff:
                 front(L["sub"][1])
                 act = B.act[l.ff][:m]
-                N.linear(xa, L["up"], act[:, :l.ff], "gelu_erf", status_ptr=st)
+                N.linear(xa, L["up"], act[:, :l.ff], "gelu_erf", status_ptr=st, fixed=True)
                 y, before = self._product(B, act, L["down"], m), L["sub"][1]
             if probe is not None:                  # the sum of the streams as the layer leaves them
                 t = torch.empty_like(x, memory_format=torch.contiguous_format)

@@ -36,7 +36,7 @@ from .checkpoint import pad8
 from .stream_decoder import ATTN_ROWS, BF16, F32, StreamDecoder, StreamRows
 
 KERNEL_UNITS = ("misc", "post_norm", "linear_f32", "window_attn", "decode_gqa", "fa_prefill", "moe_rows", "moe_prefill", "tc_grouped", "decode_post_norm", "decode_moe",
-                "sampling", "tc_gemm", "tc_gemm_2sm")
+                "sampling", "tc_gemm", "tc_gemm_rows", "tc_gemm_2sm")
 MIXERS = ("attention", "attention_2")
 ALPHA = 1.702              # of the limited units
 

@@ -9,8 +9,8 @@ re-reads the whole model 64 times per 512 tokens. This path runs a chunk as matr
 * attention through the split-KV kernels of the decode path with one query row per token (causality comes from
   the per-row positions), 64 query rows per launch;
 * the MoE through a device-side dispatch (routes sorted by expert, 128-row tile table), the grouped expert GEMM
-  with the SwiGLU epilogue, the grouped down GEMM and a score-weighted combine; the shared expert rides on the same
-  grouped kernel with a single "expert"; across ranks the partial outputs are summed by a pull all-reduce.
+  with the SwiGLU epilogue, the grouped down GEMM and a score-weighted combine; the shared expert is two dense
+  products; across ranks the partial outputs are summed by a pull all-reduce.
 
 It shares the KV cache, the page table and the weights with ``MlaMoeDecoder`` and leaves the cache exactly as
 token-by-token decoding would (same normalisation and rotary kernel), so decode continues from it.
@@ -27,6 +27,7 @@ import torch
 from ..ops import decode as K
 from ..ops import gemm as G
 from ..ops import prefill as P
+from ..ops import stream_norm as N
 from .mla_moe import BF16, MlaMoeDecoder
 
 
@@ -45,8 +46,7 @@ class MlaMoePrefill:
         self.slots = torch.zeros(M, dtype=torch.int32, device=dev)
         self.x_sym = fab.symmetric_empty((M, c.hidden)) if fab.world > 1 else None
         self.x = self.x_sym.tensor if self.x_sym is not None else e(M, c.hidden)
-        Mpad = (M + 127) // 128 * 128     # whole 128-row tiles of the one-expert group are stored
-        self.h = torch.zeros(Mpad, c.hidden, dtype=BF16, device=dev)
+        self.h = e(M, c.hidden)
         self.qkv = e(M, c.q_lora + c.kv_lora + c.rope)
         self.qn = e(M, c.q_lora)
         self.q = e(M, hl * c.qk_dim)
@@ -62,15 +62,8 @@ class MlaMoePrefill:
         self.act = e(R, c.expert_ffn)
         self.y = e(R, c.hidden)
         fs = c.shared_ffn // fab.world
-        self.sact = e(Mpad, fs)
-        self.sd = e(Mpad, c.hidden)
-        # the shared expert as a one-expert group over all rows of the chunk (static tile table)
-        nt = (M + 127) // 128
-        st = torch.zeros(nt, 4, dtype=torch.int32)
-        for i in range(nt):
-            st[i, 1], st[i, 2] = i * 128, 128
-        self.shared_tiles = st.to(dev)
-        self.shared_ntiles = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.sact = e(M, fs)
+        self.sd = e(M, c.hidden)
         # block-scaled fp8 experts: the tensor-core kernels take bf16 operands, so one layer's expert matrices are widened into
         # this scratch right before the layer's grouped GEMMs (read 1 byte, write 2 per weight: a fraction of the GEMMs' time
         # for chunks of a few hundred rows and up)
@@ -157,7 +150,7 @@ class MlaMoePrefill:
         x = self._layers_graphed(m)
         xn = K.rmsnorm(x.index_select(0, select), d.w["final_norm"], c.eps)
         self.launches += 2
-        return G.gemm(xn, d.w["lm_head"], out_f32=True, status_ptr=d.fabric.desc.status)
+        return G.gemm(xn, d.w["lm_head"], out_f32=True, status_ptr=d.fabric.desc.status, fixed=True)
 
     def _layers(self, m: int) -> torch.Tensor:
         """Embedding + all layers over the ``m`` rows staged in ``tokens / positions / slots``; returns the hidden rows."""
@@ -167,12 +160,11 @@ class MlaMoePrefill:
         x, h = self.x[:m], self.h[:m]
         n_launch = 0
         K.embedding(tok, w["embed"], out=x, status_ptr=st)
-        self.shared_ntiles.fill_((m + 127) // 128)
         for l in range(c.layers):
             p = f"layers.{l}."
             # ---- attention ----
             K.rmsnorm(x, w[p + "attn_norm"], c.eps, out=h)
-            qkv = G.gemm(h, w[p + "qkv_a"], out=self.qkv[:m], status_ptr=st)
+            qkv = G.gemm(h, w[p + "qkv_a"], out=self.qkv[:m], status_ptr=st, fixed=True)
             if d.kv_int8:
                 K.mla_kv_write_q8(qkv[:, c.q_lora:], w[p + "kv_a_norm"], pos, sl, d.page_table, d.caches[l], eps=c.eps, theta=c.theta,
                                   status_ptr=st)
@@ -180,7 +172,7 @@ class MlaMoePrefill:
                 K.mla_kv_write(qkv[:, c.q_lora:], w[p + "kv_a_norm"], pos, sl, d.page_table, d.caches[l], latent=c.kv_lora,
                                rope=c.rope, eps=c.eps, theta=c.theta, status_ptr=st)
             K.rmsnorm(qkv[:, :c.q_lora], w[p + "q_a_norm"], c.eps, out=self.qn[:m])
-            q = G.gemm(self.qn[:m], w[p + "q_b"], out=self.q[:m], status_ptr=st)
+            q = G.gemm(self.qn[:m], w[p + "q_b"], out=self.q[:m], status_ptr=st, fixed=True)
             q_lat, o_lat, attn = self.q_lat[:m], self.o_lat[:m], self.attn[:m]
             if self.tc_attention and self._contig is not None:
                 pos0, slot = self._contig
@@ -188,7 +180,7 @@ class MlaMoePrefill:
                 rows = (ctx + 63) // 64 * 64
                 kvb = w[p + "kv_b"].view(hl * (c.nope + c.vdim), c.kv_lora)
                 P.mla_ctx_gather(d.caches[l], d.page_table, slot, ctx, self.ctx_lat[:rows], self.ctx_pe[:rows], status_ptr=st)
-                G.gemm(self.ctx_lat[:rows], kvb, out=self.kv_up[:rows], status_ptr=st)
+                G.gemm(self.ctx_lat[:rows], kvb, out=self.kv_up[:rows], status_ptr=st, fixed=True)
                 G.gemm(kvb, self.ctx_lat[:rows], out=self.kvt[:, :rows], status_ptr=st)
                 P.mla_q_rope_inplace(q, pos, heads=hl, nope=c.nope, rope=c.rope, theta=c.theta)
                 P.fa_prefill(q, self.kv_up, self.kvt, attn, heads=hl, q_head_stride=c.qk_dim, k_head_stride=c.nope + c.vdim,
@@ -200,7 +192,7 @@ class MlaMoePrefill:
             if fab.world > 1:
                 G.gemm_allreduce(attn, w[p + "o_proj"], fab, self._sym_rows(m), residual=x)
             else:
-                G.gemm(attn, w[p + "o_proj"], residual=x, out=x, status_ptr=st)
+                G.gemm(attn, w[p + "o_proj"], residual=x, out=x, status_ptr=st, fixed=True)
             # ---- MoE ----
             P.router_block(x, w[p + "router"], c.topk, self.ids[:m], self.wts[:m], norm_w=w[p + "ffn_norm"], eps=c.eps,
                            scoring=c.scoring, scale=c.route_scale, xn=h)
@@ -214,11 +206,8 @@ class MlaMoePrefill:
             P.grouped_gemm(self.xp, ew["gate_up"], self.route.tiles, self.route.num_tiles, self.act, swiglu=True, status_ptr=st)
             P.grouped_gemm(self.act, ew["down"], self.route.tiles, self.route.num_tiles, self.y, status_ptr=st)
             sgu, sdn = ew["shared_gate_up"], ew["shared_down"]
-            if m >= 256 and (sgu.shape[0] // 2) % 32 == 0:
-                G.gemm_swiglu(h, sgu, out=self.sact[:m], status_ptr=st)      # the shared expert's gate | up on CTA pairs
-            else:
-                P.grouped_gemm(h, sgu.unsqueeze(0), self.shared_tiles, self.shared_ntiles, self.sact[:m], swiglu=True, status_ptr=st)
-            G.gemm(self.sact[:m], sdn, out=self.sd[:m], status_ptr=st)
+            N.gated_linear(h, sgu, N.SILU, self.sact[:m], status_ptr=st, fixed=self.w8 is None)
+            G.gemm(self.sact[:m], sdn, out=self.sd[:m], status_ptr=st, fixed=self.w8 is None)       # the widened copy is written in this very chain
             if fab.world > 1:
                 part = self.parts[self._calls & 1]
                 self._calls += 1
@@ -239,7 +228,7 @@ class MlaMoePrefill:
         p = f"layers.{l}."
         pos, sl = self.positions[:m], self.slots[:m]
         for hh in range(hl):
-            G.gemm(q[:, hh * c.qk_dim: hh * c.qk_dim + c.nope], self.w_uk_t[l][hh], out=q_lat[:, hh, :c.kv_lora], status_ptr=st)
+            G.gemm(q[:, hh * c.qk_dim: hh * c.qk_dim + c.nope], self.w_uk_t[l][hh], out=q_lat[:, hh, :c.kv_lora], status_ptr=st, fixed=True)
         P.mla_q_rope(q, pos, q_lat, nope=c.nope, rope=c.rope, theta=c.theta)
         for q0 in range(0, m, self.QC):
             q1 = min(m, q0 + self.QC)
@@ -248,7 +237,7 @@ class MlaMoePrefill:
             P.mla_merge(self.scratch, pos[q0:q1], o_lat[q0:q1], window=c.window, keys_per_split=d.kps, max_splits=d.max_splits)
         kvb = w[p + "kv_b"]
         for hh in range(hl):
-            G.gemm(o_lat[:, hh, :], kvb[hh, c.nope:, :], out=attn[:, hh * c.vdim:(hh + 1) * c.vdim], status_ptr=st)
+            G.gemm(o_lat[:, hh, :], kvb[hh, c.nope:, :], out=attn[:, hh * c.vdim:(hh + 1) * c.vdim], status_ptr=st, fixed=True)
 
     def _sym_rows(self, m: int):
         """The symmetric activation buffer restricted to ``m`` rows (same peer pointers, smaller shape)."""

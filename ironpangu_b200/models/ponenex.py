@@ -30,7 +30,7 @@ from .checkpoint import pad8
 from .stream_decoder import ATTN_ROWS, BF16, F32, StreamDecoder, StreamRows
 
 KERNEL_UNITS = ("misc", "post_norm", "linear_f32", "latent_attn", "tc_heads", "moe_rows", "moe_prefill", "tc_grouped", "decode_post_norm", "window_attn",
-                "fa_prefill", "decode_moe", "sampling", "tc_gemm", "tc_gemm_2sm")
+                "fa_prefill", "decode_moe", "sampling", "tc_gemm", "tc_gemm_rows", "tc_gemm_2sm")
 
 
 # ---------------------------------------------------------------------------------------------------------------------------
@@ -251,9 +251,9 @@ class PonenexDecoder(StreamDecoder):
         for i, L in enumerate(self.layers):
             mix, ff, after = L["mix"], L["ff"], self._next_gain(i, final)
             s = mix.shape
-            N.linear(xa, mix.w_in, lat.proj[:m, :s.in_cols], status_ptr=st)
+            N.linear(xa, mix.w_in, lat.proj[:m, :s.in_cols], status_ptr=st, fixed=True)
             mix.mix(lat, m, B.rotary.get(s.rot_dims, s.rot_base), pos, slot, plan, self.page_table, c.eps, st)
-            N.linear(lat.mixed[s.heads * s.vdim][:m], mix.w_o, y, status_ptr=st)
+            N.linear(lat.mixed[s.heads * s.vdim][:m], mix.w_o, y, status_ptr=st, fixed=True)
             N.post_norm_add(y, L["norm1b"], c.eps, x, xa, after if ff is None else L["norm2"])
             if ff is not None:
                 ff.rows(B.experts, m, xa, L["norm2b"], after, c.eps, B.x[:m], st)

@@ -156,7 +156,7 @@ class StreamRows:
         xn = torch.zeros(select.numel(), self.B.xa.shape[1], dtype=d.dtype, device=tokens.device)
         N.rms_rows(self.B.x[:m], d.final_norm, c.eps, xn, select.to(torch.int32))
         logits = torch.empty(select.numel(), c.vocab, dtype=F32, device=tokens.device)
-        N.linear(xn, d.head, logits, status_ptr=d.fabric.desc.status, cap=d.logit_cap)
+        N.linear(xn, d.head, logits, status_ptr=d.fabric.desc.status, cap=d.logit_cap, fixed=True)
         return logits
 
     def forward(self, tokens: torch.Tensor, pos0: int, slot: int = 0) -> torch.Tensor:

@@ -256,7 +256,7 @@ class LatentMixer:
         lat, rot, k, vt = B.lat[s.latent_cols][:rows], B.rot[:rows], B.k[H * n1][:rows], B.vt[H]
         check(lib.ifab_latent_gather(self.cache.data_ptr(), table.data_ptr(), slot, table.shape[1], pt, pages, first, ctx, rows, s.latent_cols, s.rot_cols, 64,
                                      lat.data_ptr(), rot.data_ptr(), status_ptr, _s()), "latent_gather")
-        N.linear(lat, self.w_k, k, status_ptr=status_ptr)
+        N.linear(lat, self.w_k, k, status_ptr=status_ptr, fixed=True)
         N.linear(self.w_v, lat, vt[:, :rows], status_ptr=status_ptr)
         q, out, gate = self._q(B)[lo:lo + n], B.mixed[H * s.vdim][lo:lo + n], B.proj[lo:lo + n, s.gate_off:]
         check(lib.ifab_fa_window_bf16(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), rot.data_ptr(), rot.stride(0), 64, vt.data_ptr(), vt.stride(0),
@@ -268,7 +268,7 @@ class LatentMixer:
         s = self.shape
         q = self._q(B)[:m]
         self.prepare(B, m, rope, pos, slot, table, eps, status_ptr)
-        N.linear(B.cq[s.q_rank][:m], self.w_uq, q, status_ptr=status_ptr)
+        N.linear(B.cq[s.q_rank][:m], self.w_uq, q, status_ptr=status_ptr, fixed=True)
         self.rotate(q, rope)
         runs = plan.runs if plan is not None and self.tiles else []
         step = plan.step_positions if runs else pos

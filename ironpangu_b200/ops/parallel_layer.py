@@ -57,14 +57,14 @@ class Join:
         """The unit's part of the operand for any number of rows."""
         m = xa.shape[0]
         if self.F:
-            N.gated_linear(xa, self.gate_up, self.unit, self.operand(B, m)[:, self.at:], None if B.pair is None else B.pair[:m, :2 * self.F], status_ptr)
+            N.gated_linear(xa, self.gate_up, self.unit, self.operand(B, m)[:, self.at:], None if B.pair is None else B.pair[:m, :2 * self.F], status_ptr, fixed=True)
 
     def rows(self, B: "JoinBuffers", m: int, y: torch.Tensor, status_ptr) -> torch.Tensor:
         """The product and its bias in f32: in ``y``, or for few rows as parts of a sum ``[parts, m, padded width]``; returns which."""
         width, k = self.w.shape
         n = 1 if B.parts is None else N.split_count(m, width, k)
         if n == 1:
-            N.linear(self.operand(B, m), self.w, y[:, :width], bias=self.bias, status_ptr=status_ptr)
+            N.linear(self.operand(B, m), self.w, y[:, :width], bias=self.bias, status_ptr=status_ptr, fixed=True)
             return y
         parts = B.parts[:n, :m]
         N.split_linear(self.operand(B, m), self.w, parts[:, :, :width], self.bias, status_ptr)

@@ -126,7 +126,7 @@ class RoutedExperts:
         D = self.gate_up.shape[2]
         n = self.w_router.shape[0]
         logits, ids, wts, route = B.logits[:m, :n], B.ids[s.top][:m], B.wts[s.top][:m], B.route[s.top, s.experts]
-        N.linear(xa, self.w_router, logits, status_ptr=status_ptr)
+        N.linear(xa, self.w_router, logits, status_ptr=status_ptr, fixed=True)
         check(lib.ifab_moe_route(logits.data_ptr(), logits.stride(0), self.bias.data_ptr(), m, s.experts, s.top, *s.rule, ids.data_ptr(),
                                  wts.data_ptr(), B.shared_w.data_ptr() if s.shared_ff else None, _s()), "moe_route")
         P.moe_dispatch(ids, 0, s.experts, route)
@@ -145,10 +145,10 @@ class RoutedExperts:
             if s.shared_ff:
                 sact, sh = B.sact[s.shared_ff], B.sy
                 if m >= 256 and sact.shape[1] % 32 == 0:
-                    N.gated_linear(xa, self.shared_gate_up, s.unit, sact[:m], status_ptr=status_ptr)
+                    N.gated_linear(xa, self.shared_gate_up, s.unit, sact[:m], status_ptr=status_ptr, fixed=True)
                 else:
                     P.grouped_gemm(xa, self.shared_gate_up[None], B.row_tiles, B.row_ntiles, sact, unit=s.unit, status_ptr=status_ptr)
-                N.linear(sact[:m], self.shared_down, sh[:m], status_ptr=status_ptr)
+                N.linear(sact[:m], self.shared_down, sh[:m], status_ptr=status_ptr, fixed=True)
         check(lib.ifab_moe_combine_norm(y.data_ptr(), y.stride(0), route.route_row.data_ptr(), wts.data_ptr(), s.top, _p(sh), 0 if sh is None else sh.stride(0),
                                         B.shared_w.data_ptr() if s.shared_ff else None, _p(gain), _p(next_gain), eps, _p(base), *N._parts(base),
                                         _p(extra), 0 if extra is None else extra.stride(0), x.data_ptr(), x.stride(0), xa.data_ptr(), xa.stride(0), _f32(xa), m, s.width, _s()), "moe_combine_norm")

@@ -140,9 +140,10 @@ def gemv_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[str] = None, status_ptr: Optional[int] = None,
-           bias: Optional[torch.Tensor] = None, cap: float = 0.0) -> None:
+           bias: Optional[torch.Tensor] = None, cap: float = 0.0, fixed: bool = False) -> None:
     """``out = act(x @ w.T + bias)`` for any number of rows: the tensor-core GEMM for bf16 operands (bf16 or f32 result), true f32 otherwise.
-    ``bias``: f32 ``[N]``; ``cap`` > 0: ``cap * tanh(out / cap)`` at the end."""
+    ``bias``: f32 ``[N]``; ``cap`` > 0: ``cap * tanh(out / cap)`` at the end. ``fixed``: no kernel of the stream writes ``w`` (a model's weights), so
+    that reading it may begin before the kernel ahead has ended."""
     T, K = x.shape
     N = w.shape[0]
     assert w.shape[1] == K and x.dtype == w.dtype and x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
@@ -151,8 +152,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[st
         check(_lib.load().ifab_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _p(bias), cap, T, N, K,
                                           ACTIVATIONS[act], _s()), "linear_f32")
     else:
-        check(_lib.load().ifab_gemm_epilogue_bf16(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _f32(out), None, 0,
-                                                  _p(bias), ACTIVATIONS[act], cap, T, N, K, status_ptr, _s()), "gemm_epilogue")
+        fn = _lib.load().ifab_gemm_fixed_bf16 if fixed else _lib.load().ifab_gemm_epilogue_bf16
+        check(fn(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _f32(out), None, 0, _p(bias), ACTIVATIONS[act], cap, T, N, K,
+                 status_ptr, _s()), "gemm_epilogue")
 
 
 def split_count(rows: int, n: int, k: int) -> int:
@@ -174,9 +176,10 @@ def split_linear(x: torch.Tensor, w: torch.Tensor, parts: torch.Tensor, bias: Op
                                            status_ptr, _s()), "gemm_split")
 
 
-def gated_linear(x: torch.Tensor, w: torch.Tensor, unit: GatedUnit, out: torch.Tensor, pair: Optional[torch.Tensor] = None, status_ptr: Optional[int] = None) -> None:
+def gated_linear(x: torch.Tensor, w: torch.Tensor, unit: GatedUnit, out: torch.Tensor, pair: Optional[torch.Tensor] = None, status_ptr: Optional[int] = None,
+                 fixed: bool = False) -> None:
     """``out`` ``[T, F]`` = the gated unit of ``x @ gate.T`` and ``x @ up.T`` with ``w`` = [gate | up] ``[2 F, K]``: one launch for bf16; in f32 the
-    two projections go through ``pair`` ``[T, 2 F]``."""
+    two projections go through ``pair`` ``[T, 2 F]``. ``fixed`` as for :func:`linear`."""
     T, K = x.shape
     F = w.shape[0] // 2
     assert w.shape == (2 * F, K) and out.shape == (T, F) and x.dtype == w.dtype == out.dtype and out.stride(1) == 1 and x.stride(1) == 1
@@ -184,5 +187,5 @@ def gated_linear(x: torch.Tensor, w: torch.Tensor, unit: GatedUnit, out: torch.T
         linear(x, w, pair)
         gated_rows(pair, unit, out)
     else:
-        check(_lib.load().ifab_gemm_gated_bf16(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), *unit.args, T, F, K, status_ptr,
-                                               _s()), "gemm_gated")
+        fn = _lib.load().ifab_gemm_gated_fixed_bf16 if fixed else _lib.load().ifab_gemm_gated_bf16
+        check(fn(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), *unit.args, T, F, K, status_ptr, _s()), "gemm_gated")

@@ -285,7 +285,7 @@ class GroupedAttention:
         return (z(page_tokens, s.dim), z(page_tokens, s.vdim)) + ((z(m, s.dim), z(m, s.vdim)) if m else ())
 
     def project(self, B: GroupedBuffers, xa: torch.Tensor, status_ptr) -> None:
-        N.linear(xa, self.w_in, B.proj[:xa.shape[0], :self.shape.in_cols], bias=self.b_in, status_ptr=status_ptr)
+        N.linear(xa, self.w_in, B.proj[:xa.shape[0], :self.shape.in_cols], bias=self.b_in, status_ptr=status_ptr, fixed=True)
 
     def attend(self, B: GroupedBuffers, m: int, pages: tuple, rope, pos, slot, plan, table, eps: float, out: torch.Tensor, status_ptr) -> None:
         """``m`` rows of a packed step (``plan``), or decode rows (None), from ``B.proj`` to ``out`` ``[m, >= heads * vdim]``."""
