@@ -8,6 +8,7 @@
 //   moe_gate_up_kernel        one CTA column per route: gate/up rows of the routed expert, gated unit
 //   moe_down_allreduce_kernel score-weighted sum of the local experts' down projections (+ the
 //                             tensor-parallel shard of the shared expert) + one-shot all-reduce
+//   argmax_rows_kernel        the same selection over logits of a tensor-core product (three rows and more)
 //   lm_head_argmax_kernel     vocabulary-sharded logits + greedy selection; the last CTA exchanges
 //                             (value, index) pairs with the peers so every rank ends with the token
 //
@@ -403,66 +404,19 @@ struct HeadParams {
   float cap;           // > 0: logits are cap tanh(logit / cap)
 };
 
-template <int T, int R>
-__global__ void __launch_bounds__(256) lm_head_argmax_kernel(HeadParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* xs = reinterpret_cast<bf16*>(smem_raw);
-  __shared__ float red[T * 33];
-  __shared__ float bestv[8][T];
-  __shared__ int besti[8][T];
-  __shared__ int is_last;
-  grid_dep_launch();
+// The end of both kernels below: the CTA that arrives last picks every token's largest logit out of the CTAs' (`partial`, [grid][T]; ties to the
+// lowest id), with `world` ranks among theirs. All threads of a CTA of 256.
+template <int T>
+__device__ __forceinline__ void finish_argmax(const HeadParams& p, int* is_last) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * 8 + warp) * R;
-  const bf16* rows[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) rows[r] = (n0 + r < p.V) ? p.w + (size_t)(n0 + r) * p.K : nullptr;
-  RowBatch<R> pf;
-  prefetch_rows<R>(rows, p.K, pf);
-  grid_dep_wait();
-  stage_x<T>(xs, p.x, p.ldx, 0, p.T, p.K, p.norm_w, p.eps, false, red);
-  {
-    float acc[R][T];
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int t = 0; t < T; ++t) acc[r][t] = 0.f;
-    warp_rows_dot<T, R>(rows, xs, p.K, acc, pf);
-    warp_reduce_acc<T, R>(acc);
-    if (lane == 0) {
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        float bv = -INFINITY;
-        int bi = 0x7fffffff;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (n0 + r >= p.V) continue;
-          if (p.cap > 0.f) acc[r][t] = soft_limit<true>(acc[r][t], p.cap);
-          if (p.logits && t < p.T) p.logits[(size_t)t * p.V + n0 + r] = acc[r][t];
-          if (acc[r][t] > bv) { bv = acc[r][t]; bi = p.vocab_offset + n0 + r; }
-        }
-        bestv[warp][t] = bv;
-        besti[warp][t] = bi;
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < T) {
-    const int t = threadIdx.x;
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int w = 0; w < 8; ++w)
-      if (bestv[w][t] > bv || (bestv[w][t] == bv && besti[w][t] < bi)) { bv = bestv[w][t]; bi = besti[w][t]; }
-    p.partial[(size_t)blockIdx.x * T + t] = make_float2(bv, __int_as_float(bi));
-  }
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     const uint32_t tk = atomicAdd(p.done, 1u);
-    is_last = (tk == gridDim.x - 1);
+    *is_last = (tk == gridDim.x - 1);
   }
   __syncthreads();
-  if (!is_last) return;
+  if (!*is_last) return;
   __threadfence();
   // final reduction over CTAs: warp t handles token t
   const uint64_t epoch = *reinterpret_cast<volatile uint64_t*>(p.seq) + 1;
@@ -524,6 +478,86 @@ __global__ void __launch_bounds__(256) lm_head_argmax_kernel(HeadParams p) {
     *p.seq = epoch;
     __threadfence();
   }
+}
+
+template <int T, int R>
+__global__ void __launch_bounds__(256) lm_head_argmax_kernel(HeadParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16* xs = reinterpret_cast<bf16*>(smem_raw);
+  __shared__ float red[T * 33];
+  __shared__ float bestv[8][T];
+  __shared__ int besti[8][T];
+  __shared__ int is_last;
+  grid_dep_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * 8 + warp) * R;
+  const bf16* rows[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) rows[r] = (n0 + r < p.V) ? p.w + (size_t)(n0 + r) * p.K : nullptr;
+  RowBatch<R> pf;
+  prefetch_rows<R>(rows, p.K, pf);
+  grid_dep_wait();
+  stage_x<T>(xs, p.x, p.ldx, 0, p.T, p.K, p.norm_w, p.eps, false, red);
+  {
+    float acc[R][T];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int t = 0; t < T; ++t) acc[r][t] = 0.f;
+    warp_rows_dot<T, R>(rows, xs, p.K, acc, pf);
+    warp_reduce_acc<T, R>(acc);
+    if (lane == 0) {
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        float bv = -INFINITY;
+        int bi = 0x7fffffff;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (n0 + r >= p.V) continue;
+          if (p.cap > 0.f) acc[r][t] = soft_limit<true>(acc[r][t], p.cap);
+          if (p.logits && t < p.T) p.logits[(size_t)t * p.V + n0 + r] = acc[r][t];
+          if (acc[r][t] > bv) { bv = acc[r][t]; bi = p.vocab_offset + n0 + r; }
+        }
+        bestv[warp][t] = bv;
+        besti[warp][t] = bi;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < T) {
+    const int t = threadIdx.x;
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+    for (int w = 0; w < 8; ++w)
+      if (bestv[w][t] > bv || (bestv[w][t] == bv && besti[w][t] < bi)) { bv = bestv[w][t]; bi = besti[w][t]; }
+    p.partial[(size_t)blockIdx.x * T + t] = make_float2(bv, __int_as_float(bi));
+  }
+  finish_argmax<T>(p, &is_last);
+}
+
+// The largest of the logits that a product has left in p.logits: 1024 columns a CTA, a warp per token.
+__global__ void __launch_bounds__(256) argmax_rows_kernel(HeadParams p) {
+  __shared__ int is_last;
+  grid_dep_launch();
+  grid_dep_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, v0 = blockIdx.x * 1024, end = min(p.V, v0 + 1024);
+  float bv = -INFINITY;
+  int bi = 0x7fffffff;
+  if (warp < p.T) {
+    const float* row = p.logits + (size_t)warp * p.V;
+    for (int c = v0 + lane; c < end; c += 32) {
+      const float v = row[c];
+      if (v > bv) { bv = v; bi = p.vocab_offset + c; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+    }
+  }
+  if (lane == 0) p.partial[(size_t)blockIdx.x * 8 + warp] = make_float2(bv, __int_as_float(bi));
+  finish_argmax<8>(p, &is_last);
 }
 
 template <int T, int R>
@@ -634,6 +668,22 @@ extern "C" int ifab_lm_head_capped_argmax(const void* x, long ldx, const void* n
   if (int rc = fabric_view(fab, &p.fv)) return rc;
   p.seq = fab->seq; p.done = fab->done;
   cudaStream_t s = (cudaStream_t)stream;
+  // From three rows on the products above are bound by FMAs (8 rows of 153600 x 4096: 1048 us), the tensor-core product by the stream of the matrix
+  // (201 us, and 10 us for the norm ahead of it and the selection behind): it wants the logits stored, and room for the normalised rows behind the partial maxima.
+  const unsigned ctas = (unsigned)((V_local + 1023) / 1024);
+  const uint64_t maxima = (uint64_t)ctas * 8 * sizeof(float2), rows = norm_w ? (uint64_t)T * K * sizeof(bf16) : 0;
+  const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w | (uintptr_t)partial | (uintptr_t)(ldx * sizeof(bf16));
+  if (T >= 3 && logits && maxima + rows <= partial_bytes && bits % 16 == 0) {
+    const void* a = x;
+    long lda = ldx;
+    if (norm_w) {
+      a = reinterpret_cast<char*>(partial) + maxima;
+      lda = K;
+      if (int rc = ifab_rmsnorm_bf16(x, ldx, norm_w, const_cast<void*>(a), K, T, K, eps, 0, stream)) return rc;
+    }
+    if (int rc = ifab_gemm_fixed_bf16(a, lda, w, K, logits, V_local, 1, nullptr, 0, nullptr, 0, cap, T, V_local, K, fab->status, stream)) return rc;
+    return launch_chain(argmax_rows_kernel, dim3(ctas), dim3(256), 0, s, p);
+  }
   if (T <= 1) return launch_head<1, 4>(p, partial_bytes, s);
   if (T <= 2) return launch_head<2, 4>(p, partial_bytes, s);
   if (T <= 4) return launch_head<4, 4>(p, partial_bytes, s);
