@@ -357,7 +357,12 @@ class FalinexDecoder(StreamDecoder):
             elif long:
                 rec.chunks(proj, L["state"], pos, plan.table, rope, o, B.scratch)
             if not alone:
-                rec.step(proj, L["state"], pos if plan is None else plan.step_positions, slot, rope, o)
+                # beside long runs only the stretches of rows that hold short ones: a launch over all rows is mostly CTAs of rows that the tiles take
+                # (5 rows beside 1500 in 18 layers: 8.7 ms a step, 7.8 ms so)
+                stretches = [(0, m)] if not long else plan.groups if len(plan.groups) <= 4 else [(plan.groups[0][0], plan.groups[-1][1])]
+                steps = pos if plan is None else plan.step_positions
+                for lo, hi in stretches:
+                    rec.step(proj[lo:hi], L["state"], steps[lo:hi], slot[lo:hi], None if rope is None else rope[lo:hi], o[lo:hi])
             if norm:
                 N.group_norm_gate(o, gate, L["gate_act"], self.cfg.eps, B.mixed[hv][:m], L["groups"], L["gain"])
             return
