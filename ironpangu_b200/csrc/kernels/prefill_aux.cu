@@ -75,16 +75,18 @@ __global__ void __launch_bounds__(72) mla_ctx_gather_kernel(const bf16* cache, c
 
 // Keys and values 0 .. ctx - 1 of one sequence slot out of the paged GQA caches [pages, page_tokens, kv_heads * hd]: the keys as
 // dense rows k[rows, W] (W = kv_heads * hd), the values TRANSPOSED as vt[W, ld] with one column per key - the operand layouts of
-// the tensor-core prompt attention. Rows / columns from ctx up to `rows` are zero. One CTA per 32 keys: the values go through a
+// the tensor-core prompt attention. Rows / columns from ctx up to `rows` are zero. One CTA per 32 keys and 128 columns: the values go through a
 // shared-memory tile so that both the reads (along a cache row) and the writes (32 consecutive keys of one column) coalesce.
+// Bound by latency at short contexts (4 MB at 509 keys), so the columns are split over CTAs too (bands of 128) and everything moves in 16-byte
+// pieces where widths and addresses allow it (`wide`): 509 keys of 512 columns 16.2 us with one CTA per 32 keys and 2-byte pieces, 2.2 us so; 4096 keys 37 -> 5.1 us.
 __global__ void __launch_bounds__(256) gqa_ctx_gather_kernel(const bf16* k_cache, const bf16* v_cache, const int32_t* page_table, int slot,
                                                              int max_pages, int page_tokens, int num_pages, int ctx, int W, bf16* k, bf16* vt,
-                                                             long ldvt, uint32_t* status) {
-  __shared__ bf16 tile[32][256 + 2];
+                                                             long ldvt, int wide, uint32_t* status) {
+  __shared__ bf16 tile[32][128 + 2];
   __shared__ long src_row[32];
   grid_dep_launch();
   grid_dep_wait();
-  const int j0 = blockIdx.x * 32, t = threadIdx.x;
+  const int j0 = blockIdx.x * 32, c0 = blockIdx.y * 128, t = threadIdx.x, width = min(128, W - c0);
   if (t < 32) {
     const int j = j0 + t;
     long row = -1;
@@ -95,23 +97,49 @@ __global__ void __launch_bounds__(256) gqa_ctx_gather_kernel(const bf16* k_cache
     src_row[t] = row;
   }
   __syncthreads();
-  for (int c0 = 0; c0 < W; c0 += 256) {
-    const int c = c0 + t;
-    for (int kk = 0; kk < 32; ++kk) {
-      const long row = src_row[kk];
-      bf16 kv = __float2bfloat16_rn(0.f), vv = kv;
-      if (row >= 0 && c < W) {
-        kv = k_cache[row * W + c];
-        vv = v_cache[row * W + c];
-      }
-      if (c < W) k[(long)(j0 + kk) * W + c] = kv;
-      tile[kk][t] = vv;
+  if (wide) {
+    uint4 kv[2], vv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = t + u * 256, c = (i & 15) * 8;
+      const long row = src_row[i >> 4];
+      const bool live = row >= 0 && c < width;
+      kv[u] = live ? *reinterpret_cast<const uint4*>(k_cache + row * W + c0 + c) : make_uint4(0, 0, 0, 0);
+      vv[u] = live ? *reinterpret_cast<const uint4*>(v_cache + row * W + c0 + c) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = t + u * 256, kk = i >> 4, c = (i & 15) * 8;
+      if (c < width) *reinterpret_cast<uint4*>(k + (long)(j0 + kk) * W + c0 + c) = kv[u];
+      uint32_t* w = reinterpret_cast<uint32_t*>(&tile[kk][c]);
+      w[0] = vv[u].x;
+      w[1] = vv[u].y;
+      w[2] = vv[u].z;
+      w[3] = vv[u].w;
     }
     __syncthreads();
-    const int key = t & 31;
-    for (int cc = t >> 5; cc < 256 && c0 + cc < W; cc += 8) vt[(long)(c0 + cc) * ldvt + j0 + key] = tile[key][cc];
-    __syncthreads();
+    for (int i = t; i < width * 4; i += 256) {
+      const int c = i >> 2, k0 = (i & 3) * 8;
+      union { bf16 h[8]; uint4 u; } o;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o.h[j] = tile[k0 + j][c];
+      *reinterpret_cast<uint4*>(vt + (long)(c0 + c) * ldvt + j0 + k0) = o.u;
+    }
+    return;
   }
+  for (int i = t; i < 32 * width; i += 256) {
+    const int kk = i / width, c = i - kk * width;
+    const long row = src_row[kk];
+    bf16 kv = __float2bfloat16_rn(0.f), vv = kv;
+    if (row >= 0) {
+      kv = k_cache[row * W + c0 + c];
+      vv = v_cache[row * W + c0 + c];
+    }
+    k[(long)(j0 + kk) * W + c0 + c] = kv;
+    tile[kk][c] = vv;
+  }
+  __syncthreads();
+  for (int i = t; i < 32 * width; i += 256) vt[(long)(c0 + (i >> 5)) * ldvt + j0 + (i & 31)] = tile[i & 31][i >> 5];
 }
 
 struct MergeParams {
@@ -408,8 +436,10 @@ extern "C" int ifab_mla_q_rope_inplace(void* q, long ldq, const int32_t* positio
 extern "C" int ifab_gqa_ctx_gather(const void* k_cache, const void* v_cache, const int32_t* page_table, int slot, int max_pages, int page_tokens,
                                    int num_pages, int ctx, int rows, int width, void* k, void* vt, long ldvt, uint32_t* status, void* stream) {
   if (ctx < 1 || rows < ctx || rows % 32 || slot < 0 || width < 1 || ldvt < rows) return -1;
-  return launch_chain(gqa_ctx_gather_kernel, dim3(rows / 32), dim3(256), 0, (cudaStream_t)stream, (const bf16*)k_cache, (const bf16*)v_cache,
-                      page_table, slot, max_pages, page_tokens, num_pages, ctx, width, (bf16*)k, (bf16*)vt, ldvt, status);
+  const uintptr_t bits = (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)k | (uintptr_t)vt;
+  return launch_chain(gqa_ctx_gather_kernel, dim3(rows / 32, (width + 127) / 128), dim3(256), 0, (cudaStream_t)stream, (const bf16*)k_cache,
+                      (const bf16*)v_cache, page_table, slot, max_pages, page_tokens, num_pages, ctx, width, (bf16*)k, (bf16*)vt, ldvt,
+                      (int)(bits % 16 == 0 && width % 8 == 0 && ldvt % 8 == 0), status);
 }
 
 extern "C" int ifab_mla_ctx_gather(const void* cache, const int32_t* page_table, int slot, int max_pages, int page_tokens, int num_pages, int ctx,
