@@ -13,6 +13,7 @@
 // sequences and prefill chunks share one launch). Reference counterparts: attention_qk_prepare /
 // paged_attention_prepare composites (native/src/inferfabric_acl.cpp:1236-1433).
 #include "attn_rule.cuh"
+#include "mma16816.cuh"
 #include "gemv.cuh"
 #include "rope.cuh"
 #include "ifab_kernels.h"
@@ -36,43 +37,72 @@ __device__ __forceinline__ long row_of(int pos, int slot, const int32_t* page_ta
   return (long)page * page_tokens + (pos % page_tokens);
 }
 
-// grid T, 256 threads
+// grid T, 256 threads. Bound by latency (a row is 6 KB): the angles are formed once per pair and not once per head, everything moves in 16-byte
+// pieces, and rotated keys go to the row and to the page from registers. 20 heads of 128: 1 row 4.6 -> 2.6 us, 509 rows 9.1 -> 3.9, 2048 rows 17.6 -> 8.2.
 __global__ void __launch_bounds__(256) gqa_rope_kv_write_kernel(bf16* qkv, long ld, const int32_t* positions, const int32_t* slots,
                                                                 const int32_t* page_table, int max_pages, int page_tokens,
                                                                 bf16* k_cache, bf16* v_cache, int num_pages, int Hq, int Hkv, int hd,
                                                                 int rot, float theta, uint32_t* status) {
+  extern __shared__ __align__(16) float cs[];      // [half] cos, then [half] sin
   grid_dep_launch();
   grid_dep_wait();
   const int t = blockIdx.x;
   const int pos = positions[t];
   if (pos < 0) return;
   bf16* row = qkv + (long)t * ld;
-  const int half = rot / 2;
-  // rotate q heads and k heads: (Hq + Hkv) * half pairs
+  const int half = rot / 2, kv_elems = Hkv * hd;
+  const long r = row_of(pos, slots[t], page_table, max_pages, page_tokens, num_pages);
+  if (r < 0 && threadIdx.x == 0 && status) atomicOr(status, IFAB_STATUS_BAD_INDEX);
+  bf16 *kdst = k_cache + r * kv_elems, *vdst = v_cache + r * kv_elems;
+  const bf16* vsrc = row + (long)(Hq + Hkv) * hd;
+  if (r >= 0)
+    for (int c = threadIdx.x; c < kv_elems / 8; c += blockDim.x) reinterpret_cast<uint4*>(vdst)[c] = reinterpret_cast<const uint4*>(vsrc)[c];
+  for (int i = threadIdx.x; i < half; i += blockDim.x) rope_cs(pos, i, rot, theta, &cs[i], &cs[half + i]);
+  __syncthreads();
+  if (half % 8 == 0) {
+    const int chunks = half / 8;
+    for (int i = threadIdx.x; i < (Hq + Hkv) * chunks; i += blockDim.x) {
+      const int h = i / chunks, j = (i - h * chunks) * 8;
+      bf16* p = row + (long)h * hd + j;
+      float a[8], b[8], x[8], y[8];
+      unpack8(*reinterpret_cast<const uint4*>(p), a);
+      unpack8(*reinterpret_cast<const uint4*>(p + half), b);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float c = cs[j + e], s = cs[half + j + e];
+        x[e] = a[e] * c - b[e] * s;
+        y[e] = b[e] * c + a[e] * s;
+      }
+      const uint4 lo = pack8(x), hi = pack8(y);
+      *reinterpret_cast<uint4*>(p) = lo;
+      *reinterpret_cast<uint4*>(p + half) = hi;
+      if (h >= Hq && r >= 0) {
+        bf16* k = kdst + (long)(h - Hq) * hd + j;
+        *reinterpret_cast<uint4*>(k) = lo;
+        *reinterpret_cast<uint4*>(k + half) = hi;
+      }
+    }
+    if (r >= 0 && rot < hd) {        // key columns that do not turn
+      const int rest = (hd - rot) / 8;
+      for (int i = threadIdx.x; i < Hkv * rest; i += blockDim.x) {
+        const long at = (long)(i / rest) * hd + rot + (i % rest) * 8;
+        *reinterpret_cast<uint4*>(kdst + at) = *reinterpret_cast<const uint4*>(row + (long)Hq * hd + at);
+      }
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < (Hq + Hkv) * half; i += blockDim.x) {
     const int h = i / half, j = i % half;
     bf16* p = row + (long)h * hd;
-    float c, s;
-    rope_cs(pos, j, rot, theta, &c, &s);
+    const float c = cs[j], s = cs[half + j];
     const float a = __bfloat162float(p[j]), b = __bfloat162float(p[j + half]);
     p[j] = __float2bfloat16_rn(a * c - b * s);
     p[j + half] = __float2bfloat16_rn(b * c + a * s);
   }
   __syncthreads();
-  const long r = row_of(pos, slots[t], page_table, max_pages, page_tokens, num_pages);
-  if (r < 0) {
-    if (threadIdx.x == 0 && status) atomicOr(status, IFAB_STATUS_BAD_INDEX);
-    return;
-  }
-  const int kv_elems = Hkv * hd;
+  if (r < 0) return;
   const uint4* ksrc = reinterpret_cast<const uint4*>(row + (long)Hq * hd);
-  const uint4* vsrc = reinterpret_cast<const uint4*>(row + (long)(Hq + Hkv) * hd);
-  uint4* kdst = reinterpret_cast<uint4*>(k_cache + r * kv_elems);
-  uint4* vdst = reinterpret_cast<uint4*>(v_cache + r * kv_elems);
-  for (int c = threadIdx.x; c < kv_elems / 8; c += blockDim.x) {
-    kdst[c] = ksrc[c];
-    vdst[c] = vsrc[c];
-  }
+  for (int c = threadIdx.x; c < kv_elems / 8; c += blockDim.x) reinterpret_cast<uint4*>(kdst)[c] = ksrc[c];
 }
 
 struct GqaParams {
@@ -230,45 +260,31 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 //            weight and the sum stays f32; the two halves of C are added at the end
 //
 // Bound by the stream of keys and values: a key costs a warp two instructions, where products on the CUDA cores (eight lanes to a key) cost 40 and
-// bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 87 us (3.8 TB/s); 8 rows of 1900 keys 46 -> 19 us, one row of
-// 2000 keys 14.8 -> 10.1 us, merge included. What is in flight per SM: two CTAs x
-// four warps x two stages of 8 KB, twice what the HBM's latency asks for.
+// bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 77 us (4.3 TB/s); 8 rows of 1900 keys 46 -> 13 us, one row of
+// 2000 keys 14.8 -> 10.4 us, merge included. Three CTAs an
+// SM x four warps with one stage of 8 KB in flight beside the one in use.
 template <int HD>
 struct MmaSplit {
-  static constexpr int KEYS = 16, WARPS = 4, STAGES = 3, CH = HD / 8;      // CH: 16-byte chunks of a row
+  static constexpr int KEYS = 16, WARPS = 4, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
   static constexpr int ROW = HD * 2, STAGE = 2 * KEYS * ROW;
   static constexpr int SMEM = WARPS * STAGES * STAGE;
 };
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// 16 bytes, or zeros where `live` is false
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-// two weights as (values, remainders)
-__device__ __forceinline__ void two_terms(float a, float b, uint32_t* hi, uint32_t* lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  const float2 f = __bfloat1622float2(h);
-  *hi = *reinterpret_cast<const uint32_t*>(&h);
-  *lo = pack_bf16(a - f.x, b - f.y);
+__device__ __forceinline__ float peer_float(const float* mine, uint32_t rank) {
+  uint32_t at;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr(mine)), "r"(rank));
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
 }
 
-template <int HD>
-__global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p) {
+// CLUSTER: the splits of a (row, kv head) are one cluster (at most eight) and merge their parts over distributed shared memory into `out`; otherwise
+// the parts go to the scratch and gqa_merge_kernel follows.
+template <int HD, bool CLUSTER>
+__global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
   using S = MmaSplit<HD>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep_launch();
@@ -278,7 +294,7 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p) {
   if (pos < 0) return;
   const Seen seen(p, pos);
   const int n = seen.n, per = p.per_split(n), k_begin = split * per;
-  if (k_begin >= n) return;
+  if (!CLUSTER && k_begin >= n) return;
   const int k_end = min(n, k_begin + per);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2, G = p.Hq / p.Hkv;
   const int slot = p.slots[t];
@@ -423,6 +439,7 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p) {
   for (int j = 0; j < HD / 8; ++j)
     *reinterpret_cast<float2*>(sm_acc + (warp * 8 + g) * HD + 8 * j + c2) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
   __syncthreads();
+  float* part = sm_acc + S::WARPS * 8 * HD;        // CLUSTER: this split's [G][HD], then maxima and sums
   for (int h = 0; h < G; ++h) {
     float M = -INFINITY;
 #pragma unroll
@@ -433,18 +450,48 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p) {
       wgt[w] = sm_m[w * 8 + h] == -INFINITY ? 0.f : __expf(sm_m[w * 8 + h] - M);
       L += wgt[w] * sm_l[w * 8 + h];
     }
-    float* out = p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2);
+    float* to = CLUSTER ? part + h * HD : p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2);
     for (int c = threadIdx.x; c < HD; c += 128) {
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < S::WARPS; ++w) v += wgt[w] * sm_acc[(w * 8 + h) * HD + c];
-      out[c] = v;
+      to[c] = v;
     }
     if (threadIdx.x == 0) {
-      out[HD] = M;
-      out[HD + 1] = L;
+      (CLUSTER ? part + 8 * HD + h : to + HD)[0] = M;
+      (CLUSTER ? part + 8 * HD + 8 + h : to + HD + 1)[0] = L;
     }
   }
+  if (!CLUSTER) return;
+  cluster_barrier();
+  const int parts = p.max_splits;
+  for (int e = split * 128 + threadIdx.x; e < G * HD; e += parts * 128) {
+    const int h = e / HD, c = e - h * HD, head = kvh * G + h;
+    float pm[8], pl[8], pv[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < parts) {
+        pm[r] = peer_float(part + 8 * HD + h, r);
+        pl[r] = peer_float(part + 8 * HD + 8 + h, r);
+        pv[r] = peer_float(part + e, r);
+      }
+    float M = p.sink ? p.sink[head] : -INFINITY;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < parts) M = fmaxf(M, pm[r]);
+    float L = p.sink ? __expf(p.sink[head] - M) : 0.f, v = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < parts && pm[r] != -INFINITY) {
+        const float w = __expf(pm[r] - M);
+        L += w * pl[r];
+        v += w * pv[r];
+      }
+    v *= L > 0.f ? p.factor / L : 0.f;
+    if (p.gate) v *= activate<true>(__bfloat162float(p.gate[(long)t * p.ldg + (p.gate_head ? head : (long)head * HD + c)]), p.gate_act);
+    res[(long)t * ldo + (long)head * HD + c] = __float2bfloat16_rn(v);
+  }
+  cluster_barrier();           // the parts stay until every split has read them
 }
 
 // grid (Hq, T), HD threads
@@ -497,11 +544,17 @@ int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   return launch_merge<HD>(p, out, ldo, s);
 }
 template <int HD>
-int launch_mma(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
+int launch_mma(const GqaParams& p, bool cluster, bf16* out, long ldo, cudaStream_t s) {
   constexpr int smem = MmaSplit<HD>::SMEM;
-  auto k = gqa_split_mma_kernel<HD>;
+  const dim3 grid(p.max_splits, p.Hkv, p.T);
+  if (cluster) {
+    auto k = gqa_split_mma_kernel<HD, true>;
+    if (int rc = opt_in_smem(k, smem)) return rc;
+    return launch_chain_cluster(k, grid, dim3(128), (unsigned)p.max_splits, smem, s, p, out, ldo);
+  }
+  auto k = gqa_split_mma_kernel<HD, false>;
   if (int rc = opt_in_smem(k, smem)) return rc;
-  if (int rc = launch_chain(k, dim3(p.max_splits, p.Hkv, p.T), dim3(128), smem, s, p)) return rc;
+  if (int rc = launch_chain(k, grid, dim3(128), smem, s, p, out, ldo)) return rc;
   return launch_merge<HD>(p, out, ldo, s);
 }
 
@@ -509,13 +562,22 @@ template <int HD>
 int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
   const int G = p.Hq / p.Hkv;
   if (G != 1 && G != 2 && G != 4 && G != 8) return -1;
-  // Many rows fill the chip by themselves: then fewer splits, each longer, so that a CTA's start and end and the merge weigh less. Three waves of
-  // two CTAs per SM even out rows of unequal length.
-  const int rows = p.T > 0 ? p.T * p.Hkv : 1, want = (888 + rows - 1) / rows;
-  p.max_splits = p.max_splits < want ? p.max_splits : want;
+  // Many rows fill the chip by themselves: then fewer splits, each longer, so that a CTA's start and end and the merge weigh less: as many CTAs as two
+  // to an SM (three fit). 64 rows of 2560 keys: 77 us with 2 splits, 89 with 4; 27 rows of 1024: 20 us with 2, 35 with 8; 8 rows of 1900: 13 us with 8.
+  const int rows = p.T > 0 ? p.T * p.Hkv : 1, asked = p.max_splits, want = (296 + rows - 1) / rows;
+  p.max_splits = asked < want ? asked : want;
   if constexpr (HD <= 128) {
     const uintptr_t bits = (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (p.ahead.pool > 0 ? (uintptr_t)p.ahead.k | (uintptr_t)p.ahead.v : 0);
-    if (bits % 16 == 0) return launch_mma<HD>(p, out, ldo, s);
+    if (bits % 16 == 0) {
+      // A cluster of up to eight splits merges by itself, which saves the merge's launch. A few rows with long contexts take more splits than that: from
+      // about 512 keys in each of eight on, more CTAs are worth the second launch (one row, four kv heads).
+      const bool cluster = rows >= 16 || (long)p.kps * asked <= 4096;
+      if (cluster) {
+        p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
+        while (p.max_splits > asked) p.max_splits /= 2;
+      }
+      return launch_mma<HD>(p, cluster, out, ldo, s);
+    }
   }
   switch (G) {
     case 1: return launch_gqa<HD, 1>(p, out, ldo, s);
@@ -532,7 +594,7 @@ extern "C" int ifab_gqa_rope_kv_write(void* qkv, long ld, const int32_t* positio
                                       int num_pages, int T, int Hq, int Hkv, int head_dim, int rotary_dim, float theta,
                                       uint32_t* status, void* stream) {
   if (head_dim % 8 || rotary_dim % 2 || rotary_dim > head_dim || ld % 8) return -1;
-  return launch_chain(gqa_rope_kv_write_kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, (bf16*)qkv, ld, positions, slots,
+  return launch_chain(gqa_rope_kv_write_kernel, dim3(T), dim3(256), (size_t)rotary_dim * sizeof(float), (cudaStream_t)stream, (bf16*)qkv, ld, positions, slots,
                       page_table, max_pages, page_tokens, (bf16*)k_cache, (bf16*)v_cache, num_pages, Hq, Hkv, head_dim, rotary_dim,
                       theta, status);
 }
