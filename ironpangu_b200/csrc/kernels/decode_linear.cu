@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(GemvParams p) {
     for (int r = 0; r < R; ++r) rows[r] = (n0 + r < p.N) ? p.w + (long)(n0 + r) * p.K : nullptr;
     RowBatch<R> pf;
     prefetch_rows<R>(rows, p.K, pf);
+    request_gain(p.norm_w, p.K);
     grid_dep_wait();
     stage_x<T>(xs, p.x, p.ldx, t0, p.T, p.K, p.norm_w, p.eps, p.zero_centered != 0, red);
     if (n0 >= p.N) return;
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(GemvParams p) {
     }
     RowBatch<2 * R> pf;
     prefetch_rows<2 * R>(rows, p.K, pf);
+    request_gain(p.norm_w, p.K);
     grid_dep_wait();
     stage_x<T>(xs, p.x, p.ldx, t0, p.T, p.K, p.norm_w, p.eps, p.zero_centered != 0, red);
     if (n0 >= p.N) return;

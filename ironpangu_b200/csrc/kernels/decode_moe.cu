@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(256) router_topk_kernel(RouterParams p) {
     const int c = threadIdx.x + j * 256;
     pf[j] = c < quads ? __ldg(wr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  request_gain(p.norm_w, p.D);
   grid_dep_wait();
   stage_x<T>(xs, p.x, p.ldx, 0, p.T, p.D, p.norm_w, p.eps, false, red);
   if (p.xn && blockIdx.x == 0) {
@@ -496,6 +497,7 @@ __global__ void __launch_bounds__(256) lm_head_argmax_kernel(HeadParams p) {
   for (int r = 0; r < R; ++r) rows[r] = (n0 + r < p.V) ? p.w + (size_t)(n0 + r) * p.K : nullptr;
   RowBatch<R> pf;
   prefetch_rows<R>(rows, p.K, pf);
+  request_gain(p.norm_w, p.K);
   grid_dep_wait();
   stage_x<T>(xs, p.x, p.ldx, 0, p.T, p.K, p.norm_w, p.eps, false, red);
   {

@@ -43,6 +43,11 @@ __device__ __forceinline__ void prefetch_rows(const bf16* const (&wrow)[R], int 
   }
 }
 
+// ask L2 for the gains of a norm (weights: before the wait for the producer of the rows)
+__device__ __forceinline__ void request_gain(const bf16* norm_w, int K) {
+  if (norm_w != nullptr && (int)threadIdx.x * 64 < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(norm_w + threadIdx.x * 64));
+}
+
 // Stage T rows of x (bf16, K columns, row stride ldx) into shared memory. When norm_w != nullptr the
 // rows are RMS-normalised on the way: y = bf16(x * rsqrt(mean(x^2) + eps) * (w or 1+w)).
 // All threads of the block participate; ends with __syncthreads().
@@ -52,6 +57,54 @@ __device__ __forceinline__ void stage_x(bf16* xs, const bf16* __restrict__ x, lo
                                         float* red /* >= T*33 floats */) {
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int chunks = K >> 3;
+  // One or two rows of up to 16 columns a thread: row and gain are requested together and stay in registers, one barrier between the sums and the
+  // scaling. (Through shared memory the gains were a second trip to HBM behind three barriers: the four
+  // linears of a layer, one row of 2048 columns, 35.5 us against 30.4.)
+  constexpr int NV = 2;
+  if (T <= 2 && norm_w != nullptr && chunks <= NV * nthr) {
+    uint4 v[T][NV], gain[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = tid + i * nthr;
+      gain[i] = c < chunks ? *reinterpret_cast<const uint4*>(norm_w + c * 8) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int t = 0; t < T; ++t)
+        v[t][i] = c < chunks && t0 + t < t_total ? *reinterpret_cast<const uint4*>(x + (long)(t0 + t) * ldx + c * 8) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        float f[8];
+        unpack8(v[t][i], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+      }
+      ss = warp_sum(ss);
+      if ((tid & 31) == 0) red[t * 33 + (tid >> 5)] = ss;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      float sum = 0.f;
+      for (int w = 0; w < (nthr >> 5); ++w) sum += red[t * 33 + w];
+      const float inv = rsqrtf(sum / (float)K + eps);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = tid + i * nthr;
+        if (c >= chunks) break;
+        float f[8], g[8];
+        unpack8(v[t][i], f);
+        unpack8(gain[i], g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = f[e] * inv * (zero_centered ? 1.f + g[e] : g[e]);
+        *reinterpret_cast<uint4*>(xs + t * K + c * 8) = pack8(f);
+      }
+    }
+    __syncthreads();
+    return;
+  }
   for (int t = 0; t < T; ++t) {
     const bool live = (t0 + t) < t_total;
     const bf16* xr = x + (long)(t0 + t) * ldx;
