@@ -152,6 +152,8 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // 2-D bf16 row-major tensor [rows, cols] (cols contiguous, row stride ld elements), box = box_rows x 64
 // columns with the 128-byte swizzle. Returns 0 or a negative/CUDA error code.
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
+// tc_gemm_rows.cu
+bool rows_better(int M, int N, int K, int F);
 // 3-D: [batch, rows, cols] with batch stride `bstride` elements (grouped / per-expert weights)
 int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t batch, uint64_t rows, uint64_t cols, uint64_t ld,
                       uint64_t bstride, uint32_t box_rows);

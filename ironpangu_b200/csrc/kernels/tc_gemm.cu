@@ -13,7 +13,7 @@
 // holds the live rows only.
 // A and B are both K-major ("NT"), which is how activations [tokens, K] and weights [out, K] are
 // stored everywhere in this library, so no transposes are needed. M, N and K tails are handled by
-// TMA zero fill plus masked stores. Used from 129 rows on (fewer: tc_gemm_rows.cu; 256 and up with as many columns: tc_gemm_2sm.cu); the
+// TMA zero fill plus masked stores. Used where neither tc_gemm_rows.cu (few rows) nor tc_gemm_2sm.cu (256 and up with as many columns) is; the
 // reference's counterpart is aclnnMatmul on [T<=4096, K] activations (token_executor.h:387-456).
 #include <cstdlib>
 
@@ -225,21 +225,23 @@ namespace {
 int gemm_epilogue(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias, int act,
                   float cap, int fixed, int M, int N, int K, uint32_t* status, void* stream) {
   if (M < 1 || N < 1 || K < 8 || K % 8 || lda % 8 || ldb % 8 || cap < 0.f) return -1;
-  // a single tile row (decode steps, short prompts) is bound by the stream of B: tc_gemm_rows.cu
-  if (M <= BM)
+  // Few rows (decode steps, short prompts) are bound by the stream of B: tc_gemm_rows.cu. From 33 to 128 rows of a matrix wide enough to fill the chip
+  // without sharing K the sum over a cluster is only a detour: N 151936, K 2048, 64 rows 134 us there and 127 here, 128 rows 172 and 138 (27 rows 114 and 120).
+  // From 256 rows on only for weights: a plain product keeps the order of its sums that the CTA pairs and the one-CTA kernel share.
+  const bool wide = M > 32 && M <= BM && (N + 127) / 128 > 296;
+  if (!wide && (M < 256 || (fixed && rows_better(M, N, K, 0))))
     return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, 0.f, 0.f, 0, fixed, M, N, K, status, stream);
   // from 256 x 256 up: CTA pairs (tcgen05.mma cta_group::2; same accumulation order, same bits) - persistent with two
   // accumulators when there is more than one tile per SM pair, one tile per pair otherwise
-  if (M >= 256 && N >= 256 && N % 32 == 0 && two_sm_enabled()) {
-    const long tiles = (long)((M + 255) / 256) * ((N + 255) / 256);
-    return ifab_gemm_epilogue_bf16_2sm(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, tiles > 74, M, N, K, status, stream);
-  }
+  if (M >= 256 && N >= 256 && N % 32 == 0 && two_sm_enabled())
+    return ifab_gemm_epilogue_bf16_2sm(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, -1, M, N, K, status, stream);
   CUtensorMap ta, tb;
-  const int BN = N > 128 ? 256 : 128;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)BM)) return rc;
+  const int BN = N > 128 && !wide ? 256 : 128, a_rows = wide ? (M + 7) / 8 * 8 : BM;
+  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN)) return rc;
-  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, BM, act, bias, cap, 0, {}, 0, 0};
+  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, a_rows, act, bias, cap, 0, {}, 0, 0};
   cudaStream_t s = (cudaStream_t)stream;
+  if (wide) return launch<128, 3>(ta, tb, p, s);
   return BN == 256 ? launch<256, 4>(ta, tb, p, s) : launch<128, 6>(ta, tb, p, s);
 }
 
@@ -247,7 +249,7 @@ int gemm_gated(const void* a, long lda, const void* b, long ldb, void* c, long l
                uint32_t* status, void* stream) {
   const GatedUnit gu{unit, limit, alpha};
   if (M < 1 || F < 8 || F % 8 || K < 8 || K % 8 || lda % 8 || ldb % 8 || !gated_ok(gu)) return -1;
-  if (M <= BM) return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, status, stream);
+  if (M < 256 || (fixed && rows_better(M, 2 * F, K, F))) return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, status, stream);
   if (M >= 256 && F >= 128 && F % 32 == 0 && two_sm_enabled())
     return ifab_gemm_gated_bf16_2sm(a, lda, b, ldb, c, ldc, unit, limit, alpha, M, F, K, status, stream);
   CUtensorMap ta, tb;

@@ -26,11 +26,14 @@ using namespace ifab::tc;
 
 namespace {
 
-constexpr int TN = 256;                         // tile N (both CTAs together), also the accumulator's TMEM columns
-constexpr int HALF_N = TN / 2;                  // B rows a CTA supplies
-constexpr int STAGES2 = 6;
-constexpr int A2_BYTES = BM * BK * 2, B2_BYTES = HALF_N * BK * 2, STAGE2_BYTES = A2_BYTES + B2_BYTES;
-constexpr int SMEM2 = STAGES2 * STAGE2_BYTES + 1024 + 256;
+// TN: columns of a pair's tile (both CTAs together), also the accumulator's TMEM columns. A CTA supplies TN / 2 rows of B.
+template <int TN>
+struct Cfg2 {
+  static constexpr int HALF_N = TN / 2, STAGES2 = TN == 256 ? 6 : TN == 192 ? 7 : 8;
+  static constexpr int A2_BYTES = BM * BK * 2, STAGE2_BYTES = A2_BYTES + HALF_N * BK * 2;
+  static constexpr int SMEM2 = STAGES2 * STAGE2_BYTES + 1024 + 256;
+  static constexpr int COLS = TN <= 128 ? 128 : 256;          // an accumulator's share of tensor memory (powers of two)
+};
 
 struct Gemm2Params {
   void* c; long ldc; int out_f32;
@@ -139,8 +142,11 @@ __device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int
 }
 
 // grid (2 * M / 256, N / 256), clusters of 2 along x; 192 threads
+template <int TN>
 __global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                                           Gemm2Params p) {
+  using C2 = Cfg2<TN>;
+  constexpr int HALF_N = C2::HALF_N, STAGES2 = C2::STAGES2, A2_BYTES = C2::A2_BYTES, STAGE2_BYTES = C2::STAGE2_BYTES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES2 * STAGE2_BYTES);
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant_
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
   }
-  if (warp == 1) tmem_alloc_pair(tmem_slot, TN);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, C2::COLS);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                            // the peer's barriers and tensor memory exist before anything is signalled or issued
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant_
   cluster_sync_all();                            // nobody reads the peer's shared or tensor memory any more
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, TN);
+    tmem_dealloc_pair(tmem_base, C2::COLS);
   }
 }
 
@@ -259,8 +265,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 
 // grid (2 * pairs), clusters of 2; 192 threads
+template <int TN>
 __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                                                      Gemm2Params p) {
+  using C2 = Cfg2<TN>;
+  constexpr int HALF_N = C2::HALF_N, STAGES2 = C2::STAGES2, A2_BYTES = C2::A2_BYTES, STAGE2_BYTES = C2::STAGE2_BYTES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES2 * STAGE2_BYTES);
@@ -291,7 +300,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
   }
-  if (warp == 1) tmem_alloc_pair(tmem_slot, 2 * TN);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 2 * C2::COLS);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();
@@ -330,7 +339,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
       // the accumulator half must have been drained by the epilogue of tile j - 2
       if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1, p.spin_limit)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t d = tmem_base + (uint32_t)(b * TN);
+      const uint32_t d = tmem_base + (uint32_t)(b * C2::COLS);
       for (int kb = 0; kb < num_kb && ok; ++kb, ++it) {
         const int s = (int)(it % STAGES2);
         if (!mbar_wait(&full[s], (it / STAGES2) & 1, p.spin_limit) || *abort_flag) { ok = false; break; }
@@ -366,7 +375,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
       tile_coords(t, tiles_m, tiles_n, &tm, &tn);
       const int m0 = tm * 2 * BM + (int)rank * BM, n0 = F > 0 ? tn * HALF_N : tn * TN;
       const int row = m0 + q * 32 + lane;
-      const uint32_t tm_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TN);
+      const uint32_t tm_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * C2::COLS);
       if (F > 0) {
 #pragma unroll 1
         for (int c0 = 0; c0 < HALF_N; c0 += 32) {
@@ -397,14 +406,55 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, 2 * TN);
+    tmem_dealloc_pair(tmem_base, 2 * C2::COLS);
   }
+}
+
+int pairs_of_device() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::max(1, sms / 2);
+}
+// Columns of a tile: of 256, 192 and 128 the width whose waves of tiles over the pairs take least. A K block costs a pair what it loads - 128 rows of A
+// and TN / 2 of B in each CTA, about 87 GB/s an SM - rather than what it multiplies, so narrow tiles gain less than their width: 2048 x 3072 (K 2048)
+// 32.5 us by 256, 30.3 by 192, 39.7 by 128; 2048 x 8192 56.7, 64.8, 83.6; 1024 x 2048 (K 6144, residual) 42.5, 41.7, 37.8.
+int tile_width(int M, int N, int pairs) {
+  int best = 256;
+  long least = 0;
+  for (int tn : {256, 192, 128}) {
+    const long tiles = (long)((M + 255) / 256) * ((N + tn - 1) / tn), cost = (tiles + pairs - 1) / pairs * (256 + tn);
+    if (!least || cost < least) least = cost, best = tn;
+  }
+  return best;
+}
+template <int TN>
+int launch_2sm(const void* a, long lda, const void* b, long ldb, const Gemm2Params& p, int persistent, int pairs, cudaStream_t s) {
+  CUtensorMap ta, tb;
+  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)lda, BM)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb, TN / 2)) return rc;
+  const int cols = p.swiglu_f > 0 ? (p.swiglu_f + TN / 2 - 1) / (TN / 2) : (p.N + TN - 1) / TN, tiles = (p.M + 255) / 256 * cols;
+  constexpr int smem = Cfg2<TN>::SMEM2;
+  if (persistent < 0) persistent = tiles > pairs;
+  if (!persistent) {
+    auto k = tc_gemm_2sm_kernel<TN>;
+    if (int rc = opt_in_smem(k, smem)) return rc;
+    return launch_chain_cluster(k, dim3(2 * ((p.M + 255) / 256), cols), dim3(192), 2, (size_t)smem, s, ta, tb, p);
+  }
+  auto k = tc_gemm_2sm_persistent_kernel<TN>;
+  if (int rc = opt_in_smem(k, smem)) return rc;
+  return launch_chain_cluster(k, dim3(2 * std::max(1, std::min(tiles, pairs))), dim3(192), 2, (size_t)smem, s, ta, tb, p);
+}
+int dispatch_2sm(const void* a, long lda, const void* b, long ldb, const Gemm2Params& p, int persistent, cudaStream_t s) {
+  const int pairs = pairs_of_device(), tn = tile_width(p.M, p.N, pairs);
+  return tn == 256 ? launch_2sm<256>(a, lda, b, ldb, p, persistent, pairs, s) : tn == 192 ? launch_2sm<192>(a, lda, b, ldb, p, persistent, pairs, s)
+                                                                                           : launch_2sm<128>(a, lda, b, ldb, p, persistent, pairs, s);
 }
 
 }  // namespace
 
-// C[M,N] = act(A[M,K] * B[N,K]^T (+ residual)) with CTA pairs on 256 x 256 tiles. N % 32 == 0, K % 8 == 0. `persistent`: one CTA pair per
-// SM pair walks the tiles with two accumulators in tensor memory, else one pair per tile.
+// C[M,N] = act(A[M,K] * B[N,K]^T (+ residual)) with CTA pairs on tiles of 256 rows. N % 32 == 0, K % 8 == 0. `persistent` 1: one CTA pair per
+// SM pair walks the tiles with two accumulators in tensor memory; 0: one pair per tile; -1: the former where there are more tiles than pairs.
 extern "C" int ifab_gemm_act_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                       int act, int persistent, int M, int N, int K, uint32_t* status, void* stream) {
   return ifab_gemm_epilogue_bf16_2sm(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, nullptr, act, 0.f, persistent, M, N, K, status, stream);
@@ -412,22 +462,8 @@ extern "C" int ifab_gemm_act_bf16_2sm(const void* a, long lda, const void* b, lo
 extern "C" int ifab_gemm_epilogue_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                            const float* bias, int act, float cap, int persistent, int M, int N, int K, uint32_t* status, void* stream) {
   if (M < 1 || N < 32 || N % 32 || K < 8 || K % 8 || lda % 8 || ldb % 8) return -1;
-  CUtensorMap ta, tb;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, HALF_N)) return rc;
-  Gemm2Params p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, 0, act, bias, cap, {}};
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
-  if (!persistent) {
-    if (int rc = opt_in_smem(tc_gemm_2sm_kernel, SMEM2)) return rc;
-    dim3 grid(2 * ((M + 255) / 256), (N + 255) / 256);
-    return launch_chain_cluster(tc_gemm_2sm_kernel, grid, dim3(192), 2, (size_t)SMEM2, (cudaStream_t)stream, ta, tb, p);
-  }
-  if (int rc = opt_in_smem(tc_gemm_2sm_persistent_kernel, SMEM2)) return rc;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int pairs = std::max(1, std::min(tiles, sms / 2));
-  return launch_chain_cluster(tc_gemm_2sm_persistent_kernel, dim3(2 * pairs), dim3(192), 2, (size_t)SMEM2, (cudaStream_t)stream, ta, tb, p);
+  const Gemm2Params p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, 0, act, bias, cap, {}};
+  return dispatch_2sm(a, lda, b, ldb, p, persistent, (cudaStream_t)stream);
 }
 extern "C" int ifab_gemm_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                   int M, int N, int K, uint32_t* status, void* stream) {
@@ -448,15 +484,6 @@ extern "C" int ifab_gemm_gated_bf16_2sm(const void* a, long lda, const void* b, 
                                         int K, uint32_t* status, void* stream) {
   const GatedUnit gu{unit, limit, alpha};
   if (!gated_ok(gu) || M < 1 || F < 32 || F % 32 || K < 8 || K % 8 || lda % 8 || ldb % 8) return -1;
-  CUtensorMap ta, tb;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, HALF_N)) return rc;
-  Gemm2Params p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, F, 0, nullptr, 0.f, gu};
-  if (int rc = opt_in_smem(tc_gemm_2sm_persistent_kernel, SMEM2)) return rc;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = ((M + 255) / 256) * ((F + HALF_N - 1) / HALF_N);
-  const int pairs = std::max(1, std::min(tiles, sms / 2));
-  return launch_chain_cluster(tc_gemm_2sm_persistent_kernel, dim3(2 * pairs), dim3(192), 2, (size_t)SMEM2, (cudaStream_t)stream, ta, tb, p);
+  const Gemm2Params p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, F, 0, nullptr, 0.f, gu};
+  return dispatch_2sm(a, lda, b, ldb, p, 1, (cudaStream_t)stream);
 }

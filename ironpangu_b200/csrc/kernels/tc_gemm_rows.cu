@@ -144,6 +144,9 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
     for (; ahead < min(nk, C::STAGES); ++ahead) load_w(ahead);
   __syncwarp();
   grid_dep_wait();
+  if (warp == 0 && lane == 0)
+    for (int kb = 0; kb < ahead; ++kb) load_a(kb);
+  __syncwarp();
   if (warp == 1) tmem_alloc(tmem_slot, C::COLS);
   tc_fence_before();
   __syncthreads();
@@ -152,8 +155,7 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0 && lane == 0) {
-    int issued = ahead, acts = 0;
-    for (; acts < ahead; ++acts) load_a(acts);
+    int issued = ahead;
     for (int kb = ahead; kb < nk; ++kb) {
       if (kb >= C::STAGES && !mbar_wait(&empty[kb % C::STAGES], (kb / C::STAGES - 1) & 1, p.spin_limit)) *abort_flag = 1;
       if (*abort_flag) break;
@@ -235,6 +237,16 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
   cluster_sync();                    // the parts stay until every CTA has read them
 }
 
+int blocks_of(int K) { return (K + BK - 1) / BK; }
+// CTAs of a tile's cluster: as many as fit two to an SM over all tiles, with at least eight K blocks (128 KB of weights) in each - below that the start
+// and the sum outweigh the stream (8 rows, N 3072 K 2048: 7.3 us by 8, 5.8 by 4). Powers of two: clusters of 3 or 6 leave SMs of a GPC idle (200
+// rows, N 3072: 16.9 us by 6, 11.7 by 4).
+int splits_of(int tiles, int blocks) {
+  int splits = 8;
+  while (splits > 1 && (tiles * splits > 296 || blocks < 8 * splits || (blocks + splits - 1) / splits * (splits - 1) >= blocks)) splits /= 2;
+  return splits;
+}
+
 template <int TOK>
 int launch(const void* a, long lda, const void* b, long ldb, RowsParams p, cudaStream_t s) {
   auto k = tc_gemm_rows_kernel<TOK>;
@@ -245,16 +257,21 @@ int launch(const void* a, long lda, const void* b, long ldb, RowsParams p, cudaS
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)lda, (uint32_t)p.box)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, b, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb, p.F > 0 ? FT / 2 : FT)) return rc;
   const int tiles = p.F > 0 ? (p.F + FT / 2 - 1) / (FT / 2) : (p.N + FT - 1) / FT, ty = (p.M + TOK - 1) / TOK;
-  // As many CTAs as fit two to an SM, with at least four K blocks (64 KB of weights) in each: below that the start and the sum outweigh the stream.
-  const int blocks = (p.K + BK - 1) / BK;
-  int splits = 296 / (tiles * ty);
-  splits = splits < 1 ? 1 : splits > 8 ? 8 : splits;
-  while (splits > 1 && (blocks < 4 * splits || (blocks + splits - 1) / splits * (splits - 1) >= blocks)) --splits;
-  p.splits = splits;
-  return launch_chain_cluster(k, dim3(tiles * splits, ty), dim3(192), (unsigned)splits, (size_t)smem, s, ta, tw, p);
+  p.splits = splits_of(tiles * ty, blocks_of(p.K));
+  return launch_chain_cluster(k, dim3(tiles * p.splits, ty), dim3(192), (unsigned)p.splits, (size_t)smem, s, ta, tw, p);
 }
 
 }  // namespace
+
+// Whether a product of M >= 256 rows is better here than on CTA pairs (tc_gemm_2sm.cu): by the K blocks an SM has to load one after the other (32 KB and 0.37 us
+// each in both), and only where sharing K saves 32 of them - the sum over the cluster costs what it saves below that. 509 x 2048: K 6144 20.7 us here, 34.6 there;
+// K 2048 13.6 and 14.3; 300 x 3072 (K 2048) 17.1 and 15.2.
+bool ifab::tc::rows_better(int M, int N, int K, int F) {
+  const int ty = (M + 127) / 128, tiles = F > 0 ? (F + FT / 2 - 1) / (FT / 2) : (N + FT - 1) / FT, blocks = blocks_of(K), splits = splits_of(tiles * ty, blocks);
+  const long here = (long)((blocks + splits - 1) / splits) * ((tiles * ty * splits + 147) / 148);
+  const long pairs = (long)((M + 255) / 256) * ((N + 255) / 256), there = (pairs + 73) / 74 * blocks;
+  return M <= 1024 && there - here >= 32;
+}
 
 // The caller has checked shapes and strides (tc_gemm.cu); F > 0: gated, N = 2 F.
 extern "C" int ifab_gemm_rows_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,

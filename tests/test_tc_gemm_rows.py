@@ -16,11 +16,13 @@ def _slack(a, b):
 
 
 @pytest.mark.parametrize("fixed", [False, True])
-@pytest.mark.parametrize("M", [1, 7, 8, 16, 17, 33, 64, 65, 127, 128])
-@pytest.mark.parametrize("N,K", [(8, 8), (100, 72), (128, 64), (129, 520), (1000, 1152), (3072, 2048)])
+@pytest.mark.parametrize("M", [1, 7, 8, 16, 17, 33, 64, 65, 127, 128, 129, 200, 255, 300])
+@pytest.mark.parametrize("N,K", [(8, 8), (100, 72), (128, 64), (129, 520), (1000, 1152), (2048, 6144), (3072, 2048)])
 def test_any_rows_columns_and_depth(M, N, K, fixed):
     from ironpangu_b200.ops import gemm as G
 
+    if M >= 256 and not (fixed and (N, K) == (2048, 6144)):
+        pytest.skip("another kernel's")
     g = torch.Generator(device="cuda").manual_seed(M * 7 + N + K)
     a, b = _rand(g, M, K + 8)[:, :K], _rand(g, N, K)
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
@@ -37,7 +39,7 @@ def test_any_rows_columns_and_depth(M, N, K, fixed):
     assert int(status) == 0
 
 
-@pytest.mark.parametrize("M", [1, 9, 64, 100])
+@pytest.mark.parametrize("M", [1, 9, 64, 100, 190])
 @pytest.mark.parametrize("F,K", [(8, 64), (72, 136), (192, 1024), (1000, 512)])
 def test_gated_units_and_epilogues(M, F, K):
     from ironpangu_b200.ops import stream_norm as N
