@@ -456,6 +456,9 @@ class PlanEngine:
         self.launches_per_forward = (per_token - (4 * len(self.head_groups) if self.fused_head else 0)
                                      - (2 * len(self.moe_groups) if self.fused_moe else 0) - (4 * len(self.gqa_groups) if self.fused_gqa else 0))
         self._describe()
+        from ..models.mla_moe import MlaMoeConfig
+        self._norm_rows = (torch.empty(self.T, (max(self.cfg.hidden, self.cfg.q_lora) + 7) // 8 * 8, dtype=torch.bfloat16, device=self.tokens.device)
+                           if isinstance(self.cfg, MlaMoeConfig) else None)
 
     def _describe(self) -> None:
         """What the program says about the model, in the vocabulary of the hand-wired decoder (``models/mla_moe.py``): a
@@ -686,6 +689,8 @@ class PlanEngine:
         head = (self.fused_head if self.fuse_override is None else (self.fuse_override and self.can_fuse_head)) and T <= self.fused_head_rows
         moe = self.fused_moe and T <= 2
         gqa = self.fused_gqa
+        # the hand-wired decoder's rule (models/mla_moe.py): dense linears of three and more rows as tensor-core products
+        product = self._norm_rows is not None and T >= 3 and self.world == 1 and fab.world == 1
         probe = self.probe
         for k, i in enumerate(self.ins):
             op, a, ins = i["op"], i["attrs"], i["inputs"]
@@ -750,7 +755,13 @@ class PlanEngine:
                 V[k] = src[:, s:s + w]
             elif op == "linear":
                 name = a["weight"] + ("|" + a["paired_weight"] if "paired_weight" in a else "")
-                K.gemv(val(ins[0]), self._param(name), norm_w=norm_w, eps=eps, swiglu=a.get("activation") == "swiglu", out=val(k))
+                x, swiglu = val(ins[0]), a.get("activation") == "swiglu"
+                if product:
+                    K.linear_product(x, self._param(name), val(k), norm_w=norm_w, eps=eps, swiglu=swiglu, norm_out=self._norm_rows[:T, :x.shape[1]], status_ptr=st)
+                else:
+                    K.gemv(x, self._param(name), norm_w=norm_w, eps=eps, swiglu=swiglu, out=val(k))
+            elif op == "linear_allreduce" and product:
+                K.linear_product(val(ins[0]), self._param(a["weight"]), val(k), residual=val(ins[1]) if len(ins) > 1 else None, status_ptr=st)
             elif op == "linear_allreduce":
                 res = val(ins[1]) if len(ins) > 1 else None
                 K.gemv_allreduce(val(ins[0]), self._param(a["weight"]), fab, residual=res, out=val(k))
