@@ -207,6 +207,17 @@ __global__ void __launch_bounds__(256) moe_down_allreduce_kernel(DownParams p) {
   __shared__ int s_n;
   grid_dep_launch();
   grid_dep_wait();
+  if (gridDim.y > 1) {              // one rank: a CTA per token (T == 1)
+    const int t = blockIdx.y;
+    p.act += (size_t)t * (p.topk + 1) * p.ldact;
+    p.ids += t * p.topk;
+    p.wts += t * p.topk;
+    if (p.shared_w) p.shared_w += t;
+    if (p.residual) p.residual += t * p.ldr;
+    if (p.y_f32) p.y_f32 += t * p.ldy;
+    else p.y += t * p.ldy;
+    p.T = 1;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nbase = blockIdx.x * RPC, n0 = nbase + warp * R;
   if (threadIdx.x == 0) timed_out = 0;
@@ -378,12 +389,13 @@ __global__ void __launch_bounds__(256) moe_down_allreduce_kernel(DownParams p) {
                                  &timed_out);
 }
 
+// `tokens` > 1 (one rank, T == 1): a CTA per token and 8 R columns
 template <int T, int R>
-int launch_down(const DownParams& p, cudaStream_t s) {
+int launch_down(const DownParams& p, cudaStream_t s, int tokens = 1) {
   const size_t smem = (size_t)(p.topk * p.F + max(p.F, p.Fs)) * sizeof(bf16);
   auto k = moe_down_allreduce_kernel<T, R>;
   if (int rc = opt_in_smem(k, smem)) return rc;
-  dim3 grid((p.D + 8 * R - 1) / (8 * R));
+  dim3 grid((p.D + 8 * R - 1) / (8 * R), tokens);
   return launch_chain(k, grid, dim3(256), smem, s, p);
 }
 template <int T>
@@ -615,6 +627,7 @@ extern "C" int ifab_moe_gate_up_unit_decode(const void* x, long ldx, const void*
 namespace {
 int run_down(const DownParams& p, cudaStream_t s) {
   if (p.T <= 1) return dispatch_down<1>(p, s);
+  if (p.fv.world == 1 || p.y_f32) return launch_down<1, 2>(p, s, p.T);
   if (p.T <= 2) return dispatch_down<2>(p, s);
   if (p.T <= 4) return dispatch_down<4>(p, s);
   return dispatch_down<8>(p, s);
@@ -671,7 +684,8 @@ extern "C" int ifab_lm_head_capped_argmax(const void* x, long ldx, const void* n
   p.seq = fab->seq; p.done = fab->done;
   cudaStream_t s = (cudaStream_t)stream;
   // From three rows on the products above are bound by FMAs (8 rows of 153600 x 4096: 1048 us), the tensor-core product by the stream of the matrix
-  // (201 us, and 10 us for the norm ahead of it and the selection behind): it wants the logits stored, and room for the normalised rows behind the partial maxima.
+  // (201 us, and 10 us for the norm ahead of it and the selection behind; one row gains nothing, its kernel's loads start under the kernel before): it wants the
+  // logits stored, and room for the normalised rows behind the partial maxima.
   const unsigned ctas = (unsigned)((V_local + 1023) / 1024);
   const uint64_t maxima = (uint64_t)ctas * 8 * sizeof(float2), rows = norm_w ? (uint64_t)T * K * sizeof(bf16) : 0;
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w | (uintptr_t)partial | (uintptr_t)(ldx * sizeof(bf16));

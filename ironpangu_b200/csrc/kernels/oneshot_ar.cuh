@@ -92,7 +92,7 @@ __device__ __forceinline__ void oneshot_allreduce_slab(const float* slab, const 
   if (threadIdx.x == 0) {
     __threadfence();
     const uint32_t ticket = atomicAdd(done, 1u);
-    if (ticket == gridDim.x - 1) {
+    if (ticket == gridDim.x * gridDim.y - 1) {
       *done = 0;
       if (zero_on_last) *zero_on_last = 0;   // a counter of the calling kernel that every CTA has passed by now
       *seq = epoch;
