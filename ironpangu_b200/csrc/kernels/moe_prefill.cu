@@ -31,9 +31,11 @@ struct RouterBlockParams {
   int M, D, E, topk, scoring, renorm; float scale;
 };
 
-// one CTA per T tokens (8, or 4 when that is what fills the SMs); warps stride over the experts, then warp t selects for token t
+// one CTA per T tokens (8, or 4 when that is what fills the SMs); warps stride over the experts, then warp t selects for token t. Bound by the latency of
+// the router's rows in L2 (each CTA reads all of them), so sixteen warps with eight loads each in flight: 512 tokens, 96 experts x 4096: 84.6 us with
+// eight warps, 54.5 us with sixteen.
 template <int T>
-__global__ void __launch_bounds__(256) router_block_kernel(RouterBlockParams p) {
+__global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* xs = reinterpret_cast<bf16*>(smem_raw);               // [8][D] normalised
   float* lg = reinterpret_cast<float*>(xs + (size_t)T * p.D); // [8][E]
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(256) router_block_kernel(RouterBlockParams p) 
     }
   }
   const int quads = p.D >> 2;
-  for (int e = warp; e < p.E; e += 8) {
+  for (int e = warp; e < p.E; e += 16) {
     const float4* wr = reinterpret_cast<const float4*>(p.w + (long)e * p.D);
     float acc[T];
 #pragma unroll
@@ -337,11 +339,11 @@ extern "C" int ifab_router_block(const void* x, long ldx, const void* norm_w, fl
   if ((M + 7) / 8 >= 148) {
     const size_t smem = (size_t)8 * D * sizeof(bf16) + (size_t)8 * E * sizeof(float);
     if (int rc = opt_in_smem(router_block_kernel<8>, smem)) return rc;
-    return launch_chain(router_block_kernel<8>, dim3((M + 7) / 8), dim3(256), smem, (cudaStream_t)stream, p);
+    return launch_chain(router_block_kernel<8>, dim3((M + 7) / 8), dim3(512), smem, (cudaStream_t)stream, p);
   }
   const size_t smem = (size_t)4 * D * sizeof(bf16) + (size_t)4 * E * sizeof(float);
   if (int rc = opt_in_smem(router_block_kernel<4>, smem)) return rc;
-  return launch_chain(router_block_kernel<4>, dim3((M + 3) / 4), dim3(256), smem, (cudaStream_t)stream, p);
+  return launch_chain(router_block_kernel<4>, dim3((M + 3) / 4), dim3(512), smem, (cudaStream_t)stream, p);
 }
 
 extern "C" int ifab_moe_dispatch(const int32_t* ids, int M, int topk, int e0, int e_local, int32_t* counts, int32_t* route_row,

@@ -36,20 +36,23 @@ __global__ void __launch_bounds__(64) mla_q_rope_kernel(const bf16* q, long ldq,
 }
 
 // rotary columns of every head of a [T, H * (nope + rope)] query matrix, rotated in place (thread i owns the pair i, i + rope / 2)
-__global__ void __launch_bounds__(64) mla_q_rope_inplace_kernel(bf16* q, long ldq, const int32_t* positions, int nope, int rope, float theta) {
+// One CTA per row: the angles once for all heads (a CTA per head and row: 512 rows of 32 heads took 18.9 us).
+__global__ void __launch_bounds__(256) mla_q_rope_inplace_kernel(bf16* q, long ldq, const int32_t* positions, int H, int nope, int rope, float theta) {
+  extern __shared__ float cs[];          // [half] cos, then [half] sin
   grid_dep_launch();
   grid_dep_wait();
-  const int h = blockIdx.x, t = blockIdx.y;
-  const int half = rope / 2;
-  const int i = threadIdx.x;
-  if (i >= half) return;
+  const int t = blockIdx.x, half = rope / 2;
   const int pos = positions[t];
-  bf16* qr = q + (long)t * ldq + (long)h * (nope + rope) + nope;
-  float c, s;
-  rope_cos_sin(pos < 0 ? 0 : pos, i, rope, theta, &c, &s);
-  const float a = __bfloat162float(qr[i]), b = __bfloat162float(qr[i + half]);
-  qr[i] = __float2bfloat16_rn(a * c - b * s);
-  qr[i + half] = __float2bfloat16_rn(b * c + a * s);
+  for (int i = threadIdx.x; i < half; i += blockDim.x) rope_cos_sin(pos < 0 ? 0 : pos, i, rope, theta, &cs[i], &cs[half + i]);
+  __syncthreads();
+  for (int j = threadIdx.x; j < H * half; j += blockDim.x) {
+    const int h = j / half, i = j - h * half;
+    bf16* qr = q + (long)t * ldq + (long)h * (nope + rope) + nope;
+    const float c = cs[i], s = cs[half + i];
+    const float a = __bfloat162float(qr[i]), b = __bfloat162float(qr[i + half]);
+    qr[i] = __float2bfloat16_rn(a * c - b * s);
+    qr[i + half] = __float2bfloat16_rn(b * c + a * s);
+  }
 }
 
 // The latent cache rows of keys 0 .. ctx - 1 of one sequence slot, copied out of their pages into two dense matrices: the
@@ -429,7 +432,7 @@ extern "C" int ifab_allreduce_rows_nvls(void* part_local, void* part_mc, const v
 
 extern "C" int ifab_mla_q_rope_inplace(void* q, long ldq, const int32_t* positions, int T, int H, int nope, int rope, float theta, void* stream) {
   if (rope != ROPE || T < 1 || H < 1) return -1;
-  return launch_chain(mla_q_rope_inplace_kernel, dim3(H, T), dim3(64), 0, (cudaStream_t)stream, (bf16*)q, ldq, positions, nope, rope, theta);
+  return launch_chain(mla_q_rope_inplace_kernel, dim3(T), dim3(256), (size_t)rope * sizeof(float), (cudaStream_t)stream, (bf16*)q, ldq, positions, H, nope, rope, theta);
 }
 
 // lat: [rows, 512], pe: [rows, 64] (rows >= ctx; the tail is zeroed)
