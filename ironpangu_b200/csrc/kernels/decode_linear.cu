@@ -112,15 +112,17 @@ int launch_gemv(const GemvParams& p, cudaStream_t s) {
 
 template <int T>
 int dispatch_rows(const GemvParams& p, cudaStream_t s) {
-  // pick rows-per-warp so that small N still spreads over the 148 SMs
-  const int n = p.N * (p.mode ? 2 : 1);
+  // Rows per warp: the fewest that leave no more CTAs than run at once, two on an SM (a second wave of a quarter of the CTAs costs as much as the first). Many
+  // columns that take several waves anyway: four rows, whose loads are in flight together. One row, K 2048, us: N 3072 6.4 by one, 4.1 by two; N 8192 13.2, 9.2
+  // by two, 6.9 by four; gated 6144 11.4 by two pairs, 9.7 by three.
   if (p.mode) {
-    if (n >= 148 * 8 * 4 * 2) return launch_gemv<T, 2>(p, s);
-    return launch_gemv<T, 1>(p, s);
+    if (p.N <= 296 * 8) return launch_gemv<T, 1>(p, s);
+    if (p.N <= 296 * 16 || p.N > 296 * 24) return launch_gemv<T, 2>(p, s);
+    return launch_gemv<T, 3>(p, s);
   }
-  if (n >= 148 * 8 * 4 * 2) return launch_gemv<T, 4>(p, s);
-  if (n >= 148 * 8 * 2 * 2) return launch_gemv<T, 2>(p, s);
-  return launch_gemv<T, 1>(p, s);
+  if (p.N <= 296 * 8) return launch_gemv<T, 1>(p, s);
+  if (p.N <= 296 * 16) return launch_gemv<T, 2>(p, s);
+  return launch_gemv<T, 4>(p, s);
 }
 
 // ----------------------------------------------------------------------------------------------

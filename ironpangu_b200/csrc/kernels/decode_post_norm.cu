@@ -56,6 +56,65 @@ __device__ __forceinline__ void stage_operand(const Params& p, bf16* xs, float* 
   const int groups = PRO == GROUP ? p.groups : 1, n = K / groups;
   const float* src = PRO == GROUP ? p.o : p.y;
   const long lds = PRO == GROUP ? p.ldo : p.ldy;
+  // One row of up to 8 columns a thread: everything the operand is made of is requested at once and stays in registers across the sums. (Read again
+  // behind the barriers, rows, gains and gates were a second trip to L2 or HBM: a step of the 2B
+  // falinex model 1168 us, 1070 so; with 16 columns a thread the registers cost more than that, 1318.) Groups of 128 columns are a warp's share.
+  constexpr int NV = 2;
+  if (T == 1 && K <= NV * 4 * nthr && (PRO == POST ? src && p.norm_w && !p.norm2_w && !p.extra : groups == 1 || n == 128)) {
+    const long r = t0;
+    const bf16* gate = p.gate + r * p.ldg;
+    const bool wide = PRO == GROUP && ((reinterpret_cast<uintptr_t>(gate) & 7) | (reinterpret_cast<uintptr_t>(p.gain) & 15)) == 0;
+    float4 v[NV], a[NV], b[NV];          // a: residual or gate, b: gains
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (tid + i * nthr) * 4;
+      v[i] = a[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      b[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (c >= K || r >= p.T) continue;
+      v[i] = *reinterpret_cast<const float4*>(src + r * lds + c);
+      if (PRO == POST) {
+        a[i] = *reinterpret_cast<const float4*>(p.x_in + r * p.ldr + c);
+        b[i] = *reinterpret_cast<const float4*>(p.norm_w + c);
+      } else if (wide) {
+        const uint2 u = *reinterpret_cast<const uint2*>(gate + c);
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        a[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+        if (p.gain) b[i] = *reinterpret_cast<const float4*>(p.gain + c);
+      } else {
+        a[i] = make_float4(__bfloat162float(gate[c]), __bfloat162float(gate[c + 1]), __bfloat162float(gate[c + 2]), __bfloat162float(gate[c + 3]));
+        if (p.gain) b[i] = make_float4(p.gain[c], p.gain[c + 1], p.gain[c + 2], p.gain[c + 3]);
+      }
+    }
+    float part[NV], iv[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) part[i] = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    if (groups == 1) {
+      float ss = warp_sum(part[0] + part[1]);
+      if (lane == 0) red[warp] = ss;
+      __syncthreads();
+      ss = 0.f;
+      for (int i = 0; i < nwarp; ++i) ss += red[i];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) iv[i] = 1.f / sqrtf(ss / (float)K + p.eps);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) iv[i] = 1.f / sqrtf(warp_sum(part[i]) / (float)n + p.eps);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (tid + i * nthr) * 4;
+      if (c >= K) break;
+      float f[4] = {v[i].x * iv[i] * b[i].x, v[i].y * iv[i] * b[i].y, v[i].z * iv[i] * b[i].z, v[i].w * iv[i] * b[i].w};
+      const float o[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = PRO == POST ? o[j] + f[j] : f[j] * activate<true>(o[j], p.gate_act);
+      if (PRO == POST && blockIdx.x == 0 && r < p.T) *reinterpret_cast<float4*>(p.x_out + r * p.ldr + c) = make_float4(f[0], f[1], f[2], f[3]);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+      *reinterpret_cast<uint2*>(xs + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    __syncthreads();
+    return;
+  }
   if (PRO == POST && !p.norm_w) {
     // nothing to divide by
   } else if (groups == 1) {

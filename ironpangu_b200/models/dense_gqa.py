@@ -175,6 +175,13 @@ class DenseDecoder:
         self.launches_per_forward = 2 + 8 * c.layers
         self._graph = None
 
+    def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor) -> None:
+        """``x += a @ w.T`` summed over the ranks (one rank: the same bits without the call counter)."""
+        if self.fabric.world == 1:
+            K.gemv(a, w, residual=x, out=x)
+        else:
+            K.gemv_allreduce(a, w, self.fabric, residual=x, out=x)
+
     def forward(self, T: Optional[int] = None, sample: bool = True) -> torch.Tensor:
         c, w, fab = self.cfg, self.w, self.fabric
         T = self.T if T is None else T
@@ -191,9 +198,9 @@ class DenseDecoder:
                                    kv_heads=self.hk, head_dim=c.head_dim, scale=1.0 / math.sqrt(c.head_dim),
                                    keys_per_split=self.kps, max_splits=self.max_splits, scratch=self.scratch,
                                    out=self.attn[:T], status_ptr=st)
-            K.gemv_allreduce(self.attn[:T], w[p + "o_proj"], fab, residual=x, out=x)
+            self._row_parallel(self.attn[:T], w[p + "o_proj"], x)
             K.gemv(x, w[p + "gate_up"], norm_w=w[p + "ffn_norm"], eps=c.eps, swiglu=True, out=self.act[:T])
-            K.gemv_allreduce(self.act[:T], w[p + "down"], fab, residual=x, out=x)
+            self._row_parallel(self.act[:T], w[p + "down"], x)
         if sample:
             K.lm_head_argmax(x, w["lm_head"], fab, norm_w=w["final_norm"], eps=c.eps, vocab_offset=self.rank * self.vl,
                              partial=self.partial, logits=None if self.logits is None else self.logits[:T],
