@@ -264,13 +264,13 @@ int launch(const void* a, long lda, const void* b, long ldb, RowsParams p, cudaS
 }  // namespace
 
 // Whether a product of M >= 256 rows is better here than on CTA pairs (tc_gemm_2sm.cu): by the K blocks an SM has to load one after the other (32 KB and 0.37 us
-// each in both), and only where sharing K saves 32 of them - the sum over the cluster costs what it saves below that. 509 x 2048: K 6144 20.7 us here, 34.6 there;
-// K 2048 13.6 and 14.3; 300 x 3072 (K 2048) 17.1 and 15.2.
+// each in both), and only where sharing K saves 16 of them - the sum over the cluster costs what it saves below that. 509 x 2048: K 6144 20.7 us here, 34.6 there;
+// K 2048 13.6 and 14.3; 509 x 3072 (K 2048, nothing saved) 18.3 and 15.6.
 bool ifab::tc::rows_better(int M, int N, int K, int F) {
   const int ty = (M + 127) / 128, tiles = F > 0 ? (F + FT / 2 - 1) / (FT / 2) : (N + FT - 1) / FT, blocks = blocks_of(K), splits = splits_of(tiles * ty, blocks);
   const long here = (long)((blocks + splits - 1) / splits) * ((tiles * ty * splits + 147) / 148);
   const long pairs = (long)((M + 255) / 256) * ((N + 255) / 256), there = (pairs + 73) / 74 * blocks;
-  return M <= 1024 && there - here >= 32;
+  return M <= 1024 && there - here >= 16;
 }
 
 // The caller has checked shapes and strides (tc_gemm.cu); F > 0: gated, N = 2 F.
