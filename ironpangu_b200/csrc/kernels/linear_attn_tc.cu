@@ -110,9 +110,10 @@ __device__ __forceinline__ void finish8(const LaParams& p, const bf16* head, con
       f[2 * i] = f[2 * i] * r.t[i].x + sign * g[2 * i] * r.t[i].y;
       f[2 * i + 1] = f[2 * i + 1] * r.t[i].z + sign * g[2 * i + 1] * r.t[i].w;
     }
-  } else if (p.act) {
+  } else if (p.act) {             // values of the activation type, before and after
+    activate_all<true, 8>(f, p.act);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = activated(p, __float2bfloat16_rn(f[i]));
+    for (int i = 0; i < 8; ++i) f[i] = bf16_round(f[i]);
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) f[i] *= scale;
@@ -427,12 +428,15 @@ __global__ void __launch_bounds__(THREADS, 1) la_tile_out_kernel(TileParams p) {
       for (int x = 0; x < 32; x += 8) {
         if (c0 + x >= a.e) break;
         float f[8], g[8];
-        if (wide) unpack8(*reinterpret_cast<const uint4*>(gr + x), g);
+        if (wide) {
+          unpack8(*reinterpret_cast<const uint4*>(gr + x), g);
+        } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (!wide) g[k] = c0 + x + k < a.e ? to_f32(gr[x + k]) : 0.f;
-          f[k] = o[x + k] * inv * activate<true>(g[k], p.gate_act);
+          for (int k = 0; k < 8; ++k) g[k] = c0 + x + k < a.e ? to_f32(gr[x + k]) : 0.f;
         }
+        activate_all<true, 8>(g, p.gate_act);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = o[x + k] * inv * g[k];
         if (wide) {
           *reinterpret_cast<uint4*>(dst + x) = pack8(f);
         } else {
@@ -450,7 +454,7 @@ __global__ void __launch_bounds__(THREADS, 1) la_tile_out_kernel(TileParams p) {
         if (c0 + x < a.e) *reinterpret_cast<float4*>(dst + x) = make_float4(o[x], o[x + 1], o[x + 2], o[x + 3]);
     } else {
 #pragma unroll
-      for (int x = 0; x < 64; ++x)
+      for (int x = 0; x < 32; ++x)
         if (c0 + x < a.e) dst[x] = o[x];
     }
   }

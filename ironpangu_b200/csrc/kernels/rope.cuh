@@ -74,6 +74,31 @@ __device__ __forceinline__ float activate(float z, int act) {
   }
 }
 
+// the same of N values: the choice outside, so that the values' chains run side by side instead of a branch ahead of each, which made the epilogue of a
+// 256 x 256 tile longer than its product (1505 x 6144, K 2048: GELU 75.7 us, 34.7 so; 34.4 without an activation)
+template <bool FAST, int N>
+__device__ __forceinline__ void activate_all(float* v, int act) {
+  switch (act) {
+    case 1:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = v[i] * sigmoid_f32<FAST>(v[i]);
+      break;
+    case 2:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = sigmoid_f32<FAST>(v[i]);
+      break;
+    case 3:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = gelu_tanh_f32<FAST>(v[i]);
+      break;
+    case 4:
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = gelu_erf_f32<FAST>(v[i]);
+      break;
+    default: break;
+  }
+}
+
 // What a gated feed-forward makes of its two projections: 0 silu(g) u, 1 relu(g) u, 2 g' sigmoid(alpha g') (u' + 1) with g' = min(g, limit) and
 // u' = u within [-limit, limit]
 struct GatedUnit {
@@ -91,11 +116,25 @@ __device__ __forceinline__ float gated_value(float g, float u, const GatedUnit& 
 }
 // the same of projections that count as bf16 rows for SiLU units (the form of the kernels that store them). The division is the fast one: the full one
 // branches, which keeps the compiler from working on more than one value of an epilogue at a time (a 128 x 128 tile then took 25 us, more than its
-// product at K = 2048: 2048 rows of 2 x 6144 columns 151 us, 92 so); 1 + exp(-g) beyond 2^126 gives 0, the limit.
+// product at K = 2048: 2048 rows of 2 x 6144 columns 151 us, 92 with it); 1 + exp(-g) beyond 2^126 gives 0, the limit.
 __device__ __forceinline__ float gated_bf16(float g, float u, const GatedUnit& unit) {
   if (unit.kind) return gated_value<true>(g, u, unit);
   g = bf16_round(g);
   return __fdividef(g, 1.f + __expf(-g)) * bf16_round(u);
+}
+// the same of N values, the kind chosen once (2048 rows of 2 x 6144 columns, K 2048: 92 us with the choice at every value, 81 so)
+template <int N>
+__device__ __forceinline__ void gated_all(float* g, const float* u, const GatedUnit& unit) {
+  if (unit.kind == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const float x = bf16_round(g[i]);
+      g[i] = __fdividef(x, 1.f + __expf(-x)) * bf16_round(u[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) g[i] = gated_value<true>(g[i], u[i], unit);
+  }
 }
 __host__ __forceinline__ bool gated_ok(const GatedUnit& u) { return u.kind >= 0 && u.kind <= 2 && (u.kind != 2 || u.limit > 0.f); }
 

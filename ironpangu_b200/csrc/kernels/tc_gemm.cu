@@ -52,10 +52,7 @@ __device__ __forceinline__ void store_row32(const GemmParams& p, int row, int co
     const bf16* r = p.residual + (long)row * p.ldr + col;
     for (int i = 0; i < nvalid; ++i) v[i] = bf16_round(v[i]) + __bfloat162float(r[i]);
   }
-  if (p.act) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = activate<true>(v[i], p.act);
-  }
+  activate_all<true, 32>(v, p.act);
   if (p.cap > 0.f) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = soft_limit<true>(v[i], p.cap);

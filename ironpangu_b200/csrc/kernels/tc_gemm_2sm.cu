@@ -114,10 +114,7 @@ __device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int
       for (int i = 0; i < 32; ++i) v[i] = bf16_round(v[i]) + __bfloat162float(r[i]);
     }
   }
-  if (p.act) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = activate<true>(v[i], p.act);
-  }
+  activate_all<true, 32>(v, p.act);
   if (p.cap > 0.f) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = soft_limit<true>(v[i], p.cap);
@@ -383,8 +380,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
           tmem_ld_32x32(tm_row + (uint32_t)c0, v);
           tmem_ld_32x32(tm_row + (uint32_t)(HALF_N + c0), u);
           tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = gated_bf16(v[i], u[i], p.unit);
+          gated_all<32>(v, u, p.unit);
           store_row32_2(p, row, n0 + c0, v);
         }
       } else {
