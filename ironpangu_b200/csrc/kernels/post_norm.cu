@@ -51,7 +51,8 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const int32_t* ids, con
   for (int c = threadIdx.x; c < D; c += blockDim.x) xa[(long)t * lda + c] = from_f32<A>(to_f32(table[(long)id * ldt + c]) * scale * inv * w[c]);
 }
 
-// one CTA per row
+// one CTA per row. Rows of up to 2048 columns that fill the chip by themselves (four to an SM) take 128 threads, whose reductions are half as deep: 1505 x 2048
+// 7.7 us with 256 threads, 6.9 us so; below that a row's own chain counts, 27 x 2048 2.2 us with 256 threads and 3.0 us with 128.
 template <typename A>
 __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* y, long ldy, int parts, long part_stride, const float* w, const float* w2, float eps, float* x, long ldx,
                                                             const float* extra, long lde, A* xa, long lda, int D) {
@@ -63,12 +64,12 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* y, long
   const float* er = extra ? extra + (long)t * lde : nullptr;
   float* xr = x + (long)t * ldx;
   A* ar = xa + (long)t * lda;
-  if (D % 4 == 0 && ldy % 4 == 0 && ldx % 4 == 0 && lda % 4 == 0 && lde % 4 == 0 && part_stride % 4 == 0 && D <= 256 * 16) {     // the row stays in registers between the passes
+  if (D % 4 == 0 && ldy % 4 == 0 && ldx % 4 == 0 && lda % 4 == 0 && lde % 4 == 0 && part_stride % 4 == 0 && D <= (int)blockDim.x * 16) {     // the row stays in registers between the passes
     float4 v[4], r[4], g[4];
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int c = (threadIdx.x + i * 256) * 4;
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
       v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       r[i] = v[i];
       g[i] = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* y, long
     ss = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int c = (threadIdx.x + i * 256) * 4;
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
       r[i].x += v[i].x * inv * g[i].x;
       r[i].y += v[i].y * inv * g[i].y;
       r[i].z += v[i].z * inv * g[i].z;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* y, long
     const float inv2 = w2 ? 1.f / sqrtf(block_sum(ss, red) / (float)D + eps) : 1.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int c = (threadIdx.x + i * 256) * 4;
+      const int c = (threadIdx.x + i * blockDim.x) * 4;
       if (c >= D) break;
       float f[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
       if (w2) {
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(256) rms_rows_kernel(const float* x, long ldx,
 // one warp per (row, group) for narrow groups, one CTA per row for a single wide one: grid (ceil(groups / WPB), rows)
 template <typename A, int WARPS_PER_GROUP>
 __global__ void __launch_bounds__(256) group_norm_gate_kernel(const float* o, long ldo, const float* w, float eps, const A* gate, long ldg, int act,
-                                                              A* y, long ldy, int groups, int n) {
+                                                              A* y, long ldy, int groups, int n, int wide) {
   __shared__ float red[33];
   grid_dep_launch();
   grid_dep_wait();
@@ -173,6 +174,42 @@ __global__ void __launch_bounds__(256) group_norm_gate_kernel(const float* o, lo
   if (WARPS_PER_GROUP == 1 && g >= groups) return;
   const float* r = o + (long)t * ldo + (long)g * n;
   float ss = 0.f;
+  // bf16 rows in pieces of four, kept in registers between the sum and the scaling (rows of 2048 columns, 1505 of them: heads of 128 7.6 us element by element,
+  // 5.5 so; one group 8.2 and 4.8; 27 of them: 2.6 and 1.7; 3.8 and 2.1)
+  constexpr int NV = WARPS_PER_GROUP == 1 ? 1 : 2;
+  if (sizeof(A) == 2 && n <= NV * 4 * TPG && wide) {
+    float4 v[NV];
+    uint2 u[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i0 + i * TPG) * 4;
+      v[i] = c < n ? *reinterpret_cast<const float4*>(r + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      u[i] = c < n ? *reinterpret_cast<const uint2*>(gate + (long)t * ldg + (long)g * n + c) : make_uint2(0u, 0u);
+      ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    }
+    ss = WARPS_PER_GROUP == 1 ? warp_sum(ss) : block_sum(ss, red);
+    const float inv = 1.f / sqrtf(ss / (float)n + eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = (i0 + i * TPG) * 4;
+      if (c >= n) break;
+      float f[4] = {v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv};
+      if (w) {
+        const float4 h = *reinterpret_cast<const float4*>(w + (long)g * n + c);
+        f[0] *= h.x;
+        f[1] *= h.y;
+        f[2] *= h.z;
+        f[3] *= h.w;
+      }
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[i].x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[i].y));
+      float a[4] = {lo.x, lo.y, hi.x, hi.y};
+      activate_all<true, 4>(a, act);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] *= a[e];
+      store4(y + (long)t * ldy + (long)g * n + c, f);
+    }
+    return;
+  }
   for (int c = i0; c < n; c += TPG) ss += r[c] * r[c];
   ss = WARPS_PER_GROUP == 1 ? warp_sum(ss) : block_sum(ss, red);
   const float inv = 1.f / sqrtf(ss / (float)n + eps);
@@ -211,10 +248,11 @@ int embed(const int32_t* ids, const void* table, long ldt, float scale, const fl
 template <typename A>
 int group_norm(const float* o, long ldo, const float* w, float eps, const void* gate, long ldg, int act, void* y, long ldy, int T, int groups, int n,
                cudaStream_t s) {
+  const int wide = ((ldo | ldg | ldy | n) & 3) == 0 && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && (((uintptr_t)gate | (uintptr_t)y) & 7) == 0;
   if (n > 512)
-    return launch_chain(group_norm_gate_kernel<A, 8>, dim3(groups, T), dim3(256), 0, s, o, ldo, w, eps, (const A*)gate, ldg, act, (A*)y, ldy, groups, n);
+    return launch_chain(group_norm_gate_kernel<A, 8>, dim3(groups, T), dim3(256), 0, s, o, ldo, w, eps, (const A*)gate, ldg, act, (A*)y, ldy, groups, n, wide);
   return launch_chain(group_norm_gate_kernel<A, 1>, dim3((groups + 7) / 8, T), dim3(256), 0, s, o, ldo, w, eps, (const A*)gate, ldg, act, (A*)y, ldy,
-                      groups, n);
+                      groups, n, wide);
 }
 
 }  // namespace
@@ -234,8 +272,9 @@ extern "C" int ifab_post_norm_add(const float* y, long ldy, int parts, long part
   if (T < 1 || D < 1 || parts < 1) return -1;
   if (!y) parts = 1;
   cudaStream_t s = (cudaStream_t)stream;
-  return f32 ? launch_chain(post_norm_add_kernel<float>, dim3(T), dim3(256), 0, s, y, ldy, parts, part_stride, w, w2, eps, x, ldx, extra, lde, (float*)xa, lda, D)
-             : launch_chain(post_norm_add_kernel<bf16>, dim3(T), dim3(256), 0, s, y, ldy, parts, part_stride, w, w2, eps, x, ldx, extra, lde, (bf16*)xa, lda, D);
+  const dim3 threads(D <= 2048 && T >= 4 * 148 ? 128 : 256);
+  return f32 ? launch_chain(post_norm_add_kernel<float>, dim3(T), threads, 0, s, y, ldy, parts, part_stride, w, w2, eps, x, ldx, extra, lde, (float*)xa, lda, D)
+             : launch_chain(post_norm_add_kernel<bf16>, dim3(T), threads, 0, s, y, ldy, parts, part_stride, w, w2, eps, x, ldx, extra, lde, (bf16*)xa, lda, D);
 }
 
 // y [T, F] = unit(gu[:, c], gu[:, up + c])
