@@ -255,14 +255,17 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 // one (row, kv head); every warp streams 16 keys and values at a time through a ring of its own in shared memory (cp.async, 16 bytes, no barrier
 // among the warps) and keeps a running maximum, sum and output, merged at the end.
 //
-//   scores   m16n8k16: the group's query rows are rows 0-7 AND 8-15 of A (so both halves of C hold them), keys are columns
-//   values   the weights enter as two bf16 terms, value in rows 0-7 and remainder in rows 8-15 of A: one product carries 16 bits of a
-//            weight and the sum stays f32; the two halves of C are added at the end
+//   scores   m16n8k16: the group's query rows are rows 0-7 AND 8-15 of A (so both halves of C hold them), keys are columns. Groups of up to four are there
+//            twice in each half
+//   values   the weights enter as three bf16 terms that hold all of their 24 bits; the sum is f32 and the rows of C that belong to a head are added at the
+//            end. Up to four heads: the terms are rows 0-3, 8-11 and 4-7 of one product (a lane has the weights of its row, so it only picks a
+//            term). Eight (WIDE): the first two terms are rows 0-7 and 8-15, and in a second product half of the third is in both
 //
 // Bound by the stream of keys and values: a key costs a warp two instructions, where products on the CUDA cores (eight lanes to a key) cost 40 and
 // bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 77 us (4.3 TB/s); 8 rows of 1900 keys 46 -> 13 us, one row of
-// 2000 keys 14.8 -> 10.4 us, merge included. Three CTAs an
-// SM x four warps with one stage of 8 KB in flight beside the one in use.
+// 2000 keys 14.8 -> 10.4 us, merge included. Two CTAs an SM (registers) x four warps
+// with one stage of 8 KB in flight beside the one in use. The third term costs groups of up to four nothing (64 rows of up to 4096 keys 91.6 us without it, 89.9
+// with), groups of eight their second product (over one kv head 33.2 and 37.6 us).
 template <int HD>
 struct MmaSplit {
   static constexpr int KEYS = 16, WARPS = 4, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
@@ -283,7 +286,7 @@ __device__ __forceinline__ float peer_float(const float* mine, uint32_t rank) {
 
 // CLUSTER: the splits of a (row, kv head) are one cluster (at most eight) and merge their parts over distributed shared memory into `out`; otherwise
 // the parts go to the scratch and gqa_merge_kernel follows.
-template <int HD, bool CLUSTER>
+template <int HD, bool CLUSTER, bool WIDE>
 __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
   using S = MmaSplit<HD>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -296,20 +299,20 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
   const int n = seen.n, per = p.per_split(n), k_begin = split * per;
   if (!CLUSTER && k_begin >= n) return;
   const int k_end = min(n, k_begin + per);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2, G = p.Hq / p.Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2, G = p.Hq / p.Hkv, gh = WIDE ? g : g & 3;      // gh: this lane's head of the group
   const int slot = p.slots[t];
   const bool ruled = !p.rule.plain();
-  const float slope = p.rule.slopes && g < G ? p.rule.slopes[kvh * G + g] : 0.f;
-  // query row g: columns 16 i + c2 + {0, 1} and + 8
+  const float slope = p.rule.slopes && gh < G ? p.rule.slopes[kvh * G + gh] : 0.f;
+  // query row of head gh: columns 16 i + c2 + {0, 1} and + 8
   uint32_t q[HD / 16][2];
   {
-    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + (g < G ? g : 0)) * HD + c2;
+    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + (gh < G ? gh : 0)) * HD + c2;
 #pragma unroll
     for (int i = 0; i < HD / 16; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const bf16 *e = qh + 16 * i + 8 * j;
-        q[i][j] = g < G ? (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16 : 0u;
+        q[i][j] = gh < G ? (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16 : 0u;
       }
   }
   float acc[HD / 8][4], m = -INFINITY, l = 0.f;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
         mma16816(s[0], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[0], b[1]);
         mma16816(s[1], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[2], b[3]);
       }
-      // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against query row g
+      // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against head gh
       float w[4];
       float mn = m;
 #pragma unroll
@@ -408,19 +411,24 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        w[j] = w[j] == -INFINITY ? 0.f : __expf(w[j] - m);
+        w[j] = w[j] == -INFINITY ? LEAST_WEIGHT : weight_of(w[j] - m);
         l += w[j];
       }
-      uint32_t a0, a1, a2, a3;
-      two_terms(w[0], w[1], &a0, &a1);
-      two_terms(w[2], w[3], &a2, &a3);
+      uint32_t lo[3], hi[3];                     // terms of the weights of keys c2, c2 + 1 and of keys c2 + 8, c2 + 9
+      three_terms(w[0], w[1], lo, WIDE ? 0.5f : 1.f);
+      three_terms(w[2], w[3], hi, WIDE ? 0.5f : 1.f);
+      const uint32_t lo0 = WIDE || g < 4 ? lo[0] : lo[2], hi0 = WIDE || g < 4 ? hi[0] : hi[2];
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) {
         uint32_t b[4];
         const int key = ((lane >> 3) & 1) * 8 + (lane & 7), ch = 2 * j + (lane >> 4);
         ldsm4t(vb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
-        mma16816(acc[2 * j], a0, a1, a2, a3, b[0], b[1]);
-        mma16816(acc[2 * j + 1], a0, a1, a2, a3, b[2], b[3]);
+        mma16816(acc[2 * j], lo0, lo[1], hi0, hi[1], b[0], b[1]);
+        mma16816(acc[2 * j + 1], lo0, lo[1], hi0, hi[1], b[2], b[3]);
+        if (WIDE) {
+          mma16816(acc[2 * j], lo[2], lo[2], hi[2], hi[2], b[0], b[1]);
+          mma16816(acc[2 * j + 1], lo[2], lo[2], hi[2], hi[2], b[2], b[3]);
+        }
       }
       __syncwarp();            // the stage is read: a later round may overwrite it
     }
@@ -436,8 +444,18 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
     sm_l[warp * 8 + g] = l;
   }
 #pragma unroll
-  for (int j = 0; j < HD / 8; ++j)
-    *reinterpret_cast<float2*>(sm_acc + (warp * 8 + g) * HD + 8 * j + c2) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
+  for (int j = 0; j < HD / 8; ++j) {
+    float2 v = make_float2(acc[j][0], acc[j][1]);
+    if (WIDE || g < 4) {       // rows 12-15 of groups up to four are nobody's
+      v.x += acc[j][2];
+      v.y += acc[j][3];
+    }
+    if (!WIDE) {               // rows 4-7: the third term
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+    }
+    if (WIDE || g < 4) *reinterpret_cast<float2*>(sm_acc + (warp * 8 + g) * HD + 8 * j + c2) = v;
+  }
   __syncthreads();
   float* part = sm_acc + S::WARPS * 8 * HD;        // CLUSTER: this split's [G][HD], then maxima and sums
   for (int h = 0; h < G; ++h) {
@@ -543,16 +561,16 @@ int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   if (int rc = launch_chain(k, grid, dim3(256), smem, s, p)) return rc;
   return launch_merge<HD>(p, out, ldo, s);
 }
-template <int HD>
+template <int HD, bool WIDE>
 int launch_mma(const GqaParams& p, bool cluster, bf16* out, long ldo, cudaStream_t s) {
   constexpr int smem = MmaSplit<HD>::SMEM;
   const dim3 grid(p.max_splits, p.Hkv, p.T);
   if (cluster) {
-    auto k = gqa_split_mma_kernel<HD, true>;
+    auto k = gqa_split_mma_kernel<HD, true, WIDE>;
     if (int rc = opt_in_smem(k, smem)) return rc;
     return launch_chain_cluster(k, grid, dim3(128), (unsigned)p.max_splits, smem, s, p, out, ldo);
   }
-  auto k = gqa_split_mma_kernel<HD, false>;
+  auto k = gqa_split_mma_kernel<HD, false, WIDE>;
   if (int rc = opt_in_smem(k, smem)) return rc;
   if (int rc = launch_chain(k, grid, dim3(128), smem, s, p, out, ldo)) return rc;
   return launch_merge<HD>(p, out, ldo, s);
@@ -563,7 +581,7 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
   const int G = p.Hq / p.Hkv;
   if (G != 1 && G != 2 && G != 4 && G != 8) return -1;
   // Many rows fill the chip by themselves: then fewer splits, each longer, so that a CTA's start and end and the merge weigh less: as many CTAs as two
-  // to an SM (three fit). 64 rows of 2560 keys: 77 us with 2 splits, 89 with 4; 27 rows of 1024: 20 us with 2, 35 with 8; 8 rows of 1900: 13 us with 8.
+  // to an SM. 64 rows of 2560 keys: 77 us with 2 splits, 89 with 4; 27 rows of 1024: 20 us with 2, 35 with 8; 8 rows of 1900: 13 us with 8.
   const int rows = p.T > 0 ? p.T * p.Hkv : 1, asked = p.max_splits, want = (296 + rows - 1) / rows;
   p.max_splits = asked < want ? asked : want;
   if constexpr (HD <= 128) {
@@ -576,7 +594,7 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
       }
-      return launch_mma<HD>(p, cluster, out, ldo, s);
+      return G == 8 ? launch_mma<HD, true>(p, cluster, out, ldo, s) : launch_mma<HD, false>(p, cluster, out, ldo, s);
     }
   }
   switch (G) {

@@ -316,13 +316,14 @@ __global__ void __launch_bounds__(256) mla_split_kernel(AttnParams p) {
 
 // The same on the tensor cores (bf16 caches): a CTA of eight warps takes HM x 16 heads of one (split, row) over tiles of 32 keys, which come through two
 // stages of shared memory (cp.async). Scores: warp w has head tile w % HM and eight keys (HM = 1: half the warps idle), m16n8k16 over the 576 columns; softmax: eight threads to a
-// head, weights as two bf16 terms through shared memory; values: 64 latent columns per warp for all heads, both terms into the same f32 sums.
+// head, weights as three bf16 terms through shared memory; values: 64 latent columns per warp for all heads, all terms into the same f32 sums.
 // Bound by latency at decode sizes (three barriers a tile); with products on the CUDA cores, four heads to a CTA, every key's row was read and multiplied by eight CTAs
-// and FMAs bound it: 8 rows of up to 1024 keys, 32 heads: 74 us before, 12 us.
+// and FMAs bound it: 8 rows of up to 1024 keys, 32 heads: 74 us before, 12 us (a third term of the
+// weights costs 4 % of it).
 template <int HM>
 struct MlaTile {
   static constexpr int KEYS = 32, HEADS = 16 * HM, PITCH = ROW * 2, PP = 80;      // bytes of a row of Q / K, of weights
-  static constexpr int Q_OFF = 0, K_OFF = HEADS * PITCH, P_OFF = K_OFF + 2 * KEYS * PITCH, S_OFF = P_OFF + 2 * HEADS * PP;
+  static constexpr int Q_OFF = 0, K_OFF = HEADS * PITCH, P_OFF = K_OFF + 2 * KEYS * PITCH, S_OFF = P_OFF + 3 * HEADS * PP;
   static constexpr int SMEM = S_OFF + HEADS * 33 * 4 + HEADS * 4;                 // scores [heads][33], factors [heads]
 };
 template <int HM>
@@ -425,15 +426,15 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
       l *= corr;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        w[e] = w[e] == -INFINITY ? 0.f : __expf(w[e] - m);
+        w[e] = w[e] == -INFINITY ? LEAST_WEIGHT : weight_of(w[e] - m);
         l += w[e];
       }
-      uint32_t hi[2], lo[2];
-      two_terms(w[0], w[1], &hi[0], &lo[0]);
-      two_terms(w[2], w[3], &hi[1], &lo[1]);
+      uint32_t lo[3], hi[3];
+      three_terms(w[0], w[1], lo);
+      three_terms(w[2], w[3], hi);
       unsigned char* to = smem_raw + C::P_OFF + h * C::PP + sub * 8;
-      *reinterpret_cast<uint2*>(to) = make_uint2(hi[0], hi[1]);
-      *reinterpret_cast<uint2*>(to + C::HEADS * C::PP) = make_uint2(lo[0], lo[1]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(to + e * C::HEADS * C::PP) = make_uint2(lo[e], hi[e]);
       if (sub == 0) factor[h] = corr;
     }
     __syncthreads();
@@ -451,11 +452,11 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
     }
 #pragma unroll
     for (int kk = 0; kk < 2; ++kk) {
-      uint32_t a[HM][2][4];
+      uint32_t a[HM][3][4];
 #pragma unroll
       for (int mt = 0; mt < HM; ++mt)
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
+        for (int e = 0; e < 3; ++e)
           ldsm4(pb + e * C::HEADS * C::PP + (mt * 16 + (lane & 15)) * C::PP + kk * 32 + (lane >> 4) * 16, a[mt][e]);
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
 #pragma unroll
         for (int mt = 0; mt < HM; ++mt)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
+          for (int e = 0; e < 3; ++e) {
             mma16816(acc[mt][2 * n], a[mt][e][0], a[mt][e][1], a[mt][e][2], a[mt][e][3], b[0], b[1]);
             mma16816(acc[mt][2 * n + 1], a[mt][e][0], a[mt][e][1], a[mt][e][2], a[mt][e][3], b[2], b[3]);
           }

@@ -1,5 +1,5 @@
 // Warp-level pieces of the decode attention kernels: 16-byte asynchronous copies into shared memory, ldmatrix, the m16n8k16 bf16 product and weights as
-// two bf16 terms. (Decode attention is bound by its keys' bytes; these products keep up with them at sixteen query rows.)
+// three bf16 terms. (Decode attention is bound by its keys' bytes; these products keep up with them at sixteen query rows.)
 #pragma once
 #include "common.cuh"
 
@@ -21,16 +21,23 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
+// Weights of a softmax as three bf16 terms each, which add up to all 24 bits of a weight. The first two are cut off below the value, not rounded to it, so that
+// no term is 0 and none is negative: an infinite value of a key then stays infinite (inf * 0 is NaN, as is inf - inf). For that a weight is at least e^-62,
+// from where on every term is a normal bf16 value; beside the weight of 1 that each softmax has, that is nothing, and so it serves for keys that are not there,
+// too, whose values are read as zeros.
+constexpr float LEAST_WEIGHT = 1.18e-27f;
+__device__ __forceinline__ float weight_of(float x) {       // e^x; NaN stays NaN
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-62.f));
+  return __expf(x);
 }
-// two weights as (values, remainders)
-__device__ __forceinline__ void two_terms(float a, float b, uint32_t* hi, uint32_t* lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  const float2 f = __bfloat1622float2(h);
-  *hi = *reinterpret_cast<const uint32_t*>(&h);
-  *lo = pack_bf16(a - f.x, b - f.y);
+__device__ __forceinline__ float cut(float w) { return __uint_as_float((__float_as_uint(w) - 1u) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
+// `last`: a power of two that the third term is multiplied by
+__device__ __forceinline__ void three_terms(float a, float b, uint32_t (&t)[3], float last = 1.f) {
+  const float a0 = cut(a), b0 = cut(b), ra = a - a0, rb = b - b0, a1 = cut(ra), b1 = cut(rb);
+  t[0] = upper_halves(a0, b0);
+  t[1] = upper_halves(a1, b1);
+  t[2] = upper_halves((ra - a1) * last, (rb - b1) * last);
 }
 
 }  // namespace ifab
