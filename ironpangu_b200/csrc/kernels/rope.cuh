@@ -114,23 +114,24 @@ __device__ __forceinline__ float gated_value(float g, float u, const GatedUnit& 
   }
   return g * sigmoid_f32<FAST>(g) * u;
 }
-// the same of projections that count as bf16 rows for SiLU units (the form of the kernels that store them). The division is the fast one: the full one
-// branches, which keeps the compiler from working on more than one value of an epilogue at a time (a 128 x 128 tile then took 25 us, more than its
-// product at K = 2048: 2048 rows of 2 x 6144 columns 151 us, 92 with it); 1 + exp(-g) beyond 2^126 gives 0, the limit.
+// SiLU with a quotient that is rounded but in rare cases, without the branch of the full division, which keeps the compiler from working on more than one value
+// of an epilogue at a time (a 128 x 128 tile then takes 25 us, more than its product at K = 2048): the fast quotient, and once more of what it leaves over
+// (iterative refinement). The divisor lies between 1 and 2, so nothing overflows.
+__device__ __forceinline__ float silu_f32(float x) {
+  const float e = __expf(-fabsf(x)), d = 1.f + e, n = x < 0.f ? x * e : x, q = __fdividef(n, d);
+  return fabsf(x) < INFINITY ? q + __fdividef(fmaf(-q, d, n), d) : q;
+}
+// the gated unit of projections that count as bf16 rows for SiLU units (the form of the kernels that store them)
 __device__ __forceinline__ float gated_bf16(float g, float u, const GatedUnit& unit) {
   if (unit.kind) return gated_value<true>(g, u, unit);
-  g = bf16_round(g);
-  return __fdividef(g, 1.f + __expf(-g)) * bf16_round(u);
+  return silu_f32(bf16_round(g)) * bf16_round(u);
 }
 // the same of N values, the kind chosen once (2048 rows of 2 x 6144 columns, K 2048: 92 us with the choice at every value, 81 so)
 template <int N>
 __device__ __forceinline__ void gated_all(float* g, const float* u, const GatedUnit& unit) {
   if (unit.kind == 0) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const float x = bf16_round(g[i]);
-      g[i] = __fdividef(x, 1.f + __expf(-x)) * bf16_round(u[i]);
-    }
+    for (int i = 0; i < N; ++i) g[i] = silu_f32(bf16_round(g[i])) * bf16_round(u[i]);
   } else {
 #pragma unroll
     for (int i = 0; i < N; ++i) g[i] = gated_value<true>(g[i], u[i], unit);
