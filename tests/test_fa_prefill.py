@@ -107,3 +107,19 @@ def test_mla_prompt_path_with_tensor_core_attention_matches_oracle():
     torch.testing.assert_close(dec.logits[0], ref[296], rtol=3e-2, atol=3e-2)
     assert fab.status() == 0
     fab.close()
+
+
+def test_weights_below_the_normal_range_count():
+    """A key of weight 2^-130 beside one of weight 1: its value of 2^127 adds 2^-3, its infinite value stays infinite."""
+    from ironpangu_b200.ops import prefill as P
+
+    m, ctx, rows = 3, 8, 64
+    q, k, vt, out = (torch.zeros(*s, dtype=torch.bfloat16, device="cuda") for s in ((m, 128), (rows, 128), (128, rows), (m, 128)))
+    q[:, 0] = 1
+    k[:ctx, 0] = -8192                              # nothing of the others
+    k[0, 0], k[1, 0] = 0, -130
+    vt[0, 1], vt[1, 1], vt[2, 0] = float("inf"), 2.0 ** 127, 3
+    P.fa_prefill(q, k, vt, out, heads=1, q_head_stride=128, k_head_stride=128, vt_head_stride=128, vt_row0=0, d1=128, d2=0, kv_group=1, ctx=ctx, pos0=ctx - m,
+                 scale=0.6931471805599453)
+    assert bool((out[:, 0] == float("inf")).all()), out[:, 0]
+    torch.testing.assert_close(out[:, 1:3].float(), torch.tensor([[0.125, 3.0]], device="cuda").expand(m, 2), rtol=2 ** -7, atol=0)
