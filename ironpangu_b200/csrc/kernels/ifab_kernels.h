@@ -84,7 +84,8 @@ int ifab_gemm_fixed_bf16(const void* a, long lda, const void* b, long ldb, void*
 int ifab_gemm_gated_fixed_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int M, int F, int K,
                                uint32_t* status, void* stream);
 int ifab_gemm_rows_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias,
-                        int act, float cap, int unit, float limit, float alpha, int F, int fixed, int M, int N, int K, uint32_t* status, void* stream);
+                        int act, float cap, int unit, float limit, float alpha, int F, int fixed, int M, int N, int K, uint32_t spin_limit, uint32_t* status,
+                        void* stream);
 int ifab_gemm_epilogue_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias,
                             int act, float cap, int M, int N, int K, uint32_t* status, void* stream);
 int ifab_gemm_epilogue_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,

@@ -27,6 +27,8 @@ using namespace ifab::tc;
 
 namespace {
 
+constexpr uint32_t SPIN_LIMIT = 4000000u;       // polls of a wait
+
 struct GemmParams {
   void* c; long ldc; int out_f32;
   const bf16* residual; long ldr;
@@ -227,7 +229,7 @@ int gemm_epilogue(const void* a, long lda, const void* b, long ldb, void* c, lon
   // From 256 rows on only for weights: a plain product keeps the order of its sums that the CTA pairs and the one-CTA kernel share.
   const bool wide = M > 32 && M <= BM && (N + 127) / 128 > 296;
   if (!wide && (M < 256 || (fixed && rows_better(M, N, K, 0))))
-    return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, 0.f, 0.f, 0, fixed, M, N, K, status, stream);
+    return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, 0.f, 0.f, 0, fixed, M, N, K, SPIN_LIMIT, status, stream);
   // from 256 x 256 up: CTA pairs (tcgen05.mma cta_group::2; same accumulation order, same bits) - persistent with two
   // accumulators when there is more than one tile per SM pair, one tile per pair otherwise
   if (M >= 256 && N >= 256 && N % 32 == 0 && two_sm_enabled())
@@ -236,7 +238,7 @@ int gemm_epilogue(const void* a, long lda, const void* b, long ldb, void* c, lon
   const int BN = N > 128 && !wide ? 256 : 128, a_rows = wide ? (M + 7) / 8 * 8 : BM;
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN)) return rc;
-  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, a_rows, act, bias, cap, 0, {}, 0, 0};
+  GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, SPIN_LIMIT, a_rows, act, bias, cap, 0, {}, 0, 0};
   cudaStream_t s = (cudaStream_t)stream;
   if (wide) return launch<128, 3>(ta, tb, p, s);
   return BN == 256 ? launch<256, 4>(ta, tb, p, s) : launch<128, 6>(ta, tb, p, s);
@@ -246,13 +248,14 @@ int gemm_gated(const void* a, long lda, const void* b, long ldb, void* c, long l
                uint32_t* status, void* stream) {
   const GatedUnit gu{unit, limit, alpha};
   if (M < 1 || F < 8 || F % 8 || K < 8 || K % 8 || lda % 8 || ldb % 8 || !gated_ok(gu)) return -1;
-  if (M < 256 || (fixed && rows_better(M, 2 * F, K, F))) return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, status, stream);
+  if (M < 256 || (fixed && rows_better(M, 2 * F, K, F)))
+    return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, SPIN_LIMIT, status, stream);
   if (M >= 256 && F >= 128 && F % 32 == 0 && two_sm_enabled())
     return ifab_gemm_gated_bf16_2sm(a, lda, b, ldb, c, ldc, unit, limit, alpha, M, F, K, status, stream);
   CUtensorMap ta, tb;
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)BM)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, 128)) return rc;
-  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, BM, 0, nullptr, 0.f, F, gu, 0, 0};
+  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, SPIN_LIMIT, BM, 0, nullptr, 0.f, F, gu, 0, 0};
   return launch<256, 4, true>(ta, tb, p, (cudaStream_t)stream);
 }
 }  // namespace
@@ -291,7 +294,7 @@ extern "C" int ifab_gemm_split_bf16(const void* a, long lda, const void* b, long
   const int a_rows = (M + 7) / 8 * 8;
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN)) return rc;
-  GemmParams p{c, ldc, 1, nullptr, 0, M, N, K, status, 4000000u, a_rows, 0, bias, 0.f, 0, {}, per, part_stride};
+  GemmParams p{c, ldc, 1, nullptr, 0, M, N, K, status, SPIN_LIMIT, a_rows, 0, bias, 0.f, 0, {}, per, part_stride};
   cudaStream_t s = (cudaStream_t)stream;
   return BN == 128 ? launch<128, 3>(ta, tb, p, s) : BN == 64 ? launch<64, 4>(ta, tb, p, s) : launch<32, 5>(ta, tb, p, s);
 }

@@ -14,6 +14,8 @@
 // the preceding kernel: they stream in while that one ends.
 // Tensor memory is allocated after that wait and the next kernel admitted after the allocation, so no CTA that holds columns ever waits for a
 // grid that still wants some.
+// Every wait is bounded. One that runs out raises the CTA's flag and the status word; the warps that read the accumulator then wait for what the CTA has started
+// (copies into its ring, products that read it) and leave NaN as their part of the sum, so that the whole tile is NaN.
 #include "attn_rule.cuh"
 #include "rope.cuh"
 #include "tc_gemm_core.cuh"
@@ -25,6 +27,7 @@ using namespace ifab::tc;
 namespace {
 
 constexpr int FT = 128;            // features of a tile (gated: 64 gate rows and their 64 up rows)
+constexpr uint32_t DRAIN = 4000000u;   // limit of the waits for what a CTA that gives up has started
 
 template <int TOK>
 struct RowsCfg {
@@ -111,6 +114,7 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
   uint64_t *empty = full + C::STAGES, *acc_full = empty + C::STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* requested = abort_flag + 1;      // K blocks whose copies were requested, once no more will be; until then -1
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int part = blockIdx.x % p.splits, tile = blockIdx.x / p.splits;
   const bool gated = p.F > 0;
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
     }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
+    *requested = -1;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_w);
@@ -163,10 +168,8 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
       load_a(kb);
       issued = kb + 1;
     }
-    if (*abort_flag) {               // every copy must land before the CTA may exit
-      for (int kb = max(0, issued - C::STAGES); kb < issued; ++kb) mbar_wait(&full[kb % C::STAGES], (kb / C::STAGES) & 1, p.spin_limit);
-      if (p.status) atomicOr(p.status, IFAB_STATUS_MBAR_TIMEOUT);
-    }
+    *requested = issued;
+    if (*abort_flag && p.status) atomicOr(p.status, IFAB_STATUS_MBAR_TIMEOUT);
   } else if (warp == 1 && lane == 0) {
     constexpr uint32_t idesc = umma_idesc_bf16(FT, TOK);
     for (int kb = 0; kb < nk; ++kb) {
@@ -192,10 +195,19 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
   if (warp >= 2) {
     const bool ready = mbar_wait(acc_full, 0, p.spin_limit);
     tc_fence_after();
-    if (!ready) *abort_flag = 1;
+    if (!ready) {                    // this limit is for the whole sum, those above are for a block each: either may be the first to run out
+      *abort_flag = 1;
+      if (lane == 0 && p.status) atomicOr(p.status, IFAB_STATUS_MBAR_TIMEOUT);
+    }
     const int f = (warp & 3) * 32 + lane;
     const uint32_t tm = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-    if (!*abort_flag)
+    if (__any_sync(0xffffffffu, *abort_flag)) {
+      for (uint32_t i = 0; i < DRAIN && *requested < 0; ++i) __nanosleep(64);
+      const int n = *requested;
+      for (int kb = max(0, n - C::STAGES); kb < n; ++kb) mbar_wait(&full[kb % C::STAGES], (kb / C::STAGES) & 1, DRAIN);
+      mbar_wait(acc_full, 0, DRAIN);
+      for (int t = 0; t < tokens; ++t) sum[t * FT + f] = __int_as_float(0x7fffffff);
+    } else {
       for (int c0 = 0; c0 < tokens; c0 += 32) {
         float v[32];
         tmem_ld_32x32(tm + (uint32_t)c0, v);
@@ -204,6 +216,7 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
         for (int i = 0; i < 32; ++i)
           if (c0 + i < tokens) sum[(c0 + i) * FT + f] = nk > 0 ? v[i] : 0.f;
       }
+    }
   }
   tc_fence_before();
   cluster_sync();
@@ -273,12 +286,12 @@ bool ifab::tc::rows_better(int M, int N, int K, int F) {
   return M <= 1024 && there - here >= 16;
 }
 
-// The caller has checked shapes and strides (tc_gemm.cu); F > 0: gated, N = 2 F.
+// The caller has checked shapes and strides (tc_gemm.cu); F > 0: gated, N = 2 F. spin_limit: polls of a wait.
 extern "C" int ifab_gemm_rows_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                    const float* bias, int act, float cap, int unit, float limit, float alpha, int F, int fixed, int M, int N, int K,
-                                   uint32_t* status, void* stream) {
+                                   uint32_t spin_limit, uint32_t* status, void* stream) {
   if (M < 1 || N < 1 || K < 8 || K % 8 || lda % 8 || ldb % 8 || (F > 0 && N != 2 * F)) return -1;
-  RowsParams p{c, ldc, out_f32, (const bf16*)residual, ldr, bias, act, cap, M, N, K, F, {unit, limit, alpha}, 1, 0, fixed, status, 4000000u};
+  RowsParams p{c, ldc, out_f32, (const bf16*)residual, ldr, bias, act, cap, M, N, K, F, {unit, limit, alpha}, 1, 0, fixed, status, spin_limit};
   cudaStream_t s = (cudaStream_t)stream;
   if (M <= 16) return launch<16>(a, lda, b, ldb, p, s);
   if (M <= 32) return launch<32>(a, lda, b, ldb, p, s);
