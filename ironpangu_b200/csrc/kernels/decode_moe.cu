@@ -451,9 +451,9 @@ __device__ __forceinline__ void finish_argmax(const HeadParams& p, int* is_last)
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
     if (world > 1) {
-      // exchange: slot [parity][src rank][t] in every peer's staging area
+      // exchange: slot [parity][src rank][t] of eight tokens a rank in every peer's staging area, whichever kernel and T a rank's own operands lead to
       if (lane < world) {
-        float2* dst = reinterpret_cast<float2*>(p.fv.data[lane] + (size_t)par * p.fv.data_half_bytes) + rank * T + t;
+        float2* dst = reinterpret_cast<float2*>(p.fv.data[lane] + (size_t)par * p.fv.data_half_bytes) + rank * 8 + t;
         *dst = make_float2(bv, __int_as_float(bi));
       }
     } else if (lane == 0) {
@@ -477,7 +477,7 @@ __device__ __forceinline__ void finish_argmax(const HeadParams& p, int* is_last)
       float bv = -INFINITY;
       int bi = 0x7fffffff;
       for (int q = 0; q < world; ++q) {
-        const float2 v = __ldcg(src + q * T + t);
+        const float2 v = __ldcg(src + q * 8 + t);
         const int vi = __float_as_int(v.y);
         if (v.x > bv || (v.x == bv && vi < bi)) { bv = v.x; bi = vi; }
       }

@@ -61,6 +61,10 @@ def main():
     ids = K.lm_head_argmax(x, w[rank * vl:(rank + 1) * vl].contiguous(), fab, norm_w=nw, vocab_offset=rank * vl)
     ref = (rmsnorm_ref(x, nw, 1e-5) @ w.float().T).argmax(-1)
     assert torch.equal(ids.long(), ref), (ids, ref)
+    for kept in (True, rank == 0):                  # on every rank, on one only: the ranks' kernels may differ
+        ids = K.lm_head_argmax(x, w[rank * vl:(rank + 1) * vl].contiguous(), fab, norm_w=nw, vocab_offset=rank * vl,
+                               logits=torch.empty(T, vl, device="cuda") if kept else None)
+        assert torch.equal(ids.long(), ref), (kept, ids, ref)
     print(f"rank {rank}: ok lm_head_argmax", flush=True)
 
     # 3. tiny model, TP = EP = world ---------------------------------------------------------------
