@@ -574,14 +574,16 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(HeadParams p) {
   finish_argmax<8>(p, &is_last);
 }
 
+// what either form of the head asks of its sizes and of the room for the partial maxima: that of the kernel above
+template <int T, int R>
+int head_fits(const HeadParams& p, uint64_t partial_bytes) {
+  if (int rc = opt_in_smem(lm_head_argmax_kernel<T, R>, (size_t)T * p.K * sizeof(bf16))) return rc;
+  return (uint64_t)((p.V + 8 * R - 1) / (8 * R)) * T * sizeof(float2) > partial_bytes ? -5 : 0;
+}
 template <int T, int R>
 int launch_head(const HeadParams& p, uint64_t partial_bytes, cudaStream_t s) {
-  const size_t smem = (size_t)T * p.K * sizeof(bf16);
-  auto k = lm_head_argmax_kernel<T, R>;
-  if (int rc = opt_in_smem(k, smem)) return rc;
-  dim3 grid((p.V + 8 * R - 1) / (8 * R));
-  if ((uint64_t)grid.x * T * sizeof(float2) > partial_bytes) return -5;
-  return launch_chain(k, grid, dim3(256), smem, s, p);
+  if (int rc = head_fits<T, R>(p, partial_bytes)) return rc;
+  return launch_chain(lm_head_argmax_kernel<T, R>, dim3((p.V + 8 * R - 1) / (8 * R)), dim3(256), (size_t)T * p.K * sizeof(bf16), s, p);
 }
 
 }  // namespace
@@ -690,6 +692,7 @@ extern "C" int ifab_lm_head_capped_argmax(const void* x, long ldx, const void* n
   const uint64_t maxima = (uint64_t)ctas * 8 * sizeof(float2), rows = norm_w ? (uint64_t)T * K * sizeof(bf16) : 0;
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w | (uintptr_t)partial | (uintptr_t)(ldx * sizeof(bf16));
   if (T >= 3 && logits && maxima + rows <= partial_bytes && bits % 16 == 0) {
+    if (int rc = T <= 4 ? head_fits<4, 4>(p, partial_bytes) : head_fits<8, 2>(p, partial_bytes)) return rc;
     const void* a = x;
     long lda = ldx;
     if (norm_w) {

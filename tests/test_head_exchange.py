@@ -36,3 +36,25 @@ def test_candidates_lie_where_every_form_of_the_head_looks(T, kept):
     torch.testing.assert_close(value(sent)[:T], ref.max(-1).values, rtol=1e-4, atol=1e-3)
     assert fab.status() == 0
     fab.close()
+
+
+@pytest.mark.parametrize("T", [3, 4, 8])
+def test_room_for_the_maxima_is_asked_for_in_either_form(T):
+    """Logits kept or not, the same partial buffer is too small (and the same is large enough)."""
+    from ironpangu_b200.ops import decode as K
+    from ironpangu_b200.parallel.fabric import Fabric
+
+    fab = Fabric(0, 1)
+    V, D = 1000, 64
+    x, w = torch.randn(T, D, device="cuda").to(BF16), torch.randn(V, D, device="cuda").to(BF16)
+    need = (V + 31) // 32 * 4 * 8 if T <= 4 else (V + 15) // 16 * 8 * 8
+    ids = {}
+    for logits in (None, torch.empty(T, V, device="cuda")):
+        with pytest.raises(RuntimeError):
+            K.lm_head_argmax(x, w, fab, norm_w=torch.ones(D, device="cuda", dtype=BF16), logits=logits, partial=torch.empty(need // 4 - 2, device="cuda"))
+        ids[logits is None] = K.lm_head_argmax(x, w, fab, norm_w=torch.ones(D, device="cuda", dtype=BF16), logits=logits, partial=torch.empty(need // 4, device="cuda"))
+    ref = torch.nn.functional.rms_norm(x.float(), (D,), eps=1e-5).to(BF16).float() @ w.float().T
+    for i in ids.values():                          # any of the nearly largest: both forms add up in an order of their own
+        assert bool((ref.gather(1, i.long()[:, None])[:, 0] >= ref.max(-1).values - 1e-2).all())
+    assert fab.status() == 0
+    fab.close()
