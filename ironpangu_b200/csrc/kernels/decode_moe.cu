@@ -629,7 +629,7 @@ extern "C" int ifab_moe_gate_up_unit_decode(const void* x, long ldx, const void*
 namespace {
 int run_down(const DownParams& p, cudaStream_t s) {
   if (p.T <= 1) return dispatch_down<1>(p, s);
-  if (p.fv.world == 1 || p.y_f32) return launch_down<1, 2>(p, s, p.T);
+  if (p.fv.world == 1 || p.y_f32) return (p.D + 31) / 32 <= 296 ? launch_down<1, 2>(p, s, p.T) : -2;        // rows as wide as the other forms take
   if (p.T <= 2) return dispatch_down<2>(p, s);
   if (p.T <= 4) return dispatch_down<4>(p, s);
   return dispatch_down<8>(p, s);

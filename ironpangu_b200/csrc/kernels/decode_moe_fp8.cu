@@ -476,7 +476,7 @@ extern "C" int ifab_moe_down_allreduce_decode_fp8(const void* act, const int32_t
   if ((size_t)fab->world * 296 > fab->flag_half_words) return -4;
   cudaStream_t s = (cudaStream_t)stream;
   if (T <= 1) return dispatch_down8<1>(p, s);
-  if (fab->world == 1) return launch_down8<1, 4>(p, s, T);
+  if (fab->world == 1) return (D + 31) / 32 <= 296 ? launch_down8<1, 4>(p, s, T) : -2;       // rows as wide as the other forms take
   if (T <= 2) return dispatch_down8<2>(p, s);
   if (T <= 4) return dispatch_down8<4>(p, s);
   return dispatch_down8<8>(p, s);

@@ -37,3 +37,27 @@ def test_tokens_together_equal_tokens_alone(fp8, T, E, topk, D, F, Fs):
         assert torch.equal(down(act, 0, T), torch.cat([down(act, t, t + 1) for t in range(T)]))
     assert fab.status() == 0
     fab.close()
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("T", [1, 2, 8])
+def test_rows_too_wide_are_refused_for_any_number_of_tokens(fp8, T):
+    """Rows of the down projection: 296 CTAs of 32 columns at the most, at one rank too."""
+    from ironpangu_b200.ops import decode as K
+    from ironpangu_b200.parallel.fabric import Fabric
+
+    fab = Fabric(0, 1)
+    E, topk, F = 2, 1, 32
+    fn = K.moe_down_allreduce_fp8 if fp8 else K.moe_down_allreduce
+    for D in (296 * 32, 296 * 32 + 8):
+        dn = torch.zeros(E, D, F, dtype=BF16, device="cuda")
+        args = (torch.zeros(T, topk + 1, F, dtype=BF16, device="cuda"), torch.zeros(T, topk, dtype=torch.int32, device="cuda"), torch.ones(T, topk, device="cuda"),
+                K.quantize_fp8_block(dn) if fp8 else dn, 0, fab)
+        out = torch.ones(T, D, dtype=BF16, device="cuda")
+        if D > 296 * 32:
+            with pytest.raises(RuntimeError):
+                fn(*args, out=out)
+        else:
+            fn(*args, out=out)
+            assert int(out.count_nonzero()) == 0
+    fab.close()
