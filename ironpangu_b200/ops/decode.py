@@ -84,8 +84,9 @@ def linear_product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, norm_
                    residual: Optional[torch.Tensor] = None, swiglu: bool = False, norm_out: Optional[torch.Tensor] = None,
                    status_ptr: Optional[int] = None) -> torch.Tensor:
     """:func:`gemv` as a tensor-core product of a model's weights: the better form from three rows on, where FMAs bound the streaming one (8 rows, 4096 x 4096:
-    28.6 us against 14.7). ``norm_out``: room for the normalised rows."""
+    28.6 us against 14.7). ``norm_out``: room for the normalised rows, ``[T, K]``."""
     T, K = x.shape
+    assert norm_w is None or norm_out is None or norm_out.shape == x.shape
     assert w.shape[1] == K and w.is_contiguous() and w.dtype == BF16 and x.dtype == BF16
     xn = x if norm_w is None else rmsnorm(x, norm_w, eps, out=norm_out)
     lib, st = _lib.load(), _stream()

@@ -460,6 +460,11 @@ class PlanEngine:
         self._norm_rows = (torch.empty(self.T, (max(self.cfg.hidden, self.cfg.q_lora) + 7) // 8 * 8, dtype=torch.bfloat16, device=self.tokens.device)
                            if isinstance(self.cfg, MlaMoeConfig) else None)
 
+    def _takes_product(self, width: int, normed: bool, units: int) -> bool:
+        """Whether a linear of ``width`` columns (with ``units`` gated results, 0: none) fits the tensor-core form: its normalised rows into the room
+        that is kept for them, gated results in whole pieces of eight. The streaming form takes any."""
+        return (not normed or width <= self._norm_rows.shape[1]) and units % 8 == 0
+
     def _describe(self) -> None:
         """What the program says about the model, in the vocabulary of the hand-wired decoder (``models/mla_moe.py``): a
         configuration record and the parameters by role. The prompt executor (``models/mla_moe_prefill.py``) and the batch
@@ -756,7 +761,7 @@ class PlanEngine:
             elif op == "linear":
                 name = a["weight"] + ("|" + a["paired_weight"] if "paired_weight" in a else "")
                 x, swiglu = val(ins[0]), a.get("activation") == "swiglu"
-                if product:
+                if product and self._takes_product(x.shape[1], norm_w is not None, val(k).shape[1] if swiglu else 0):
                     K.linear_product(x, self._param(name), val(k), norm_w=norm_w, eps=eps, swiglu=swiglu, norm_out=self._norm_rows[:T, :x.shape[1]], status_ptr=st)
                 else:
                     K.gemv(x, self._param(name), norm_w=norm_w, eps=eps, swiglu=swiglu, out=val(k))
