@@ -154,6 +154,9 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 // tc_gemm_rows.cu
 bool rows_better(int M, int N, int K, int F);
+// tc_gemm_2sm.cu: SMs of the current device; rows of A and B that a CTA of a pair loads per K block, over all its tiles of an M x N product
+int device_sms();
+long pair_loads(int M, int N);
 // 3-D: [batch, rows, cols] with batch stride `bstride` elements (grouped / per-expert weights)
 int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t batch, uint64_t rows, uint64_t cols, uint64_t ld,
                       uint64_t bstride, uint32_t box_rows);

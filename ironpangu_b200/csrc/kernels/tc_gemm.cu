@@ -13,7 +13,7 @@
 // holds the live rows only.
 // A and B are both K-major ("NT"), which is how activations [tokens, K] and weights [out, K] are
 // stored everywhere in this library, so no transposes are needed. M, N and K tails are handled by
-// TMA zero fill plus masked stores. Used where neither tc_gemm_rows.cu (few rows) nor tc_gemm_2sm.cu (256 and up with as many columns) is; the
+// TMA zero fill plus masked stores. Used where neither tc_gemm_rows.cu (few rows) nor tc_gemm_2sm.cu (CTA pairs, from 129 rows on) is better; the
 // reference's counterpart is aclnnMatmul on [T<=4096, K] activations (token_executor.h:387-456).
 #include <cstdlib>
 
@@ -221,26 +221,37 @@ extern "C" int ifab_gemm_act_bf16(const void* a, long lda, const void* b, long l
 }
 
 namespace {
+// Whether a product of up to 128 rows is better off without shared K, a CTA a tile (its box of A holds the live rows only): a matrix wide enough for an SM a
+// tile of 128 columns from `least` rows on (the sum over a cluster is only a detour there: N 151936 K 2048 64 rows 134 us and 127 here, 27 rows 114 and 120; N 32000
+// K 1024 64 rows 20.4 and 18.7), and, where the rows are many beside K, one of a quarter of that (N 12288 K 1024 128 rows 15.8 us and 12.6, K 2048 100 rows 19.4 and
+// 18.3; N 6144 K 1536 128 rows 12.8 and 12.1, 64 rows 10.6 and 11.3).
+bool one_tile_row(int M, int tiles, int K, int least, int per_k = 48) { return tiles > device_sms() ? M > least : 4 * tiles > device_sms() && (long)M * 1024 > (long)per_k * K; }
+// columns of its tiles: the narrowest that all run at once, two on an SM
+int narrow_tile(int N, int least = 32) {
+  int n = least;
+  while (n < 128 && (N + n - 1) / n > 2 * device_sms()) n *= 2;
+  return n;
+}
+
 int gemm_epilogue(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias, int act,
                   float cap, int fixed, int M, int N, int K, uint32_t* status, void* stream) {
   if (M < 1 || N < 1 || K < 8 || K % 8 || lda % 8 || ldb % 8 || cap < 0.f) return -1;
-  // Few rows (decode steps, short prompts) are bound by the stream of B: tc_gemm_rows.cu. From 33 to 128 rows of a matrix wide enough to fill the chip
-  // without sharing K the sum over a cluster is only a detour: N 151936, K 2048, 64 rows 134 us there and 127 here, 128 rows 172 and 138 (27 rows 114 and 120).
-  // From 256 rows on only for weights: a plain product keeps the order of its sums that the CTA pairs and the one-CTA kernel share.
-  const bool wide = M > 32 && M <= BM && (N + 127) / 128 > 296;
-  if (!wide && (M < 256 || (fixed && rows_better(M, N, K, 0))))
+  // Few rows (decode steps, short prompts) are bound by the stream of B: tc_gemm_rows.cu. Above 128 rows by what has to be loaded, and from 256 rows on only for
+  // weights: a plain product keeps the order of its sums that the CTA pairs and the one-CTA kernel share.
+  const bool alone = M <= BM && one_tile_row(M, (N + 127) / 128, K, 32);
+  if (M <= BM ? !alone : (M < 256 || fixed) && rows_better(M, N, K, 0))
     return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, 0.f, 0.f, 0, fixed, M, N, K, SPIN_LIMIT, status, stream);
-  // from 256 x 256 up: CTA pairs (tcgen05.mma cta_group::2; same accumulation order, same bits) - persistent with two
-  // accumulators when there is more than one tile per SM pair, one tile per pair otherwise
-  if (M >= 256 && N >= 256 && N % 32 == 0 && two_sm_enabled())
+  // CTA pairs (tcgen05.mma cta_group::2; same accumulation order, same bits) - persistent with two accumulators when there is more than one tile per SM
+  // pair, one tile per pair otherwise
+  if (M > BM && N >= 256 && N % 32 == 0 && two_sm_enabled())
     return ifab_gemm_epilogue_bf16_2sm(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, -1, M, N, K, status, stream);
   CUtensorMap ta, tb;
-  const int BN = N > 128 && !wide ? 256 : 128, a_rows = wide ? (M + 7) / 8 * 8 : BM;
+  const int BN = alone ? narrow_tile(N) : N > 128 ? 256 : 128, a_rows = alone ? (M + 7) / 8 * 8 : BM;
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
   if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN)) return rc;
   GemmParams p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, SPIN_LIMIT, a_rows, act, bias, cap, 0, {}, 0, 0};
   cudaStream_t s = (cudaStream_t)stream;
-  if (wide) return launch<128, 3>(ta, tb, p, s);
+  if (alone) return BN == 32 ? launch<32, 5>(ta, tb, p, s) : BN == 64 ? launch<64, 4>(ta, tb, p, s) : launch<128, 3>(ta, tb, p, s);
   return BN == 256 ? launch<256, 4>(ta, tb, p, s) : launch<128, 6>(ta, tb, p, s);
 }
 
@@ -248,15 +259,19 @@ int gemm_gated(const void* a, long lda, const void* b, long ldb, void* c, long l
                uint32_t* status, void* stream) {
   const GatedUnit gu{unit, limit, alpha};
   if (M < 1 || F < 8 || F % 8 || K < 8 || K % 8 || lda % 8 || ldb % 8 || !gated_ok(gu)) return -1;
-  if (M < 256 || (fixed && rows_better(M, 2 * F, K, F)))
+  const bool alone = M <= BM && one_tile_row(M, (F + 63) / 64, K, 96, 64);      // F 4096 K 1024: 64 rows 8.9 us shared, 9.3 here; 128 rows 11.5 and 10.1
+  if (M <= BM ? !alone : (M < 256 || fixed) && rows_better(M, 2 * F, K, F))
     return ifab_gemm_rows_bf16(a, lda, b, ldb, c, ldc, 0, nullptr, 0, nullptr, 0, 0.f, unit, limit, alpha, F, fixed, M, 2 * F, K, SPIN_LIMIT, status, stream);
-  if (M >= 256 && F >= 128 && F % 32 == 0 && two_sm_enabled())
+  if (M > BM && F >= 128 && F % 32 == 0 && two_sm_enabled())
     return ifab_gemm_gated_bf16_2sm(a, lda, b, ldb, c, ldc, unit, limit, alpha, M, F, K, status, stream);
+  const int BN = alone ? narrow_tile(2 * F, 64) : 256, a_rows = alone ? (M + 7) / 8 * 8 : BM;
   CUtensorMap ta, tb;
-  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)BM)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, 128)) return rc;
-  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, SPIN_LIMIT, BM, 0, nullptr, 0.f, F, gu, 0, 0};
-  return launch<256, 4, true>(ta, tb, p, (cudaStream_t)stream);
+  if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, (uint32_t)a_rows)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tb, b, (uint64_t)2 * F, (uint64_t)K, (uint64_t)ldb, (uint32_t)(BN / 2))) return rc;
+  GemmParams p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, SPIN_LIMIT, a_rows, 0, nullptr, 0.f, F, gu, 0, 0};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (alone) return BN == 64 ? launch<64, 4, true>(ta, tb, p, s) : launch<128, 3, true>(ta, tb, p, s);
+  return launch<256, 4, true>(ta, tb, p, s);
 }
 }  // namespace
 
@@ -272,7 +287,7 @@ extern "C" int ifab_gemm_fixed_bf16(const void* a, long lda, const void* b, long
 }
 
 // C[M, F] (bf16) = unit(A gate^T, A up^T) with B = [gate rows | up rows] ([2 F, K]) and the gated units of rope.cuh (0 SiLU, 1 ReLU, 2 limited). F % 8
-// == 0. Rows from 256 on go to the CTA pairs where F % 32 == 0.
+// == 0. Rows from 129 on go to the CTA pairs where F % 32 == 0 and that is the better form.
 extern "C" int ifab_gemm_gated_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int M, int F,
                                     int K, uint32_t* status, void* stream) {
   return gemm_gated(a, lda, b, ldb, c, ldc, unit, limit, alpha, 0, M, F, K, status, stream);

@@ -406,22 +406,18 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
   }
 }
 
-int pairs_of_device() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, sms / 2);
-}
+int pairs_of_device() { return std::max(1, device_sms() / 2); }
 // Columns of a tile: of 256, 192 and 128 the width whose waves of tiles over the pairs take least. A K block costs a pair what it loads - 128 rows of A
 // and TN / 2 of B in each CTA, about 87 GB/s an SM - rather than what it multiplies, so narrow tiles gain less than their width: 2048 x 3072 (K 2048)
 // 32.5 us by 256, 30.3 by 192, 39.7 by 128; 2048 x 8192 56.7, 64.8, 83.6; 1024 x 2048 (K 6144, residual) 42.5, 41.7, 37.8.
-int tile_width(int M, int N, int pairs) {
+int tile_width(int M, int N, int pairs, long* loads = nullptr) {
   int best = 256;
   long least = 0;
   for (int tn : {256, 192, 128}) {
     const long tiles = (long)((M + 255) / 256) * ((N + tn - 1) / tn), cost = (tiles + pairs - 1) / pairs * (256 + tn);
     if (!least || cost < least) least = cost, best = tn;
   }
+  if (loads) *loads = least;
   return best;
 }
 template <int TN>
@@ -448,6 +444,18 @@ int dispatch_2sm(const void* a, long lda, const void* b, long ldb, const Gemm2Pa
 }
 
 }  // namespace
+
+int ifab::tc::device_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+long ifab::tc::pair_loads(int M, int N) {
+  long loads = 0;
+  tile_width(M, N, pairs_of_device(), &loads);
+  return loads;
+}
 
 // C[M,N] = act(A[M,K] * B[N,K]^T (+ residual)) with CTA pairs on tiles of 256 rows. N % 32 == 0, K % 8 == 0. `persistent` 1: one CTA pair per
 // SM pair walks the tiles with two accumulators in tensor memory; 0: one pair per tile; -1: the former where there are more tiles than pairs.

@@ -16,6 +16,8 @@
 // grid that still wants some.
 // Every wait is bounded. One that runs out raises the CTA's flag and the status word; the warps that read the accumulator then wait for what the CTA has started
 // (copies into its ring, products that read it) and leave NaN as their part of the sum, so that the whole tile is NaN.
+#include <algorithm>
+
 #include "attn_rule.cuh"
 #include "rope.cuh"
 #include "tc_gemm_core.cuh"
@@ -251,12 +253,24 @@ __global__ void __launch_bounds__(192) tc_gemm_rows_kernel(const __grid_constant
 }
 
 int blocks_of(int K) { return (K + BK - 1) / BK; }
-// CTAs of a tile's cluster: as many as fit two to an SM over all tiles, with at least eight K blocks (128 KB of weights) in each - below that the start
-// and the sum outweigh the stream (8 rows, N 3072 K 2048: 7.3 us by 8, 5.8 by 4). Powers of two: clusters of 3 or 6 leave SMs of a GPC idle (200
-// rows, N 3072: 16.9 us by 6, 11.7 by 4).
-int splits_of(int tiles, int blocks) {
+// CTAs of a tile's cluster, a power of two (clusters of 3 or 6 leave SMs of a GPC idle: 200 rows, N 3072: 16.9 us by 6, 11.7 by 4), the most that pay:
+//   eight K blocks each   while all CTAs run at once, two on an SM. Larger clusters do not pack the GPCs: 256 CTAs by 8 (200 rows, N 2112 K 4096: 272 of them
+//                         19.3 us, 136 by 4 16.0), 280 by 4 (384 rows, N 3072 K 2048: 288 of them 21.6, 144 by 2 15.4)
+//   six                   by up to 4 (200 rows, N 4096 K 1536: 14.2 us by 2, 11.3 by 4)
+//   four                  while every CTA has an SM to itself, by 8 less than half a chip (16 rows, K 2048: N 1024 6.0 us by 4, 5.0 by 8; N 2048 6.2 and 7.0;
+//                         K 1024: N 1024 6.3 by 2, 4.5 by 4); from 65 rows on, whose blocks are twice as large, two of them by 8 (128 rows, N 1024 K 1024: 8.1 us
+//                         by 4, 7.1 by 8)
+int splits_of(int M, int tiles, int blocks) {
+  const int sms = device_sms();
   int splits = 8;
-  while (splits > 1 && (tiles * splits > 296 || blocks < 8 * splits || (blocks + splits - 1) / splits * (splits - 1) >= blocks)) splits /= 2;
+  for (; splits > 1; splits /= 2) {
+    const long ctas = (long)tiles * splits * 148;
+    if ((blocks + splits - 1) / splits * (splits - 1) >= blocks) continue;        // a CTA without work
+    if (blocks >= 8 * splits && ctas <= (splits == 8 ? 256 : splits == 4 ? 280 : 296) * sms) break;
+    if (blocks >= 6 * splits && splits <= 4 && ctas <= 256 * sms) break;
+    if (splits < 8 && blocks >= 4 * splits && ctas <= 148 * sms) break;
+    if (splits == 8 && blocks >= (M > 64 ? 2 : 4) * 8 && ctas <= 64 * sms) break;
+  }
   return splits;
 }
 
@@ -270,20 +284,20 @@ int launch(const void* a, long lda, const void* b, long ldb, RowsParams p, cudaS
   if (int rc = make_tmap_bf16_2d(&ta, a, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)lda, (uint32_t)p.box)) return rc;
   if (int rc = make_tmap_bf16_2d(&tw, b, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb, p.F > 0 ? FT / 2 : FT)) return rc;
   const int tiles = p.F > 0 ? (p.F + FT / 2 - 1) / (FT / 2) : (p.N + FT - 1) / FT, ty = (p.M + TOK - 1) / TOK;
-  p.splits = splits_of(tiles * ty, blocks_of(p.K));
+  p.splits = splits_of(p.M, tiles * ty, blocks_of(p.K));
   return launch_chain_cluster(k, dim3(tiles * p.splits, ty), dim3(192), (unsigned)p.splits, (size_t)smem, s, ta, tw, p);
 }
 
 }  // namespace
 
-// Whether a product of M >= 256 rows is better here than on CTA pairs (tc_gemm_2sm.cu): by the K blocks an SM has to load one after the other (32 KB and 0.37 us
-// each in both), and only where sharing K saves 16 of them - the sum over the cluster costs what it saves below that. 509 x 2048: K 6144 20.7 us here, 34.6 there;
-// K 2048 13.6 and 14.3; 509 x 3072 (K 2048, nothing saved) 18.3 and 15.6.
+// Whether a product of more than 128 rows is better here than on CTA pairs (tc_gemm_2sm.cu), by what an SM or pair has to load one after the other: a K block is
+// 32 KB here, 128 rows of A and half a tile's columns a CTA there, at about 0.37 us per 32 KB in both. From 256 rows on only where that saves eight blocks.
+// us here / there: 255 rows 2048 x 6144 16.6 / 34.6, 3072 x 2048 13.1 / 15.3, 8192 x 2048 18.4 / 15.3, 12288 x 2048 29.4 / 19.2; 509 rows 2048 x 6144 19.7 / 34.9,
+// 2048 x 2048 13.1 / 14.6, 3072 x 2048 18.3 / 15.7.
 bool ifab::tc::rows_better(int M, int N, int K, int F) {
-  const int ty = (M + 127) / 128, tiles = F > 0 ? (F + FT / 2 - 1) / (FT / 2) : (N + FT - 1) / FT, blocks = blocks_of(K), splits = splits_of(tiles * ty, blocks);
-  const long here = (long)((blocks + splits - 1) / splits) * ((tiles * ty * splits + 147) / 148);
-  const long pairs = (long)((M + 255) / 256) * ((N + 255) / 256), there = (pairs + 73) / 74 * blocks;
-  return M <= 1024 && there - here >= 16;
+  const int sms = device_sms(), blocks = blocks_of(K), tiles = (F > 0 ? (F + FT / 2 - 1) / (FT / 2) : (N + FT - 1) / FT) * ((M + 127) / 128), splits = splits_of(M, tiles, blocks);
+  const long here = (long)((blocks + splits - 1) / splits) * 2 * 256 * std::max(sms, tiles * splits) / sms, there = blocks * pair_loads(M, N);
+  return M <= 1024 && there - here >= (M < 256 ? 0 : 8 * 2 * 256);
 }
 
 // The caller has checked shapes and strides (tc_gemm.cu); F > 0: gated, N = 2 F. spin_limit: polls of a wait.
