@@ -264,8 +264,10 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 // Bound by the stream of keys and values: a key costs a warp two instructions, where products on the CUDA cores (eight lanes to a key) cost 40 and
 // bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 77 us (4.3 TB/s); 8 rows of 1900 keys 46 -> 13 us, one row of
 // 2000 keys 14.8 -> 10.4 us, merge included. Two CTAs an SM (registers) x four warps
-// with one stage of 8 KB in flight beside the one in use. The third term costs groups of up to four nothing (64 rows of up to 4096 keys 91.6 us without it, 89.9
-// with), groups of eight their second product (over one kv head 33.2 and 37.6 us).
+// with one stage of 8 KB in flight beside the one in use.
+// Every product of sixteen is added to its f32 sum outside the tensor core, scores in two sums each: the tensor core cuts off what it adds up, and chains of its
+// products left results 0.6e-6 to 1.9e-6 off, where these are 2.5e-7 to 4.2e-7 and FMAs 2.4e-7 to 4.4e-7. Against two terms of a weight and chains: 64 rows of up
+// to 4096 keys 91.2 -> 92.8 us; groups of eight (over one kv head) 32.9 -> 35.0 us.
 template <int HD>
 struct MmaSplit {
   static constexpr int KEYS = 16, WARPS = 4, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
@@ -287,7 +289,7 @@ __device__ __forceinline__ float peer_float(const float* mine, uint32_t rank) {
 // CLUSTER: the splits of a (row, kv head) are one cluster (at most eight) and merge their parts over distributed shared memory into `out`; otherwise
 // the parts go to the scratch and gqa_merge_kernel follows.
 template <int HD, bool CLUSTER, bool WIDE>
-__global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
+__global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
   using S = MmaSplit<HD>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep_launch();
@@ -378,14 +380,19 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
       asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
       __syncwarp();
       const uint32_t kb = ring + st * S::STAGE, vb = kb + S::KEYS * S::ROW;
-      float s[2][4] = {};
+      float s[2][4] = {};                        // [keys c2 .. / c2 + 8 ..][two sums each: of even and of odd pieces of the columns]
 #pragma unroll
       for (int kk = 0; kk < HD / 16; ++kk) {
         uint32_t b[4];
         const int key = (lane >> 4) * 8 + (lane & 7), ch = 2 * kk + ((lane >> 3) & 1);
         ldsm4(kb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
-        mma16816(s[0], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[0], b[1]);
-        mma16816(s[1], q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[2], b[3]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float d[4];
+          mma16816_alone(d, q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[2 * h], b[2 * h + 1]);
+          s[h][2 * (kk & 1)] += d[0];
+          s[h][2 * (kk & 1) + 1] += d[1];
+        }
       }
       // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against head gh
       float w[4];
@@ -393,7 +400,7 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = c2 + (j >> 1) * 8 + (j & 1);
-        w[j] = s[j >> 1][j & 1] * p.scale;
+        w[j] = (s[j >> 1][j & 1] + s[j >> 1][2 + (j & 1)]) * p.scale;
         if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
         if (__shfl_sync(0xffffffffu, at[st], key) < 0) w[j] = -INFINITY;
         mn = fmaxf(mn, w[j]);
@@ -423,11 +430,13 @@ __global__ void __launch_bounds__(128) gqa_split_mma_kernel(GqaParams p, bf16* r
         uint32_t b[4];
         const int key = ((lane >> 3) & 1) * 8 + (lane & 7), ch = 2 * j + (lane >> 4);
         ldsm4t(vb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
-        mma16816(acc[2 * j], lo0, lo[1], hi0, hi[1], b[0], b[1]);
-        mma16816(acc[2 * j + 1], lo0, lo[1], hi0, hi[1], b[2], b[3]);
-        if (WIDE) {
-          mma16816(acc[2 * j], lo[2], lo[2], hi[2], hi[2], b[0], b[1]);
-          mma16816(acc[2 * j + 1], lo[2], lo[2], hi[2], hi[2], b[2], b[3]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float d[4];
+          mma16816_alone(d, lo0, lo[1], hi0, hi[1], b[2 * h], b[2 * h + 1]);
+          if (WIDE) mma16816(d, lo[2], lo[2], hi[2], hi[2], b[2 * h], b[2 * h + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[2 * j + h][e] += d[e];
         }
       }
       __syncwarp();            // the stage is read: a later round may overwrite it

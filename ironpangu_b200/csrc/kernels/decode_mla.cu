@@ -83,13 +83,15 @@ __global__ void __launch_bounds__(128) mla_kv_write_kernel(const bf16* kv, long 
 // ------------------------------------------------------------------------------------------------
 // grid (H, T, latent/128), 256 threads. A CTA produces 128 latent columns of one head: thread
 // (ds, cg) = (tid / 16, tid % 16) owns 8 columns [cg*8, cg*8+8) and the 8 q_nope elements
-// [ds*8, ds*8+8); its 8 weight loads (16 bytes each) are issued before the dependency wait, the 16
+// [ds*8, ds*8+8); its 8 weight loads (16 bytes each) are issued before the dependency wait, the
 // d-slices are then summed through shared memory. CTA z == 0 also rotates the rope part.
+// For 32, 64 and 128 elements the parts (nope / 32 elements each) and the tree of their sums are those of the one-launch kernel of one and two rows
+// (decode_mla_head.cu): in another order one query element in a few thousand rounds to another bf16, and a sequence's tokens then depend on the steps it shares.
 __global__ void __launch_bounds__(256) mla_q_absorb_kernel(const bf16* q, long ldq, const bf16* w_kvb, float theta,
                                                            const int32_t* positions, bf16* q_lat, int H, int nope,
                                                            int rope, int latent, int vdim) {
   __shared__ float qs[256];
-  __shared__ float part[16][129];
+  __shared__ float part[32][129];
   grid_dep_launch();
   const int h = blockIdx.x, t = blockIdx.y, cbase = blockIdx.z * 128;
   const int cg = threadIdx.x & 15, ds = threadIdx.x >> 4;
@@ -108,27 +110,59 @@ __global__ void __launch_bounds__(256) mla_q_absorb_kernel(const bf16* q, long l
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-  for (int d0 = ds * 8; d0 < nope; d0 += 128) {
+  const int each = nope >> 5;
+  const bool tree = nope == 32 * each && (each == 1 || each == 2 || each == 4);
+  if (tree) {
+    if (ds * 8 < nope)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int d = d0 + j;
-      if (d >= nope) break;
-      float wf[8];
-      unpack8(d0 == ds * 8 ? wv[j] : ld_stream16(W + (long)d * latent), wf);
-      const float qd = qs[d];
+      for (int j = 0; j < 8; ++j) {
+        const int d = ds * 8 + j;
+        float wf[8];
+        unpack8(wv[j], wf);
+        const float qd = qs[d];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = fmaf(qd, wf[i], acc[i]);
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(qd, wf[i], acc[i]);
+        if ((d + 1) % each) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          part[d / each][cg * 8 + i] = acc[i];
+          acc[i] = 0.f;
+        }
+      }
+  } else
+    for (int d0 = ds * 8; d0 < nope; d0 += 128) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int d = d0 + j;
+        if (d >= nope) break;
+        float wf[8];
+        unpack8(d0 == ds * 8 ? wv[j] : ld_stream16(W + (long)d * latent), wf);
+        const float qd = qs[d];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(qd, wf[i], acc[i]);
+      }
     }
-  }
+  if (!tree) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) part[ds][cg * 8 + i] = acc[i];
+    for (int i = 0; i < 8; ++i) part[ds][cg * 8 + i] = acc[i];
+  }
   __syncthreads();
   bf16* out = q_lat + ((long)t * H + h) * (latent + rope);
   if (threadIdx.x < 128) {
-    float v = 0.f;
+    float v[32];
+    if (tree) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v += part[k][threadIdx.x];
-    out[cbase + threadIdx.x] = __float2bfloat16_rn(v);
+      for (int k = 0; k < 32; ++k) v[k] = part[k][threadIdx.x];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; ++k) v[k] += v[k + o];
+    } else {
+      v[0] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[0] += part[k][threadIdx.x];
+    }
+    out[cbase + threadIdx.x] = __float2bfloat16_rn(v[0]);
   }
   const int half = rope / 2;
   if (blockIdx.z == 0 && (int)threadIdx.x >= 128 && (int)threadIdx.x - 128 < half) {
@@ -318,8 +352,10 @@ __global__ void __launch_bounds__(256) mla_split_kernel(AttnParams p) {
 // stages of shared memory (cp.async). Scores: warp w has head tile w % HM and eight keys (HM = 1: half the warps idle), m16n8k16 over the 576 columns; softmax: eight threads to a
 // head, weights as three bf16 terms through shared memory; values: 64 latent columns per warp for all heads, all terms into the same f32 sums.
 // Bound by latency at decode sizes (three barriers a tile); with products on the CUDA cores, four heads to a CTA, every key's row was read and multiplied by eight CTAs
-// and FMAs bound it: 8 rows of up to 1024 keys, 32 heads: 74 us before, 12 us (a third term of the
-// weights costs 4 % of it).
+// and FMAs bound it: 8 rows of up to 1024 keys, 32 heads: 74 us before, 12 us.
+// Every product of sixteen is added to its f32 sum outside the tensor core, which cuts off what it adds up: scores as four sums, the first terms' products apart from
+// those of the remainders. Results are 1.0e-7 to 2.0e-7 off, those of FMAs 1.2e-7 to 2.2e-7, chains of products with two terms 1.5e-6 to 2.9e-6; it costs a tenth of
+// the kernel (8 rows of up to 1024 keys, merge included, 20.1 -> 22.4 us).
 template <int HM>
 struct MlaTile {
   static constexpr int KEYS = 32, HEADS = 16 * HM, PITCH = ROW * 2, PP = 80;      // bytes of a row of Q / K, of weights
@@ -327,7 +363,7 @@ struct MlaTile {
   static constexpr int SMEM = S_OFF + HEADS * 33 * 4 + HEADS * 4;                 // scores [heads][33], factors [heads]
 };
 template <int HM>
-__global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
+__global__ void __launch_bounds__(256, HM == 1 ? 2 : 1) mla_split_mma_kernel(AttnParams p) {
   using C = MlaTile<HM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep_launch();
@@ -393,7 +429,7 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
     const uint32_t kb = smem_addr(smem_raw + C::K_OFF + st * C::KEYS * C::PITCH);
     if (warp < 4 * HM) {
       const int mt = warp % HM, n0 = warp / HM * 8;
-      float s[2][4] = {};                        // two chains
+      float s[4][4] = {};                        // four sums of nine pieces
 #pragma unroll 6
       for (int kk = 0; kk < ROW / 32; ++kk) {
         uint32_t b[4], a[4];
@@ -401,14 +437,17 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           ldsm4(at(qb, mt * 16 + (lane & 15), 4 * kk + 2 * e + (lane >> 4)), a);
-          mma16816(s[e], a[0], a[1], a[2], a[3], b[2 * e], b[2 * e + 1]);
+          float d[4];
+          mma16816_alone(d, a[0], a[1], a[2], a[3], b[2 * e], b[2 * e + 1]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) s[2 * (kk & 1) + e][i] += d[i];
         }
       }
       const int row = mt * 16 + (lane >> 2), col = n0 + (lane & 3) * 2;
-      sc[row * 33 + col] = s[0][0] + s[1][0];
-      sc[row * 33 + col + 1] = s[0][1] + s[1][1];
-      sc[(row + 8) * 33 + col] = s[0][2] + s[1][2];
-      sc[(row + 8) * 33 + col + 1] = s[0][3] + s[1][3];
+      sc[row * 33 + col] = (s[0][0] + s[1][0]) + (s[2][0] + s[3][0]);
+      sc[row * 33 + col + 1] = (s[0][1] + s[1][1]) + (s[2][1] + s[3][1]);
+      sc[(row + 8) * 33 + col] = (s[0][2] + s[1][2]) + (s[2][2] + s[3][2]);
+      sc[(row + 8) * 33 + col + 1] = (s[0][3] + s[1][3]) + (s[2][3] + s[3][3]);
     }
     __syncthreads();
     if (threadIdx.x < C::HEADS * 8) {
@@ -465,9 +504,13 @@ __global__ void __launch_bounds__(256) mla_split_mma_kernel(AttnParams p) {
 #pragma unroll
         for (int mt = 0; mt < HM; ++mt)
 #pragma unroll
-          for (int e = 0; e < 3; ++e) {
-            mma16816(acc[mt][2 * n], a[mt][e][0], a[mt][e][1], a[mt][e][2], a[mt][e][3], b[0], b[1]);
-            mma16816(acc[mt][2 * n + 1], a[mt][e][0], a[mt][e][1], a[mt][e][2], a[mt][e][3], b[2], b[3]);
+          for (int h = 0; h < 2; ++h) {
+            float d[4], r[4];
+            mma16816_alone(d, a[mt][0][0], a[mt][0][1], a[mt][0][2], a[mt][0][3], b[2 * h], b[2 * h + 1]);
+            mma16816_alone(r, a[mt][2][0], a[mt][2][1], a[mt][2][2], a[mt][2][3], b[2 * h], b[2 * h + 1]);
+            mma16816(r, a[mt][1][0], a[mt][1][1], a[mt][1][2], a[mt][1][3], b[2 * h], b[2 * h + 1]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[mt][2 * n + h][i] += d[i] + r[i];
           }
       }
     }
@@ -533,11 +576,11 @@ __global__ void __launch_bounds__(256) mla_merge_vup_kernel(AttnParams p, const 
     Ls = L;
   }
   __syncthreads();
-  const float invL = Ls > 0.f ? 1.f / Ls : 0.f;
+  const float L = Ls;
   for (int c = threadIdx.x; c < LATENT; c += blockDim.x) {
     float v = 0.f;
     for (int s = 0; s < ns; ++s) v += wgt[s] * base[(long)s * (LATENT + 2) + c];
-    os[c] = __float2bfloat16_rn(v * invL);
+    os[c] = __float2bfloat16_rn(L > 0.f ? v / L : 0.f);        // as the one-launch kernel divides
   }
   __syncthreads();
   for (int j0 = warp * RV, it = 0; j0 < vdim; j0 += 8 * RV, ++it) {

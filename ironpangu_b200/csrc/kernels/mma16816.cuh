@@ -1,4 +1,4 @@
-// Warp-level pieces of the decode attention kernels: 16-byte asynchronous copies into shared memory, ldmatrix, the m16n8k16 bf16 product and weights as
+// Warp-level pieces of the decode attention kernels and the greedy head: 16-byte asynchronous copies into shared memory, ldmatrix, the m16n8k16 bf16 product and weights as
 // three bf16 terms. (Decode attention is bound by its keys' bytes; these products keep up with them at sixteen query rows.)
 #pragma once
 #include "common.cuh"
@@ -20,6 +20,18 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// one product alone
+__device__ __forceinline__ void mma16816_alone(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ float two_sum(float& s, float b) {      // s += b; what the rounding leaves over (Knuth, The Art of Computer Programming 2, 4.2.2)
+  const float a = s;
+  s = a + b;
+  const float c = s - a;
+  return (a - (s - c)) + (b - c);
 }
 // Weights of a softmax as three bf16 terms each, which add up to all 24 bits of a weight. The first two are cut off below the value, not rounded to it, so that
 // no term is 0 and none is negative: an infinite value of a key then stays infinite (inf * 0 is NaN, as is inf - inf). For that a weight is at least e^-62,

@@ -152,3 +152,28 @@ def test_few_rows_of_long_contexts(hd, kv, group, contexts):
         want = torch.einsum("hn,nhd->hd", a, v[max(0, c - window):]).reshape(-1) * torch.sigmoid(gate[t].double())
         torch.testing.assert_close(seen[t].double(), want, rtol=2 ** -8, atol=2e-5)
     assert int(status) == 0
+
+
+@pytest.mark.parametrize("kv,group,hd,n,kps,splits", [(4, 4, 128, 500, 128, 64), (4, 2, 128, 3000, 128, 64), (1, 8, 128, 4000, 128, 64), (4, 4, 64, 6000, 128, 64), (1, 4, 128, 6000, 4000, 2)])
+def test_parts_are_f32_sums(kv, group, hd, n, kps, splits):
+    """Maxima, sums and outputs of the splits as they lie in the scratch, before any rounding to bf16, against double precision."""
+    from ironpangu_b200.ops import decode as K
+
+    g = torch.Generator(device="cuda").manual_seed(n + hd)
+    pages, H = (n + 15) // 16, kv * group
+    kc, vc, q = (torch.randn(*s, generator=g, device="cuda").to(BF16) for s in ((pages, 16, kv, hd), (pages, 16, kv, hd), (1, H * hd)))
+    q *= 2
+    table, pos, slot = torch.arange(pages, dtype=torch.int32, device="cuda").view(1, -1), torch.tensor([n - 1], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    scratch = torch.full((H * splits * (hd + 2),), float("nan"), device="cuda")
+    K.gqa_decode_attention(q, kc, vc, pos, slot, table, heads=H, kv_heads=kv, head_dim=hd, scale=hd ** -0.5, keys_per_split=kps, max_splits=splits, scratch=scratch)
+    most = min(splits, (296 + kv - 1) // kv)                                   # of one row
+    parts = scratch[:H * most * (hd + 2)].view(H, most, hd + 2).double()
+    parts = parts[:, ~parts[0, :, hd].isnan()]
+    w = torch.exp(parts[..., hd] - parts[..., hd].max(-1, keepdim=True).values)
+    out = (w[..., None] * parts[..., :hd]).sum(1) / (w * parts[..., hd + 1]).sum(-1)[:, None]
+    k, v = (x.view(-1, kv, hd)[:n].double() for x in (kc, vc))
+    s = torch.einsum("gjd,ngd->gjn", q.view(kv, group, hd).double(), k) * hd ** -0.5
+    ref = torch.einsum("gjn,ngd->gjd", torch.softmax(s, -1), v).reshape(H, hd)
+    # scores of up to 10 with a few roundings to 2^-24 of them, weights 2^-21 off at most: 4e-7 as f32 sums in any order are; where the tensor cores add up along a
+    # whole row, cutting off, 6e-7 to 2e-6
+    assert float((out - ref).norm() / ref.norm()) < 5.5e-7
