@@ -259,7 +259,7 @@ class MlaMoeDecoder:
         self.scratch = e(T * self.hl * self.max_splits * (c.kv_lora + 2), dt=torch.float32)
         self.logits_r = e(T, c.experts, dt=torch.float32)
         self.route_ids = e(T, c.topk, dt=torch.int32)
-        self.xn, self.qn = e(T, c.hidden), e(T, c.q_lora)
+        self.xn = e(T, c.hidden)
         self.route_w = e(T, c.topk, dt=torch.float32)
         self.act = torch.zeros(T, c.topk + 1, c.expert_ffn, dtype=BF16, device=dev)
         self.partial = e(((self.vl + 7) // 8) * 8 * 2, dt=torch.float32)
@@ -286,19 +286,12 @@ class MlaMoeDecoder:
         return self.next_ids[:T]
 
     # -- one step ----------------------------------------------------------------------------------
-    def product_rows(self, T: int) -> bool:
-        """Whether a step's dense linears run as tensor-core products; between ranks the streaming ones carry the all-reduce."""
-        return T >= 3 and self.world == 1 and self.fabric.world == 1
-
     def _ffn(self, l: int, T: int) -> None:
         """o_proj + all-reduce, router, expert FFN + all-reduce of layer ``l`` (consumes ``self.attn``, updates ``self.x``)."""
         c, w, fab = self.cfg, self.w, self.fabric
         p = f"layers.{l}."
         x, attn = self.x[:T], self.attn[:T]
-        if self.product_rows(T):
-            K.linear_product(attn, w[p + "o_proj"], x, residual=x, status_ptr=fab.desc.status)
-        else:
-            K.gemv_allreduce(attn, w[p + "o_proj"], fab, residual=x, out=x)
+        K.gemv_allreduce(attn, w[p + "o_proj"], fab, residual=x, out=x)
         if self.fused_moe and T <= 2:
             K.moe_block(x, w[p + "router"], w[p + "gate_up"], w[p + "down"], self.rank * self.el, c.topk, fab, sync=self.moe_sync,
                         norm_w=w[p + "ffn_norm"], eps=c.eps, scoring=c.scoring, scale=c.route_scale,
@@ -327,15 +320,11 @@ class MlaMoeDecoder:
         tok, pos, slot = self.tokens[:T], self.positions[:T], self.slots[:T]
         x = self.x[:T]
         st = fab.desc.status
-        rows = self.product_rows(T)
         K.embedding(tok, w["embed"], out=x, status_ptr=st)
         for l in range(c.layers):
             p = f"layers.{l}."
             qkv = self.qkv[:T]
-            if rows:
-                K.linear_product(x, w[p + "qkv_a"], qkv, norm_w=w[p + "attn_norm"], eps=c.eps, norm_out=self.xn[:T], status_ptr=st)
-            else:
-                K.gemv(x, w[p + "qkv_a"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv)
+            K.gemv(x, w[p + "qkv_a"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv)
             fuse = self.fused_head if self.fuse_override is None else (self.fuse_override and self.can_fuse_head)
             if fuse and T <= self.fused_head_rows:
                 K.mla_head_decode(qkv, w[p + "q_a_norm"], w[p + "kv_a_norm"], w[p + "q_b"], w[p + "kv_b"], self.caches[l], pos, slot,
@@ -351,10 +340,7 @@ class MlaMoeDecoder:
                 K.mla_kv_write(qkv[:, c.q_lora:], w[p + "kv_a_norm"], pos, slot, self.page_table, self.caches[l],
                                latent=c.kv_lora, rope=c.rope, eps=c.eps, theta=c.theta, status_ptr=st)
             q = self.q[:T]
-            if rows:
-                K.linear_product(qkv[:, :c.q_lora], w[p + "q_b"], q, norm_w=w[p + "q_a_norm"], eps=c.eps, norm_out=self.qn[:T], status_ptr=st)
-            else:
-                K.gemv(qkv[:, :c.q_lora], w[p + "q_b"], norm_w=w[p + "q_a_norm"], eps=c.eps, out=q)
+            K.gemv(qkv[:, :c.q_lora], w[p + "q_b"], norm_w=w[p + "q_a_norm"], eps=c.eps, out=q)
             q_lat = self.q_lat[:T]
             K.mla_q_absorb(q, w[p + "kv_b"], pos, nope=c.nope, rope=c.rope, theta=c.theta, out=q_lat)
             attn = self.attn[:T]

@@ -80,25 +80,6 @@ def gemv(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] = N
     return out
 
 
-def linear_product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-5,
-                   residual: Optional[torch.Tensor] = None, swiglu: bool = False, norm_out: Optional[torch.Tensor] = None,
-                   status_ptr: Optional[int] = None) -> torch.Tensor:
-    """:func:`gemv` as a tensor-core product of a model's weights: the better form from three rows on, where FMAs bound the streaming one (8 rows, 4096 x 4096:
-    28.6 us against 14.7). ``norm_out``: room for the normalised rows, ``[T, K]``."""
-    T, K = x.shape
-    assert norm_w is None or norm_out is None or norm_out.shape == x.shape
-    assert w.shape[1] == K and w.is_contiguous() and w.dtype == BF16 and x.dtype == BF16
-    xn = x if norm_w is None else rmsnorm(x, norm_w, eps, out=norm_out)
-    lib, st = _lib.load(), _stream()
-    if swiglu:
-        check(lib.ifab_gemm_gated_fixed_bf16(xn.data_ptr(), _rows(xn), w.data_ptr(), K, out.data_ptr(), _rows(out), 0, 0.0, 1.0, T, w.shape[0] // 2, K, status_ptr, st),
-              "linear_product")
-    else:
-        check(lib.ifab_gemm_fixed_bf16(xn.data_ptr(), _rows(xn), w.data_ptr(), K, out.data_ptr(), _rows(out), int(out.dtype == torch.float32), _ptr(residual),
-                                       0 if residual is None else _rows(residual), None, 0, 0.0, T, w.shape[0], K, status_ptr, st), "linear_product")
-    return out
-
-
 def gemv_allreduce(x: torch.Tensor, w: torch.Tensor, fabric, *, residual: Optional[torch.Tensor] = None,
                    out: Optional[torch.Tensor] = None, out_f32: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Row-parallel linear fused with a one-shot all-reduce: ``y = sum_r x_r @ w_r.T (+ residual)``."""

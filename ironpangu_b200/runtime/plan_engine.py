@@ -456,14 +456,6 @@ class PlanEngine:
         self.launches_per_forward = (per_token - (4 * len(self.head_groups) if self.fused_head else 0)
                                      - (2 * len(self.moe_groups) if self.fused_moe else 0) - (4 * len(self.gqa_groups) if self.fused_gqa else 0))
         self._describe()
-        from ..models.mla_moe import MlaMoeConfig
-        self._norm_rows = (torch.empty(self.T, (max(self.cfg.hidden, self.cfg.q_lora) + 7) // 8 * 8, dtype=torch.bfloat16, device=self.tokens.device)
-                           if isinstance(self.cfg, MlaMoeConfig) else None)
-
-    def _takes_product(self, width: int, normed: bool, units: int) -> bool:
-        """Whether a linear of ``width`` columns (with ``units`` gated results, 0: none) fits the tensor-core form: its normalised rows into the room
-        that is kept for them, gated results in whole pieces of eight. The streaming form takes any."""
-        return (not normed or width <= self._norm_rows.shape[1]) and units % 8 == 0
 
     def _describe(self) -> None:
         """What the program says about the model, in the vocabulary of the hand-wired decoder (``models/mla_moe.py``): a
@@ -694,8 +686,6 @@ class PlanEngine:
         head = (self.fused_head if self.fuse_override is None else (self.fuse_override and self.can_fuse_head)) and T <= self.fused_head_rows
         moe = self.fused_moe and T <= 2
         gqa = self.fused_gqa
-        # the hand-wired decoder's rule (models/mla_moe.py): dense linears of three and more rows as tensor-core products
-        product = self._norm_rows is not None and T >= 3 and self.world == 1 and fab.world == 1
         probe = self.probe
         for k, i in enumerate(self.ins):
             op, a, ins = i["op"], i["attrs"], i["inputs"]
@@ -760,13 +750,7 @@ class PlanEngine:
                 V[k] = src[:, s:s + w]
             elif op == "linear":
                 name = a["weight"] + ("|" + a["paired_weight"] if "paired_weight" in a else "")
-                x, swiglu = val(ins[0]), a.get("activation") == "swiglu"
-                if product and self._takes_product(x.shape[1], norm_w is not None, val(k).shape[1] if swiglu else 0):
-                    K.linear_product(x, self._param(name), val(k), norm_w=norm_w, eps=eps, swiglu=swiglu, norm_out=self._norm_rows[:T, :x.shape[1]], status_ptr=st)
-                else:
-                    K.gemv(x, self._param(name), norm_w=norm_w, eps=eps, swiglu=swiglu, out=val(k))
-            elif op == "linear_allreduce" and product:
-                K.linear_product(val(ins[0]), self._param(a["weight"]), val(k), residual=val(ins[1]) if len(ins) > 1 else None, status_ptr=st)
+                K.gemv(val(ins[0]), self._param(name), norm_w=norm_w, eps=eps, swiglu=a.get("activation") == "swiglu", out=val(k))
             elif op == "linear_allreduce":
                 res = val(ins[1]) if len(ins) > 1 else None
                 K.gemv_allreduce(val(ins[0]), self._param(a["weight"]), fab, residual=res, out=val(k))
