@@ -1,5 +1,5 @@
-"""Row kernels at the edges of their pieces: the gated group norm in pieces of four and element by element, the output norm at the width where a row's
-CTA grows from 128 to 256 threads, against PyTorch in double precision."""
+"""Row kernels at the edges of their pieces: the gated group norm in pieces of four and element by element, the output norm at the widths and
+numbers of rows where a row's CTA changes between 128 and 256 threads, against PyTorch in double precision."""
 import pytest
 import torch
 
@@ -29,16 +29,24 @@ def test_gated_group_norm(groups, n, off):
 
 
 @pytest.mark.parametrize("D", [4, 508, 512, 516, 2044, 2046, 2048, 2052, 4096, 4100])
-def test_output_norm(D):
+@pytest.mark.parametrize("T", [3, 591, 592, 700])              # 128 threads to a row from 592 rows on (four to an SM of 148), for up to 2048 columns
+def test_output_norm(T, D):
     from ironpangu_b200.ops import stream_norm as N
 
-    T, eps = 3, 1e-3
+    eps = 1e-3
     g = torch.Generator().manual_seed(D)
     y, x, w, w2 = torch.randn(T, D, generator=g), torch.randn(T, D, generator=g), torch.rand(D, generator=g) + 0.5, torch.rand(D, generator=g) + 0.5
-    rms = lambda v: v / (v.square().mean(-1, keepdim=True) + eps).sqrt()
-    want = x.double() + rms(y.double()) * w.double()
-    xd, xa = x.cuda(), torch.zeros(T, D, device="cuda")
-    N.post_norm_add(y.cuda(), w.cuda(), eps, xd, xa, w2.cuda())
-    # f32: a sum of D squares in pieces (a few 2^-24 of it), four roundings of terms up to 6
-    torch.testing.assert_close(xd.cpu().double(), want, rtol=2e-6, atol=2e-6)
-    torch.testing.assert_close(xa.cpu().double(), rms(want) * w2.double(), rtol=4e-6, atol=4e-6)
+    inv = lambda v: 1 / (v.square().mean(-1, keepdim=True) + eps).sqrt()
+    want = x.double() + y.double() * inv(y.double()) * w.double()
+    scale = inv(want) * w2.double()
+    for second in (True, False):
+        for dt in (torch.float32, BF16):
+            xd, xa = x.cuda(), torch.zeros(T, D, dtype=dt, device="cuda")
+            N.post_norm_add(y.cuda(), w.cuda(), eps, xd, xa, w2.cuda() if second else None)
+            # f32: terms up to 8 with a relative error of 6 x 2^-24 (sum of squares in pieces, root, quotient, two products) and the rounding of a sum up to 13
+            e = 6 * 2 ** -24 * 8 + 2 ** -24 * 13
+            torch.testing.assert_close(xd.cpu().double(), want, rtol=0, atol=e)
+            out, err = (want * scale, e * scale + 6 * 2 ** -24 * (want * scale).abs()) if second else (want, torch.full_like(want, e))
+            if dt is BF16:
+                err = err + 2 ** -8 * out.abs()
+            assert bool(((xa.cpu().double() - out).abs() <= err).all())
