@@ -73,12 +73,10 @@ int ifab_moe_down_allreduce_decode_fp8(const void* act, const int32_t* ids, cons
 /* ---- tensor-core GEMM (tcgen05 + TMEM + TMA): C[M,N] = A[M,K] * B[N,K]^T (+ residual) ---- */
 int ifab_gemm_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual,
                    long ldr, int M, int N, int K, uint32_t* status, void* stream);
-/* the same with an activation of the result in the epilogue: 0 none, 1 SiLU, 2 sigmoid, 3 GELU (tanh form) */
-int ifab_gemm_act_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, int act,
-                       int M, int N, int K, uint32_t* status, void* stream);
+/* on CTA pairs, with an activation of the result in the epilogue: 0 none, 1 SiLU, 2 sigmoid, 3 GELU (tanh form), 4 GELU (erf form) */
 int ifab_gemm_act_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, int act,
                            int persistent, int M, int N, int K, uint32_t* status, void* stream);
-/* the same with a bias [N] (f32, or null) and, for cap > 0, a soft limit cap tanh(result / cap) after the activation */
+/* the same with a bias [N] (f32, or null) and, for cap > 0, a soft limit cap tanh(result / cap) after the activation; fixed: no kernel of the stream writes b */
 int ifab_gemm_fixed_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr, const float* bias,
                          int act, float cap, int M, int N, int K, uint32_t* status, void* stream);
 int ifab_gemm_gated_fixed_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int unit, float limit, float alpha, int M, int F, int K,

@@ -211,13 +211,7 @@ static bool two_sm_enabled() {
 // C[M,N] = A[M,K] * B[N,K]^T (+ residual). A: row stride lda, B: row stride ldb (elements), K % 8 == 0.
 extern "C" int ifab_gemm_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32,
                               const void* residual, long ldr, int M, int N, int K, uint32_t* status, void* stream) {
-  return ifab_gemm_act_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, 0, M, N, K, status, stream);
-}
-
-// The same with an activation of the result in the epilogue (1 SiLU, 2 sigmoid, 3 GELU in the tanh form).
-extern "C" int ifab_gemm_act_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
-                                  int act, int M, int N, int K, uint32_t* status, void* stream) {
-  return ifab_gemm_epilogue_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, nullptr, act, 0.f, M, N, K, status, stream);
+  return ifab_gemm_epilogue_bf16(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, nullptr, 0, 0.f, M, N, K, status, stream);
 }
 
 namespace {
@@ -275,7 +269,7 @@ int gemm_gated(const void* a, long lda, const void* b, long ldb, void* c, long l
 }
 }  // namespace
 
-// The same with a bias [N] in f32 (or null) and, for cap > 0, a soft limit of the result (cap tanh(result / cap)) after the activation.
+// The same with a bias [N] in f32 (or null), an activation of the result (rope.cuh) and, for cap > 0, a soft limit of the result (cap tanh(result / cap)) after it.
 extern "C" int ifab_gemm_epilogue_bf16(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                        const float* bias, int act, float cap, int M, int N, int K, uint32_t* status, void* stream) {
   return gemm_epilogue(a, lda, b, ldb, c, ldc, out_f32, residual, ldr, bias, act, cap, 0, M, N, K, status, stream);

@@ -13,7 +13,7 @@
 // Six stages of 32 KB. No TMA load is multicast: every CTA fetches its own tiles. Every mbarrier wait is bounded; a wait that
 // runs out raises the CTA's abort flag and a status bit, and both CTAs still meet at the closing cluster barrier.
 // Shapes: N % 32 == 0 (rows are stored 32 columns at a time), K % 8 == 0; M, N and K tails by TMA zero fill and masked stores.
-// `ifab_gemm_bf16` uses these kernels from 256 rows and 256 columns up; below that a pair's 256 x 256 tile is mostly padding.
+// `ifab_gemm_bf16` uses these kernels from 129 rows and 256 columns up, but where the cluster form has less to load (tc_gemm_rows.cu).
 #include <algorithm>
 
 #include "attn_rule.cuh"

@@ -21,10 +21,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, residual: Optional[torch.Tensor] =
     assert b.shape[1] == K and a.dtype == BF16 and b.dtype == BF16 and a.stride(1) == 1 and b.stride(1) == 1
     if out is None:
         out = torch.empty(M, N, dtype=torch.float32 if out_f32 else BF16, device=a.device)
-    fn = _lib.load().ifab_gemm_fixed_bf16 if fixed else _lib.load().ifab_gemm_epilogue_bf16
+    fn = _lib.load().ifab_gemm_fixed_bf16 if fixed else _lib.load().ifab_gemm_bf16
     check(fn(a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(), out.stride(0), int(out.dtype == torch.float32),
-             None if residual is None else residual.data_ptr(), 0 if residual is None else residual.stride(0), None, 0, 0.0, M, N, K, status_ptr,
-             torch.cuda.current_stream().cuda_stream), "gemm")
+             None if residual is None else residual.data_ptr(), 0 if residual is None else residual.stride(0), *((None, 0, 0.0) if fixed else ()), M, N, K,
+             status_ptr, torch.cuda.current_stream().cuda_stream), "gemm")
     return out
 
 
