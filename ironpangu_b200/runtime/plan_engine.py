@@ -452,7 +452,6 @@ class PlanEngine:
         self._head_members = {m: k for k, g in self.head_groups.items() for m in g["members"]}
         self._moe_members = {m: k for k, g in self.moe_groups.items() for m in g["members"]}
         per_token = self.program["launches_per_token"] + sum(1 for i in self.ins if i["op"] == "mla_attention")
-        per_token += sum(1 for i in self.ins if i["op"] == "paged_attention")        # split + merge
         self.launches_per_forward = (per_token - (4 * len(self.head_groups) if self.fused_head else 0)
                                      - (2 * len(self.moe_groups) if self.fused_moe else 0) - (4 * len(self.gqa_groups) if self.fused_gqa else 0))
         self._describe()
