@@ -115,8 +115,6 @@ int dispatch_rows(const GemvParams& p, cudaStream_t s) {
   // Rows per warp: the fewest that leave no more CTAs than run at once, two on an SM (a second wave of a quarter of the CTAs costs as much as the first). Many
   // columns that take several waves anyway: four rows, whose loads are in flight together. One row, K 2048, us: N 3072 6.4 by one, 4.1 by two; N 8192 13.2, 9.2
   // by two, 6.9 by four; gated 6144 11.4 by two pairs, 9.7 by three.
-  // The lines are those of one row. Of more rows other shares are better at some widths (K 2048, by one, two, three, four: two rows N 6144 12.6, 11.2, 7.1, 11.4;
-  // eight rows N 3072 28.1, 24.2, 13.6, 16.1; two rows gated N 3072 9.4, 12.5, 10.1).
   if (p.mode) {
     if (p.N <= 296 * 8) return launch_gemv<T, 1>(p, s);
     if (p.N <= 296 * 16 || p.N > 296 * 24) return launch_gemv<T, 2>(p, s);
