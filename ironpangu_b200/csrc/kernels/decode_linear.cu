@@ -110,19 +110,33 @@ int launch_gemv(const GemvParams& p, cudaStream_t s) {
   return launch_chain(k, grid, dim3(256), smem, s, p);
 }
 
+// Rows (or pairs of them) of the matrix to a warp.
+//   one row of x        the fewest that leave no more CTAs than run at once, two on an SM (a second wave of a quarter of the CTAs costs as much as the first). Many
+//                       columns that take several waves anyway: four rows, whose loads are in flight together. K 2048, us: N 3072 6.4 by one, 4.1 by two;
+//                       N 8192 13.2, 9.2 by two, 6.9 by four; gated 6144 11.4 by two pairs, 9.7 by three
+//   two to eight        a row's operands in registers serve more products, so that three and four are better as soon as one does not fill the chip: whichever has
+//                       the least to do in its waves, of which eight rows get one CTA an SM (registers). K 2048, us by one, two, three, four: two rows N 3072 8.4,
+//                       7.5, 6.1, 6.0, N 6144 12.6, 11.2, 7.1, 11.4; four rows N 6144 25.1, 17.4, 11.3, 18.3, N 8192 32.5, 19.7, 19.4, 18.8; eight rows N 3072
+//                       28.1, 24.2, 13.6, 16.1, N 4096 31.8, 24.4, 26.4, 16.5. Pairs, by one, two, three: two rows N 3072 9.4, 12.5, 10.1, N 12288 27.6, 32.3, 22.9; four rows N 8192 35.2, 26.4, 29.2; eight rows N 3072 30.0, 30.5, 20.1
 template <int T>
 int dispatch_rows(const GemvParams& p, cudaStream_t s) {
-  // Rows per warp: the fewest that leave no more CTAs than run at once, two on an SM (a second wave of a quarter of the CTAs costs as much as the first). Many
-  // columns that take several waves anyway: four rows, whose loads are in flight together. One row, K 2048, us: N 3072 6.4 by one, 4.1 by two; N 8192 13.2, 9.2
-  // by two, 6.9 by four; gated 6144 11.4 by two pairs, 9.7 by three.
-  if (p.mode) {
-    if (p.N <= 296 * 8) return launch_gemv<T, 1>(p, s);
-    if (p.N <= 296 * 16 || p.N > 296 * 24) return launch_gemv<T, 2>(p, s);
-    return launch_gemv<T, 3>(p, s);
-  }
   if (p.N <= 296 * 8) return launch_gemv<T, 1>(p, s);
-  if (p.N <= 296 * 16) return launch_gemv<T, 2>(p, s);
-  return launch_gemv<T, 4>(p, s);
+  if constexpr (T == 1) {
+    if (p.mode) {
+      if (p.N <= 296 * 16 || p.N > 296 * 24) return launch_gemv<T, 2>(p, s);
+      return launch_gemv<T, 3>(p, s);
+    }
+    if (p.N <= 296 * 16) return launch_gemv<T, 2>(p, s);
+    return launch_gemv<T, 4>(p, s);
+  } else {
+    auto waves_of = [&](int r) { return ((p.N + 8 * r - 1) / (8 * r) + (T == 8 ? 147 : 295)) / (T == 8 ? 148 : 296) * r; };
+    if (p.mode) {
+      if (T == 2) return p.N <= 296 * 16 ? launch_gemv<T, 1>(p, s) : launch_gemv<T, 3>(p, s);
+      return waves_of(2) < waves_of(3) ? launch_gemv<T, 2>(p, s) : launch_gemv<T, 3>(p, s);
+    }
+    if (T < 8 && p.N <= 296 * 16) return launch_gemv<T, 4>(p, s);
+    return waves_of(3) < waves_of(4) ? launch_gemv<T, 3>(p, s) : launch_gemv<T, 4>(p, s);
+  }
 }
 
 // ----------------------------------------------------------------------------------------------
