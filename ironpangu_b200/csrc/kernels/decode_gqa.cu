@@ -105,6 +105,11 @@ __global__ void __launch_bounds__(256) gqa_rope_kv_write_kernel(bf16* qkv, long 
   for (int c = threadIdx.x; c < kv_elems / 8; c += blockDim.x) reinterpret_cast<uint4*>(kdst)[c] = ksrc[c];
 }
 
+int log2_of(int v) {
+  int k = 0;
+  while (k < 30 && (1 << k) < v) ++k;
+  return v > 0 && (1 << k) == v ? k : -1;
+}
 struct GqaParams {
   const bf16* q; long ldq; const bf16* k_cache; const bf16* v_cache;
   const int32_t* positions; const int32_t* slots; const int32_t* page_table;
@@ -119,16 +124,22 @@ struct GqaParams {
   ScoreRule rule;
   AheadRule ahead;                                // entries that count as the first keys of a row
   float factor;                                   // of the result
+  int order;                                      // rows by how much they see
+  int group, page_shift, split_shift;             // Hq / Hkv; logarithms of page_tokens and max_splits (-1: none): divisions are most of a short row's start
   // keys of a split of a row that sees n: an even share, at least kps, whole rounds of a CTA (64 keys)
-  __device__ __forceinline__ int per_split(int n) const { return (max(kps, (n + max_splits - 1) / max_splits) + 63) / 64 * 64; }
+  __device__ __forceinline__ int per_split(int n) const {
+    const int share = split_shift >= 0 ? (n + max_splits - 1) >> split_shift : (n + max_splits - 1) / max_splits;
+    return (max(kps, share) + 63) / 64 * 64;
+  }
 };
 
 // what a row sees: entries ahead of its window, then the positions first .. pos
 struct Seen {
   int first, ahead, n;
-  __device__ __forceinline__ Seen(const GqaParams& p, int pos) : first(first_key(pos, p.window, p.rule.chunked)) {
+  // `pages`: counted from the sixteen positions on that the first lies among
+  __device__ __forceinline__ Seen(const GqaParams& p, int pos, bool pages = false) : first(first_key(pos, p.window, p.rule.chunked)) {
     ahead = p.ahead.count(first);
-    n = ahead + pos + 1 - first;
+    n = ahead + pos + 1 - (pages ? first & ~15 : first);
   }
 };
 // row of key k of what a row sees; `pooled`: in the caches of the blocks
@@ -261,71 +272,99 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 //            end. Up to four heads: the terms are rows 0-3, 8-11 and 4-7 of one product (a lane has the weights of its row, so it only picks a
 //            term). Eight (WIDE): the first two terms are rows 0-7 and 8-15, and in a second product half of the third is in both
 //
-// Bound by the stream of keys and values: a key costs a warp two instructions, where products on the CUDA cores (eight lanes to a key) cost 40 and
-// bound the kernel. 16 query heads over 4: 64 rows of 2560 keys (335 MB) 376 us before, 77 us (4.3 TB/s); 8 rows of 1900 keys 46 -> 13 us, one row of
-// 2000 keys 14.8 -> 10.4 us, merge included. Two CTAs an SM (registers) x four warps
-// with one stage of 8 KB in flight beside the one in use.
+// Bound by the stream of keys and values while all CTAs run (a tile of 16 keys takes a warp 1100 clocks and about as long again until the next one is there), and by what
+// comes before and behind: rows' order, the start's chain of loads (position, page, keys: divisions are shifts, the pages of 32 tiles one trip, the query's columns
+// requested behind them) and the merge (a warp a head; parts pushed to the CTA that adds them up, one cluster barrier). 16 query heads over 4: 64 rows of 2560
+// keys (335 MB) 376 us on the CUDA cores, 96 before these, 75 now (4.5 TB/s); 64 rows of 1250, 32 heads 65 -> 49; one row of 2000 keys 10.8 -> 8.0, of
+// 4000 16.2 -> 11.0; 8 rows of 1900 15.7 -> 15.5. A third stage of keys or a third CTA an SM gave nothing.
+// PAGES: where pages hold a multiple of 16 positions a tile is 16 positions from a multiple of 16 on: rows one behind the other, one page to look up, no masks inside.
 // Every product of sixteen is added to its f32 sum outside the tensor core, scores in two sums each: the tensor core cuts off what it adds up, and chains of its
 // products left results 0.6e-6 to 1.9e-6 off, where these are 2.5e-7 to 4.2e-7 and FMAs 2.4e-7 to 4.4e-7. Against two terms of a weight and chains: 64 rows of up
 // to 4096 keys 91.2 -> 92.8 us; groups of eight (over one kv head) 32.9 -> 35.0 us.
-template <int HD>
+template <int HD, int W>
 struct MmaSplit {
-  static constexpr int KEYS = 16, WARPS = 4, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
+  static constexpr int KEYS = 16, WARPS = W, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
   static constexpr int ROW = HD * 2, STAGE = 2 * KEYS * ROW;
-  static constexpr int SMEM = WARPS * STAGES * STAGE;
+  static constexpr int RINGS = WARPS * STAGES * STAGE, SMEM = RINGS + (8 * HD + 8 * 8 * 2) * 4;
 };
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float peer_float(const float* mine, uint32_t rank) {
+__device__ __forceinline__ uint32_t peer_addr(const float* mine, uint32_t rank) {
   uint32_t at;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr(mine)), "r"(rank));
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-  return v;
+  return at;
+}
+__device__ __forceinline__ void st_peer4(float* mine, uint32_t rank, const float4& v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(peer_addr(mine, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void st_peer2(float* mine, uint32_t rank, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer_addr(mine, rank)), "f"(a), "f"(b) : "memory");
 }
 
 // CLUSTER: the splits of a (row, kv head) are one cluster (at most eight) and merge their parts over distributed shared memory into `out`; otherwise
 // the parts go to the scratch and gqa_merge_kernel follows.
-template <int HD, bool CLUSTER, bool WIDE>
-__global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
-  using S = MmaSplit<HD>;
+template <int HD, bool CLUSTER, bool WIDE, bool PAGES, int W>
+__global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
+  using S = MmaSplit<HD, W>;
+  constexpr int NT = 32 * W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep_launch();
   grid_dep_wait();
-  const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
-  const int pos = p.positions[t];
+  const int split = blockIdx.x, kvh = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int t = blockIdx.z;
+  if (p.order) {                   // the rows that see most first: a long one that starts last is what a launch waits for
+    __shared__ int s_n[NT], s_t;
+    const int mine = threadIdx.x < p.T ? p.positions[threadIdx.x] : -1;
+    const int seen_n = mine < 0 ? 0 : Seen(p, mine).n;
+    s_n[threadIdx.x] = seen_n;
+    __syncthreads();
+    int before = 0;
+    for (int i = 0; i < p.T; ++i) before += s_n[i] > seen_n || (s_n[i] == seen_n && i < (int)threadIdx.x);
+    if (threadIdx.x < p.T && before == t) s_t = threadIdx.x;
+    __syncthreads();
+    t = s_t;
+  }
+  const int pos = p.positions[t], slot = p.slots[t];
   if (pos < 0) return;
-  const Seen seen(p, pos);
+  if (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  const Seen seen(p, pos, PAGES);
   const int n = seen.n, per = p.per_split(n), k_begin = split * per;
   if (!CLUSTER && k_begin >= n) return;
   const int k_end = min(n, k_begin + per);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2, G = p.Hq / p.Hkv, gh = WIDE ? g : g & 3;      // gh: this lane's head of the group
-  const int slot = p.slots[t];
+  const int g = lane >> 2, c2 = (lane & 3) * 2, G = p.group, gh = WIDE ? g : g & 3;      // gh: this lane's head of the group
   const bool ruled = !p.rule.plain();
   const float slope = p.rule.slopes && gh < G ? p.rule.slopes[kvh * G + gh] : 0.f;
-  // query row of head gh: columns 16 i + c2 + {0, 1} and + 8
-  uint32_t q[HD / 16][2];
-  {
-    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + (gh < G ? gh : 0)) * HD + c2;
+  float acc[HD / 8][2], m = -INFINITY, l = 0.f;
 #pragma unroll
-    for (int i = 0; i < HD / 16; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const bf16 *e = qh + 16 * i + 8 * j;
-        q[i][j] = gh < G ? (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16 : 0u;
-      }
-  }
-  float acc[HD / 8][4], m = -INFINITY, l = 0.f;
-#pragma unroll
-  for (int i = 0; i < HD / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  for (int i = 0; i < HD / 8; ++i) acc[i][0] = acc[i][1] = 0.f;
 
   const uint32_t ring = smem_addr(smem_raw) + warp * S::STAGES * S::STAGE;
   const long kv_elems = (long)p.Hkv * HD;
   const int first = k_begin + warp * S::KEYS, stride = S::WARPS * S::KEYS;
-  // where key `first + i * stride + (lane & 15)` lies: 2 * row + (1: among the blocks); -1: nowhere
+  // PAGES: sixteen positions that lie one behind the other in a page, from a multiple of sixteen on (first row; -1: nowhere). Keys ahead of the first one and behind
+  // the last one are not there
+  const int base = PAGES ? (seen.first & ~15) + first : 0;
+  auto there = [&](int i, int key) { return base + i * stride + key >= seen.first && base + i * stride + key <= pos; };
+  const int tiles = first < k_end ? (k_end - first + stride - 1) / stride : 0;
+  // pages of 32 tiles, one a lane: one trip to memory for all of them
+  auto page_of = [&](int i) {
+    const int at = base + i * stride;
+    if (i >= tiles || at > pos) return -1;
+    const int lp = p.page_shift >= 0 ? at >> p.page_shift : at / p.page_tokens, page = lp < p.max_pages ? p.page_table[(long)slot * p.max_pages + lp] : -1;
+    if (page >= 0 && page < p.num_pages) return page;
+    if (p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
+    return -1;
+  };
+  int page = PAGES ? page_of(lane) : 0;
+  // where key `first + i * stride + (lane & 15)` lies: 2 * row + (1: among the blocks); -1: nowhere. PAGES: the tile's first row
   auto locate = [&](int i) -> long {
+    if (PAGES) {
+      if (i && (i & 31) == 0) page = page_of(i + lane);
+      const int at = base + i * stride, its = __shfl_sync(0xffffffffu, page, i & 31);
+      return its < 0 ? -1 : (long)its * p.page_tokens + (p.page_shift >= 0 ? at & (p.page_tokens - 1) : at % p.page_tokens);
+    }
     const int k = first + i * stride + (lane & 15);
     if (k >= k_end) return -1;
     bool pooled;
@@ -336,22 +375,39 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
     }
     return 2 * r + pooled;
   };
-  auto load = [&](int stage, long where) {
-    const uint32_t base = ring + stage * S::STAGE;
+  auto load = [&](int stage, int i, long where) {
+    const uint32_t dst0 = ring + stage * S::STAGE;
     const int ch = lane % S::CH;
+    if (PAGES) {
+      constexpr int STEP = 32 / S::CH;
+      const int key0 = lane / S::CH;
+      const long at = (where < 0 ? 0 : where + key0) * kv_elems + (long)kvh * HD + ch * 8;
+      const bool whole = where >= 0 && there(i, 0) && there(i, S::KEYS - 1);
 #pragma unroll
-    for (int i = 0; i < S::KEYS * S::CH / 32; ++i) {
-      const int key = lane / S::CH + i * (32 / S::CH);
-      const long w = __shfl_sync(0xffffffffu, where, key);
-      const long at = w < 0 ? 0 : (w >> 1) * kv_elems + (long)kvh * HD + ch * 8;
-      const bf16* kb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.k : p.k_cache;
-      const bf16* vb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.v : p.v_cache;
-      const uint32_t dst = base + key * S::ROW + ((ch ^ (key & 7)) << 4);
-      copy16(dst, kb + at, w >= 0);
-      copy16(dst + S::KEYS * S::ROW, vb + at, w >= 0);
+      for (int j = 0; j < S::KEYS / STEP; ++j) {
+        const int key = key0 + j * STEP;
+        const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
+        const bool live = whole || (where >= 0 && there(i, key));
+        const long off = live ? at + (long)j * STEP * kv_elems : 0;
+        copy16(dst, p.k_cache + off, live);
+        copy16(dst + S::KEYS * S::ROW, p.v_cache + off, live);
+      }
+      return;
+    }
+    if constexpr (!PAGES) {
+#pragma unroll
+      for (int j = 0; j < S::KEYS * S::CH / 32; ++j) {
+        const int key = lane / S::CH + j * (32 / S::CH);
+        const long w = __shfl_sync(0xffffffffu, where, key);
+        const long at = w < 0 ? 0 : (w >> 1) * kv_elems + (long)kvh * HD + ch * 8;
+        const bf16* kb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.k : p.k_cache;
+        const bf16* vb = w >= 0 && (w & 1) ? (const bf16*)p.ahead.v : p.v_cache;
+        const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
+        copy16(dst, kb + at, w >= 0);
+        copy16(dst + S::KEYS * S::ROW, vb + at, w >= 0);
+      }
     }
   };
-  const int tiles = first < k_end ? (k_end - first + stride - 1) / stride : 0;
   long at[S::STAGES];          // of the tiles in the ring, by stage
 #pragma unroll
   for (int i = 0; i < S::STAGES; ++i) at[i] = -1;
@@ -359,9 +415,22 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
   for (int i = 0; i < S::STAGES - 1; ++i) {
     if (i < tiles) {
       at[i] = locate(i);
-      load(i, at[i]);
+      load(i, i, at[i]);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // query row of head gh: columns 16 i + c2 + {0, 1} and + 8
+  uint32_t q[HD / 16][2];
+  {
+    const bf16* qh = p.q + (long)t * p.ldq + (long)(kvh * G + (gh < G ? gh : 0)) * HD + c2;
+    const bool pairs = (reinterpret_cast<uintptr_t>(qh) & 3) == 0;
+#pragma unroll
+    for (int i = 0; i < HD / 16; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const bf16 *e = qh + 16 * i + 8 * j;
+        q[i][j] = gh >= G ? 0u : pairs ? *reinterpret_cast<const uint32_t*>(e) : (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16;
+      }
   }
   long next = S::STAGES - 1 < tiles ? locate(S::STAGES - 1) : -1;
   for (int i0 = 0; i0 < tiles; i0 += S::STAGES) {
@@ -373,36 +442,50 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
       const int to = (st + AHEAD) % S::STAGES;
       if (i + AHEAD < tiles) {
         at[to] = next;
-        load(to, next);
+        load(to, i + AHEAD, next);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       next = i + AHEAD + 1 < tiles ? locate(i + AHEAD + 1) : -1;
       asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
       __syncwarp();
       const uint32_t kb = ring + st * S::STAGE, vb = kb + S::KEYS * S::ROW;
+      uint32_t b[HD / 16][4];
       float s[2][4] = {};                        // [keys c2 .. / c2 + 8 ..][two sums each: of even and of odd pieces of the columns]
 #pragma unroll
-      for (int kk = 0; kk < HD / 16; ++kk) {
-        uint32_t b[4];
+      for (int kk = 0; kk < HD / 16; ++kk) {       // all of a tile's operands requested together: one after the other their latencies were most of its time
         const int key = (lane >> 4) * 8 + (lane & 7), ch = 2 * kk + ((lane >> 3) & 1);
-        ldsm4(kb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
+        ldsm4(kb + key * S::ROW + ((ch ^ (key & 7)) << 4), b[kk]);
+      }
+#pragma unroll
+      for (int kk = 0; kk < HD / 16; ++kk) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float d[4];
-          mma16816_alone(d, q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[2 * h], b[2 * h + 1]);
+          mma16816_alone(d, q[kk][0], q[kk][0], q[kk][1], q[kk][1], b[kk][2 * h], b[kk][2 * h + 1]);
           s[h][2 * (kk & 1)] += d[0];
           s[h][2 * (kk & 1) + 1] += d[1];
         }
       }
+#pragma unroll
+      for (int j = 0; j < HD / 16; ++j) {
+        const int key = ((lane >> 3) & 1) * 8 + (lane & 7), ch = 2 * j + (lane >> 4);
+        ldsm4t(vb + key * S::ROW + ((ch ^ (key & 7)) << 4), b[j]);
+      }
       // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against head gh
       float w[4];
       float mn = m;
+      const bool whole = PAGES && at[st] >= 0 && there(i, 0) && there(i, S::KEYS - 1);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = c2 + (j >> 1) * 8 + (j & 1);
         w[j] = (s[j >> 1][j & 1] + s[j >> 1][2 + (j & 1)]) * p.scale;
-        if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
-        if (__shfl_sync(0xffffffffu, at[st], key) < 0) w[j] = -INFINITY;
+        if (PAGES) {
+          if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, pos - (base + i * stride + key));
+          if (!whole && (at[st] < 0 || !there(i, key))) w[j] = -INFINITY;
+        } else {
+          if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
+          if (__shfl_sync(0xffffffffu, at[st], key) < 0) w[j] = -INFINITY;
+        }
         mn = fmaxf(mn, w[j]);
       }
       mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
@@ -413,7 +496,7 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
 #pragma unroll
         for (int j = 0; j < HD / 8; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[j][e] *= corr;
+          for (int e = 0; e < 2; ++e) acc[j][e] *= corr;
         m = mn;
       }
 #pragma unroll
@@ -427,16 +510,16 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
       const uint32_t lo0 = WIDE || g < 4 ? lo[0] : lo[2], hi0 = WIDE || g < 4 ? hi[0] : hi[2];
 #pragma unroll
       for (int j = 0; j < HD / 16; ++j) {
-        uint32_t b[4];
-        const int key = ((lane >> 3) & 1) * 8 + (lane & 7), ch = 2 * j + (lane >> 4);
-        ldsm4t(vb + key * S::ROW + ((ch ^ (key & 7)) << 4), b);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float d[4];
-          mma16816_alone(d, lo0, lo[1], hi0, hi[1], b[2 * h], b[2 * h + 1]);
-          if (WIDE) mma16816(d, lo[2], lo[2], hi[2], hi[2], b[2 * h], b[2 * h + 1]);
+          mma16816_alone(d, lo0, lo[1], hi0, hi[1], b[j][2 * h], b[j][2 * h + 1]);
+          if (WIDE) mma16816(d, lo[2], lo[2], hi[2], hi[2], b[j][2 * h], b[j][2 * h + 1]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[2 * j + h][e] += d[e];
+          for (int e = 0; e < 2; ++e) {
+            acc[2 * j + h][e] += d[e];
+            if (WIDE || g < 4) acc[2 * j + h][e] += d[2 + e];        // rows 12-15 of groups up to four are nobody's
+          }
         }
       }
       __syncwarp();            // the stage is read: a later round may overwrite it
@@ -455,10 +538,6 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
 #pragma unroll
   for (int j = 0; j < HD / 8; ++j) {
     float2 v = make_float2(acc[j][0], acc[j][1]);
-    if (WIDE || g < 4) {       // rows 12-15 of groups up to four are nobody's
-      v.x += acc[j][2];
-      v.y += acc[j][3];
-    }
     if (!WIDE) {               // rows 4-7: the third term
       v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
       v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
@@ -466,41 +545,63 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
     if (WIDE || g < 4) *reinterpret_cast<float2*>(sm_acc + (warp * 8 + g) * HD + 8 * j + c2) = v;
   }
   __syncthreads();
-  float* part = sm_acc + S::WARPS * 8 * HD;        // CLUSTER: this split's [G][HD], then maxima and sums
-  for (int h = 0; h < G; ++h) {
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < S::WARPS; ++w) M = fmaxf(M, sm_m[w * 8 + h]);
-    float wgt[S::WARPS], L = 0.f;
+  // A warp merges a head at a time. CLUSTER: what the warp has goes to the CTA of the cluster that will put the parts of these columns together: its memory behind
+  // the rings, [splits][its columns], then maxima and sums [splits][8] (pushed, so that the one barrier is all there is to wait for).
+  const int parts = p.max_splits, mine = G * HD / parts;
+  float* got = reinterpret_cast<float*>(smem_raw + S::RINGS);
+  if (CLUSTER) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // all CTAs of the cluster run
+  for (int h = warp; h < G; h += S::WARPS) {
+    float wgt[S::WARPS], M = -INFINITY, L = 0.f;
 #pragma unroll
     for (int w = 0; w < S::WARPS; ++w) {
-      wgt[w] = sm_m[w * 8 + h] == -INFINITY ? 0.f : __expf(sm_m[w * 8 + h] - M);
+      wgt[w] = sm_m[w * 8 + h];
+      M = fmaxf(M, wgt[w]);
+    }
+#pragma unroll
+    for (int w = 0; w < S::WARPS; ++w) {
+      wgt[w] = wgt[w] == -INFINITY ? 0.f : __expf(wgt[w] - M);
       L += wgt[w] * sm_l[w * 8 + h];
     }
-    float* to = CLUSTER ? part + h * HD : p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2);
-    for (int c = threadIdx.x; c < HD; c += 128) {
-      float v = 0.f;
+    if (lane * 4 < HD) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int w = 0; w < S::WARPS; ++w) v += wgt[w] * sm_acc[(w * 8 + h) * HD + c];
-      to[c] = v;
+      for (int w = 0; w < S::WARPS; ++w) {
+        const float4 a = *reinterpret_cast<const float4*>(sm_acc + (w * 8 + h) * HD + lane * 4);
+        v.x += wgt[w] * a.x;
+        v.y += wgt[w] * a.y;
+        v.z += wgt[w] * a.z;
+        v.w += wgt[w] * a.w;
+      }
+      if (CLUSTER) {
+        const int e = h * HD + lane * 4, to = e / mine;
+        st_peer4(got + split * mine + e - to * mine, to, v);
+      } else {
+        float* to = p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2) + lane * 4;
+        to[0] = v.x;
+        to[1] = v.y;
+        to[2] = v.z;
+        to[3] = v.w;
+      }
     }
-    if (threadIdx.x == 0) {
-      (CLUSTER ? part + 8 * HD + h : to + HD)[0] = M;
-      (CLUSTER ? part + 8 * HD + 8 + h : to + HD + 1)[0] = L;
+    if (CLUSTER) {
+      if (lane < parts) st_peer2(got + G * HD + (split * 8 + h) * 2, lane, M, L);
+    } else if (lane == 0) {
+      float* to = p.scratch + (((long)t * p.Hq + kvh * G + h) * p.max_splits + split) * (HD + 2) + HD;
+      to[0] = M;
+      to[1] = L;
     }
   }
   if (!CLUSTER) return;
   cluster_barrier();
-  const int parts = p.max_splits;
-  for (int e = split * 128 + threadIdx.x; e < G * HD; e += parts * 128) {
-    const int h = e / HD, c = e - h * HD, head = kvh * G + h;
+  for (int i = threadIdx.x; i < mine; i += NT) {
+    const int e = split * mine + i, h = e / HD, c = e - h * HD, head = kvh * G + h;
     float pm[8], pl[8], pv[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
       if (r < parts) {
-        pm[r] = peer_float(part + 8 * HD + h, r);
-        pl[r] = peer_float(part + 8 * HD + 8 + h, r);
-        pv[r] = peer_float(part + e, r);
+        pm[r] = got[G * HD + (r * 8 + h) * 2];
+        pl[r] = got[G * HD + (r * 8 + h) * 2 + 1];
+        pv[r] = got[r * mine + i];
       }
     float M = p.sink ? p.sink[head] : -INFINITY;
 #pragma unroll
@@ -518,12 +619,11 @@ __global__ void __launch_bounds__(128, HD == 64 ? 4 : 2) gqa_split_mma_kernel(Gq
     if (p.gate) v *= activate<true>(__bfloat162float(p.gate[(long)t * p.ldg + (p.gate_head ? head : (long)head * HD + c)]), p.gate_act);
     res[(long)t * ldo + (long)head * HD + c] = __float2bfloat16_rn(v);
   }
-  cluster_barrier();           // the parts stay until every split has read them
 }
 
 // grid (Hq, T), HD threads
 template <int HD>
-__global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
+__global__ void gqa_merge_kernel(GqaParams p, int pages, bf16* out, long ldo) {
   __shared__ float wgt[64];
   __shared__ float Ls;
   grid_dep_launch();
@@ -531,7 +631,7 @@ __global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
   const int h = blockIdx.x, t = blockIdx.y;
   const int pos = p.positions[t];
   if (pos < 0) return;
-  const int n = Seen(p, pos).n;
+  const int n = Seen(p, pos, pages != 0).n;
   const int per = p.per_split(n), ns = (n + per - 1) / per;
   const float* base = p.scratch + ((long)t * p.Hq + h) * p.max_splits * (HD + 2);
   if (threadIdx.x < 32) {      // up to 64 splits: two per lane
@@ -558,8 +658,8 @@ __global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
 }
 
 template <int HD>
-int launch_merge(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
-  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, out, ldo);
+int launch_merge(const GqaParams& p, int pages, bf16* out, long ldo, cudaStream_t s) {
+  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, pages, out, ldo);
 }
 template <int HD, int G>
 int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
@@ -568,21 +668,21 @@ int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   if (int rc = opt_in_smem(k, smem)) return rc;
   dim3 grid(p.max_splits, p.Hkv, p.T);
   if (int rc = launch_chain(k, grid, dim3(256), smem, s, p)) return rc;
-  return launch_merge<HD>(p, out, ldo, s);
+  return launch_merge<HD>(p, 0, out, ldo, s);
 }
-template <int HD, bool WIDE>
-int launch_mma(const GqaParams& p, bool cluster, bf16* out, long ldo, cudaStream_t s) {
-  constexpr int smem = MmaSplit<HD>::SMEM;
+template <int HD, bool CLUSTER, bool WIDE, bool PAGES, int W>
+int launch_split(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
+  constexpr int smem = MmaSplit<HD, W>::SMEM;
   const dim3 grid(p.max_splits, p.Hkv, p.T);
-  if (cluster) {
-    auto k = gqa_split_mma_kernel<HD, true, WIDE>;
-    if (int rc = opt_in_smem(k, smem)) return rc;
-    return launch_chain_cluster(k, grid, dim3(128), (unsigned)p.max_splits, smem, s, p, out, ldo);
-  }
-  auto k = gqa_split_mma_kernel<HD, false, WIDE>;
+  auto k = gqa_split_mma_kernel<HD, CLUSTER, WIDE, PAGES, W>;
   if (int rc = opt_in_smem(k, smem)) return rc;
-  if (int rc = launch_chain(k, grid, dim3(128), smem, s, p, out, ldo)) return rc;
-  return launch_merge<HD>(p, out, ldo, s);
+  return CLUSTER ? launch_chain_cluster(k, grid, dim3(32 * W), (unsigned)p.max_splits, smem, s, p, out, ldo) : launch_chain(k, grid, dim3(32 * W), smem, s, p, out, ldo);
+}
+template <int HD, bool WIDE, bool PAGES>
+int launch_mma(const GqaParams& p, bool cluster, int warps, bf16* out, long ldo, cudaStream_t s) {
+  if (cluster) return warps == 8 ? launch_split<HD, true, WIDE, PAGES, 8>(p, out, ldo, s) : launch_split<HD, true, WIDE, PAGES, 4>(p, out, ldo, s);
+  if (int rc = launch_split<HD, false, WIDE, PAGES, 4>(p, out, ldo, s)) return rc;
+  return launch_merge<HD>(p, PAGES, out, ldo, s);
 }
 
 template <int HD>
@@ -603,7 +703,14 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
       }
-      return G == 8 ? launch_mma<HD, true>(p, cluster, out, ldo, s) : launch_mma<HD, false>(p, cluster, out, ldo, s);
+      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight).
+      const int warps = cluster && rows * p.max_splits <= 148 ? 8 : 4;
+      p.split_shift = log2_of(p.max_splits);
+      // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so
+      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > 296;
+      if (p.page_tokens % 16 == 0 && !p.ahead.any())
+        return G == 8 ? launch_mma<HD, true, true>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, true>(p, cluster, warps, out, ldo, s);
+      return G == 8 ? launch_mma<HD, true, false>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, false>(p, cluster, warps, out, ldo, s);
     }
   }
   switch (G) {
@@ -650,7 +757,7 @@ extern "C" int ifab_gqa_window_attention(const void* q, long ldq, const void* k_
   if ((uint64_t)T * Hq * max_splits * (head_dim + 2) * sizeof(float) > scratch_bytes) return -5;
   GqaParams p{(const bf16*)q, ldq, (const bf16*)k_cache, (const bf16*)v_cache, positions, slots, page_table,
               max_pages, page_tokens, num_pages, scale, window, T, Hq, Hkv, keys_per_split, max_splits, scratch, status, sink, (const bf16*)gate, ldg,
-              gate_act, gate_per_head, {cap, slopes, chunked}, ahead, factor};
+              gate_act, gate_per_head, {cap, slopes, chunked}, ahead, factor, 0, Hq / Hkv, log2_of(page_tokens), -1};
   cudaStream_t s = (cudaStream_t)stream;
   switch (head_dim) {
     case 64: return dispatch_g<64>(p, (bf16*)out, ldo, s);

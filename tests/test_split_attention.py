@@ -177,3 +177,44 @@ def test_parts_are_f32_sums(kv, group, hd, n, kps, splits):
     # scores of up to 10 with a few roundings to 2^-24 of them, weights 2^-21 off at most: 4e-7 as f32 sums in any order are; where the tensor cores add up along a
     # whole row, cutting off, 6e-7 to 2e-6
     assert float((out - ref).norm() / ref.norm()) < 5.5e-7
+
+
+# tiles of sixteen positions in pages that hold a multiple of them (16, 32, 48) and in others (24); windows that begin inside a tile; more than 32 tiles a warp (one
+# split of 5000 keys); more CTAs than run at once, of rows of very different lengths (60 rows) and rows that are not there
+@pytest.mark.parametrize("page,kv,group,hd,contexts,window,splits", [
+    (16, 2, 4, 128, [5000], 0, 1), (32, 1, 8, 128, [5000, 40], 0, 1), (24, 2, 4, 128, [700, 33], 0, 8), (48, 2, 2, 64, [700, 48, 49], 0, 8),
+    (16, 4, 4, 128, [1000, 65, 64, 17, 16, 3], 65, 8), (32, 2, 8, 64, [200, 31, 33], 33, 8), (16, 4, 4, 128, [17 * i + 1 if i % 7 else 0 for i in range(60)], 0, 64),
+    (16, 4, 2, 64, [2000 - 30 * i for i in range(60)], 500, 8)])
+def test_pages_windows_and_order(page, kv, group, hd, contexts, window, splits):
+    from ironpangu_b200.ops.window_attn import gqa_window
+
+    g = torch.Generator(device="cuda").manual_seed(page + hd + len(contexts))
+    T, H = len(contexts), kv * group
+    most = (max(contexts) + page - 1) // page
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(BF16)
+    kc, vc, q = rand(T * most, page, kv, hd), rand(T * most, page, kv, hd), rand(T, H * hd)
+    table = torch.randperm(T * most, generator=g, device="cuda").int().view(T, most)
+    pos = torch.tensor([c - 1 for c in contexts], dtype=torch.int32, device="cuda")
+    slots = torch.arange(T, dtype=torch.int32, device="cuda")
+    for t, c in enumerate(contexts):                     # what a row does not see must not count, whatever it holds
+        if c and window and c > window:
+            gone = (c - window) // page
+            table[t, :gone] = -1
+        rest = torch.arange(c, most * page, device="cuda")
+        rows = table[t].long().clamp(min=0)[rest // page] * page + rest % page
+        kc.view(-1, kv, hd)[rows] = float("nan")
+        vc.view(-1, kv, hd)[rows] = float("nan")
+    out = torch.full((T, H * hd), 7.0, dtype=BF16, device="cuda")
+    scratch = torch.empty(T * H * 64 * (hd + 2), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gqa_window(q, kc, vc, pos, slots, table, heads=H, window=window or max(contexts), scale=hd ** -0.5, splits=splits, scratch=scratch, out=out, status_ptr=status.data_ptr())
+    for t, c in enumerate(contexts):
+        if c == 0:
+            assert bool((out[t] == 7).all())
+            continue
+        at = torch.arange(max(0, c - window) if window else 0, c, device="cuda")
+        rows = table[t].long()[at // page] * page + at % page
+        ref = _reference(q[t].view(H, hd), kc.view(-1, kv, hd)[rows], vc.view(-1, kv, hd)[rows], hd ** -0.5).reshape(-1)
+        # a rounding to bf16 (at most 2^-8 of the value); f32 scores, weights and sums (2^-18 of values up to 5 is ample)
+        torch.testing.assert_close(out[t].double(), ref, rtol=2 ** -8, atol=2e-5)
+    assert int(status) == 0
