@@ -1,6 +1,7 @@
 // Decode-time (M = 1..8 tokens per tile) linear layers for sm_100a.
 //
 //   gemv_kernel            y = act(norm(x) W^T) (+ residual)         column-parallel / replicated linears
+//   rows_kernel            the same as a stream through rings in shared memory (row_stream.cuh): the dense decoder's linears
 //   gemv_allreduce_kernel  y = sum_ranks(x_r W_r^T) + residual       row-parallel linear fused with a
 //                          one-shot all-reduce over NVLink peer memory (push partial tiles to every
 //                          peer, bounded flag wait, rank-ordered f32 sum) - no separate collective launch
@@ -9,6 +10,8 @@
 // HcclAllReduce (native/src/token_executor.h:374-404); here both are one kernel.
 #include "gemv.cuh"
 #include "oneshot_ar.cuh"
+#include "row_stream.cuh"
+#include "tc_common.cuh"
 #include "ifab_kernels.h"
 
 using namespace ifab;
@@ -139,6 +142,58 @@ int dispatch_rows(const GemvParams& p, cudaStream_t s) {
   }
 }
 
+// Shared memory of the two kinds: two CTAs with a norm never fit an SM together, nor three of any, but one with and one without do. A layer's linears alternate between
+// the kinds, so every SM has one CTA of each of two kernels; where two CTAs of a kernel fit, an SM that became free early took two and another one none (2B
+// layer 36 us).
+constexpr int SMEM_NORM = 126976, SMEM_PLAIN = 102912;
+template <int MR, bool GATED, bool NORM>
+using RowsStream = RowStream<MR, NORM ? (MR == 8 ? 10 : 12) : 8, NORM ? (MR == 8 ? 4 : 6) : (MR == 8 ? 3 : 5), MR == 8 ? 33792 : NORM ? 18432 : 13312, GATED>;
+
+// grid (a CTA for each SM, tiles of MR rows of x)
+template <int MR, bool GATED, bool NORM>
+__global__ void __launch_bounds__(RS_WARPS * 32, 2) rows_kernel(GemvParams p) {
+  using S = RowsStream<MR, GATED, NORM>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float sums[RS_WARPS * 8];
+  grid_dep_launch();
+  const int t0 = blockIdx.y * MR, T = min(MR, p.T - t0);
+  S stream;
+  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x)}, smem);
+  BfRows<MR, NORM> x{p.x + (long)t0 * p.ldx, p.ldx, p.norm_w, p.eps, p.zero_centered, T};
+  x.early(stream);
+  grid_dep_wait();
+  float first_res = 0.f;          // requested here: behind the sums it was one more trip to L2
+  int ft, fn;
+  if (!GATED && p.residual && stream.first_result(T, &ft, &fn)) first_res = __bfloat162float(p.residual[(long)(t0 + ft) * p.ldr + fn]);
+  x.prepare(stream, sums);
+  auto out = [&](int t, int n, float v, float u, bool first) {
+    if (GATED) {
+      const float g = bf16_round(v);
+      reinterpret_cast<bf16*>(p.y)[(long)(t0 + t) * p.ldy + n] = __float2bfloat16_rn(silu(g) * bf16_round(u));
+      return;
+    }
+    if (p.residual) v = bf16_round(v) + (first ? first_res : __bfloat162float(p.residual[(long)(t0 + t) * p.ldr + n]));
+    if (p.out_f32) reinterpret_cast<float*>(p.y)[(long)(t0 + t) * p.ldy + n] = v;
+    else reinterpret_cast<bf16*>(p.y)[(long)(t0 + t) * p.ldy + n] = __float2bfloat16_rn(v);
+  };
+  stream.run(x, T, out);
+}
+
+template <int MR, bool GATED, bool NORM>
+int launch_rows(const GemvParams& p, cudaStream_t s) {
+  constexpr int smem = NORM ? SMEM_NORM : SMEM_PLAIN;
+  static_assert(RowsStream<MR, GATED, NORM>::SMEM <= smem, "ring, sums and rows");
+  auto k = rows_kernel<MR, GATED, NORM>;
+  if (int rc = opt_in_smem(k, smem)) return rc;
+  if (int rc = (int)cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+  return launch_chain(k, dim3(tc::device_sms(), (p.T + MR - 1) / MR), dim3(RS_WARPS * 32), (size_t)smem, s, p);
+}
+template <int MR>
+int dispatch_rows_stream(const GemvParams& p, cudaStream_t s) {
+  if (p.mode) return p.norm_w ? launch_rows<MR, true, true>(p, s) : launch_rows<MR, true, false>(p, s);
+  return p.norm_w ? launch_rows<MR, false, true>(p, s) : launch_rows<MR, false, false>(p, s);
+}
+
 // ----------------------------------------------------------------------------------------------
 // Row-parallel linear + one-shot all-reduce (protocol in oneshot_ar.cuh).
 // Every CTA owns a slab of 8*R output columns for all T tokens; only same-index CTAs of the ranks
@@ -226,6 +281,16 @@ extern "C" int ifab_gemv_bf16(const void* x, long ldx, const void* w, const void
   if (T <= 2) return dispatch_rows<2>(p, s);
   if (T <= 4) return dispatch_rows<4>(p, s);
   return dispatch_rows<8>(p, s);
+}
+
+// The same by rings in shared memory (row_stream.cuh), for chains of kernels that leave L1 alone: a ring wants most of an SM's memory as shared memory, and kernels that
+// keep 128 KB of loads in flight in registers (the experts' and the form above) lose a quarter of their rate beside it. x, w and norm_w on 16 bytes.
+extern "C" int ifab_gemv_rows_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, int zero_centered, const void* residual, long ldr, void* y,
+                                   long ldy, int out_f32, int T, int N, int K, int mode, void* stream) {
+  const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w;
+  if (T < 1 || N < 1 || K < 8 || K % 8 != 0 || ldx % 8 != 0 || bits % 16 != 0 || mode < 0 || mode > 1 || (mode && (residual || out_f32))) return -1;
+  GemvParams p{(const bf16*)x, ldx, (const bf16*)w, (const bf16*)norm_w, eps, zero_centered, (const bf16*)residual, ldr, y, ldy, out_f32, T, N, K, mode};
+  return T <= 2 ? dispatch_rows_stream<2>(p, (cudaStream_t)stream) : dispatch_rows_stream<8>(p, (cudaStream_t)stream);
 }
 
 extern "C" int ifab_gemv_allreduce_bf16(const void* x, long ldx, const void* w, const void* residual, long ldr,

@@ -19,6 +19,8 @@
 #include "oneshot_ar.cuh"
 #include "moe_select.cuh"
 #include "rope.cuh"
+#include "row_stream.cuh"
+#include "tc_common.cuh"
 #include "ifab_kernels.h"
 
 using namespace ifab;
@@ -493,58 +495,57 @@ __device__ __forceinline__ void finish_argmax(const HeadParams& p, int* is_last)
   }
 }
 
-template <int T, int R>
-__global__ void __launch_bounds__(256) lm_head_argmax_kernel(HeadParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* xs = reinterpret_cast<bf16*>(smem_raw);
-  __shared__ float red[T * 33];
+// The head as a stream through rings (row_stream.cuh), a CTA an SM: no more CTAs than run at once, so no wave ends with an SM idle and the partial maxima are few.
+// One row of 151936 x 2048 (622 MB) 104.4 -> 103 us alone; behind a step's kernels, whose end it fills its rings under, 117 -> 104.
+constexpr int HEAD_SMEM = 126976;
+template <int T, bool NORM>
+using HeadStream = RowStream<T <= 2 ? 2 : 8, T <= 2 ? 12 : 10, T <= 2 ? 6 : 4, T <= 2 ? 18432 : 33792, false>;
+template <int T, bool NORM>
+__global__ void __launch_bounds__(256, 1) lm_head_argmax_kernel(HeadParams p) {
+  using S = HeadStream<T, NORM>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float sums[RS_WARPS * 8];
   __shared__ float bestv[8][T];
   __shared__ int besti[8][T];
   __shared__ int is_last;
   grid_dep_launch();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (blockIdx.x * 8 + warp) * R;
-  const bf16* rows[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) rows[r] = (n0 + r < p.V) ? p.w + (size_t)(n0 + r) * p.K : nullptr;
-  RowBatch<R> pf;
-  prefetch_rows<R>(rows, p.K, pf);
-  request_gain(p.norm_w, p.K);
+  S stream;
+  stream.start(RowShare{p.w, p.V, p.K, (int)((long)p.V * blockIdx.x / gridDim.x), (int)((long)p.V * (blockIdx.x + 1) / gridDim.x)}, smem);
+  BfRows<T <= 2 ? 2 : 8, NORM> x{p.x, p.ldx, p.norm_w, p.eps, 0, p.T};
+  x.early(stream);
   grid_dep_wait();
-  stage_x<T>(xs, p.x, p.ldx, 0, p.T, p.K, p.norm_w, p.eps, false, red);
-  {
-    float acc[R][T];
+  x.prepare(stream, sums);
+  float bv[T];
+  int bi[T];
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+  for (int t = 0; t < T; ++t) bv[t] = -INFINITY, bi[t] = 0x7fffffff;
+  auto out = [&](int t, int n, float v, float, bool) {        // a thread's columns of a row ascend
+    if (p.cap > 0.f) v = soft_limit<true>(v, p.cap);
+    if (p.logits) p.logits[(size_t)t * p.V + n] = v;
 #pragma unroll
-      for (int t = 0; t < T; ++t) acc[r][t] = 0.f;
-    warp_rows_dot<T, R>(rows, xs, p.K, acc, pf);
-    warp_reduce_acc<T, R>(acc);
-    if (lane == 0) {
+    for (int i = 0; i < T; ++i)
+      if (i == t && v > bv[i]) bv[i] = v, bi[i] = p.vocab_offset + n;
+  };
+  stream.run(x, p.T, out);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        float bv = -INFINITY;
-        int bi = 0x7fffffff;
+  for (int t = 0; t < T; ++t) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (n0 + r >= p.V) continue;
-          if (p.cap > 0.f) acc[r][t] = soft_limit<true>(acc[r][t], p.cap);
-          if (p.logits && t < p.T) p.logits[(size_t)t * p.V + n0 + r] = acc[r][t];
-          if (acc[r][t] > bv) { bv = acc[r][t]; bi = p.vocab_offset + n0 + r; }
-        }
-        bestv[warp][t] = bv;
-        besti[warp][t] = bi;
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv[t], o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi[t], o);
+      if (ov > bv[t] || (ov == bv[t] && oi < bi[t])) bv[t] = ov, bi[t] = oi;
     }
+    if (lane == 0) bestv[warp][t] = bv[t], besti[warp][t] = bi[t];
   }
   __syncthreads();
   if (threadIdx.x < T) {
     const int t = threadIdx.x;
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
+    float v = -INFINITY;
+    int id = 0x7fffffff;
     for (int w = 0; w < 8; ++w)
-      if (bestv[w][t] > bv || (bestv[w][t] == bv && besti[w][t] < bi)) { bv = bestv[w][t]; bi = besti[w][t]; }
-    p.partial[(size_t)blockIdx.x * T + t] = make_float2(bv, __int_as_float(bi));
+      if (bestv[w][t] > v || (bestv[w][t] == v && besti[w][t] < id)) v = bestv[w][t], id = besti[w][t];
+    p.partial[(size_t)blockIdx.x * T + t] = make_float2(v, __int_as_float(id));
   }
   finish_argmax<T>(p, &is_last);
 }
@@ -574,16 +575,24 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(HeadParams p) {
   finish_argmax<8>(p, &is_last);
 }
 
-// what either form of the head asks of its sizes and of the room for the partial maxima: that of the kernel above
-template <int T, int R>
-int head_fits(const HeadParams& p, uint64_t partial_bytes) {
-  if (int rc = opt_in_smem(lm_head_argmax_kernel<T, R>, (size_t)T * p.K * sizeof(bf16))) return rc;
-  return (uint64_t)((p.V + 8 * R - 1) / (8 * R)) * T * sizeof(float2) > partial_bytes ? -5 : 0;
+// What either form of the head asks of its sizes and of the room for the partial maxima: a place a token for every `rows` rows of the matrix
+int head_fits(const HeadParams& p, int T, int rows, uint64_t partial_bytes) {
+  if ((size_t)T * (p.K * sizeof(bf16) + 33 * 4 + 64) > 232448) return (int)cudaErrorInvalidValue;
+  return (uint64_t)((p.V + rows - 1) / rows) * T * sizeof(float2) > partial_bytes ? -5 : 0;
 }
-template <int T, int R>
-int launch_head(const HeadParams& p, uint64_t partial_bytes, cudaStream_t s) {
-  if (int rc = head_fits<T, R>(p, partial_bytes)) return rc;
-  return launch_chain(lm_head_argmax_kernel<T, R>, dim3((p.V + 8 * R - 1) / (8 * R)), dim3(256), (size_t)T * p.K * sizeof(bf16), s, p);
+template <int T, bool NORM>
+int launch_head(const HeadParams& p, int rows, cudaStream_t s) {
+  static_assert(HeadStream<T, NORM>::SMEM <= HEAD_SMEM, "ring, sums and rows");
+  auto k = lm_head_argmax_kernel<T, NORM>;
+  if (int rc = opt_in_smem(k, HEAD_SMEM)) return rc;
+  if (int rc = (int)cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+  return launch_chain(k, dim3(min(tc::device_sms(), (p.V + rows - 1) / rows)), dim3(256), (size_t)HEAD_SMEM, s, p);
+}
+template <int T>
+int dispatch_head(const HeadParams& p, uint64_t partial_bytes, cudaStream_t s) {
+  constexpr int rows = T <= 4 ? 32 : 16;
+  if (int rc = head_fits(p, T, rows, partial_bytes)) return rc;
+  return p.norm_w ? launch_head<T, true>(p, rows, s) : launch_head<T, false>(p, rows, s);
 }
 
 }  // namespace
@@ -692,7 +701,7 @@ extern "C" int ifab_lm_head_capped_argmax(const void* x, long ldx, const void* n
   const uint64_t maxima = (uint64_t)ctas * 8 * sizeof(float2), rows = norm_w ? (uint64_t)T * K * sizeof(bf16) : 0;
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w | (uintptr_t)partial | (uintptr_t)(ldx * sizeof(bf16));
   if (T >= 3 && logits && maxima + rows <= partial_bytes && bits % 16 == 0) {
-    if (int rc = T <= 4 ? head_fits<4, 4>(p, partial_bytes) : head_fits<8, 2>(p, partial_bytes)) return rc;
+    if (int rc = T <= 4 ? head_fits(p, 4, 32, partial_bytes) : head_fits(p, 8, 16, partial_bytes)) return rc;
     const void* a = x;
     long lda = ldx;
     if (norm_w) {
@@ -703,8 +712,8 @@ extern "C" int ifab_lm_head_capped_argmax(const void* x, long ldx, const void* n
     if (int rc = ifab_gemm_fixed_bf16(a, lda, w, K, logits, V_local, 1, nullptr, 0, nullptr, 0, cap, T, V_local, K, fab->status, stream)) return rc;
     return launch_chain(argmax_rows_kernel, dim3(ctas), dim3(256), 0, s, p);
   }
-  if (T <= 1) return launch_head<1, 4>(p, partial_bytes, s);
-  if (T <= 2) return launch_head<2, 4>(p, partial_bytes, s);
-  if (T <= 4) return launch_head<4, 4>(p, partial_bytes, s);
-  return launch_head<8, 2>(p, partial_bytes, s);
+  if (T <= 1) return dispatch_head<1>(p, partial_bytes, s);
+  if (T <= 2) return dispatch_head<2>(p, partial_bytes, s);
+  if (T <= 4) return dispatch_head<4>(p, partial_bytes, s);
+  return dispatch_head<8>(p, partial_bytes, s);
 }

@@ -55,6 +55,8 @@ int ifab_rmsnorm_bf16(const void* x, long ldx, const void* w, void* y, long ldy,
 int ifab_gemv_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, int zero_centered,
                    const void* residual, long ldr, void* y, long ldy, int out_f32, int T, int N, int K, int mode,
                    void* stream);
+int ifab_gemv_rows_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, int zero_centered, const void* residual, long ldr, void* y, long ldy,
+                        int out_f32, int T, int N, int K, int mode, void* stream);
 int ifab_gemv_allreduce_bf16(const void* x, long ldx, const void* w, const void* residual, long ldr, void* y, long ldy,
                              void* y_f32, int T, int N, int K, const IfabFabric* fab, void* stream);
 

@@ -178,7 +178,7 @@ class DenseDecoder:
     def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor) -> None:
         """``x += a @ w.T`` summed over the ranks (one rank: the same bits without the call counter)."""
         if self.fabric.world == 1:
-            K.gemv(a, w, residual=x, out=x)
+            K.gemv(a, w, residual=x, out=x, rings=True)
         else:
             K.gemv_allreduce(a, w, self.fabric, residual=x, out=x)
 
@@ -191,7 +191,7 @@ class DenseDecoder:
         for l in range(c.layers):
             p = f"layers.{l}."
             qkv = self.qkv[:T]
-            K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv)
+            K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv, rings=fab.world == 1)
             K.gqa_rope_kv_write(qkv, pos, slot, self.page_table, self.k_cache[l], self.v_cache[l], heads=self.hq,
                                 kv_heads=self.hk, head_dim=c.head_dim, theta=c.theta, status_ptr=st)
             K.gqa_decode_attention(qkv, self.k_cache[l], self.v_cache[l], pos, slot, self.page_table, heads=self.hq,
@@ -199,7 +199,7 @@ class DenseDecoder:
                                    keys_per_split=self.kps, max_splits=self.max_splits, scratch=self.scratch,
                                    out=self.attn[:T], status_ptr=st)
             self._row_parallel(self.attn[:T], w[p + "o_proj"], x)
-            K.gemv(x, w[p + "gate_up"], norm_w=w[p + "ffn_norm"], eps=c.eps, swiglu=True, out=self.act[:T])
+            K.gemv(x, w[p + "gate_up"], norm_w=w[p + "ffn_norm"], eps=c.eps, swiglu=True, out=self.act[:T], rings=fab.world == 1)
             self._row_parallel(self.act[:T], w[p + "down"], x)
         if sample:
             K.lm_head_argmax(x, w["lm_head"], fab, norm_w=w["final_norm"], eps=c.eps, vocab_offset=self.rank * self.vl,

@@ -117,9 +117,17 @@ class DensePrefill:
         self.slots[:m].copy_(slots)
         x = self._layers_graphed(m)
         xs = x.index_select(0, select)
+        if xs.shape[0] <= 2 and self._few(xs.shape[0], d.w["lm_head"]):      # 151936 x 2048, 8 rows: 146 us so, 104 as norm and product
+            self.launches += 1
+            return K.gemv(xs, d.w["lm_head"], norm_w=d.w["final_norm"], eps=c.eps, out_f32=True, rings=True)
         xn = K.rmsnorm(xs, d.w["final_norm"], c.eps)
         self.launches += 2
         return G.gemm(xn, d.w["lm_head"], out_f32=True, status_ptr=d.fabric.desc.status, fixed=True)
+
+    def _few(self, m: int, w: torch.Tensor) -> bool:
+        """Whether ``m`` rows go through the streaming linears (one tile of eight rows, which the weights pass once, and the norm ahead of them in the same
+        launch): 2B model, 8 rows, a layer's four linears and two norms 40 us as products, 28 so."""
+        return m <= 8 and self.dec.fabric.world == 1 and w.is_contiguous()
 
     def _layers_graphed(self, m: int) -> torch.Tensor:
         if m > self.graph_rows_max:
@@ -164,23 +172,34 @@ class DensePrefill:
         scale = 1.0 / math.sqrt(c.head_dim)
         for l in range(c.layers):
             p = f"layers.{l}."
-            K.rmsnorm(x, w[p + "attn_norm"], c.eps, out=h)
-            qkv = G.gemm(h, w[p + "qkv"], out=self.qkv[:m], status_ptr=st, fixed=True)
+            if self._few(m, w[p + "qkv"]):
+                qkv = K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=self.qkv[:m], rings=True)
+            else:
+                K.rmsnorm(x, w[p + "attn_norm"], c.eps, out=h)
+                qkv = G.gemm(h, w[p + "qkv"], out=self.qkv[:m], status_ptr=st, fixed=True)
             K.gqa_rope_kv_write(qkv, pos, sl, d.page_table, d.k_cache[l], d.v_cache[l], heads=d.hq, kv_heads=d.hk,
                                 head_dim=c.head_dim, theta=c.theta, status_ptr=st)
             self._attention(l, m, qkv, pos, sl, scale, st)
             if fab.world > 1:
                 G.gemm_allreduce(self.attn[:m], w[p + "o_proj"], fab, self._sym_rows(m), residual=x)
+            elif self._few(m, w[p + "o_proj"]):
+                K.gemv(self.attn[:m], w[p + "o_proj"], residual=x, out=x, rings=True)
             else:
                 G.gemm(self.attn[:m], w[p + "o_proj"], residual=x, out=x, status_ptr=st, fixed=True)
-            K.rmsnorm(x, w[p + "ffn_norm"], c.eps, out=h)
-            if m >= 256:
+            few = self._few(m, w[p + "gate_up"])
+            if not few:
+                K.rmsnorm(x, w[p + "ffn_norm"], c.eps, out=h)
+            if few:
+                K.gemv(x, w[p + "gate_up"], norm_w=w[p + "ffn_norm"], eps=c.eps, swiglu=True, out=self.act[:m], rings=True)
+            elif m >= 256:
                 # whole 256-row tile pairs: the packed gate | up projection and its activation on CTA pairs, one persistent launch
                 G.gemm_swiglu(h, w[p + "gate_up"], out=self.act[:m], status_ptr=st)
             else:
                 N.gated_linear(h, w[p + "gate_up"], N.SILU, self.act[:m], status_ptr=st, fixed=True)
             if fab.world > 1:
                 G.gemm_allreduce(self.act[:m], w[p + "down"], fab, self._sym_rows(m), residual=x)
+            elif self._few(m, w[p + "down"]):
+                K.gemv(self.act[:m], w[p + "down"], residual=x, out=x, rings=True)
             else:
                 G.gemm(self.act[:m], w[p + "down"], residual=x, out=x, status_ptr=st, fixed=True)
         self.launches = 1 + c.layers * (8 + 2 * ((m + self.QC - 1) // self.QC))

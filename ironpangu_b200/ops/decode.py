@@ -63,18 +63,20 @@ def swiglu_rows(gu: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.T
 
 def gemv(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-5,
          zero_centered: bool = False, residual: Optional[torch.Tensor] = None, swiglu: bool = False,
-         out_f32: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+         out_f32: bool = False, out: Optional[torch.Tensor] = None, rings: bool = False) -> torch.Tensor:
     """``y = act(norm(x) @ w.T) (+ residual)`` for a few tokens (decode).
 
     ``w`` is ``[N, K]`` (or ``[2N, K]`` = gate rows then up rows when ``swiglu``). ``norm_w`` fuses an
-    RMSNorm of ``x`` into the prologue."""
+    RMSNorm of ``x`` into the prologue. ``rings``: the weights stream through shared memory, eight rows as fast as one; for steps without
+    kernels that stream through L1 (expert weights)."""
     T, K = x.shape
     rows = w.shape[0]
     assert w.shape[1] == K and w.is_contiguous() and w.dtype == BF16 and x.dtype == BF16
     N = rows // 2 if swiglu else rows
     if out is None:
         out = torch.empty(T, N, dtype=torch.float32 if out_f32 else BF16, device=x.device)
-    check(_lib.load().ifab_gemv_bf16(x.data_ptr(), _rows(x), w.data_ptr(), _ptr(norm_w), eps, int(zero_centered),
+    fn = _lib.load().ifab_gemv_rows_bf16 if rings else _lib.load().ifab_gemv_bf16
+    check(fn(x.data_ptr(), _rows(x), w.data_ptr(), _ptr(norm_w), eps, int(zero_centered),
                                      _ptr(residual), _rows(residual) if residual is not None else 0, out.data_ptr(),
                                      _rows(out), int(out.dtype == torch.float32), T, N, K, int(swiglu), _stream()), "gemv")
     return out

@@ -416,6 +416,8 @@ class PlanEngine:
             width = max(self._gqa_packed[k].shape[0] for k in self.gqa_groups)
             self._gqa_qkv = torch.empty(self.T, width, dtype=BF16, device=self.fabric.device)     # read by attention while the workspace holds its splits
         self.fused_gqa = bool(self.gqa_groups) and self._fused_gqa_option is not False
+        # programs of grouped-query layers and linears: the hand-wired decoder's form of the linears (and its bits)
+        self._rings = self.world == 1 and bool(self.gqa_groups) and not any(i["op"].startswith(("moe_", "latent_", "mla_")) for i in self.ins)
         self.fused_ctx_limit = 2048
         can_head = bool(self.head_groups) and all(g["ok"] for g in self.head_groups.values())
         self.fused_head = (can_head and self.max_context <= self.fused_ctx_limit) if fused_head is None else (bool(fused_head) and can_head)
@@ -721,7 +723,7 @@ class PlanEngine:
                 wq = self._gqa_packed[k]
                 qkv = self._gqa_qkv[:T, :wq.shape[0]]
                 kc, vc = self._kv_of[g["cache"]]
-                K.gemv(val(g["x"]), wq, norm_w=self._param(g["norm"], g["norm_optional"]) if g["norm"] else None, eps=g["eps"], out=qkv)
+                K.gemv(val(g["x"]), wq, norm_w=self._param(g["norm"], g["norm_optional"]) if g["norm"] else None, eps=g["eps"], out=qkv, rings=self._rings)
                 K.gqa_rope_kv_write(qkv, pos, slot, self.page_table, kc, vc, heads=H, kv_heads=KVH, head_dim=hd, rotary_dim=g["rotary_dim"],
                                     theta=g["theta"], status_ptr=st)
                 K.gqa_decode_attention(qkv, kc, vc, pos, slot, self.page_table, heads=H, kv_heads=KVH, head_dim=hd, scale=float(a["scale"]),
@@ -749,10 +751,13 @@ class PlanEngine:
                 V[k] = src[:, s:s + w]
             elif op == "linear":
                 name = a["weight"] + ("|" + a["paired_weight"] if "paired_weight" in a else "")
-                K.gemv(val(ins[0]), self._param(name), norm_w=norm_w, eps=eps, swiglu=a.get("activation") == "swiglu", out=val(k))
+                K.gemv(val(ins[0]), self._param(name), norm_w=norm_w, eps=eps, swiglu=a.get("activation") == "swiglu", out=val(k), rings=self._rings)
             elif op == "linear_allreduce":
                 res = val(ins[1]) if len(ins) > 1 else None
-                K.gemv_allreduce(val(ins[0]), self._param(a["weight"]), fab, residual=res, out=val(k))
+                if self._rings:
+                    K.gemv(val(ins[0]), self._param(a["weight"]), residual=res, out=val(k), rings=True)
+                else:
+                    K.gemv_allreduce(val(ins[0]), self._param(a["weight"]), fab, residual=res, out=val(k))
             elif op == "norm":
                 K.rmsnorm(val(ins[0]), self._param(a["weight"]), float(a["eps"]), out=val(k))
             elif op == "mla_kv_write":

@@ -1,0 +1,66 @@
+"""Linears of one to eight rows as a stream through rings, at the edges of their shares: more SMs than rows of the matrix, remainders of eight rows, of a warp's columns and of
+a ring; rows of x that fit shared memory and that do not."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+@pytest.mark.parametrize("gated,norm", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("N,K,T", [(1, 8, 2), (7, 520, 1), (147, 1024, 8), (149, 1032, 3), (2368, 1544, 5), (2999, 2048, 8), (5000, 264, 2), (300, 6144, 8), (300, 16384, 8), (64, 16392, 1), (9000, 512, 11)])
+def test_shares_and_remainders(N, K, T, gated, norm):
+    from ironpangu_b200.ops import decode as D
+
+    g = torch.Generator(device="cuda").manual_seed(N + K + T)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w = rand(T, K + 8).to(BF16)[:, :K], (rand(N * (1 + gated), K) * K ** -0.5).to(BF16)
+    gain = (rand(K) * 0.1 + 1).to(BF16) if norm else None
+    operand = x.float()
+    if norm:
+        operand = (operand * torch.rsqrt(operand.square().mean(-1, keepdim=True) + 1e-6) * gain.float()).to(BF16).float()
+    ref = operand.double() @ w.double().T
+    # f32 sums; a norm in f32 may round an operand to the next bf16 value (2^-8 of it) in another order of its sum: a few of K
+    slack = float((operand.double().abs() @ w.double().abs().T).max()) * (2.0 ** -20 + (2.0 ** -8 * K ** -0.5 if norm else 0.0)) + 1e-6
+    if gated:
+        out = torch.full((T + 1, N + 3), 7.0, dtype=BF16, device="cuda")
+        D.gemv(x, w, norm_w=gain, eps=1e-6, swiglu=True, out=out[:T, :N], rings=True)
+        gate, up = ref[:, :N], ref[:, N:]
+        want = torch.nn.functional.silu(gate) * up
+        bound = 1.02 * 2.0 ** -8 * (1.1 * gate.abs() * up.abs() + 2 * want.abs()) + slack * (2 * up.abs() + 2 * gate.abs() + 1)
+        assert bool(((out[:T, :N].double() - want).abs() <= bound).all())
+    else:
+        out = torch.full((T + 1, N + 3), 7.0, device="cuda")
+        D.gemv(x, w, norm_w=gain, eps=1e-6, out=out[:T, :N], rings=True)
+        torch.testing.assert_close(out[:T, :N].double(), ref, rtol=0, atol=slack)
+        res = rand(T, N).to(BF16)
+        y = res.clone()
+        D.gemv(x, w, norm_w=gain, eps=1e-6, residual=y, out=y, rings=True)          # in place
+        want = ref + res.double()
+        assert bool(((y.double() - want).abs() <= 2.0 ** -8 * (ref.abs() + want.abs()) + slack).all())
+    assert bool((out[T:] == 7).all()) and bool((out[:, N:] == 7).all())
+    alone = torch.cat([D.gemv(x[t:t + 1], w, norm_w=gain, eps=1e-6, swiglu=gated, rings=True) for t in range(T)])
+    assert torch.equal(D.gemv(x, w, norm_w=gain, eps=1e-6, swiglu=gated, rings=True), alone)          # the bits that a row has alone
+
+
+@pytest.mark.parametrize("T,V,K", [(1, 31, 64), (1, 33, 1032), (2, 5000, 512), (3, 700, 520), (8, 17, 64), (8, 9000, 4104)])
+def test_greedy_head(T, V, K):
+    from ironpangu_b200.ops import decode as D
+    from ironpangu_b200.parallel.fabric import Fabric
+
+    g = torch.Generator(device="cuda").manual_seed(T + V + K)
+    x, w = torch.randn(T, K, generator=g, device="cuda").to(BF16), (torch.randn(V, K, generator=g, device="cuda") * K ** -0.5).to(BF16)
+    w[V // 2] = w[0]                                     # equal logits: the lowest id
+    fab = Fabric(0, 1)
+    for keep in (True, False):
+        logits = torch.full((T, V), 7.0, device="cuda") if keep else None
+        ids = D.lm_head_argmax(x, w, fab, logits=logits)
+        ref = x.double() @ w.double().T
+        slack = float((x.double().abs() @ w.double().abs().T).max()) * 2.0 ** -20 + 1e-6
+        best = ref.max(-1).values
+        assert bool((best - ref.gather(1, ids.long()[:, None])[:, 0] <= 2 * slack).all())
+        assert not bool((ids == V // 2).any()) or V // 2 == 0
+        if keep:
+            torch.testing.assert_close(logits.double(), ref, rtol=0, atol=slack)
+    assert fab.status() == 0
+    fab.close()
