@@ -17,6 +17,8 @@
 #include "gemv.cuh"
 #include "moe_select.cuh"
 #include "rope.cuh"
+#include "row_stream.cuh"
+#include "tc_common.cuh"
 #include "ifab_kernels.h"
 
 using namespace ifab;
@@ -277,6 +279,76 @@ __global__ void __launch_bounds__(256) gemv_operand_kernel(Params p) {
   if (p.shared_w && lane == 0) p.shared_w[warp] = sigmoid_f32(__ldcg(logits + p.E));
 }
 
+// The same as a stream through rings (row_stream.cuh), one or two rows: for steps without kernels that stream through L1 (see there). The operand is staged by the form
+// above, so an output projection behind a group norm and a down projection fit an SM beside an input projection behind an output norm.
+// 2B falinex, one row, us from one kernel's end to the next's: input and up projections 8.4 -> 6.6, down projection 8.0 -> 6.0, output projection behind a group norm
+// 5.9 -> 4.6.
+constexpr int OPERAND_SMEM = 126976, PLAIN_SMEM = 102912;
+template <int PRO>
+using OperandStream = RowStream<2, PRO == POST ? 12 : 8, PRO == POST ? 6 : 5, PRO == POST ? 18432 : 16768, false>;
+template <int T>
+struct StagedRows {
+  struct Raw {};
+  uint32_t at;
+  template <class S>
+  __device__ __forceinline__ void load(const S&, int, Raw&) const {}
+  template <class S>
+  __device__ __forceinline__ void operand(const S& s, int k, const Raw&, uint4 (&a)[RS_STEPS]) const {
+    const int t = s.lane >> 2, c0 = k * s.chunk + s.col;
+#pragma unroll
+    for (int u = 0; u < RS_STEPS; ++u) {
+      a[u] = make_uint4(0, 0, 0, 0);
+      if (t < T && u < s.steps && c0 + s.at_step(u) < s.s.K) a[u] = ld_shared16(at + (t * s.s.K + c0 + s.at_step(u)) * 2);
+    }
+  }
+};
+
+template <int T, int PRO>
+__global__ void __launch_bounds__(256, 2) rows_operand_kernel(Params p) {
+  using S = OperandStream<PRO>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float red[T * 8];
+  grid_dep_launch();
+  S stream;
+  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x)}, smem);
+  auto out = [&](int t, int n, float v, float, bool) {
+    if (p.out_bias) v += p.out_bias[n];
+    if (p.addend) v += p.addend[(long)t * p.ldadd + n];
+    v = activate<true>(v, p.act);
+    if (p.out_f32) reinterpret_cast<float*>(p.z)[(long)t * p.ldz + n] = v;
+    else reinterpret_cast<bf16*>(p.z)[(long)t * p.ldz + n] = __float2bfloat16_rn(v);
+  };
+  if constexpr (PRO == PLAIN) {
+    BfRows<2, false> x{p.x, p.ldx, nullptr, 0.f, 0, p.T};
+    x.early(stream);
+    grid_dep_wait();
+    x.prepare(stream, red);
+    stream.run(x, p.T, out);
+  } else {
+    grid_dep_wait();
+    bf16* xs = reinterpret_cast<bf16*>(smem + S::RING + S::RED);
+    stage_operand<T, PRO>(p, xs, reinterpret_cast<float*>(xs + (long)T * p.K), red, nullptr, 0);
+    StagedRows<T> x{smem_addr(xs)};
+    stream.run(x, p.T, out);
+  }
+}
+template <int T, int PRO>
+int launch_rings(const Params& p, cudaStream_t s) {
+  constexpr int smem = PRO == POST ? OPERAND_SMEM : PLAIN_SMEM;
+  static_assert(OperandStream<PRO>::SMEM <= smem, "ring, sums and rows");
+  auto k = rows_operand_kernel<T, PRO>;
+  if (int rc = opt_in_smem(k, smem)) return rc;
+  if (int rc = (int)cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+  return launch_chain(k, dim3(tc::device_sms()), dim3(256), (size_t)smem, s, p);
+}
+// what the form above takes: one or two rows, of which normalised operands fit; no second norm; matrices and plain rows on 16 bytes
+template <int PRO>
+bool rings_take(const Params& p) {
+  const size_t operand = (size_t)p.T * p.K * sizeof(bf16) + (PRO == GROUP ? (size_t)p.T * p.groups : 8) * sizeof(float);
+  return p.T >= 1 && p.T <= 2 && p.N >= 1 && p.K >= 8 && p.K % 8 == 0 && !p.norm2_w && (reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.x)) % 16 == 0 &&
+         (PRO == PLAIN || operand <= (PRO == POST ? 18432 : 16768));
+}
+
 // The front of a layer with parallel sublayers. CTAs 0 .. router_ctas - 1 hold the router's rows (f32 logits; the last of them selects), the
 // others warps of R weight rows: the projection (`w`, N rows, bf16 result with out_bias), then R / 2 pairs of the gated unit (gate rows
 // [0, F), up rows [F, 2 F) of w_gu).
@@ -386,7 +458,8 @@ int by_rows(const Params& p, cudaStream_t s) {
   return launch_one<T, 1, PRO>(p, s);
 }
 template <int PRO>
-int dispatch(const Params& p, cudaStream_t s) {
+int dispatch(const Params& p, cudaStream_t s, bool rings = false) {
+  if (rings && rings_take<PRO>(p)) return p.T == 1 ? launch_rings<1, PRO>(p, s) : launch_rings<2, PRO>(p, s);
   if (p.T < 1 || p.N < 1 || p.K < 8 || p.K % 8) return -1;
   if (p.T <= 1) return by_rows<1, PRO>(p, s);
   if (p.T <= 2) return by_rows<2, PRO>(p, s);
@@ -396,14 +469,24 @@ int dispatch(const Params& p, cudaStream_t s) {
 
 }  // namespace
 
-extern "C" int ifab_gemv_post_norm(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
+namespace {
+int run_gemv_post_norm(bool rings, const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
                                    const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
   if (ldy % 4 || ldx % 4 || x_in == x_out) return -1;
   Params p{};
   p.norm2_w = norm2_w;
   p.y = y; p.ldy = ldy; p.norm_w = norm_w; p.eps = eps; p.x_in = x_in; p.x_out = x_out; p.ldr = ldx;
   p.w = (const bf16*)w; p.z = z; p.ldz = ldz; p.out_f32 = out_f32; p.act = act; p.T = T; p.N = N; p.K = K;
-  return dispatch<POST>(p, (cudaStream_t)stream);
+  return dispatch<POST>(p, (cudaStream_t)stream, rings);
+}
+}  // namespace
+extern "C" int ifab_gemv_post_norm(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
+                                   const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
+  return run_gemv_post_norm(false, y, ldy, norm_w, norm2_w, eps, x_in, x_out, ldx, w, z, ldz, out_f32, act, T, N, K, stream);
+}
+extern "C" int ifab_gemv_post_norm_rows(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
+                                   const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
+  return run_gemv_post_norm(true, y, ldy, norm_w, norm2_w, eps, x_in, x_out, ldx, w, z, ldz, out_f32, act, T, N, K, stream);
 }
 // The router of a sublayer pair: x_out as above, xn = bf16(rms(x_out) * norm2_w), f32 logits [T, N] = xn w^T (T <= 8), then ids / wts of the chosen
 // of the first E columns and, when N = E + 1, shared_w = sigmoid(logits[:, E]). ticket: one zeroed word (left zero again)
@@ -421,23 +504,43 @@ extern "C" int ifab_router_post_norm(const float* y, long ldy, const float* norm
   p.w = (const bf16*)w; p.z = logits; p.ldz = ldz; p.out_f32 = 1; p.act = 0; p.T = T; p.N = N; p.K = K;
   return dispatch<POST>(p, (cudaStream_t)stream);
 }
-extern "C" int ifab_gemv_group_norm(const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act,
+namespace {
+int run_gemv_group_norm(bool rings, const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act,
                                     const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
   if (ldo % 4 || groups < 1 || groups > 1024 || K % groups) return -1;
   Params p{};
   p.o = o; p.ldo = ldo; p.gain = gain; p.eps = eps; p.groups = groups; p.gate = (const bf16*)gate; p.ldg = ldg; p.gate_act = gate_act;
   p.w = (const bf16*)w; p.z = z; p.ldz = ldz; p.out_f32 = out_f32; p.act = act; p.T = T; p.N = N; p.K = K;
-  return dispatch<GROUP>(p, (cudaStream_t)stream);
+  return dispatch<GROUP>(p, (cudaStream_t)stream, rings);
+}
+}  // namespace
+extern "C" int ifab_gemv_group_norm(const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act,
+                                    const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
+  return run_gemv_group_norm(false, o, ldo, gain, eps, groups, gate, ldg, gate_act, w, z, ldz, out_f32, act, T, N, K, stream);
+}
+extern "C" int ifab_gemv_group_norm_rows(const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act,
+                                    const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream) {
+  return run_gemv_group_norm(true, o, ldo, gain, eps, groups, gate, ldg, gate_act, w, z, ldz, out_f32, act, T, N, K, stream);
 }
 // z = act(x w^T + bias + addend); bias [N] and addend (f32 rows, which may be z) or null
-extern "C" int ifab_gemv_act(const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T,
+namespace {
+int run_gemv_act(bool rings, const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T,
                              int N, int K, void* stream) {
   if (ldx % 8) return -1;
   Params p{};
   p.out_bias = bias; p.addend = addend; p.ldadd = ldadd;
   p.x = (const bf16*)x; p.ldx = ldx;
   p.w = (const bf16*)w; p.z = z; p.ldz = ldz; p.out_f32 = out_f32; p.act = act; p.T = T; p.N = N; p.K = K;
-  return dispatch<PLAIN>(p, (cudaStream_t)stream);
+  return dispatch<PLAIN>(p, (cudaStream_t)stream, rings);
+}
+}  // namespace
+extern "C" int ifab_gemv_act(const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T,
+                             int N, int K, void* stream) {
+  return run_gemv_act(false, x, ldx, w, bias, addend, ldadd, z, ldz, out_f32, act, T, N, K, stream);
+}
+extern "C" int ifab_gemv_act_rows(const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T,
+                             int N, int K, void* stream) {
+  return run_gemv_act(true, x, ldx, w, bias, addend, ldadd, z, ldz, out_f32, act, T, N, K, stream);
 }
 
 // The front of a layer with parallel sublayers for T <= 2 rows: x_out = x_in (+ y) (+ extra); h = bf16(rms(x_out) * norm_w), also stored to xn when given;

@@ -327,14 +327,20 @@ int ifab_gate_rows(const void* o, long ldo, int head_stride, const void* gate, l
  * z = act(bf16(x_out) W^T), or of bf16(rms(x_out) * norm2_w) when norm2_w is given; ..._group_norm: z = act(bf16((o / rms per group [* gain]) * gate_act(gate)) W^T) */
 int ifab_gemv_post_norm(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
                         const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream);
+int ifab_gemv_post_norm_rows(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx,
+                        const void* w, void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream);
 /* the same with both norms as a router: xn = the operand, f32 logits, then ids / wts (and shared_w = sigmoid(logits[:, E]) when N = E + 1), T <= 8 */
 int ifab_router_post_norm(const float* y, long ldy, const float* norm_w, const float* norm2_w, float eps, const float* x_in, float* x_out, long ldx, void* xn,
                           long ldn, const void* w, float* logits, long ldz, const float* bias, int E, int topk, int scoring, int renorm, float scale,
                           int32_t* ids, float* wts, float* shared_w, uint32_t* ticket, int T, int N, int K, void* stream);
 int ifab_gemv_group_norm(const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act, const void* w,
                          void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream);
+int ifab_gemv_group_norm_rows(const float* o, long ldo, const float* gain, float eps, int groups, const void* gate, long ldg, int gate_act, const void* w,
+                         void* z, long ldz, int out_f32, int act, int T, int N, int K, void* stream);
 /* z = act(x W^T + bias + addend), bias and addend (f32 rows, may be z) or null */
 int ifab_gemv_act(const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T, int N,
+                  int K, void* stream);
+int ifab_gemv_act_rows(const void* x, long ldx, const void* w, const float* bias, const float* addend, long ldadd, void* z, long ldz, int out_f32, int act, int T, int N,
                   int K, void* stream);
 /* front of a layer with parallel sublayers, T <= 2: x_out = x_in (+ y) (+ extra), h = rms(x_out) * norm_w -> projection z = h W^T + bias, gated unit of
  * [gate | up] rows, router logits and selection */

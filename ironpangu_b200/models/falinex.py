@@ -421,21 +421,21 @@ class FalinexDecoder(StreamDecoder):
             mx = L["m"]
             hv, proj = mx.heads * mx.vdim, B.proj[:n]
             if owed is None:
-                N.gemv_act(xa, L["in"], proj)
+                N.gemv_act(xa, L["in"], proj, rings=True)
             else:
-                N.gemv_post_norm(y, owed, c.eps, x, x2, L["in"], proj)
+                N.gemv_post_norm(y, owed, c.eps, x, x2, L["in"], proj, rings=True)
                 x, x2 = x2, x
             self._mix(B, L, n, pos, slot, None, norm=False)
             if mx.recurrent:
-                N.gemv_group_norm(B.o[:n, :hv], proj[:, L["gate0"]:], L["gate_act"], c.eps, L["o"], y, L["groups"], L["gain"])
+                N.gemv_group_norm(B.o[:n, :hv], proj[:, L["gate0"]:], L["gate_act"], c.eps, L["o"], y, L["groups"], L["gain"], rings=True)
             else:
-                N.gemv_act(B.mixed[hv][:n], L["o"], y)
+                N.gemv_act(B.mixed[hv][:n], L["o"], y, rings=True)
             owed = L["norm1"]
             if L["ff"]:
                 act = B.act[L["ff"]][:n]
-                N.gemv_post_norm(y, owed, c.eps, x, x2, L["up"], act, "gelu_tanh")
+                N.gemv_post_norm(y, owed, c.eps, x, x2, L["up"], act, "gelu_tanh", rings=True)
                 x, x2 = x2, x
-                N.gemv_act(act, L["down"], y)
+                N.gemv_act(act, L["down"], y, rings=True)
                 owed = L["norm2"]
         N.post_norm_add(y, owed, c.eps, x, xa, self.final_norm)
 

@@ -110,32 +110,35 @@ def gate_rows(o: torch.Tensor, head_stride: int, gate: torch.Tensor, act: str, o
 
 
 def gemv_post_norm(y: torch.Tensor, norm_w: torch.Tensor, eps: float, x_in: torch.Tensor, x_out: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
-                   act: Optional[str] = None, next_norm: Optional[torch.Tensor] = None) -> None:
+                   act: Optional[str] = None, next_norm: Optional[torch.Tensor] = None, rings: bool = False) -> None:
     """``x_out = x_in + rms(y) * norm_w``; ``out = act(bf16(x_out) @ w.T)``, or of ``bf16(rms(x_out) * next_norm)``, in one launch (decode
-    rows)."""
+    rows). ``rings`` (here and below): one and two rows stream the weights through shared memory, for steps without kernels that stream through L1."""
     T, K = y.shape
     N = w.shape[0]
     assert w.shape[1] == K and w.is_contiguous() and x_in.stride(0) == x_out.stride(0)
-    check(_lib.load().ifab_gemv_post_norm(y.data_ptr(), y.stride(0), norm_w.data_ptr(), _p(next_norm), eps, x_in.data_ptr(), x_out.data_ptr(), x_in.stride(0), w.data_ptr(),
+    fn = _lib.load().ifab_gemv_post_norm_rows if rings else _lib.load().ifab_gemv_post_norm
+    check(fn(y.data_ptr(), y.stride(0), norm_w.data_ptr(), _p(next_norm), eps, x_in.data_ptr(), x_out.data_ptr(), x_in.stride(0), w.data_ptr(),
                                           out.data_ptr(), out.stride(0), _f32(out), ACTIVATIONS[act], T, N, K, _s()), "gemv_post_norm")
 
 
 def gemv_group_norm(o: torch.Tensor, gate: torch.Tensor, gate_act: str, eps: float, w: torch.Tensor, out: torch.Tensor, groups: int,
-                    gain: Optional[torch.Tensor] = None) -> None:
+                    gain: Optional[torch.Tensor] = None, rings: bool = False) -> None:
     """``out = bf16((o / rms per group [* gain]) * gate_act(gate)) @ w.T`` in one launch (decode rows)."""
     T, K = o.shape
     N = w.shape[0]
     assert w.shape[1] == K and w.is_contiguous() and gate.dtype == BF16
-    check(_lib.load().ifab_gemv_group_norm(o.data_ptr(), o.stride(0), _p(gain), eps, groups, gate.data_ptr(), gate.stride(0), ACTIVATIONS[gate_act],
+    fn = _lib.load().ifab_gemv_group_norm_rows if rings else _lib.load().ifab_gemv_group_norm
+    check(fn(o.data_ptr(), o.stride(0), _p(gain), eps, groups, gate.data_ptr(), gate.stride(0), ACTIVATIONS[gate_act],
                                            w.data_ptr(), out.data_ptr(), out.stride(0), _f32(out), 0, T, N, K, _s()), "gemv_group_norm")
 
 
 def gemv_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[str] = None, bias: Optional[torch.Tensor] = None,
-             addend: Optional[torch.Tensor] = None) -> None:
+             addend: Optional[torch.Tensor] = None, rings: bool = False) -> None:
     """``out = act(x @ w.T + bias + addend)`` for decode rows; ``bias`` f32 ``[N]``, ``addend`` f32 rows (may be ``out``)."""
     T, K = x.shape
     assert w.shape[1] == K and w.is_contiguous() and x.dtype == BF16
-    check(_lib.load().ifab_gemv_act(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), _p(addend), 0 if addend is None else addend.stride(0), out.data_ptr(),
+    fn = _lib.load().ifab_gemv_act_rows if rings else _lib.load().ifab_gemv_act
+    check(fn(x.data_ptr(), x.stride(0), w.data_ptr(), _p(bias), _p(addend), 0 if addend is None else addend.stride(0), out.data_ptr(),
                                     out.stride(0), _f32(out), ACTIVATIONS[act], T, w.shape[0], K, _s()), "gemv_act")
 
 

@@ -64,3 +64,36 @@ def test_greedy_head(T, V, K):
             torch.testing.assert_close(logits.double(), ref, rtol=0, atol=slack)
     assert fab.status() == 0
     fab.close()
+
+
+# operands made of a norm's output and a residual, of normalised groups with gates, and plain rows too long for shared memory
+@pytest.mark.parametrize("T", [1, 2, 3])
+@pytest.mark.parametrize("K,N,groups", [(192, 328, 6), (2048, 150, 16), (4096, 1000, 1), (4104, 147, 3), (9000, 77, 9)])
+def test_operands_of_norms_and_gates(T, K, N, groups):
+    from ironpangu_b200.ops import stream_norm as S
+
+    g = torch.Generator(device="cuda").manual_seed(K + N + T)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    w, y, x, gain, eps = (rand(N, K) * K ** -0.5).to(BF16), rand(T, K), rand(T, K) * 4, rand(K) * 0.1 + 1, 1e-3
+    rms = lambda v: v * torch.rsqrt(v.square().mean(-1, keepdim=True) + eps)
+
+    def check(out, operand):
+        # the operand may round to the next bf16 value (2^-8 of it) where its f32 norm ends a little off; f32 sums
+        ref, scale = operand.to(BF16).double() @ w.double().T, float((operand.double().abs() @ w.double().abs().T).max())
+        torch.testing.assert_close(out.double(), ref, rtol=0, atol=scale * (2.0 ** -20 + 2.0 ** -8 * K ** -0.5) + 1e-6)
+
+    z, x_out = torch.empty(T, N, device="cuda"), torch.empty(T, K, device="cuda")
+    S.gemv_post_norm(y, gain, eps, x, x_out, w, z, rings=True)
+    want = x.double() + rms(y.double()) * gain.double()
+    torch.testing.assert_close(x_out.double(), want, rtol=1e-5, atol=4e-6)
+    check(z, want.float())
+    gate = rand(T, K).to(BF16)
+    S.gemv_group_norm(y, gate, "sigmoid", eps, w, z, groups, gain, rings=True)
+    check(z, (rms(y.double().view(T, groups, -1)).view(T, K) * gain.double() * torch.sigmoid(gate.double())).float())
+    xb = x.to(BF16)
+    S.gemv_act(xb, w, z, rings=True)
+    check(z, xb.float())
+    bias, add = rand(N), rand(T, N)
+    out = add.clone()
+    S.gemv_act(xb, w, out, bias=bias, addend=out, rings=True)
+    torch.testing.assert_close(out, z + bias + add, rtol=1e-5, atol=1e-5)
