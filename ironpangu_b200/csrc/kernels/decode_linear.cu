@@ -147,7 +147,7 @@ int dispatch_rows(const GemvParams& p, cudaStream_t s) {
 // layer 36 us).
 constexpr int SMEM_NORM = 126976, SMEM_PLAIN = 102912;
 template <int MR, bool GATED, bool NORM>
-using RowsStream = RowStream<MR, NORM ? (MR == 8 ? 10 : 12) : 8, NORM ? (MR == 8 ? 4 : 6) : (MR == 8 ? 3 : 5), MR == 8 ? 33792 : NORM ? 18432 : 13312, GATED>;
+using RowsStream = RowStream<MR, NORM ? (MR == 8 ? 10 : 12) : 8, NORM ? (MR == 8 ? 4 : 6) : (MR == 8 ? 3 : 5), MR == 8 ? 33792 : NORM ? 18432 : 13312, GATED ? Rows::GATED : Rows::PLAIN>;
 
 // grid (a CTA for each SM, tiles of MR rows of x)
 template <int MR, bool GATED, bool NORM>
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 2) rows_kernel(GemvParams p) {
   grid_dep_launch();
   const int t0 = blockIdx.y * MR, T = min(MR, p.T - t0);
   S stream;
-  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x)}, smem);
+  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x), 0}, smem);
   BfRows<MR, NORM> x{p.x + (long)t0 * p.ldx, p.ldx, p.norm_w, p.eps, p.zero_centered, T};
   x.early(stream);
   grid_dep_wait();
@@ -192,6 +192,80 @@ template <int MR>
 int dispatch_rows_stream(const GemvParams& p, cudaStream_t s) {
   if (p.mode) return p.norm_w ? launch_rows<MR, true, true>(p, s) : launch_rows<MR, true, false>(p, s);
   return p.norm_w ? launch_rows<MR, false, true>(p, s) : launch_rows<MR, false, false>(p, s);
+}
+
+// The projection of a grouped-query layer with what comes behind it: rows of q and k are turned, keys and values go to their pages. A result is the pair of columns that a
+// rotation mixes, so no other launch has to wait for the row: 2B model, a step of one row 4.4 us a layer for the kernel that did it (decode_gqa.cu), of eight rows 3.9.
+// q lands in `y`; angles, roundings and pages are that kernel's.
+struct QkvParams {
+  GemvParams g;
+  const int32_t *positions, *slots, *page_table;
+  int max_pages, page_tokens, num_pages;
+  bf16 *k_cache, *v_cache;
+  int Hq, Hkv, half;
+  float theta;
+  uint32_t* status;
+};
+template <int MR>
+__global__ void __launch_bounds__(RS_WARPS * 32, 2) qkv_rows_kernel(QkvParams q) {
+  using S = RowStream<MR, MR == 8 ? 10 : 12, MR == 8 ? 4 : 6, MR == 8 ? 33792 : 18432, Rows::PAIRS>;
+  const GemvParams& p = q.g;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ float sums[RS_WARPS * 8];
+  grid_dep_launch();
+  S stream;
+  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x), q.half}, smem);
+  BfRows<MR, true> x{p.x, p.ldx, p.norm_w, p.eps, p.zero_centered, p.T};
+  x.early(stream);
+  grid_dep_wait();
+  // where row t's keys and values go (-1: nowhere), and the angle of pair j
+  struct Place {
+    long row;
+    float c, s;
+  };
+  auto place = [&](int t, int n) {
+    Place at{-1, 1.f, 0.f};
+    const int pos = q.positions[t], h = n / q.half, j = n - h * q.half;
+    if (pos < 0) return at;
+    if (h >= q.Hq) {
+      const int lp = pos / q.page_tokens, page = lp < q.max_pages ? q.page_table[(long)q.slots[t] * q.max_pages + lp] : -1;
+      if (page >= 0 && page < q.num_pages) at.row = (long)page * q.page_tokens + pos % q.page_tokens;
+      else if (q.status) atomicOr(q.status, IFAB_STATUS_BAD_INDEX);
+    }
+    if (h < q.Hq + q.Hkv) {
+      const float inv_freq = exp2f(-(2.f * (float)j / (float)(2 * q.half)) * log2f(q.theta));
+      sincosf((float)pos * inv_freq, &at.s, &at.c);
+      at.c = bf16_round(at.c);
+      at.s = bf16_round(at.s);
+    }
+    return at;
+  };
+  Place mine{-1, 1.f, 0.f};       // requested here: behind the sums it was two more trips to L2
+  int ft, fn;
+  if (stream.first_result(p.T, &ft, &fn)) mine = place(ft, fn);
+  x.prepare(stream, sums);
+  auto out = [&](int t, int n, float v, float u, bool first) {
+    const Place at = first ? mine : place(t, n);
+    const int h = n / q.half, j = n - h * q.half, hd = 2 * q.half;
+    const float a = bf16_round(v), b = bf16_round(u);
+    const bf16 lo = __float2bfloat16_rn(a * at.c - b * at.s), hi = __float2bfloat16_rn(b * at.c + a * at.s);
+    bf16* to = reinterpret_cast<bf16*>(p.y) + (long)t * p.ldy + h * hd + j;
+    if (h >= q.Hq) {
+      if (at.row < 0) return;
+      const bool key = h < q.Hq + q.Hkv;
+      to = (key ? q.k_cache : q.v_cache) + (at.row * q.Hkv + (h - q.Hq - (key ? 0 : q.Hkv))) * hd + j;
+    }
+    to[0] = lo;
+    to[q.half] = hi;
+  };
+  stream.run(x, p.T, out);
+}
+template <int MR>
+int launch_qkv(const QkvParams& q, cudaStream_t s) {
+  auto k = qkv_rows_kernel<MR>;
+  if (int rc = opt_in_smem(k, SMEM_NORM)) return rc;
+  if (int rc = (int)cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+  return launch_chain(k, dim3(tc::device_sms()), dim3(RS_WARPS * 32), (size_t)SMEM_NORM, s, q);
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -291,6 +365,18 @@ extern "C" int ifab_gemv_rows_bf16(const void* x, long ldx, const void* w, const
   if (T < 1 || N < 1 || K < 8 || K % 8 != 0 || ldx % 8 != 0 || bits % 16 != 0 || mode < 0 || mode > 1 || (mode && (residual || out_f32))) return -1;
   GemvParams p{(const bf16*)x, ldx, (const bf16*)w, (const bf16*)norm_w, eps, zero_centered, (const bf16*)residual, ldr, y, ldy, out_f32, T, N, K, mode};
   return T <= 2 ? dispatch_rows_stream<2>(p, (cudaStream_t)stream) : dispatch_rows_stream<8>(p, (cudaStream_t)stream);
+}
+
+// q [T, Hq * head_dim] (into y), keys and values (into their pages) of norm(x) w^T with w = [q heads | k heads | v heads] rows; all columns of a head of q and k turn.
+// One to eight rows; a row at position -1 writes its q only.
+extern "C" int ifab_qkv_rows_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, void* y, long ldy, const int32_t* positions,
+                                  const int32_t* slots, const int32_t* page_table, int max_pages, int page_tokens, void* k_cache, void* v_cache, int num_pages, int T,
+                                  int Hq, int Hkv, int head_dim, int K, float theta, uint32_t* status, void* stream) {
+  const uintptr_t bits = (uintptr_t)x | (uintptr_t)w | (uintptr_t)norm_w;
+  if (T < 1 || T > 8 || K < 8 || K % 8 != 0 || ldx % 8 != 0 || bits % 16 != 0 || !norm_w || head_dim < 2 || head_dim % 2 || Hq < 1 || Hkv < 1 || page_tokens < 1) return -1;
+  QkvParams q{{(const bf16*)x, ldx, (const bf16*)w, (const bf16*)norm_w, eps, 0, nullptr, 0, y, ldy, 0, T, (Hq + 2 * Hkv) * (head_dim / 2), K, 0},
+              positions, slots, page_table, max_pages, page_tokens, num_pages, (bf16*)k_cache, (bf16*)v_cache, Hq, Hkv, head_dim / 2, theta, status};
+  return T <= 2 ? launch_qkv<2>(q, (cudaStream_t)stream) : launch_qkv<8>(q, (cudaStream_t)stream);
 }
 
 extern "C" int ifab_gemv_allreduce_bf16(const void* x, long ldx, const void* w, const void* residual, long ldr,

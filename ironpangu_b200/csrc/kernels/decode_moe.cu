@@ -499,7 +499,7 @@ __device__ __forceinline__ void finish_argmax(const HeadParams& p, int* is_last)
 // One row of 151936 x 2048 (622 MB) 104.4 -> 103 us alone; behind a step's kernels, whose end it fills its rings under, 117 -> 104.
 constexpr int HEAD_SMEM = 126976;
 template <int T, bool NORM>
-using HeadStream = RowStream<T <= 2 ? 2 : 8, T <= 2 ? 12 : 10, T <= 2 ? 6 : 4, T <= 2 ? 18432 : 33792, false>;
+using HeadStream = RowStream<T <= 2 ? 2 : 8, T <= 2 ? 12 : 10, T <= 2 ? 6 : 4, T <= 2 ? 18432 : 33792, Rows::PLAIN>;
 template <int T, bool NORM>
 __global__ void __launch_bounds__(256, 1) lm_head_argmax_kernel(HeadParams p) {
   using S = HeadStream<T, NORM>;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(256, 1) lm_head_argmax_kernel(HeadParams p) {
   __shared__ int is_last;
   grid_dep_launch();
   S stream;
-  stream.start(RowShare{p.w, p.V, p.K, (int)((long)p.V * blockIdx.x / gridDim.x), (int)((long)p.V * (blockIdx.x + 1) / gridDim.x)}, smem);
+  stream.start(RowShare{p.w, p.V, p.K, (int)((long)p.V * blockIdx.x / gridDim.x), (int)((long)p.V * (blockIdx.x + 1) / gridDim.x), 0}, smem);
   BfRows<T <= 2 ? 2 : 8, NORM> x{p.x, p.ldx, p.norm_w, p.eps, 0, p.T};
   x.early(stream);
   grid_dep_wait();

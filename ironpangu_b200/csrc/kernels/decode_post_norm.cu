@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256) gemv_operand_kernel(Params p) {
 // 5.9 -> 4.6.
 constexpr int OPERAND_SMEM = 126976, PLAIN_SMEM = 102912;
 template <int PRO>
-using OperandStream = RowStream<2, PRO == POST ? 12 : 8, PRO == POST ? 6 : 5, PRO == POST ? 18432 : 16768, false>;
+using OperandStream = RowStream<2, PRO == POST ? 12 : 8, PRO == POST ? 6 : 5, PRO == POST ? 18432 : 16768, Rows::PLAIN>;
 template <int T>
 struct StagedRows {
   struct Raw {};
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(256, 2) rows_operand_kernel(Params p) {
   __shared__ float red[T * 8];
   grid_dep_launch();
   S stream;
-  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x)}, smem);
+  stream.start(RowShare{p.w, p.N, p.K, (int)((long)p.N * blockIdx.x / gridDim.x), (int)((long)p.N * (blockIdx.x + 1) / gridDim.x), 0}, smem);
   auto out = [&](int t, int n, float v, float, bool) {
     if (p.out_bias) v += p.out_bias[n];
     if (p.addend) v += p.addend[(long)t * p.ldadd + n];

@@ -57,6 +57,9 @@ int ifab_gemv_bf16(const void* x, long ldx, const void* w, const void* norm_w, f
                    void* stream);
 int ifab_gemv_rows_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, int zero_centered, const void* residual, long ldr, void* y, long ldy,
                         int out_f32, int T, int N, int K, int mode, void* stream);
+int ifab_qkv_rows_bf16(const void* x, long ldx, const void* w, const void* norm_w, float eps, void* y, long ldy, const int32_t* positions, const int32_t* slots,
+                       const int32_t* page_table, int max_pages, int page_tokens, void* k_cache, void* v_cache, int num_pages, int T, int Hq, int Hkv, int head_dim, int K,
+                       float theta, uint32_t* status, void* stream);
 int ifab_gemv_allreduce_bf16(const void* x, long ldx, const void* w, const void* residual, long ldr, void* y, long ldy,
                              void* y_f32, int T, int N, int K, const IfabFabric* fab, void* stream);
 

@@ -37,17 +37,20 @@ __device__ __forceinline__ uint4 ld_shared16(uint32_t at) {
 __device__ __forceinline__ void st_shared16(uint32_t at, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// a CTA's share of the product: rows lo <= n < hi of W [N, K] or, GATED, those and rows N + n of W [2 N, K]
+// A CTA's share of the product: results lo <= n < hi of N. PLAIN: of row n of W [N, K]; GATED: of rows n and N + n of W [2 N, K]; PAIRS: of the two rows that a
+// rotation turns into one another, n + n / half * half and the one half behind, of W [2 N, K]
+enum class Rows { PLAIN, GATED, PAIRS };
 struct RowShare {
   const bf16* w;
-  int N, K, lo, hi;
+  int N, K, lo, hi, half;
 };
 
-// MR: most rows of x. TB: tiles of eight rows of W that are summed up at a time (GATED: half of them gate rows, the other half the matching up rows).
+// MR: most rows of x. TB: tiles of eight rows of W that are summed up at a time (GATED and PAIRS: half of them first rows, the other half the second ones).
 // DEPTH: stages of a ring. XS: bytes for rows of x
-template <int MR, int TB, int DEPTH, int XS, bool GATED>
+template <int MR, int TB, int DEPTH, int XS, Rows KIND>
 struct RowStream {
-  static constexpr int PER = GATED ? 2 : 1, ROWS = 8 * TB / PER;      // outputs of a block of tiles
+  static constexpr bool TWO = KIND != Rows::PLAIN;
+  static constexpr int PER = TWO ? 2 : 1, ROWS = 8 * TB / PER;      // outputs of a block of tiles
   static constexpr int RING = RS_WARPS * DEPTH * RS_STAGE, RED = RS_WARPS * TB * MR * 8 * 4, SMEM = RING + RED + XS;
 
   RowShare s;
@@ -68,7 +71,13 @@ struct RowStream {
   __device__ __forceinline__ void request(int at) {
     if (pb < s.hi) {
       const int r = pb + pt / PER * 8 + (lane >> 3), left = min(steps * 32, s.K - pk * chunk - col) - (lane & 7) * 8;
-      const bf16* from = src + (long)(pt / PER * 8 + (GATED && (pt & 1) ? s.N : 0)) * s.K;
+      const bf16 *from = src + (long)(pt / PER * 8 + (KIND == Rows::GATED && (pt & 1) ? s.N : 0)) * s.K, *from4 = from + 4l * s.K;
+      if (KIND == Rows::PAIRS) {
+        const int a = min(r, s.N - 1), b = min(r + 4, s.N - 1), second = pt & 1 ? s.half : 0;
+        const bf16* at_col = s.w + pk * chunk + col + (lane & 7) * 8;
+        from = at_col + (long)(a + a / s.half * s.half + second) * s.K;
+        from4 = at_col + (long)(b + b / s.half * s.half + second) * s.K;
+      }
       // a piece lies where its reader's accesses meet no bank twice
       const uint32_t dst = ring + at * RS_STAGE + (lane >> 3) * 128 + (((lane & 7) ^ (lane >> 3)) << 4), dst4 = dst ^ 64;
       const bool row = r < s.hi, row4 = r + 4 < s.hi;
@@ -76,7 +85,7 @@ struct RowStream {
       for (int h = 0; h < RS_STEPS / 2; ++h) {
         const bool in = row && h * 64 < left, in4 = row4 && h * 64 < left;
         copy16(dst + h * 1024, in ? from + h * 64 : s.w, in);
-        copy16(dst4 + h * 1024 + 512, in4 ? from + 4l * s.K + h * 64 : s.w, in4);
+        copy16(dst4 + h * 1024 + 512, in4 ? from4 + h * 64 : s.w, in4);
       }
       if (++pt == pn) {
         pt = 0;
@@ -173,7 +182,7 @@ struct RowStream {
           constexpr int W = TB * MR * 8;
           return ((f[0] + f[W]) + (f[2 * W] + f[3 * W])) + ((f[4 * W] + f[5 * W]) + (f[6 * W] + f[7 * W]));
         };
-        out(t, n, sum(from), GATED ? sum(from + MR * 8) : 0.f, lo == s.lo && i == (int)threadIdx.x);
+        out(t, n, sum(from), TWO ? sum(from + MR * 8) : 0.f, lo == s.lo && i == (int)threadIdx.x);
       }
       if (lo + ROWS < s.hi) __syncthreads();
     }

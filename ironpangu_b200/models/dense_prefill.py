@@ -173,12 +173,14 @@ class DensePrefill:
         for l in range(c.layers):
             p = f"layers.{l}."
             if self._few(m, w[p + "qkv"]):
-                qkv = K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=self.qkv[:m], rings=True)
+                qkv = self.qkv[:m]
+                K.qkv_rows(x, w[p + "qkv"], w[p + "attn_norm"], pos, sl, d.page_table, d.k_cache[l], d.v_cache[l], heads=d.hq, kv_heads=d.hk, head_dim=c.head_dim,
+                           theta=c.theta, eps=c.eps, out=qkv, status_ptr=st)
             else:
                 K.rmsnorm(x, w[p + "attn_norm"], c.eps, out=h)
                 qkv = G.gemm(h, w[p + "qkv"], out=self.qkv[:m], status_ptr=st, fixed=True)
-            K.gqa_rope_kv_write(qkv, pos, sl, d.page_table, d.k_cache[l], d.v_cache[l], heads=d.hq, kv_heads=d.hk,
-                                head_dim=c.head_dim, theta=c.theta, status_ptr=st)
+                K.gqa_rope_kv_write(qkv, pos, sl, d.page_table, d.k_cache[l], d.v_cache[l], heads=d.hq, kv_heads=d.hk,
+                                    head_dim=c.head_dim, theta=c.theta, status_ptr=st)
             self._attention(l, m, qkv, pos, sl, scale, st)
             if fab.world > 1:
                 G.gemm_allreduce(self.attn[:m], w[p + "o_proj"], fab, self._sym_rows(m), residual=x)

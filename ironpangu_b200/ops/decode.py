@@ -82,6 +82,17 @@ def gemv(x: torch.Tensor, w: torch.Tensor, *, norm_w: Optional[torch.Tensor] = N
     return out
 
 
+def qkv_rows(x: torch.Tensor, w: torch.Tensor, norm_w: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, page_table: torch.Tensor, k_cache: torch.Tensor,
+             v_cache: torch.Tensor, *, heads: int, kv_heads: int, head_dim: int, theta: float, eps: float, out: torch.Tensor, status_ptr: Optional[int] = None) -> None:
+    """``gemv(x, w, norm_w=norm_w, rings=True)`` and :func:`gqa_rope_kv_write` behind it as one launch, for one to eight rows whose heads turn in all columns: the turned
+    query heads land in the first columns of ``out``, turned keys and values in their pages."""
+    T, K = x.shape
+    assert w.shape == ((heads + 2 * kv_heads) * head_dim, K) and w.is_contiguous() and w.dtype == x.dtype == BF16 and k_cache.is_contiguous() and v_cache.is_contiguous()
+    check(_lib.load().ifab_qkv_rows_bf16(x.data_ptr(), _rows(x), w.data_ptr(), norm_w.data_ptr(), eps, out.data_ptr(), _rows(out), positions.data_ptr(), slots.data_ptr(),
+                                         page_table.data_ptr(), page_table.shape[1], k_cache.shape[1], k_cache.data_ptr(), v_cache.data_ptr(), k_cache.shape[0], T, heads,
+                                         kv_heads, head_dim, K, theta, status_ptr, _stream()), "qkv_rows")
+
+
 def gemv_allreduce(x: torch.Tensor, w: torch.Tensor, fabric, *, residual: Optional[torch.Tensor] = None,
                    out: Optional[torch.Tensor] = None, out_f32: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Row-parallel linear fused with a one-shot all-reduce: ``y = sum_r x_r @ w_r.T (+ residual)``."""

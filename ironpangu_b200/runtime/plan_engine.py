@@ -455,7 +455,7 @@ class PlanEngine:
         self._moe_members = {m: k for k, g in self.moe_groups.items() for m in g["members"]}
         per_token = self.program["launches_per_token"] + sum(1 for i in self.ins if i["op"] == "mla_attention")
         self.launches_per_forward = (per_token - (4 * len(self.head_groups) if self.fused_head else 0)
-                                     - (2 * len(self.moe_groups) if self.fused_moe else 0) - (4 * len(self.gqa_groups) if self.fused_gqa else 0))
+                                     - (2 * len(self.moe_groups) if self.fused_moe else 0) - (sum(5 if self._turns_in_projection(g) else 4 for g in self.gqa_groups.values()) if self.fused_gqa else 0))
         self._describe()
 
     def _describe(self) -> None:
@@ -501,6 +501,10 @@ class PlanEngine:
             w[p + "gate_up"], w[p + "down"] = self._param(gu["weight"] + "|" + gu["paired_weight"]), self._param(dn["weight"])
             w[p + "shared_gate_up"] = self._param(gu["shared_weight"] + "|" + gu["shared_paired_weight"])
             w[p + "shared_down"] = self._param(dn["shared_weight"])
+
+    def _turns_in_projection(self, g: dict) -> bool:
+        """Whether a grouped-query group's rotation and page write are part of its projection's launch."""
+        return self._rings and bool(g["norm"]) and g["rotary_dim"] == int(self.ins[g["members"][-1]]["attrs"]["head_dim"])
 
     def _describe_dense(self, emb: dict, head: dict) -> None:
         """The same for a stack of {grouped-query attention, SwiGLU} layers, in the vocabulary of ``models/dense_gqa.py``: the
@@ -723,9 +727,14 @@ class PlanEngine:
                 wq = self._gqa_packed[k]
                 qkv = self._gqa_qkv[:T, :wq.shape[0]]
                 kc, vc = self._kv_of[g["cache"]]
-                K.gemv(val(g["x"]), wq, norm_w=self._param(g["norm"], g["norm_optional"]) if g["norm"] else None, eps=g["eps"], out=qkv, rings=self._rings)
-                K.gqa_rope_kv_write(qkv, pos, slot, self.page_table, kc, vc, heads=H, kv_heads=KVH, head_dim=hd, rotary_dim=g["rotary_dim"],
-                                    theta=g["theta"], status_ptr=st)
+                gain = self._param(g["norm"], g["norm_optional"]) if g["norm"] else None
+                if self._turns_in_projection(g) and T <= 8:
+                    K.qkv_rows(val(g["x"]), wq, gain, pos, slot, self.page_table, kc, vc, heads=H, kv_heads=KVH, head_dim=hd, theta=g["theta"], eps=g["eps"], out=qkv,
+                               status_ptr=st)
+                else:
+                    K.gemv(val(g["x"]), wq, norm_w=gain, eps=g["eps"], out=qkv, rings=self._rings)
+                    K.gqa_rope_kv_write(qkv, pos, slot, self.page_table, kc, vc, heads=H, kv_heads=KVH, head_dim=hd, rotary_dim=g["rotary_dim"],
+                                        theta=g["theta"], status_ptr=st)
                 K.gqa_decode_attention(qkv, kc, vc, pos, slot, self.page_table, heads=H, kv_heads=KVH, head_dim=hd, scale=float(a["scale"]),
                                        keys_per_split=self.kps, max_splits=self.max_splits, scratch=self.scratch, out=val(k), status_ptr=st)
             elif op == "kv_cache_append":

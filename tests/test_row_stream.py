@@ -97,3 +97,38 @@ def test_operands_of_norms_and_gates(T, K, N, groups):
     out = add.clone()
     S.gemv_act(xb, w, out, bias=bias, addend=out, rings=True)
     torch.testing.assert_close(out, z + bias + add, rtol=1e-5, atol=1e-5)
+
+
+# heads of 128, 64, 40 and 2 columns; shares that end inside a head; rows that are not there, in the same sequence, and on a page outside the cache
+@pytest.mark.parametrize("T,H,kv,hd,K", [(1, 16, 4, 128, 2048), (8, 8, 2, 64, 520), (3, 3, 3, 40, 256), (2, 5, 1, 2, 64)])
+def test_projection_with_rotation_and_pages(T, H, kv, hd, K):
+    from ironpangu_b200.ops import decode as D
+
+    g = torch.Generator(device="cuda").manual_seed(T + hd + K)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, gain = rand(T, K).to(BF16), (rand((H + 2 * kv) * hd, K) * K ** -0.5).to(BF16), (rand(K) * 0.1 + 1).to(BF16)
+    pages, table = 6, torch.tensor([[3, 1, 5], [0, 2, 77]], dtype=torch.int32, device="cuda")
+    pos = torch.tensor([17, 18, 3, -1, 40, 0, 31, 5][:T], dtype=torch.int32, device="cuda")
+    slots = torch.tensor([0, 0, 1, 1, 1, 1, 1, 0][:T], dtype=torch.int32, device="cuda")          # row 4 of eight: page 77
+    def cache():
+        return [torch.full((pages, 16, kv, hd), 7.0, dtype=BF16, device="cuda") for _ in range(2)]
+    (k1, v1), (k2, v2) = cache(), cache()
+    st1, st2 = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    one = torch.full((T, (H + 2 * kv) * hd), 7.0, dtype=BF16, device="cuda")
+    D.qkv_rows(x, w, gain, pos, slots, table, k1, v1, heads=H, kv_heads=kv, head_dim=hd, theta=1e4, eps=1e-6, out=one, status_ptr=st1.data_ptr())
+    two = D.gemv(x, w, norm_w=gain, eps=1e-6, rings=True)
+    if hd % 8 == 0:
+        D.gqa_rope_kv_write(two, pos, slots, table, k2, v2, heads=H, kv_heads=kv, head_dim=hd, theta=1e4, status_ptr=st2.data_ptr())
+        assert int(st1) == int(st2)
+        # the same f32 products of bf16 values, added in f32 and rounded: at most one bf16 step where a sum ends beside a boundary
+        for a, b in ((one[:, :H * hd], two[:, :H * hd]), (k1, k2), (v1, v2)):
+            torch.testing.assert_close(a.float(), b.float(), rtol=2 ** -7, atol=2.0 ** -12)
+        assert torch.equal(v1, v2)
+    else:
+        f = two.double().view(T, H + 2 * kv, hd)
+        c, s = (t.float().to(BF16).double() for t in (torch.cos(pos.double()), torch.sin(pos.double())))
+        for t in range(T):
+            if int(pos[t]) >= 0:
+                q = torch.stack([f[t, :H, 0] * c[t] - f[t, :H, 1] * s[t], f[t, :H, 1] * c[t] + f[t, :H, 0] * s[t]], -1).reshape(-1)
+                torch.testing.assert_close(one[t, :H * hd].double(), q, rtol=2 ** -7, atol=2.0 ** -12)
+    assert bool((one[:, H * hd:] == 7).all())
