@@ -12,9 +12,11 @@
 
 #include <algorithm>
 
+#include "expert_stream.cuh"
 #include "gemv.cuh"
 #include "ifab_kernels.h"
 #include "oneshot_ar.cuh"
+#include "row_stream.cuh"
 
 using namespace ifab;
 
@@ -203,6 +205,205 @@ __global__ void __launch_bounds__(256) moe_gate_up_fp8_kernel(GateUp8Params p) {
     bf16* out = p.act + ((size_t)t * (p.topk + 1) + slot) * p.F;
     out[j0] = __float2bfloat16_rn(silu(bf16_round(acc[0] * un)) * bf16_round(acc[2] * un));
     if (j0 + 1 < Fcur) out[j0 + 1] = __float2bfloat16_rn(silu(bf16_round(acc[1] * un)) * bf16_round(acc[3] * un));
+  }
+}
+
+// ---- both halves with every expert read once -----------------------------------------------------------
+// A step's tokens choose overlapping experts, and converting a weight costs more than multiplying it: here an expert's weights are read and converted once, for all of its
+// tokens, and multiplied on the tensor cores (m16n8k16 in f16, f32 sums: sixteen rows of weights against eight tokens). A CTA an SM streams its share through rings
+// like those of row_stream.cuh, sixteen rows by 256 columns (gate / up) or 32 rows by 128 (down) a warp and stage, block scales beside them; a product of a block of
+// 128 columns is scaled once. The shared expert comes first: its weights are on the way before the wait for the router.
+// Bound by the bytes of the chosen experts. 8 tokens of 8 among 96 experts and a shared one, 4096 x 1536: a token at a time on the CUDA cores
+// gate / up 212 us and down 101, so 108 (642 MB: 5.9 TB/s) and 78 (321 MB: 4.1 TB/s, half of its instructions being conversions).
+__device__ __forceinline__ void mma16816_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// four fp8 values as two pairs of f16
+__device__ __forceinline__ uint2 halves_of(uint32_t w) {
+  const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)w, __NV_E4M3), hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+// sixteen columns of sixteen rows (lane: rows g and g + 8) against eight tokens: x, x + 1 hold the lane's token's values of them
+__device__ __forceinline__ void mma_piece(float (&d)[4], const uint4& w, const uint4& w8, const uint4& x, const uint4& x1) {
+  const uint2 a = halves_of(w.x), a8 = halves_of(w8.x), b = halves_of(w.y), b8 = halves_of(w8.y), c = halves_of(w.z), c8 = halves_of(w8.z), e = halves_of(w.w), e8 = halves_of(w8.w);
+  mma16816_f16(d, a.x, a8.x, a.y, a8.y, x.x, x.y);
+  mma16816_f16(d, b.x, b8.x, b.y, b8.y, x.z, x.w);
+  mma16816_f16(d, c.x, c8.x, c.y, c8.y, x1.x, x1.y);
+  mma16816_f16(d, e.x, e8.x, e.y, e8.y, x1.z, x1.w);
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const void* src, bool live) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4 : 0) : "memory");
+}
+// where piece c (16 bytes) of row r lies within 128 bytes: a quarter of a warp writes a row and reads half of two, in either case without meeting a bank twice
+__device__ __forceinline__ int swizzled(int c, int r) { return c ^ ((r & 1) << 2 | (r >> 1 & 3)); }
+
+constexpr int XP_STAGE = 4096, XP_SCALES = 128, XP_DEPTH = 3, XP_TILES = 4;
+constexpr int XP_RING = 8 * XP_DEPTH * (XP_STAGE + XP_SCALES), XP_RED = 8 * XP_TILES * 128 * 4;
+
+// A CTA's share of gate / up: first pairs of the shared expert, then eights of pairs of the listed experts
+__global__ void __launch_bounds__(256, 1) expert_gate_up_kernel(GateUp8Params p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ RouteList list;
+  __shared__ float sums[RS_WARPS * 8];
+  __shared__ int tile_entry[XP_TILES], tile_row[XP_TILES], tile_live[XP_TILES];
+  grid_dep_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, nb = (p.D + QBLOCK - 1) / QBLOCK, chunks = (p.D + 2047) / 2048;
+  const uint32_t ring = smem_addr(smem) + warp * XP_DEPTH * (XP_STAGE + XP_SCALES);
+  float* red = reinterpret_cast<float*>(smem + XP_RING);
+  struct {
+    struct { int K; } s;
+    uint32_t xs;
+    int pitch, warp, lane;
+    __device__ bool fits(int) const { return true; }
+  } rows{{p.D}, smem_addr(smem) + XP_RING + XP_RED, (p.D * 2 + 127) / 128 * 128 + 16, warp, lane};
+  const int lo = p.w_sgu ? (int)((long)p.Fs * blockIdx.x / gridDim.x) : 0, hi = p.w_sgu ? (int)((long)p.Fs * (blockIdx.x + 1) / gridDim.x) : 0, shared_tiles = (hi - lo + 7) / 8;
+  const int eights = p.F / 8;
+  int tiles = shared_tiles, first = 0;         // of this CTA; first eight of the listed experts'
+  // the tile a cursor stands on: entry (-1: the shared expert), first pair, pairs
+  struct Cursor {
+    int i, entry, row;
+  };
+  auto begin = [&](Cursor& c) {
+    c.i = 0;
+    c.entry = shared_tiles ? -1 : first / eights;
+    c.row = shared_tiles ? lo : (first - c.entry * eights) * 8;
+  };
+  auto advance = [&](Cursor& c) {
+    if (++c.i == shared_tiles) {
+      c.entry = first / eights;
+      c.row = (first - c.entry * eights) * 8;
+    } else if ((c.row += 8) == p.F && c.entry >= 0) {
+      c.row = 0;
+      ++c.entry;
+    }
+  };
+  Cursor ask;
+  int k_ask = 0, asked = 0;
+  auto request = [&](int at) {
+    if (ask.i < tiles) {
+      const bool shared = ask.entry < 0;
+      const int F = shared ? p.Fs : p.F, live = shared ? hi - ask.row : 8;
+      const size_t e = shared ? 0 : list.expert[ask.entry];
+      const uint8_t* w = (shared ? p.w_sgu : p.w_gu + e * 2 * p.F * p.D) + (size_t)ask.row * p.D;
+      const float* sc = (shared ? p.s_sgu : p.s_gu + e * 2 * p.F * nb) + (size_t)ask.row * nb;
+      const uint32_t to = ring + at * (XP_STAGE + XP_SCALES);
+      const int col = k_ask * 2048 + warp * 256 + (lane & 7) * 16, r0 = lane >> 3;
+      const uint32_t at0 = to + r0 * 128 + swizzled(lane & 7, r0) * 16;      // rows r0 and r0 + 4 of the gate rows, the same of the up rows
+      const uint8_t* from = w + (size_t)r0 * p.D + col;
+      const size_t four = 4 * (size_t)p.D, up = (size_t)F * p.D;
+      const bool in0 = col < p.D, in1 = col + 128 < p.D;
+      // rows that are not there may hold anything (a row's sums are its own), columns that are not there are zeros
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint8_t* row = from + (i & 1 ? four : 0) + (i >= 2 ? up : 0);
+        const uint32_t dst = (i & 1 ? (at0 ^ 32) + 512 : at0) + (i >> 1) * 2048;
+        if (r0 + (i & 1) * 4 < live) {
+          copy16(dst, in0 ? row : p.w_gu, in0);
+          copy16(dst + 1024, in1 ? row + 128 : p.w_gu, in1);
+        }
+      }
+      const int r = lane >> 1, b = k_ask * 16 + warp * 2 + (lane & 1);
+      const bool in = (r & 7) < live && b < nb;
+      copy4(to + XP_STAGE + lane * 4, in ? sc + (size_t)((r & 7) + (r >= 8 ? F : 0)) * nb + b : p.s_gu, in);
+      if (++k_ask == chunks) {
+        k_ask = 0;
+        advance(ask);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  begin(ask);
+  for (; asked < XP_DEPTH && ask.i < shared_tiles; ++asked) request(asked);
+  if (p.norm_w) request_gain(p.norm_w, p.D);
+  grid_dep_wait();
+  // rows of x, normalised on request, as f16 scaled by kXScale
+  auto stage = [&](auto x) {
+    x.early(rows);
+    x.prepare(rows, sums);
+  };
+  if (p.norm_w) stage(BfRows<8, true>{p.x, p.ldx, p.norm_w, p.eps, 0, p.T});
+  else stage(BfRows<8, false>{p.x, p.ldx, nullptr, 0.f, 0, p.T});
+  list_routes(list, p.ids, p.T, p.topk, p.e0, p.e_local);
+  for (int i = threadIdx.x; i < p.T * (p.D >> 3); i += 256) {
+    const int t = i / (p.D >> 3);
+    uint4* at = reinterpret_cast<uint4*>(smem + XP_RING + XP_RED + t * rows.pitch) + (i - t * (p.D >> 3));
+    *at = bf16x8_to_scaled_f16(*at);
+  }
+  const long all = (long)list.n * eights;
+  first = (int)(all * blockIdx.x / gridDim.x);
+  tiles = shared_tiles + (int)(all * (blockIdx.x + 1) / gridDim.x) - first;
+  if (ask.i >= shared_tiles) {                 // the cursor was past the shared expert before the list was there
+    ask.entry = first / eights;
+    ask.row = (first - ask.entry * eights) * 8;
+  }
+  for (; asked < XP_DEPTH; ++asked) request(asked);
+  __syncthreads();
+  Cursor use;
+  begin(use);
+  int slot = 0;
+  const bool token = g < p.T;
+  const uint32_t xat = rows.xs + g * rows.pitch + warp * 512 + q * 32;
+  for (int i0 = 0; i0 < tiles; i0 += XP_TILES) {
+    for (int tt = 0; tt < XP_TILES && i0 + tt < tiles; ++tt) {
+      if (threadIdx.x == 0) {
+        tile_entry[tt] = use.entry;
+        tile_row[tt] = use.row;
+        tile_live[tt] = use.entry < 0 ? min(8, hi - use.row) : 8;
+      }
+      advance(use);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};     // gate row g of tokens 2 q and 2 q + 1, up row g of them
+#pragma unroll 1
+      for (int k = 0; k < chunks; ++k) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(XP_DEPTH - 1) : "memory");
+        __syncwarp();
+        const uint32_t at = ring + slot * (XP_STAGE + XP_SCALES);
+        const float2 sg = *reinterpret_cast<const float2*>(smem + (at - smem_addr(smem)) + XP_STAGE + g * 8), su = *reinterpret_cast<const float2*>(smem + (at - smem_addr(smem)) + XP_STAGE + 64 + g * 8);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t piece = at + h * 1024 + g * 128 + swizzled(q + 4 * u, g) * 16;
+            uint4 x = make_uint4(0, 0, 0, 0), x1 = x;
+            if (token && k * 2048 + warp * 256 + h * 128 + (q + 4 * u) * 16 < p.D) {
+              const uint32_t from = xat + k * 4096 + h * 256 + u * 128;
+              x = ld_shared16(from);
+              x1 = ld_shared16(from + 16);
+            }
+            mma_piece(d, ld_shared16(piece), ld_shared16(piece + 2048), x, x1);
+          }
+          const float a = h ? sg.y : sg.x, b = h ? su.y : su.x;
+          acc[0] = fmaf(a, d[0], acc[0]);
+          acc[1] = fmaf(a, d[1], acc[1]);
+          acc[2] = fmaf(b, d[2], acc[2]);
+          acc[3] = fmaf(b, d[3], acc[3]);
+        }
+        __syncwarp();                          // the stage is read
+        request(slot);
+        slot = slot + 1 == XP_DEPTH ? 0 : slot + 1;
+      }
+      *reinterpret_cast<float4*>(red + ((warp * XP_TILES + tt) * 32 + lane) * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+    __syncthreads();
+    const int n = min(XP_TILES, tiles - i0);
+    for (int i = threadIdx.x; i < n * 64; i += 256) {
+      const int tt = i >> 6, r = i & 7, t = i >> 3 & 7, entry = tile_entry[tt];
+      if (t >= p.T || r >= tile_live[tt]) continue;
+      const int s = entry < 0 ? p.topk : list.slot[entry][t];
+      if (s < 0) continue;
+      const float* from = red + (tt * 32 + r * 4 + (t >> 1)) * 4 + (t & 1);
+      float a = 0.f, b = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        a += from[w * XP_TILES * 128];
+        b += from[w * XP_TILES * 128 + 2];
+      }
+      constexpr float un = 1.f / kXScale;
+      p.act[((size_t)t * (p.topk + 1) + s) * p.F + tile_row[tt] + r] = __float2bfloat16_rn(silu(bf16_round(a * un)) * bf16_round(b * un));
+    }
+    if (i0 + XP_TILES < tiles) __syncthreads();
   }
 }
 
@@ -430,6 +631,166 @@ int dispatch_down8(const Down8Params& p, cudaStream_t s) {
   return -2;
 }
 
+// A CTA's rows of the down projection, 32 at a time, over all experts of all tokens; a warp takes every eighth block of 128 columns (which one, an expert's number says, so that
+// a token's sums do not depend on its neighbours'). One rank.
+__global__ void __launch_bounds__(256, 1) expert_down_kernel(Down8Params p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ RouteList list;
+  __shared__ float weight[RL_ROUTES][RL_TOKENS];
+  grid_dep_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int r0 = (int)((long)p.D * blockIdx.x / gridDim.x), r1 = (int)((long)p.D * (blockIdx.x + 1) / gridDim.x);
+  const uint32_t ring = smem_addr(smem) + warp * XP_DEPTH * (XP_STAGE + XP_SCALES);
+  float* red = reinterpret_cast<float*>(smem + XP_RING);
+  const int nb = (p.F + QBLOCK - 1) / QBLOCK, nbs = p.w_sdown ? (p.Fs + QBLOCK - 1) / QBLOCK : 0;
+  int n = 0;                                   // entries
+  bool known = false;
+  // a warp's blocks: of the shared expert (entry -1), then of the listed ones
+  struct Cursor {
+    int row, entry, block;
+  };
+  auto settle = [&](Cursor& c) {               // on to the next block that there is (row r1: none)
+    for (;;) {
+      if (c.entry < 0 ? c.block < nbs : c.entry < n && c.block < nb) return;
+      if (++c.entry >= n) {
+        if (!known) return;                    // the list is not there yet
+        c.entry = -1;
+        c.block = warp;
+        c.row += 32;
+        if (c.row >= r1) return;
+        continue;
+      }
+      c.block = (warp - list.expert[c.entry] * nb) & 7;
+    }
+  };
+  Cursor ask{r0, -1, warp}, use{r0, -1, warp};
+  auto request = [&](int at) {
+    const uint32_t to = ring + at * (XP_STAGE + XP_SCALES);
+    if (ask.row < r1 && (known || ask.entry < 0)) {
+      const bool shared = ask.entry < 0;
+      const int F = shared ? p.Fs : p.F, blocks = shared ? nbs : nb;
+      const size_t e = shared ? 0 : list.expert[ask.entry];
+      const uint8_t* w = (shared ? p.w_sdown : p.w_down + e * p.D * p.F) + (size_t)ask.row * F;
+      const float* sc = (shared ? p.s_sdown : p.s_down + e * p.D * nb) + (size_t)ask.row * blocks + ask.block;
+      const int live = r1 - ask.row, col = ask.block * 128 + (lane & 7) * 16, row0 = lane >> 3;
+      const bool in = col < F;
+      const uint8_t* from = in ? w + (size_t)row0 * F + col : p.w_down;
+      const size_t four = in ? 4 * (size_t)F : 0;
+      const uint32_t at0 = to + row0 * 128 + swizzled(lane & 7, row0) * 16;
+      // rows that are not there may hold anything (a row's sums are its own), columns that are not there are zeros
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (row0 + i * 4 < live) copy16((i & 1 ? at0 ^ 32 : at0) + i * 512, from, in);
+        from += four;
+      }
+      copy4(to + XP_STAGE + lane * 4, lane < live ? sc + (size_t)lane * blocks : p.s_down, lane < live);
+      ask.block += 8;
+      settle(ask);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int asked = 0;
+  settle(ask);
+  for (; asked < XP_DEPTH && ask.entry < 0 && ask.row == r0; ++asked) request(asked);
+  grid_dep_wait();
+  if (p.seq && blockIdx.x == 0 && threadIdx.x == 0) *p.seq += 1;
+  list_routes(list, p.ids, p.T, p.topk, p.e0, p.e_local);
+  for (int i = threadIdx.x; i < list.n * RL_TOKENS; i += 256) {
+    const int t = i & 7, s = list.slot[i >> 3][t];
+    weight[i >> 3][t] = s >= 0 ? p.wts[t * p.topk + s] : 0.f;
+  }
+  n = list.n;
+  known = true;
+  if (ask.entry >= 0) {                        // it had left the shared expert
+    ask.entry = -1;
+    ask.block = nbs;
+    settle(ask);
+  }
+  for (; asked < XP_DEPTH; ++asked) request(asked);
+  __syncthreads();
+  settle(use);
+  // this lane's token's values of a block: pieces q and q + 4
+  uint4 raw[4];
+  auto load = [&](const Cursor& c) {
+    const int s = g >= p.T || c.row >= r1 ? -1 : c.entry < 0 ? p.topk : list.slot[c.entry][g], F = c.entry < 0 ? p.Fs : p.F;
+    const bf16* row = p.act + ((size_t)g * (p.topk + 1) + max(s, 0)) * p.F + c.block * 128;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int col = (q + 4 * u) * 16;
+      const bool in = s >= 0 && c.block * 128 + col < F;
+      raw[2 * u] = raw[2 * u + 1] = make_uint4(0, 0, 0, 0);
+      if (in) {
+        raw[2 * u] = ld_row16(row + col);
+        raw[2 * u + 1] = ld_row16(row + col + 8);
+      }
+    }
+  };
+  load(use);
+  int slot = 0;
+  for (int row = r0; row < r1; row += 32) {
+    float acc[2][4] = {};                      // [sixteen rows][row g of tokens 2 q and 2 q + 1, row g + 8 of them]
+    while (use.row == row && (use.entry < 0 ? use.block < nbs : use.entry < n)) {
+      uint4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = bf16x8_to_scaled_f16(raw[i]);
+      float c[2];
+      bool his[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = 2 * q + i;
+        his[i] = t < p.T && (use.entry < 0 || list.slot[use.entry][t] >= 0);
+        c[i] = (use.entry < 0 ? 1.f : weight[use.entry][t]) * (1.f / kXScale);
+      }
+      use.block += 8;
+      settle(use);
+      load(use);
+      asm volatile("cp.async.wait_group %0;" ::"n"(XP_DEPTH - 1) : "memory");
+      __syncwarp();
+      const uint32_t at = ring + slot * (XP_STAGE + XP_SCALES);
+      const float* scales = reinterpret_cast<const float*>(smem + (at - smem_addr(smem)) + XP_STAGE);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t piece = at + m * 2048 + g * 128 + swizzled(q + 4 * u, g) * 16;
+          mma_piece(d, ld_shared16(piece), ld_shared16(piece + 1024), x[2 * u], x[2 * u + 1]);
+        }
+        const float a = scales[m * 16 + g], b = scales[m * 16 + 8 + g];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (his[i]) {
+            acc[m][i] = fmaf(c[i] * a, d[i], acc[m][i]);
+            acc[m][2 + i] = fmaf(c[i] * b, d[2 + i], acc[m][2 + i]);
+          }
+      }
+      __syncwarp();                            // the stage is read
+      request(slot);
+      slot = slot + 1 == XP_DEPTH ? 0 : slot + 1;
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) *reinterpret_cast<float4*>(red + ((warp * 2 + m) * 32 + lane) * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 32 * RL_TOKENS; i += 256) {
+      const int r = i & 31, t = i >> 5;
+      if (t >= p.T || row + r >= r1) continue;
+      const float* from = red + ((r >> 4) * 32 + (r & 7) * 4 + (t >> 1)) * 4 + (r >> 3 & 1) * 2 + (t & 1);
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v += from[w * 256];
+      if (p.residual) v = bf16_round(v) + __bfloat162float(p.residual[(long)t * p.ldr + row + r]);
+      p.y[(long)t * p.ldy + row + r] = __float2bfloat16_rn(v);
+    }
+    if (row + 32 < r1) __syncthreads();
+  }
+}
+int launch_expert_down(const Down8Params& p, cudaStream_t s) {
+  constexpr int smem = XP_RING + 8 * 2 * 128 * 4;
+  if (int rc = opt_in_smem(expert_down_kernel, smem)) return rc;
+  if (int rc = (int)cudaFuncSetAttribute(expert_down_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+  return launch_chain(expert_down_kernel, dim3(tc::device_sms()), dim3(256), (size_t)smem, s, p);
+}
+
 }  // namespace
 
 // w: bf16 [rows, K] (row stride ldw); q: u8 [rows, K]; scales: f32 [rows, ceil(K / 128)]
@@ -454,6 +815,24 @@ extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* 
   if (D % 16 != 0 || F % 16 != 0 || Fs % 16 != 0 || Fs > F) return -1;
   GateUp8Params p{(const bf16*)x, ldx, (const bf16*)norm_w, eps, ids, T, D, F, topk, e0, e_local,
                   (const uint8_t*)w_gu, s_gu, (const uint8_t*)w_shared_gu, s_shared_gu, Fs, (bf16*)act};
+  // by experts, up to eight tokens at a time, where their rows fit beside the rings
+  const uintptr_t bits = (uintptr_t)x | (uintptr_t)w_gu | (uintptr_t)w_shared_gu | (uintptr_t)norm_w;
+  const size_t room = 232448 - 8192 - XP_RING - XP_RED, row = (size_t)((D * 2 + 127) / 128 * 128 + 16);
+  const int at_once = (int)std::min<size_t>(RL_TOKENS, room / row);
+  if (T >= 1 && at_once >= 1 && topk >= 1 && topk <= MAX_TOPK8 && e_local >= 1 && e_local <= RL_EXPERTS && bits % 16 == 0 && ldx % 8 == 0) {
+    for (int t0 = 0; t0 < T; t0 += at_once) {
+      GateUp8Params q = p;
+      q.T = std::min(at_once, T - t0);
+      q.x += (long)t0 * ldx;
+      q.ids += t0 * topk;
+      q.act += (size_t)t0 * (topk + 1) * F;
+      const size_t smem = XP_RING + XP_RED + q.T * row;
+      if (int rc = opt_in_smem(expert_gate_up_kernel, smem)) return rc;
+      if (int rc = (int)cudaFuncSetAttribute(expert_gate_up_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
+      if (int rc = launch_chain(expert_gate_up_kernel, dim3(tc::device_sms()), dim3(256), smem, (cudaStream_t)stream, q)) return rc;
+    }
+    return 0;
+  }
   dim3 grid((F + 15) / 16, T * topk + T);
   const size_t smem = (size_t)D * sizeof(bf16);
   if (int rc = opt_in_smem(moe_gate_up_fp8_kernel, smem)) return rc;
@@ -475,6 +854,8 @@ extern "C" int ifab_moe_down_allreduce_decode_fp8(const void* act, const int32_t
   if ((size_t)fab->world * T * D * sizeof(uint64_t) > fab->ll_half_bytes) return -3;
   if ((size_t)fab->world * 296 > fab->flag_half_words) return -4;
   cudaStream_t s = (cudaStream_t)stream;
+  if (fab->world == 1 && (D + 31) / 32 <= 296 && topk >= 1 && e_local >= 1 && e_local <= RL_EXPERTS && ((uintptr_t)act | (uintptr_t)w_down | (uintptr_t)w_shared_down) % 16 == 0)
+    return launch_expert_down(p, s);
   if (T <= 1) return dispatch_down8<1>(p, s);
   if (fab->world == 1) return (D + 31) / 32 <= 296 ? launch_down8<1, 4>(p, s, T) : -2;       // rows as wide as the other forms take
   if (T <= 2) return dispatch_down8<2>(p, s);

@@ -228,6 +228,8 @@ class MlaMoeDecoder:
         c, dev = cfg, fabric.device
         assert c.heads % self.world == 0 and c.experts % self.world == 0 and c.vocab % self.world == 0
         assert c.shared_ffn % (8 * self.world) == 0
+        # linears as streams through shared memory beside expert kernels that stream so themselves; bf16 experts stream through L1
+        self.rings = expert_fp8 and fabric.world == 1
         self.hl, self.el, self.vl = c.heads // self.world, c.experts // self.world, c.vocab // self.world
         self.T = max_tokens
         self.max_context = max_context
@@ -291,7 +293,10 @@ class MlaMoeDecoder:
         c, w, fab = self.cfg, self.w, self.fabric
         p = f"layers.{l}."
         x, attn = self.x[:T], self.attn[:T]
-        K.gemv_allreduce(attn, w[p + "o_proj"], fab, residual=x, out=x)
+        if self.rings:
+            K.gemv(attn, w[p + "o_proj"], residual=x, out=x, rings=True)
+        else:
+            K.gemv_allreduce(attn, w[p + "o_proj"], fab, residual=x, out=x)
         if self.fused_moe and T <= 2:
             K.moe_block(x, w[p + "router"], w[p + "gate_up"], w[p + "down"], self.rank * self.el, c.topk, fab, sync=self.moe_sync,
                         norm_w=w[p + "ffn_norm"], eps=c.eps, scoring=c.scoring, scale=c.route_scale,
@@ -324,7 +329,7 @@ class MlaMoeDecoder:
         for l in range(c.layers):
             p = f"layers.{l}."
             qkv = self.qkv[:T]
-            K.gemv(x, w[p + "qkv_a"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv)
+            K.gemv(x, w[p + "qkv_a"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv, rings=self.rings)
             fuse = self.fused_head if self.fuse_override is None else (self.fuse_override and self.can_fuse_head)
             if fuse and T <= self.fused_head_rows:
                 K.mla_head_decode(qkv, w[p + "q_a_norm"], w[p + "kv_a_norm"], w[p + "q_b"], w[p + "kv_b"], self.caches[l], pos, slot,
@@ -340,7 +345,7 @@ class MlaMoeDecoder:
                 K.mla_kv_write(qkv[:, c.q_lora:], w[p + "kv_a_norm"], pos, slot, self.page_table, self.caches[l],
                                latent=c.kv_lora, rope=c.rope, eps=c.eps, theta=c.theta, status_ptr=st)
             q = self.q[:T]
-            K.gemv(qkv[:, :c.q_lora], w[p + "q_b"], norm_w=w[p + "q_a_norm"], eps=c.eps, out=q)
+            K.gemv(qkv[:, :c.q_lora], w[p + "q_b"], norm_w=w[p + "q_a_norm"], eps=c.eps, out=q, rings=self.rings)
             q_lat = self.q_lat[:T]
             K.mla_q_absorb(q, w[p + "kv_b"], pos, nope=c.nope, rope=c.rope, theta=c.theta, out=q_lat)
             attn = self.attn[:T]

@@ -1,0 +1,59 @@
+"""fp8 expert kernels that read an expert once for all of its tokens, where their lists and shares can go wrong: a token that names an expert twice, experts of other ranks, no
+expert at all, columns and rows that are no multiple of a stage's, more rows than a CTA has at a time."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def _wide(w):
+    q, s = w
+    K = q.shape[-1]
+    return q.view(torch.float8_e4m3fn).double() * s.double().repeat_interleave(128, -1)[..., :K]
+
+
+@pytest.mark.parametrize("T,E,topk,D,F,Fs,shared", [(8, 3, 2, 64, 16, 16, True), (5, 300, 16, 2064, 144, 80, True), (3, 40, 4, 5008, 272, 0, False), (1, 8, 8, 9472, 128, 128, True), (8, 2, 1, 4112, 1040, 16, True)])
+def test_lists_and_shares(T, E, topk, D, F, Fs, shared):
+    from ironpangu_b200.ops import decode as K
+    from ironpangu_b200.parallel.fabric import Fabric
+
+    g = torch.Generator(device="cuda").manual_seed(T + E + D)
+    rand = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.05).to(BF16)
+    x, res, gain = rand(T, D) * 20, rand(T, D) * 10, rand(D) + 1
+    gu, dn = K.quantize_fp8_block(rand(E, 2 * F, D)), K.quantize_fp8_block(rand(E, D, F))
+    sgu, sdn = (K.quantize_fp8_block(rand(2 * Fs, D)), K.quantize_fp8_block(rand(D, Fs))) if shared else (None, None)
+    ids = torch.randint(-2, E + 2, (T, topk), generator=g, device="cuda").int()          # experts of nobody's among them
+    if topk > 1:
+        ids[0, 1] = ids[0, 0] = 1                                                          # one expert twice
+    if T > 2:
+        ids[2] = -1                                                                        # none at all
+    wts = torch.rand(T, topk, generator=g, device="cuda")
+    fab = Fabric(0, 1)
+    calls = fab.calls()
+    act = K.moe_gate_up_fp8(x, ids, gu, 0, norm_w=gain, w_shared_gu=sgu, act=torch.zeros(T, topk + 1, F, dtype=BF16, device="cuda"))
+    y = K.moe_down_allreduce_fp8(act, ids, wts, dn, 0, fab, w_shared_down=sdn, residual=res)
+    assert fab.calls() == calls + 1
+    h = x.float()
+    h = (h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-5) * gain.float()).to(BF16).double()
+    GU, DN = _wide(gu), _wide(dn)
+    for t in range(T):
+        want, scale = torch.zeros(D, dtype=torch.float64, device="cuda"), torch.zeros(D, dtype=torch.float64, device="cuda")
+        routes = [(k, GU[int(ids[t, k])], DN[int(ids[t, k])], float(wts[t, k]), F) for k in range(topk) if 0 <= int(ids[t, k]) < E]
+        routes += [(topk, _wide(sgu), _wide(sdn), 1.0, Fs)] if shared else []
+        used = {r[0] for r in routes}
+        for k, wg, wd, c, f in routes:
+            gate, up = wg[:f] @ h[t], wg[f:] @ h[t]
+            a = torch.nn.functional.silu(gate) * up
+            # both projections and their product are rounded to bf16 (2^-8 of a value at most, silu at most 1.1 times as steep); operands that a norm in f32 rounds to
+            # the next bf16 value and f32 sums: 2^-8 K^-1/2 of the magnitudes
+            slack = 2.0 ** -8 * (1.1 * gate.abs() * up.abs() + 2 * a.abs()) * 1.05 + (2 * up.abs() + 2 * gate.abs() + 1) * float((wg.abs() @ h[t].abs()).max()) * 2.0 ** -8 * D ** -0.5
+            assert bool(((act[t, k, :f].double() - a).abs() <= slack).all())
+            rows = act[t, k, :f].double()
+            want += c * (wd @ rows)
+            scale += c * (wd.abs() @ rows.abs())
+        assert all(bool((act[t, k] == 0).all()) for k in range(topk + 1) if k not in used)
+        total = want + res[t].double()
+        assert bool(((y[t].double() - total).abs() <= 2.0 ** -8 * (want.abs() + total.abs()) + 2.0 ** -18 * scale + 1e-6).all())
+    assert fab.status() == 0
+    fab.close()
