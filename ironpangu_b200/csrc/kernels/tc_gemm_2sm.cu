@@ -9,9 +9,9 @@
 //                        complete on the LEADER's full barrier (its shared::cluster address, by mapa)
 //   warp 1 (both CTAs)   allocates tensor memory (cta_group::2, collectively); in the leader one elected lane issues the MMAs and
 //                        releases a stage in BOTH CTAs with tcgen05.commit...multicast::cluster
-//   warps 2-5 (both)     epilogue of this CTA's 128 rows: tcgen05.ld, convert, residual, store
-// Six stages of 32 KB. No TMA load is multicast: every CTA fetches its own tiles. Every mbarrier wait is bounded; a wait that
-// runs out raises the CTA's abort flag and a status bit, and both CTAs still meet at the closing cluster barrier.
+//   warps 2-9 (both)     epilogue of this CTA's 128 rows, two warps for 32 of them: tcgen05.ld, convert, residual, store (tile_rows)
+// Six stages of 32 KB, and 4 KB a reader through which its rows pass. No TMA load is multicast: every CTA fetches its own
+// tiles. Every mbarrier wait is bounded; a wait that runs out raises the CTA's abort flag and a status bit, and both CTAs still meet at the closing cluster barrier.
 // Shapes: N % 32 == 0 (rows are stored 32 columns at a time), K % 8 == 0; M, N and K tails by TMA zero fill and masked stores.
 // `ifab_gemm_bf16` uses these kernels from 129 rows and 256 columns up, but where the cluster form has less to load (tc_gemm_rows.cu).
 #include <algorithm>
@@ -26,12 +26,15 @@ using namespace ifab::tc;
 
 namespace {
 
+constexpr int READERS = 8, SLOT_BYTES = 4096, THREADS2 = 64 + 32 * READERS;
+
 // TN: columns of a pair's tile (both CTAs together), also the accumulator's TMEM columns. A CTA supplies TN / 2 rows of B.
 template <int TN>
 struct Cfg2 {
-  static constexpr int HALF_N = TN / 2, STAGES2 = TN == 256 ? 6 : TN == 192 ? 7 : 8;
+  static constexpr int HALF_N = TN / 2, STAGES2 = TN == 128 ? 8 : 6;
   static constexpr int A2_BYTES = BM * BK * 2, STAGE2_BYTES = A2_BYTES + HALF_N * BK * 2;
-  static constexpr int SMEM2 = STAGES2 * STAGE2_BYTES + 1024 + 256;
+  static constexpr int RING2 = STAGES2 * STAGE2_BYTES;        // then a slot for each reader's rows (tile_rows)
+  static constexpr int SMEM2 = RING2 + READERS * SLOT_BYTES + 1024 + 256;
   static constexpr int COLS = TN <= 128 ? 128 : 256;          // an accumulator's share of tensor memory (powers of two)
 };
 
@@ -41,6 +44,7 @@ struct Gemm2Params {
   int M, N, K;
   uint32_t* status;
   uint32_t spin_limit;
+  int staged;     // rows of C (and of the residual) begin on 16 bytes: whole lines by way of shared memory (tile_rows)
   int swiglu_f;   // > 0 (persistent kernel only): B = [gate rows 0..F) | up rows F..2F), C[M, F] = unit(A gate^T, A up^T)
   int act;        // activation of the result (numbers of activate(); 0: none), after bias and residual
   const float* bias; float cap;      // [N] or null; > 0: cap tanh(result / cap)
@@ -90,35 +94,39 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-__device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int col, float* v) {
-  if (row >= p.M || col >= (p.swiglu_f > 0 ? p.swiglu_f : p.N)) return;
-  if (p.bias) {
+__device__ __forceinline__ void add_bias32(const Gemm2Params& p, int col, float* v) {
+  if (!p.bias) return;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] += p.bias[col + i];
-  }
-  if (p.residual) {        // 16-byte loads: two bytes at a time a 256 x 256 tile's epilogue took 20 us (509 x 2048, K 6144: 56 us, 42 so)
-    const bf16* r = p.residual + (long)row * p.ldr + col;
-    if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      uint4 u[4];
+  for (int i = 0; i < 32; ++i) v[i] += p.bias[col + i];
+}
+__device__ __forceinline__ void add_residual8(float* v, const uint4& u) {
+  float f[8];
+  unpack8(u, f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) u[i] = reinterpret_cast<const uint4*>(r)[i];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float f[8];
-        unpack8(u[i], f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[8 * i + j] = bf16_round(v[8 * i + j]) + f[j];
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = bf16_round(v[i]) + __bfloat162float(r[i]);
-    }
-  }
+  for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j]) + f[j];
+}
+__device__ __forceinline__ void finish32(const Gemm2Params& p, float* v) {
   activate_all<true, 32>(v, p.act);
   if (p.cap > 0.f) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = soft_limit<true>(v[i], p.cap);
   }
+}
+// 32 columns of the lane's own row, straight to C
+__device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int col, float* v) {
+  if (row >= p.M || col >= (p.swiglu_f > 0 ? p.swiglu_f : p.N)) return;
+  add_bias32(p, col, v);
+  if (p.residual) {
+    const bf16* r = p.residual + (long)row * p.ldr + col;
+    if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add_residual8(v + 8 * i, reinterpret_cast<const uint4*>(r)[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = bf16_round(v[i]) + __bfloat162float(r[i]);
+    }
+  }
+  finish32(p, v);
   if (p.out_f32) {
     float* out = reinterpret_cast<float*>(p.c) + (long)row * p.ldc + col;
     if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {
@@ -138,15 +146,128 @@ __device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int
   }
 }
 
-// grid (2 * M / 256, N / 256), clusters of 2 along x; 192 threads
+// The columns a tile has of its row block: [0, width) from n0 on, less at C's edge (both multiples of 32).
+__device__ __forceinline__ int tile_cols(const Gemm2Params& p, int n0, int width) { return min(width, (p.swiglu_f > 0 ? p.swiglu_f : p.N) - n0); }
+
+// 16-byte piece `pc` of row `r` in a reader's slot (32 rows x 128 bytes); the rotation keeps both a row's pieces and a column of pieces on all banks
+__device__ __forceinline__ uint4* slot_piece(unsigned char* slot, int r, int pc) { return reinterpret_cast<uint4*>(slot) + r * 8 + (pc ^ (r & 7)); }
+// requests the residual of 32 rows x `pieces` * 8 columns into the slot, a line a row
+__device__ __forceinline__ void request_residual(const Gemm2Params& p, unsigned char* slot, int row0, int col, int pieces, int lane) {
+  const int pc = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    if (row0 + r < p.M && pc < pieces)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(slot_piece(slot, r, pc))), "l"(p.residual + (long)(row0 + r) * p.ldr + col + pc * 8)
+                   : "memory");
+  }
+}
+// the residual of the reader's first chunk of a tile, requested while the tile's products still run
+__device__ __forceinline__ void request_first(const Gemm2Params& p, unsigned char* slot, int row0, int n0, int width, int half, int lane) {
+  const int cols = tile_cols(p, n0, width), c0 = 64 * half;
+  if (p.staged && p.residual && c0 < cols) request_residual(p, slot, row0, n0 + c0, min(cols - c0, 64) >> 3, lane);
+}
+
+// A reader's part of a tile: 32 rows, every second chunk of 128 bytes of them (`half` 0 or 1: two readers share the 32 lanes of tensor memory a warp can
+// reach). A lane holds a row, so its own 16-byte stores touched 32 lines each, half a sector at a time, and with one warp a quarter of tensor memory the
+// residual's loads stood in line with them: 4.5 us a tile of 256 x 192 whatever K, 4 us more with a residual. So a finished row goes to the reader's slot, in
+// the place its residual was copied to, and leaves it as whole lines, and there are two warps for a quarter. us before -> after, (one warp a quarter):
+//   2048 x 2048, residual   K 2048 22.6 -> 19.4 (20.9), K 6144 45.0 -> 41.4 (42.8)      2048 x 3072, K 2048  31.6 -> 28.9 (28.6)
+//   1505 x 2048, f32 out    K 2048 18.9 -> 16.6 (16.6), K 6144 40.7 -> 37.8 (38.3)      2048 x (2 x 6144)    83.2 -> 81.8 (81.2; K 64: 34.4 -> 29.8 (35.3))
+// The slots take the place of the seventh stage that tiles of 192 columns had, which does not show.
+// Direct stores stay for rows that do not begin on 16 bytes, and f32 results with a residual.
+template <bool GATED>
+__device__ __forceinline__ void tile_rows(const Gemm2Params& p, uint32_t tm_row, int up, unsigned char* slot, int row0, int n0, int width, int half, int lane) {
+  if (!p.staged) {
+#pragma unroll 1
+    for (int c0 = 32 * half; c0 < width; c0 += 64) {
+      float v[32];
+      tmem_ld_32x32(tm_row + (uint32_t)c0, v);
+      if (GATED) {
+        float u[32];
+        tmem_ld_32x32(tm_row + (uint32_t)(up + c0), u);
+        tmem_ld_wait();
+        gated_all<32>(v, u, p.unit);
+      } else {
+        tmem_ld_wait();
+      }
+      store_row32_2(p, row0 + lane, n0 + c0, v);
+    }
+    return;
+  }
+  const int cols = tile_cols(p, n0, width);
+  if (!GATED && p.out_f32) {
+#pragma unroll 1
+    for (int c0 = 32 * half; c0 < cols; c0 += 64) {
+      float v[32];
+      tmem_ld_32x32(tm_row + (uint32_t)c0, v);
+      tmem_ld_wait();
+      add_bias32(p, n0 + c0, v);
+      finish32(p, v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(slot_piece(slot, lane, i)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      __syncwarp();
+      float* out = reinterpret_cast<float*>(p.c) + n0 + c0 + (lane & 7) * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3);
+        if (row0 + r < p.M) *reinterpret_cast<uint4*>(out + (long)(row0 + r) * p.ldc) = *slot_piece(slot, r, lane & 7);
+      }
+      __syncwarp();
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int c0 = 64 * half; c0 < cols; c0 += 128) {
+    const int col = n0 + c0, pieces = min(cols - c0, 64) >> 3;
+    if (!GATED && p.residual) {
+      if (c0 >= 128) request_residual(p, slot, row0, col, pieces, lane);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (4 * h >= pieces) break;
+      float v[32];
+      tmem_ld_32x32(tm_row + (uint32_t)(c0 + 32 * h), v);
+      if (GATED) {
+        float u[32];
+        tmem_ld_32x32(tm_row + (uint32_t)(up + c0 + 32 * h), u);
+        tmem_ld_wait();
+        gated_all<32>(v, u, p.unit);
+      } else {
+        tmem_ld_wait();
+      }
+      add_bias32(p, col + 32 * h, v);
+      if (!GATED && p.residual) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) add_residual8(v + 8 * i, *slot_piece(slot, lane, 4 * h + i));
+      }
+      finish32(p, v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *slot_piece(slot, lane, 4 * h + i) = pack8(v + 8 * i);
+    }
+    __syncwarp();
+    bf16* out = reinterpret_cast<bf16*>(p.c) + col + (lane & 7) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = 4 * i + (lane >> 3);
+      if (row0 + r < p.M && (lane & 7) < pieces) *reinterpret_cast<uint4*>(out + (long)(row0 + r) * p.ldc) = *slot_piece(slot, r, lane & 7);
+    }
+    __syncwarp();
+  }
+}
+
+// grid (2 * M / 256, N / 256), clusters of 2 along x; THREADS2 threads
 template <int TN>
-__global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+__global__ void __launch_bounds__(THREADS2) tc_gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                                           Gemm2Params p) {
   using C2 = Cfg2<TN>;
   constexpr int HALF_N = C2::HALF_N, STAGES2 = C2::STAGES2, A2_BYTES = C2::A2_BYTES, STAGE2_BYTES = C2::STAGE2_BYTES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES2 * STAGE2_BYTES);
+  unsigned char* slots = smem + C2::RING2;
+  uint64_t* full = reinterpret_cast<uint64_t*>(slots + READERS * SLOT_BYTES);
   uint64_t* empty = full + STAGES2;
   uint64_t* acc_full = empty + STAGES2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
@@ -213,23 +334,17 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant_
     umma_commit_pair(acc_full);                  // both CTAs' accumulators are complete (or abandoned)
   } else if (warp >= 2) {
     // ---- epilogue (both CTAs): this CTA's 128 rows ----
+    const int q = warp & 3, half = (warp - 2) >> 2, row0 = m0 + q * 32;
+    unsigned char* slot = slots + (warp - 2) * SLOT_BYTES;
+    request_first(p, slot, row0, n0, TN, half, lane);
     const bool ready = mbar_wait(acc_full, 0, p.spin_limit);
     tc_fence_after();
     if (!ready) {
       *abort_flag = 1;
       if (lane == 0 && p.status) atomicOr(p.status, IFAB_STATUS_MBAR_TIMEOUT);
     }
-    if (ready && !*abort_flag) {
-      const int q = warp & 3;
-      const int row = m0 + q * 32 + lane;
-#pragma unroll 1
-      for (int c0 = 0; c0 < TN; c0 += 32) {
-        float v[32];
-        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-        tmem_ld_wait();
-        store_row32_2(p, row, n0 + c0, v);
-      }
-    }
+    if (ready && !*abort_flag) tile_rows<false>(p, tmem_base + ((uint32_t)(q * 32) << 16), 0, slot, row0, n0, TN, half, lane);
+    else asm volatile("cp.async.wait_all;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -244,7 +359,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_kernel(const __grid_constant_
 // One CTA pair per SM pair (at most 74 pairs) walks the 256 x 256 tiles round-robin. Tensor memory holds TWO accumulators
 // (2 x 256 columns = all 512): while the epilogue warps of both CTAs drain tile j, the leader already issues the MMAs of tile
 // j + 1 into the other half, and the producers keep the stage ring full across tile boundaries. An accumulator half goes back
-// to the issuer when the eight epilogue warps of the pair (four per CTA) have arrived on the leader's acc_empty barrier.
+// to the issuer when the epilogue warps of both CTAs have arrived on the leader's acc_empty barrier.
 // Tile order of the persistent walk: groups of RASTER_M tile rows, inside a group the row index runs fastest. The 74 pairs
 // that work at the same time then share a few B tiles (each read by up to RASTER_M pairs back to back) and keep RASTER_M
 // tile rows of A in L2, instead of sweeping all of B for every tile row (at 8192^3 B alone is 128 MB - more than L2).
@@ -261,18 +376,19 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-// grid (2 * pairs), clusters of 2; 192 threads
+// grid (2 * pairs), clusters of 2; THREADS2 threads
 template <int TN>
-__global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+__global__ void __launch_bounds__(THREADS2) tc_gemm_2sm_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                                                      Gemm2Params p) {
   using C2 = Cfg2<TN>;
   constexpr int HALF_N = C2::HALF_N, STAGES2 = C2::STAGES2, A2_BYTES = C2::A2_BYTES, STAGE2_BYTES = C2::STAGE2_BYTES;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES2 * STAGE2_BYTES);
+  unsigned char* slots = smem + C2::RING2;
+  uint64_t* full = reinterpret_cast<uint64_t*>(slots + READERS * SLOT_BYTES);
   uint64_t* empty = full + STAGES2;
   uint64_t* acc_full = empty + STAGES2;          // [2], one arrival each (the leader's commit, multicast to both CTAs)
-  uint64_t* acc_empty = acc_full + 2;            // [2], used in the leader only: eight arrivals each (epilogue warps of both CTAs)
+  uint64_t* acc_empty = acc_full + 2;            // [2], used in the leader only: an arrival of every epilogue warp of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -290,7 +406,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 8);
+      mbar_init(&acc_empty[b], 2 * READERS);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -357,41 +473,26 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
     }
   } else if (warp >= 2) {
     // ---- epilogue (both CTAs) ----
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    unsigned char* slot = slots + (warp - 2) * SLOT_BYTES;
     int j = 0;
     for (int t = pair; t < tiles; t += pairs, ++j) {
       const int b = j & 1;
+      int tm, tn;
+      tile_coords(t, tiles_m, tiles_n, &tm, &tn);
+      const int row0 = tm * 2 * BM + (int)rank * BM + q * 32, n0 = F > 0 ? tn * HALF_N : tn * TN;
+      request_first(p, slot, row0, n0, F > 0 ? HALF_N : TN, half, lane);
       const bool ready = mbar_wait(&acc_full[b], (j >> 1) & 1, p.spin_limit);
       tc_fence_after();
       if (!ready || *abort_flag) {
         *abort_flag = 1;
         if (lane == 0 && p.status) atomicOr(p.status, IFAB_STATUS_MBAR_TIMEOUT);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         break;
       }
-      int tm, tn;
-      tile_coords(t, tiles_m, tiles_n, &tm, &tn);
-      const int m0 = tm * 2 * BM + (int)rank * BM, n0 = F > 0 ? tn * HALF_N : tn * TN;
-      const int row = m0 + q * 32 + lane;
       const uint32_t tm_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * C2::COLS);
-      if (F > 0) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < HALF_N; c0 += 32) {
-          float v[32], u[32];
-          tmem_ld_32x32(tm_row + (uint32_t)c0, v);
-          tmem_ld_32x32(tm_row + (uint32_t)(HALF_N + c0), u);
-          tmem_ld_wait();
-          gated_all<32>(v, u, p.unit);
-          store_row32_2(p, row, n0 + c0, v);
-        }
-      } else {
-#pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += 32) {
-          float v[32];
-          tmem_ld_32x32(tm_row + (uint32_t)c0, v);
-          tmem_ld_wait();
-          store_row32_2(p, row, n0 + c0, v);
-        }
-      }
+      if (F > 0) tile_rows<true>(p, tm_row, HALF_N, slot, row0, n0, HALF_N, half, lane);
+      else tile_rows<false>(p, tm_row, 0, slot, row0, n0, TN, half, lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[b]), 0));
@@ -406,6 +507,7 @@ __global__ void __launch_bounds__(192) tc_gemm_2sm_persistent_kernel(const __gri
   }
 }
 
+bool on_16(const void* rows, long ld, int bytes) { return reinterpret_cast<uintptr_t>(rows) % 16 == 0 && ld * bytes % 16 == 0; }
 int pairs_of_device() { return std::max(1, device_sms() / 2); }
 // Columns of a tile: of 256, 192 and 128 the width whose waves of tiles over the pairs take least. A K block costs a pair what it loads - 128 rows of A
 // and TN / 2 of B in each CTA, about 87 GB/s an SM - rather than what it multiplies, so narrow tiles gain less than their width: 2048 x 3072 (K 2048)
@@ -431,11 +533,11 @@ int launch_2sm(const void* a, long lda, const void* b, long ldb, const Gemm2Para
   if (!persistent) {
     auto k = tc_gemm_2sm_kernel<TN>;
     if (int rc = opt_in_smem(k, smem)) return rc;
-    return launch_chain_cluster(k, dim3(2 * ((p.M + 255) / 256), cols), dim3(192), 2, (size_t)smem, s, ta, tb, p);
+    return launch_chain_cluster(k, dim3(2 * ((p.M + 255) / 256), cols), dim3(THREADS2), 2, (size_t)smem, s, ta, tb, p);
   }
   auto k = tc_gemm_2sm_persistent_kernel<TN>;
   if (int rc = opt_in_smem(k, smem)) return rc;
-  return launch_chain_cluster(k, dim3(2 * std::max(1, std::min(tiles, pairs))), dim3(192), 2, (size_t)smem, s, ta, tb, p);
+  return launch_chain_cluster(k, dim3(2 * std::max(1, std::min(tiles, pairs))), dim3(THREADS2), 2, (size_t)smem, s, ta, tb, p);
 }
 int dispatch_2sm(const void* a, long lda, const void* b, long ldb, const Gemm2Params& p, int persistent, cudaStream_t s) {
   const int pairs = pairs_of_device(), tn = tile_width(p.M, p.N, pairs);
@@ -466,7 +568,8 @@ extern "C" int ifab_gemm_act_bf16_2sm(const void* a, long lda, const void* b, lo
 extern "C" int ifab_gemm_epilogue_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
                                            const float* bias, int act, float cap, int persistent, int M, int N, int K, uint32_t* status, void* stream) {
   if (M < 1 || N < 32 || N % 32 || K < 8 || K % 8 || lda % 8 || ldb % 8) return -1;
-  const Gemm2Params p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, 0, act, bias, cap, {}};
+  const int staged = on_16(c, ldc, out_f32 ? 4 : 2) && (!residual || (!out_f32 && on_16(residual, ldr, 2)));
+  const Gemm2Params p{c, ldc, out_f32, (const bf16*)residual, ldr, M, N, K, status, 4000000u, staged, 0, act, bias, cap, {}};
   return dispatch_2sm(a, lda, b, ldb, p, persistent, (cudaStream_t)stream);
 }
 extern "C" int ifab_gemm_bf16_2sm(const void* a, long lda, const void* b, long ldb, void* c, long ldc, int out_f32, const void* residual, long ldr,
@@ -488,6 +591,6 @@ extern "C" int ifab_gemm_gated_bf16_2sm(const void* a, long lda, const void* b, 
                                         int K, uint32_t* status, void* stream) {
   const GatedUnit gu{unit, limit, alpha};
   if (!gated_ok(gu) || M < 1 || F < 32 || F % 32 || K < 8 || K % 8 || lda % 8 || ldb % 8) return -1;
-  const Gemm2Params p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, F, 0, nullptr, 0.f, gu};
+  const Gemm2Params p{c, ldc, 0, nullptr, 0, M, 2 * F, K, status, 4000000u, on_16(c, ldc, 2), F, 0, nullptr, 0.f, gu};
   return dispatch_2sm(a, lda, b, ldb, p, 1, (cudaStream_t)stream);
 }

@@ -65,3 +65,43 @@ def test_two_sm_swiglu_projection(M, F, K):
     one = torch.empty(nt * 128, F, dtype=BF16, device="cuda")
     P.grouped_gemm(ap, b.unsqueeze(0), tiles.cuda(), torch.tensor([nt], dtype=torch.int32, device="cuda"), one, swiglu=True)
     assert torch.equal(out, one[:M])
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 32, 64), (255, 96, 136), (129, 288, 64), (300, 224, 72), (257, 2080, 64), (4100, 3104, 128)])
+def test_rows_by_shared_memory_are_the_direct_ones(M, N, K, persistent):
+    """Rows that begin on 16 bytes leave as whole lines by way of shared memory, others straight from the accumulator's registers: the same
+    products rounded the same way, so both are, bit for bit, the f32 results rounded, with the residual added and rounded again. Nothing
+    beside the result is written. N covers the last chunk of 32 columns in tiles of 256, 192 and 128, M the rows beyond a tile's end."""
+    from ironpangu_b200.ops.gemm import gemm_2sm, gemm_swiglu
+    g = torch.Generator(device="cuda").manual_seed(0)
+    bf = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, b, base = bf(M, K), bf(N, K), bf(M + 1, N + 16)
+    f32 = gemm_2sm(a, b, out_f32=True, status_ptr=st.data_ptr(), persistent=persistent)
+    wide = torch.full((M + 1, N + 16), 7., device="cuda")
+    gemm_2sm(a, b, out=wide[:M, 1:1 + N], status_ptr=st.data_ptr(), persistent=persistent)
+    assert torch.equal(wide[:M, 1:1 + N], f32)
+    gemm_2sm(a, b, out=wide[:M, 4:4 + N], status_ptr=st.data_ptr(), persistent=persistent)
+    assert torch.equal(wide[:M, 4:4 + N], f32) and bool((wide[:, 4 + N:] == 7.).all()) and bool((wide[M] == 7.).all())
+    for off in (8, 3):
+        c = base.clone()
+        want = base.clone()
+        want[:M, off:off + N] = (f32.to(torch.bfloat16).float() + base[:M, off:off + N].float()).to(torch.bfloat16)
+        view = c[:M, off:off + N]
+        gemm_2sm(a, b, residual=view, out=view, status_ptr=st.data_ptr(), persistent=persistent)
+        assert torch.equal(c, want)
+        view.copy_(base[:M, off:off + N])
+        gemm_2sm(a, b, out=view, status_ptr=st.data_ptr(), persistent=persistent)
+        want[:M, off:off + N] = f32.to(torch.bfloat16)
+        assert torch.equal(c, want)
+    outs = []
+    F = (N + 63) // 64 * 32
+    packed = bf(2 * F, K)
+    for off in (8, 3):
+        c = torch.full((M + 1, F + 16), 7., device="cuda", dtype=torch.bfloat16)
+        gemm_swiglu(a, packed, out=c[:M, off:off + F], status_ptr=st.data_ptr())
+        outs.append(c[:M, off:off + F].clone())
+        c[:M, off:off + F] = 7.
+        assert bool((c == 7.).all())
+    assert torch.equal(*outs) and st.item() == 0
