@@ -1,6 +1,6 @@
 // Prefill-side MoE plumbing around the grouped tcgen05 GEMM (tc_grouped.cu), for chunks of hundreds of tokens:
 //
-//   router_block_kernel   f32 router projection + top-k for blocks of 8 tokens (the decode router handles <= 8 rows
+//   router_block_kernel   f32 router projection + top-k for blocks of 8 tokens, the experts shared by a cluster (the decode router handles <= 8 rows
 //                         per launch; a prefill chunk would need 64 launches)
 //   moe_dispatch_kernel   routes of this rank's experts -> rows sorted by expert (stable: token-major inside an
 //                         expert), per-expert counts, the 128-row tile table of the grouped GEMM and, for every
@@ -29,74 +29,104 @@ struct RouterBlockParams {
   const float* w; const float* bias;
   float* logits; int32_t* ids; float* wts; bf16* xn; long ldxn;
   int M, D, E, topk, scoring, renorm; float scale;
+  int ranks;          // CTAs of a cluster
 };
 
-// one CTA per T tokens (8, or 4 when that is what fills the SMs); warps stride over the experts, then warp t selects for token t. Bound by the latency of
-// the router's rows in L2 (each CTA reads all of them), so sixteen warps with eight loads each in flight: 512 tokens, 96 experts x 4096: 84.6 us with
-// eight warps, 54.5 us with sixteen.
-template <int T>
+// the float at `at` of this CTA's shared memory, as CTA `rank` of the cluster holds it
+__device__ __forceinline__ float ld_of_rank(const float* at, int rank) {
+  uint32_t addr;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void router_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A cluster per T tokens (8; 4 where the rows of 8 don't fit), each of its CTAs a share of the experts; a warp takes EG experts at a time through all
+// columns, and after a cluster barrier warp t selects for a token from the shares' logits. Bound by the issue of its multiply-adds and by the router's rows
+// from L2. One CTA for all experts of 4 tokens read every row of the router in each of 128 CTAs (201 MB of L2 reads for 512 tokens) and unpacked the tokens'
+// bf16 columns anew for every expert; a share of the experts halves the reads, and EG experts at a time share the unpacked columns.
+// us before -> after, 96 experts x 4096: 16 tokens 49.3 -> 24.2, 256 67.6 -> 28.6, 512 82.5 -> 35.7, 1100 86.2 -> 55.1, 4096 280 -> 216; 512 tokens with 128 x 2048
+// 61.6 -> 29.7, 256 x 7168 334 -> 101. A sum's order is that of one expert and token alone, so shares and widths don't show in the results.
+template <int T, int EG>
 __global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* xs = reinterpret_cast<bf16*>(smem_raw);               // [8][D] normalised
-  float* lg = reinterpret_cast<float*>(xs + (size_t)T * p.D); // [8][E]
+  bf16* xs = reinterpret_cast<bf16*>(smem_raw);               // [T][D] normalised
+  float* lg = reinterpret_cast<float*>(xs + (size_t)T * p.D); // [T][share]
   __shared__ float red[T * 33];
   grid_dep_launch();
   grid_dep_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = blockIdx.x * T;
+  const int ranks = p.ranks, rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * T;
+  const int share = p.E / ranks, e0 = rank * share;      // ranks divides E
   stage_x<T>(xs, p.x, p.ldx, t0, p.M, p.D, p.norm_w, p.eps, false, red);
-  if (p.xn) {   // the normalised rows are reused by the expert GEMMs
-    for (int i = threadIdx.x; i < T * (p.D >> 3); i += blockDim.x) {
-      const int t = i / (p.D >> 3), c = i % (p.D >> 3);
-      if (t0 + t < p.M) *reinterpret_cast<uint4*>(p.xn + (long)(t0 + t) * p.ldxn + c * 8) = *reinterpret_cast<const uint4*>(xs + (size_t)t * p.D + c * 8);
-    }
-  }
   const int quads = p.D >> 2;
-  for (int e = warp; e < p.E; e += 16) {
-    const float4* wr = reinterpret_cast<const float4*>(p.w + (long)e * p.D);
-    float acc[T];
+  for (int first = warp * EG; first < share; first += 16 * EG) {
+    const float4* wr[EG];
 #pragma unroll
-    for (int t = 0; t < T; ++t) acc[t] = 0.f;
-    // eight 16-byte weight loads in flight per lane: issued one at a time the loop waits for L2 on every iteration
-    constexpr int G = 8;
+    for (int j = 0; j < EG; ++j) wr[j] = reinterpret_cast<const float4*>(p.w + (long)(e0 + min(first + j, share - 1)) * p.D);
+    float acc[EG][T];
+#pragma unroll
+    for (int j = 0; j < EG; ++j)
+#pragma unroll
+      for (int t = 0; t < T; ++t) acc[j][t] = 0.f;
+    // several 16-byte weight loads in flight per lane: issued one at a time the loop waits for L2 on every iteration
+    constexpr int G = EG == 1 ? 8 : EG == 2 ? 4 : EG == 3 ? 3 : 2;
     for (int c0 = lane; c0 < quads; c0 += 32 * G) {
-      float4 wv[G];
+      float4 wv[EG][G];
 #pragma unroll
-      for (int g = 0; g < G; ++g) wv[g] = (c0 + 32 * g < quads) ? __ldg(wr + c0 + 32 * g) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int j = 0; j < EG; ++j) wv[j][g] = (c0 + 32 * g < quads) ? __ldg(wr[j] + c0 + 32 * g) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const int c = c0 + 32 * g;
         if (c < quads) {
 #pragma unroll
           for (int t = 0; t < T; ++t) {
-            const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(xs + (size_t)t * p.D + c * 4);
-            const float2 a = __bfloat1622float2(xp[0]), b = __bfloat1622float2(xp[1]);
-            acc[t] += wv[g].x * a.x + wv[g].y * a.y + wv[g].z * b.x + wv[g].w * b.y;
+            const uint2 x4 = *reinterpret_cast<const uint2*>(xs + (size_t)t * p.D + c * 4);
+            const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x4.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x4.y));
+#pragma unroll
+            for (int j = 0; j < EG; ++j) acc[j][t] += wv[j][g].x * a.x + wv[j][g].y * a.y + wv[j][g].z * b.x + wv[j][g].w * b.y;
           }
         }
       }
     }
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-      const float v = warp_sum(acc[t]);
-      if (lane == 0) {
-        lg[t * p.E + e] = v;
-        if (p.logits && t0 + t < p.M) p.logits[(long)(t0 + t) * p.E + e] = v;
+    for (int j = 0; j < EG; ++j) {
+      if (first + j >= share) break;
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const float v = warp_sum(acc[j][t]);
+        if (lane == 0) {
+          lg[t * share + first + j] = v;
+          if (p.logits && t0 + t < p.M) p.logits[(long)(t0 + t) * p.E + e0 + first + j] = v;
+        }
       }
     }
   }
-  __syncthreads();
-  const int t = warp;
-  if (t >= T || t0 + t >= p.M) return;
+  router_cluster_sync();             // the logits of every share, and all CTAs' rows of x read (xn may be x)
+  if (p.xn) {   // the normalised rows are reused by the expert GEMMs
+    for (int i = threadIdx.x; i < T * (p.D >> 3); i += blockDim.x) {
+      const int t = i / (p.D >> 3), c = i % (p.D >> 3);
+      if (t % ranks == rank && t0 + t < p.M) *reinterpret_cast<uint4*>(p.xn + (long)(t0 + t) * p.ldxn + c * 8) = *reinterpret_cast<const uint4*>(xs + (size_t)t * p.D + c * 8);
+    }
+  }
+  const int t = warp * ranks + rank;
   constexpr int PER = 8;
   float score[PER], sel[PER];
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int ei = lane + 32 * i;
-    score[i] = (ei < p.E) ? lg[t * p.E + ei] : -INFINITY;
+    score[i] = (t < T && ei < p.E) ? ld_of_rank(lg + t * share + ei % share, ei / share) : -INFINITY;
     mx = fmaxf(mx, score[i]);
   }
+  router_cluster_sync();             // no CTA leaves while another reads its share
+  if (t >= T || t0 + t >= p.M) return;
   mx = warp_max(mx);
   float denom = 0.f;
 #pragma unroll
@@ -326,24 +356,35 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(CombineParams p, int q
   }
 }
 
+template <int T, int EG>
+int launch_router_of(const RouterBlockParams& p, size_t smem, cudaStream_t s) {
+  if (int rc = opt_in_smem(router_block_kernel<T, EG>, smem)) return rc;
+  return launch_chain_cluster(router_block_kernel<T, EG>, dim3((p.M + T - 1) / T * p.ranks), dim3(512), (unsigned)p.ranks, smem, s, p);
+}
+// As many CTAs (a power of two that divides the experts, up to 8) share a block's experts as leave every CTA an SM of its own (a CTA costs 16 us beside its
+// experts' 38 us at 96 x 4096, so a second wave of smaller shares gains nothing: 1200 tokens by 1 105 us, by 2 three waves of 36); a warp's experts in as few
+// passes of up to four as they take, all as wide.
+template <int T>
+int launch_router(RouterBlockParams p, cudaStream_t s) {
+  p.ranks = 1;
+  while (p.ranks < 8 && (long)((p.M + T - 1) / T) * 2 * p.ranks <= 148 && p.E % (2 * p.ranks) == 0) p.ranks *= 2;
+  const int share = p.E / p.ranks, a_warp = (share + 15) / 16, passes = (a_warp + 3) / 4, width = (a_warp + passes - 1) / passes;
+  const size_t smem = (size_t)T * p.D * sizeof(bf16) + (size_t)T * share * sizeof(float);
+  return width == 1 ? launch_router_of<T, 1>(p, smem, s) : width == 2 ? launch_router_of<T, 2>(p, smem, s) : width == 3 ? launch_router_of<T, 3>(p, smem, s)
+                                                                                                                       : launch_router_of<T, 4>(p, smem, s);
+}
+
 }  // namespace
 
 extern "C" int ifab_router_block(const void* x, long ldx, const void* norm_w, float eps, const float* w_router, const float* bias,
                                  float* logits, int32_t* ids, float* wts, void* xn, long ldxn, int M, int D, int E, int topk,
                                  int scoring, int renorm, float scale, void* stream) {
   if (M < 1 || E > 256 || topk > MAX_TOPK || topk > E || D % 8) return -1;
-  RouterBlockParams p{(const bf16*)x, ldx, (const bf16*)norm_w, eps, w_router, bias, logits, ids, wts, (bf16*)xn, ldxn,
-                      M, D, E, topk, scoring, renorm, scale};
-  // eight tokens per CTA re-read the router matrix least often; with fewer than ~150 such CTAs half the SMs idle, so chunks of
-  // up to ~1200 tokens run four tokens per CTA
-  if ((M + 7) / 8 >= 148) {
-    const size_t smem = (size_t)8 * D * sizeof(bf16) + (size_t)8 * E * sizeof(float);
-    if (int rc = opt_in_smem(router_block_kernel<8>, smem)) return rc;
-    return launch_chain(router_block_kernel<8>, dim3((M + 7) / 8), dim3(512), smem, (cudaStream_t)stream, p);
-  }
-  const size_t smem = (size_t)4 * D * sizeof(bf16) + (size_t)4 * E * sizeof(float);
-  if (int rc = opt_in_smem(router_block_kernel<4>, smem)) return rc;
-  return launch_chain(router_block_kernel<4>, dim3((M + 3) / 4), dim3(512), smem, (cudaStream_t)stream, p);
+  const RouterBlockParams p{(const bf16*)x, ldx, (const bf16*)norm_w, eps, w_router, bias, logits, ids, wts, (bf16*)xn, ldxn,
+                            M, D, E, topk, scoring, renorm, scale, 1};
+  // Rows of eight tokens up to 14000 columns; wider ones run four tokens per CTA, up to ~1200 tokens
+  if ((M + 7) / 8 >= 148 || (size_t)8 * (D * sizeof(bf16) + E * sizeof(float)) <= 224 * 1024) return launch_router<8>(p, (cudaStream_t)stream);
+  return launch_router<4>(p, (cudaStream_t)stream);
 }
 
 extern "C" int ifab_moe_dispatch(const int32_t* ids, int M, int topk, int e0, int e_local, int32_t* counts, int32_t* route_row,

@@ -108,6 +108,32 @@ def test_router_block_matches_reference():
     torch.testing.assert_close(wts, rw, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("M,E,D,topk,sigmoid", [(1, 96, 256, 6, False), (9, 7, 264, 2, True), (60, 16, 1000, 4, False), (45, 100, 520, 16, True), (300, 96, 1024, 6, False),
+                                                (333, 256, 512, 8, True), (1190, 130, 264, 6, False), (20, 64, 15000, 4, False)])
+def test_router_block_shares(M, E, D, topk, sigmoid):
+    """Every share of the experts (clusters of 8 to 1, experts that no power of two divides, one to four experts a warp) and rows too wide for blocks
+    of eight. A logit is D / 32 sums in a lane and five across lanes, so it is within (D / 32 + 8) 2^-24 of the sum of its products' magnitudes."""
+    from ironpangu_b200.ops import prefill as P
+
+    g = torch.Generator(device="cuda").manual_seed(M + E)
+    x = torch.randn(M, D, generator=g, device="cuda").to(BF16)
+    wr, bias = torch.randn(E, D, generator=g, device="cuda") * D ** -0.5, torch.randn(E, generator=g, device="cuda") * 0.1
+    logits = torch.full((M + 1, E), 7., device="cuda")
+    ids = torch.full((M + 1, topk), 7, dtype=torch.int32, device="cuda")
+    wts = torch.full((M + 1, topk), 7., device="cuda")
+    xn = x.clone()
+    P.router_block(xn, wr, topk, ids[:M], wts[:M], norm_w=torch.ones(D, dtype=BF16, device="cuda"), logits=logits[:M], xn=xn, bias=bias if sigmoid else None,
+                   scoring="sigmoid_bias_group_topk" if sigmoid else "softmax")
+    bound = (D / 32 + 8) * 2 ** -24 * (xn.double().abs() @ wr.double().abs().T)
+    assert bool(((logits[:M].double() - xn.double() @ wr.double().T).abs() <= bound).all())
+    score = torch.sigmoid(logits[:M].double()) if sigmoid else torch.softmax(logits[:M].double(), -1)
+    want = torch.topk(score + bias.double() if sigmoid else score, topk).indices
+    assert torch.equal(ids[:M].long(), want)
+    w = score.gather(1, want)
+    torch.testing.assert_close(wts[:M].double(), w / w.sum(-1, keepdim=True), rtol=1e-5, atol=1e-7)
+    assert bool((logits[M] == 7).all() and (ids[M] == 7).all() and (wts[M] == 7).all())
+
+
 @pytest.mark.parametrize("m,window", [(19, 0), (150, 0), (40, 8)])
 def test_prefill_matches_oracle_and_decode_continues(m, window):
     from ironpangu_b200.models.mla_moe import MlaMoeConfig, MlaMoeDecoder, random_full_weights, shard_weights
