@@ -3,10 +3,12 @@
 // Storage: a weight matrix [rows, K] is kept as one byte per element plus one f32 scale per 1 x 128 block of a row
 // (scales[row][ceil(K / 128)]); the represented value is fp8(w[row][k]) * scale[row][k / 128]. Decode linears are bound
 // by the HBM stream of the weights, so halving the bytes of the expert matrices - 3/4 of the bytes a token touches in a
-// mixture-of-experts layer - is what this buys; the arithmetic stays f32: every lane converts its 16-byte chunk (16
-// weights) to f32, forms the chunk's dot product with the bf16 activations staged in shared memory, and scales it once.
-// The kernels mirror the bf16 ones of decode_moe.cu (same grids, same routing inputs, same fused all-reduce), only the
-// chunk geometry differs: 16 elements per 16-byte load instead of 8.
+// mixture-of-experts layer - is what this buys. Two forms:
+//   expert_gate_up_kernel, expert_down_kernel   one rank: every listed expert is streamed through rings in shared memory once for all
+//                       tokens that chose it, its weights widened once, and multiplied on the tensor cores
+//   the kernels that mirror the bf16 ones of decode_moe.cu (same grids, same routing inputs, same fused all-reduce)   several ranks, and
+//                       sizes whose rows don't fit beside the rings: every lane converts its 16-byte chunk (16 weights), forms the
+//                       chunk's dot product with the activations staged in shared memory, and scales it once
 // Reference: W8A8 expert matrices of the 92B program (dequantising grouped matmul, native/src/token_executor.h:640-700).
 #include <cuda_fp8.h>
 

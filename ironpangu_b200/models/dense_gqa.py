@@ -3,7 +3,8 @@ decode kernels, with tensor parallelism over the fused row-parallel GEMV + all-r
 
 Per layer and step: qkv GEMV (norm prologue) -> RoPE + paged KV append -> split-KV GQA attention ->
 o_proj GEMV fused with all-reduce + residual -> gate_up GEMV (norm prologue, SwiGLU epilogue) ->
-down GEMV fused with all-reduce + residual. 6 launches per layer, no stand-alone collective.
+down GEMV fused with all-reduce + residual. 6 launches per layer, no stand-alone collective; on one
+rank 5, as the qkv launch rotates and appends, and the linears are streams through rings in shared memory.
 Query rows of different sequences (continuous batching) share every launch: each row carries its
 own position and sequence slot. Sampling is greedy (fused with the lm_head) or top-k / top-p on the
 device. The reference's dense family runs per-layer composites of vendor ops with an all-gather

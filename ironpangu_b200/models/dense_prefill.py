@@ -5,7 +5,8 @@ The decode kernels of ``DenseDecoder`` multiply at most 8 rows per pass on the C
 matrix-matrix work: the four linears of a layer on the tcgen05 GEMM (gate/up
 with the SwiGLU epilogue, the row-parallel o_proj and down projections through the fused GEMM + all-reduce kernel when the
 model is tensor parallel), rotary + cache append through the decode path's kernel, attention through its split-KV kernels
-with one query row per token (causality comes from the per-row positions), ``attn_rows`` query rows per launch.
+with one query row per token (causality comes from the per-row positions), ``attn_rows`` query rows per launch. Up to eight rows on
+one rank take the decoder's streaming linears instead (``_few``).
 It shares weights, caches and the page table with the decoder, so decode continues from the state it leaves.
 
 Sequence-parallel mode (``sequence_parallel=True``, tensor-parallel models, chunks of a multiple of ``128 * world`` rows): the
