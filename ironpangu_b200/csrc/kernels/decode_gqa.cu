@@ -703,11 +703,13 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
       }
-      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight).
-      const int warps = cluster && rows * p.max_splits <= 148 ? 8 : 4;
+      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). Sixteen
+      // clusters of eight such CTAs do not fit the GPCs at once (4 rows of 1000 keys, four kv heads of two: 11.6 us by eight, 7.9 by four).
+      const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : 148) ? 8 : 4;
       p.split_shift = log2_of(p.max_splits);
-      // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so
-      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > 296;
+      // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
+      // less than their order (60 rows of 100 keys 11.7 and 13.5)
+      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > 296 && (long)p.kps * asked > 512;
       if (p.page_tokens % 16 == 0 && !p.ahead.any())
         return G == 8 ? launch_mma<HD, true, true>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, true>(p, cluster, warps, out, ldo, s);
       return G == 8 ? launch_mma<HD, true, false>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, false>(p, cluster, warps, out, ldo, s);
