@@ -503,8 +503,9 @@ class PlanEngine:
             w[p + "shared_down"] = self._param(dn["shared_weight"])
 
     def _turns_in_projection(self, g: dict) -> bool:
-        """Whether a grouped-query group's rotation and page write are part of its projection's launch."""
-        return self._rings and bool(g["norm"]) and g["rotary_dim"] == int(self.ins[g["members"][-1]]["attrs"]["head_dim"])
+        """Whether a grouped-query group's rotation and page write are part of its projection's launch, which normalises its rows (an optional norm
+        whose gain the checkpoint lacks passes them on)."""
+        return self._rings and g["norm"] in self.P and g["rotary_dim"] == int(self.ins[g["members"][-1]]["attrs"]["head_dim"])
 
     def _describe_dense(self, emb: dict, head: dict) -> None:
         """The same for a stack of {grouped-query attention, SwiGLU} layers, in the vocabulary of ``models/dense_gqa.py``: the

@@ -101,6 +101,38 @@ def test_gpu_bundle_engine_equals_the_hand_wired_dense_decoder(tmp_path, fused):
 
 
 @pytest.mark.gpu
+def test_gpu_optional_norm_the_checkpoint_lacks(tmp_path):
+    """A projection behind an optional norm without a gain takes its rows as they are: the steps and the launches of the program without that norm."""
+    from ironpangu_b200.parallel.fabric import Fabric
+    from ironpangu_b200.runtime.plan_engine import PlanEngine
+
+    cfg = G.DenseConfig.tiny(2)
+    text = dense_gqa_source(cfg, 1, 64)
+    norm, after = f"norm(x, weight = w.input_layernorm, eps = {cfg.eps!r})", f"norm(h, weight = w.post_attention_layernorm, eps = {cfg.eps!r})"
+    assert norm in text and after in text
+    fab = Fabric(0, 1)
+    P = {k: v for k, v in G.bundle_parameters(cfg, G.random_rank_weights(cfg, 0, 1, torch.device("cuda", 0), seed=4)).items() if "layernorm" not in k}
+    engines = []
+    for name, operand in (("optional", "optional_" + norm), ("plain", "x")):
+        src = tmp_path / f"{name}.inferfabric"
+        src.write_text(text.replace(norm, operand).replace(after, "h"))
+        out = compiler.write_bundle(src, tmp_path / name, prefill_tokens=8)
+        engines.append(PlanEngine(out["dir"], None, fab, max_tokens=8, keep_logits=True, parameters=P))
+    optional, plain = engines
+    assert all(g["norm"] and g["norm_optional"] for g in optional.gqa_groups.values()) and len(optional.gqa_groups) == cfg.layers
+    assert optional.launches_per_forward == plain.launches_per_forward
+    for e in engines:
+        for at, n in ((0, 3), (3, 1), (4, 8)):
+            e.tokens[:n].copy_(torch.arange(at + 5, at + 5 + n, dtype=torch.int32))
+            e.positions[:n].copy_(torch.arange(at, at + n, dtype=torch.int32))
+            e.slots[:n].zero_()
+            e.forward(n)
+    assert torch.equal(optional.logits, plain.logits) and bool(plain.logits.isfinite().all())
+    assert int(fab.status()) == 0
+    fab.close()
+
+
+@pytest.mark.gpu
 def test_gpu_prompt_executor_runs_on_the_bundle_engine(tmp_path):
     """The dense prompt path (matrix-matrix kernels, chunks of 64 rows) reads a bundle's engine through its decoder facade: it
     leaves the same K / V pages and the same first token as on the hand-wired decoder, and decode continues from them."""
