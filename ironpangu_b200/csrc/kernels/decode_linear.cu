@@ -218,13 +218,14 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 2) qkv_rows_kernel(QkvParams q)
   BfRows<MR, true> x{p.x, p.ldx, p.norm_w, p.eps, p.zero_centered, p.T};
   x.early(stream);
   grid_dep_wait();
-  // where row t's keys and values go (-1: nowhere), and the angle of pair j
+  // where row t's keys and values go (-1: nowhere), whether the head turns (values and rows that are not there do not), and the angle of pair j
   struct Place {
     long row;
+    bool turns;
     float c, s;
   };
   auto place = [&](int t, int n) {
-    Place at{-1, 1.f, 0.f};
+    Place at{-1, false, 1.f, 0.f};
     const int pos = q.positions[t], h = n / q.half, j = n - h * q.half;
     if (pos < 0) return at;
     if (h >= q.Hq) {
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 2) qkv_rows_kernel(QkvParams q)
       else if (q.status) atomicOr(q.status, IFAB_STATUS_BAD_INDEX);
     }
     if (h < q.Hq + q.Hkv) {
+      at.turns = true;
       const float inv_freq = exp2f(-(2.f * (float)j / (float)(2 * q.half)) * log2f(q.theta));
       sincosf((float)pos * inv_freq, &at.s, &at.c);
       at.c = bf16_round(at.c);
@@ -240,15 +242,19 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 2) qkv_rows_kernel(QkvParams q)
     }
     return at;
   };
-  Place mine{-1, 1.f, 0.f};       // requested here: behind the sums it was two more trips to L2
+  Place mine{-1, false, 1.f, 0.f};       // requested here: behind the sums it was two more trips to L2
   int ft, fn;
   if (stream.first_result(p.T, &ft, &fn)) mine = place(ft, fn);
   x.prepare(stream, sums);
   auto out = [&](int t, int n, float v, float u, bool first) {
     const Place at = first ? mine : place(t, n);
     const int h = n / q.half, j = n - h * q.half, hd = 2 * q.half;
-    const float a = bf16_round(v), b = bf16_round(u);
-    const bf16 lo = __float2bfloat16_rn(a * at.c - b * at.s), hi = __float2bfloat16_rn(b * at.c + a * at.s);
+    bf16 lo = __float2bfloat16_rn(v), hi = __float2bfloat16_rn(u);
+    if (at.turns) {          // others are copied: by cosine 1 and sine 0 an infinite column would make NaN of its partner
+      const float a = __bfloat162float(lo), b = __bfloat162float(hi);
+      lo = __float2bfloat16_rn(a * at.c - b * at.s);
+      hi = __float2bfloat16_rn(b * at.c + a * at.s);
+    }
     bf16* to = reinterpret_cast<bf16*>(p.y) + (long)t * p.ldy + h * hd + j;
     if (h >= q.Hq) {
       if (at.row < 0) return;

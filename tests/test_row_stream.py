@@ -132,3 +132,28 @@ def test_projection_with_rotation_and_pages(T, H, kv, hd, K):
                 q = torch.stack([f[t, :H, 0] * c[t] - f[t, :H, 1] * s[t], f[t, :H, 1] * c[t] + f[t, :H, 0] * s[t]], -1).reshape(-1)
                 torch.testing.assert_close(one[t, :H * hd].double(), q, rtol=2 ** -7, atol=2.0 ** -12)
     assert bool((one[:, H * hd:] == 7).all())
+
+
+@pytest.mark.parametrize("T", [2, 8])
+def test_columns_that_do_not_turn_are_copied(T):
+    """Values, and queries of rows that are not there: an infinite or NaN column stays one column, as behind the projection and the rotation in launches of their own."""
+    from ironpangu_b200.ops import decode as D
+
+    H, kv, hd, K, page = 4, 2, 64, 256, 16
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, generator=g, device="cuda").to(BF16)
+    w, gain = (torch.randn((H + 2 * kv) * hd, K, generator=g, device="cuda") * K ** -0.5).to(BF16), torch.ones(K, device="cuda", dtype=BF16)
+    w[(H + kv) * hd + 3, 7] = float("inf")
+    w[(H + kv) * hd + hd + hd // 2 + 5] = float("nan")
+    w[9, 1] = float("inf")
+    table = torch.arange(T, dtype=torch.int32, device="cuda")[:, None].contiguous()
+    pos, slots = torch.arange(T, dtype=torch.int32, device="cuda") + 1, torch.arange(T, dtype=torch.int32, device="cuda")
+    pos[1] = -1
+    k1, v1, k2, v2 = (torch.full((T, page, kv, hd), 7.0, dtype=BF16, device="cuda") for _ in range(4))
+    one = torch.empty(T, (H + 2 * kv) * hd, dtype=BF16, device="cuda")
+    D.qkv_rows(x, w, gain, pos, slots, table, k1, v1, heads=H, kv_heads=kv, head_dim=hd, theta=1e4, eps=1e-6, out=one)
+    two = D.gemv(x, w, norm_w=gain, eps=1e-6, rings=True)
+    D.gqa_rope_kv_write(two, pos, slots, table, k2, v2, heads=H, kv_heads=kv, head_dim=hd, theta=1e4)
+    torch.testing.assert_close(v1, v2, rtol=0, atol=0, equal_nan=True)
+    torch.testing.assert_close(one[1, :H * hd], two[1, :H * hd], rtol=0, atol=0, equal_nan=True)
+    assert int((~v1.isfinite()).sum()) == 2 * (T - 1) and int((~one[1, :H * hd].isfinite()).sum()) == 1
