@@ -173,7 +173,7 @@ class DenseDecoder:
         self.next_ids = torch.zeros(T, dtype=torch.int32, device=dev)
         self.next_vals = torch.zeros(T, dtype=torch.float32, device=dev)
         self.logits = e(T, self.vl, dt=torch.float32) if keep_logits else None
-        self.launches_per_forward = 2 + (5 if self.world == 1 else 6) * c.layers      # one more a layer where few rows of long contexts merge their splits in a launch of their own
+        self.launches_per_forward = 2 + (5 if self.world == 1 and T <= 8 else 6) * c.layers      # one more a layer where few rows of long contexts merge their splits in a launch of their own
         self._graph = None
 
     def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor) -> None:
@@ -192,11 +192,11 @@ class DenseDecoder:
         for l in range(c.layers):
             p = f"layers.{l}."
             qkv = self.qkv[:T]
-            if fab.world == 1:
+            if fab.world == 1 and T <= 8:
                 K.qkv_rows(x, w[p + "qkv"], w[p + "attn_norm"], pos, slot, self.page_table, self.k_cache[l], self.v_cache[l], heads=self.hq, kv_heads=self.hk,
                            head_dim=c.head_dim, theta=c.theta, eps=c.eps, out=qkv, status_ptr=st)
             else:
-                K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv)
+                K.gemv(x, w[p + "qkv"], norm_w=w[p + "attn_norm"], eps=c.eps, out=qkv, rings=fab.world == 1)
                 K.gqa_rope_kv_write(qkv, pos, slot, self.page_table, self.k_cache[l], self.v_cache[l], heads=self.hq,
                                     kv_heads=self.hk, head_dim=c.head_dim, theta=c.theta, status_ptr=st)
             K.gqa_decode_attention(qkv, self.k_cache[l], self.v_cache[l], pos, slot, self.page_table, heads=self.hq,

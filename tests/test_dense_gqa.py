@@ -47,6 +47,25 @@ def test_two_interleaved_sequences_match_oracle():
     fab.close()
 
 
+def test_more_rows_than_a_tile_without_sampling():
+    """Steps without a token to choose take any number of rows: hidden rows and pages of eleven rows are those of eight and three."""
+    runs = []
+    for sizes in ((11,), (8, 3)):
+        cfg, _, fab, dec = _setup(max(sizes))
+        at = 0
+        for n in sizes:
+            dec.tokens[:n].copy_(torch.arange(at + 3, at + 3 + n, dtype=torch.int32))
+            dec.positions[:n].copy_(torch.arange(at, at + n, dtype=torch.int32))
+            dec.slots[:n].zero_()
+            dec.forward(n, sample=False)
+            at += n
+        runs.append((dec.x[:3].clone() if len(sizes) > 1 else dec.x[8:11].clone(), torch.stack(dec.k_cache), torch.stack(dec.v_cache)))
+        assert fab.status() == 0
+        fab.close()
+    for a, b in zip(*runs):
+        torch.testing.assert_close(a, b, rtol=2e-2, atol=2e-2)
+
+
 def test_graph_replay_equals_eager():
     cfg, full, fab, dec = _setup(1, 1)
     outs = []
