@@ -829,7 +829,8 @@ extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* 
       q.ids += t0 * topk;
       q.act += (size_t)t0 * (topk + 1) * F;
       const size_t smem = XP_RING + XP_RED + q.T * row;
-      if (int rc = opt_in_smem(expert_gate_up_kernel, smem)) return rc;
+      // opened for as many tokens as go at once, whatever this step's: by this step's, a thread with fewer tokens would close it for this launch
+      if (int rc = opt_in_smem(expert_gate_up_kernel, XP_RING + XP_RED + at_once * row)) return rc;
       if (int rc = (int)cudaFuncSetAttribute(expert_gate_up_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) return rc;
       if (int rc = launch_chain(expert_gate_up_kernel, dim3(tc::device_sms()), dim3(256), smem, (cudaStream_t)stream, q)) return rc;
     }

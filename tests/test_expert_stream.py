@@ -57,3 +57,34 @@ def test_lists_and_shares(T, E, topk, D, F, Fs, shared):
         assert bool(((y[t].double() - total).abs() <= 2.0 ** -8 * (want.abs() + total.abs()) + 2.0 ** -18 * scale + 1e-6).all())
     assert fab.status() == 0
     fab.close()
+
+
+def test_threads_with_steps_of_different_widths():
+    """The shared memory of a launch depends on the tokens; what the kernel is opened for does not, or one thread's launch would be refused for another's step."""
+    import threading
+    from ironpangu_b200.ops import decode as K
+
+    from ironpangu_b200.ops import _lib
+
+    E, topk, D, F = 4, 2, 4096, 16
+    q, scales = K.quantize_fp8_block((torch.randn(E, 2 * F, D, device="cuda") * 0.05).to(BF16))
+    fn, codes = _lib.load().ifab_moe_gate_up_decode_fp8, set()
+
+    def steps(T):
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            x, ids = torch.ones(T, D, dtype=BF16, device="cuda"), torch.zeros(T, topk, dtype=torch.int32, device="cuda")
+            act = torch.zeros(T, topk + 1, F, dtype=BF16, device="cuda")
+            args = (x.data_ptr(), D, None, 1e-5, ids.data_ptr(), T, D, F, topk, 0, E, q.data_ptr(), scales.data_ptr(), None, None, 0, act.data_ptr(),
+                    torch.cuda.current_stream().cuda_stream)
+            for _ in range(30):
+                for _ in range(200):
+                    codes.add(fn(*args))
+                torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=steps, args=(T,)) for T in (1, 8) * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert codes == {0}
