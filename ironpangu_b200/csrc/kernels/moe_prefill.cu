@@ -358,7 +358,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(CombineParams p, int q
 
 template <int T, int EG>
 int launch_router_of(const RouterBlockParams& p, size_t smem, cudaStream_t s) {
-  if (int rc = opt_in_smem(router_block_kernel<T, EG>, smem)) return rc;
+  // opened for all experts in a CTA, whatever this chunk's share: by the share, a thread with another chunk would close it for this launch
+  if (int rc = opt_in_smem(router_block_kernel<T, EG>, (size_t)T * (p.D * sizeof(bf16) + p.E * sizeof(float)))) return rc;
   return launch_chain_cluster(router_block_kernel<T, EG>, dim3((p.M + T - 1) / T * p.ranks), dim3(512), (unsigned)p.ranks, smem, s, p);
 }
 // As many CTAs (a power of two that divides the experts, up to 8) share a block's experts as leave every CTA an SM of its own (a CTA costs 16 us beside its

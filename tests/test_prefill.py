@@ -134,6 +134,35 @@ def test_router_block_shares(M, E, D, topk, sigmoid):
     assert bool((logits[M] == 7).all() and (ids[M] == 7).all() and (wts[M] == 7).all())
 
 
+def test_router_threads_with_chunks_of_different_lengths():
+    """The shared memory of a router's launch depends on the chunk; what the kernel is opened for does not, or one thread's launch would be refused for another's."""
+    import threading
+    from ironpangu_b200.ops import _lib
+
+    D, E, topk = 4096, 96, 8
+    wr, codes = torch.randn(E, D, device="cuda") * D ** -0.5, set()
+    fn = _lib.load().ifab_router_block
+
+    def chunks(M):
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            x = torch.ones(M, D, dtype=BF16, device="cuda")
+            ids, wts = torch.empty(M, topk, dtype=torch.int32, device="cuda"), torch.empty(M, topk, device="cuda")
+            args = (x.data_ptr(), D, None, 1e-5, wr.data_ptr(), None, None, ids.data_ptr(), wts.data_ptr(), None, 0, M, D, E, topk, 0, 1, 1.0,
+                    torch.cuda.current_stream().cuda_stream)
+            for _ in range(30):
+                for _ in range(100):
+                    codes.add(fn(*args))
+                torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=chunks, args=(M,)) for M in (400, 700) * 3]     # the same kernel, with half of the experts to a CTA and with all
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert codes == {0}
+
+
 @pytest.mark.parametrize("m,window", [(19, 0), (150, 0), (40, 8)])
 def test_prefill_matches_oracle_and_decode_continues(m, window):
     from ironpangu_b200.models.mla_moe import MlaMoeConfig, MlaMoeDecoder, random_full_weights, shard_weights
