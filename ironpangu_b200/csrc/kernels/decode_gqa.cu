@@ -12,6 +12,9 @@
 // Query rows carry their own position and sequence slot (continuous batching: rows of different
 // sequences and prefill chunks share one launch). Reference counterparts: attention_qk_prepare /
 // paged_attention_prepare composites (native/src/inferfabric_acl.cpp:1236-1433).
+#include <climits>
+#include <type_traits>
+
 #include "attn_rule.cuh"
 #include "mma16816.cuh"
 #include "gemv.cuh"
@@ -136,10 +139,9 @@ struct GqaParams {
 // what a row sees: entries ahead of its window, then the positions first .. pos
 struct Seen {
   int first, ahead, n;
-  // `pages`: counted from the sixteen positions on that the first lies among
-  __device__ __forceinline__ Seen(const GqaParams& p, int pos, bool pages = false) : first(first_key(pos, p.window, p.rule.chunked)) {
+  __device__ __forceinline__ Seen(const GqaParams& p, int pos) : first(first_key(pos, p.window, p.rule.chunked)) {
     ahead = p.ahead.count(first);
-    n = ahead + pos + 1 - (pages ? first & ~15 : first);
+    n = ahead + pos + 1 - first;
   }
 };
 // row of key k of what a row sees; `pooled`: in the caches of the blocks
@@ -277,7 +279,9 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 // requested behind them) and the merge (a warp a head; parts pushed to the CTA that adds them up, one cluster barrier). 16 query heads over 4: 64 rows of 2560
 // keys (335 MB) 376 us on the CUDA cores, 96 before these, 75 now (4.5 TB/s); 64 rows of 1250, 32 heads 65 -> 49; one row of 2000 keys 10.8 -> 8.0, of
 // 4000 16.2 -> 11.0; 8 rows of 1900 15.7 -> 15.5. A third stage of keys or a third CTA an SM gave nothing.
-// PAGES: where pages hold a multiple of 16 positions a tile is 16 positions from a multiple of 16 on: rows one behind the other, one page to look up, no masks inside.
+// PAGES: where pages hold a multiple of 16 positions a tile is rows that lie one behind the other in one page, with no masks inside; behind a window that begins inside
+// sixteen positions, the last of one page's and the first of the next one's. (Tiles from a multiple of sixteen on counted up to 15 keys more than the window has, a tile
+// more and, in whole rounds of a CTA, up to twice the share: windows of 512, eight splits, four rows of four kv heads 7.7 us so, 6.9 now, six 8.2 and 7.0.)
 // Every product of sixteen is added to its f32 sum outside the tensor core, scores in two sums each: the tensor core cuts off what it adds up, and chains of its
 // products left results 0.6e-6 to 1.9e-6 off, where these are 2.5e-7 to 4.2e-7 and FMAs 2.4e-7 to 4.4e-7. Against two terms of a weight and chains: 64 rows of up
 // to 4096 keys 91.2 -> 92.8 us; groups of eight (over one kv head) 32.9 -> 35.0 us.
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   const int pos = p.positions[t], slot = p.slots[t];
   if (pos < 0) return;
   if (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  const Seen seen(p, pos, PAGES);
+  const Seen seen(p, pos);
   const int n = seen.n, per = p.per_split(n), k_begin = split * per;
   if (!CLUSTER && k_begin >= n) return;
   const int k_end = min(n, k_begin + per);
@@ -341,58 +345,78 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   for (int i = 0; i < HD / 8; ++i) acc[i][0] = acc[i][1] = 0.f;
 
   const uint32_t ring = smem_addr(smem_raw) + warp * S::STAGES * S::STAGE;
-  const long kv_elems = (long)p.Hkv * HD;
+  const int kv_elems = p.Hkv * HD;
   const int first = k_begin + warp * S::KEYS, stride = S::WARPS * S::KEYS;
-  // PAGES: sixteen positions that lie one behind the other in a page, from a multiple of sixteen on (first row; -1: nowhere). Keys ahead of the first one and behind
-  // the last one are not there
-  const int base = PAGES ? (seen.first & ~15) + first : 0;
-  auto there = [&](int i, int key) { return base + i * stride + key >= seen.first && base + i * stride + key <= pos; };
+  // PAGES: a tile's positions are base + i * stride on; its keys before `cut` lie in the page of the first of them, the others in that of the last. Behind `pos` is nothing
+  const int base = PAGES ? seen.first + first : 0, cut = 16 - (base & 15);
+  auto there = [&](int i, int key) { return base + i * stride + key <= pos; };
   const int tiles = first < k_end ? (k_end - first + stride - 1) / stride : 0;
   // pages of 32 tiles, one a lane: one trip to memory for all of them
-  auto page_of = [&](int i) {
-    const int at = base + i * stride;
+  auto page_of = [&](int i, int key) {
+    const int at = base + i * stride + key;
     if (i >= tiles || at > pos) return -1;
     const int lp = p.page_shift >= 0 ? at >> p.page_shift : at / p.page_tokens, page = lp < p.max_pages ? p.page_table[(long)slot * p.max_pages + lp] : -1;
     if (page >= 0 && page < p.num_pages) return page;
     if (p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
     return -1;
   };
-  int page = PAGES ? page_of(lane) : 0;
-  // where key `first + i * stride + (lane & 15)` lies: 2 * row + (1: among the blocks); -1: nowhere. PAGES: the tile's first row
-  auto locate = [&](int i) -> long {
-    if (PAGES) {
-      if (i && (i & 31) == 0) page = page_of(i + lane);
-      const int at = base + i * stride, its = __shfl_sync(0xffffffffu, page, i & 31);
-      return its < 0 ? -1 : (long)its * p.page_tokens + (p.page_shift >= 0 ? at & (p.page_tokens - 1) : at % p.page_tokens);
-    }
-    const int k = first + i * stride + (lane & 15);
-    if (k >= k_end) return -1;
-    bool pooled;
-    const long r = key_row(p, seen, k, slot, &pooled);
-    if (r < 0) {
-      if (lane < 16 && p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
-      return -1;
-    }
-    return 2 * r + pooled;
+  int page = PAGES ? page_of(lane, 0) : 0, page2 = PAGES && cut < 16 ? page_of(lane, cut) : page;
+  // Where a tile lies. PAGES: its key 0 by the page of the first keys and by that of the others (rows; NOWHERE: no such page). Otherwise key `first + i * stride +
+  // (lane & 15)`: 2 * row + (1: among the blocks); -1: nowhere
+  constexpr int NOWHERE = INT_MIN;
+  struct Rows {
+    int a, b;
   };
-  auto load = [&](int stage, int i, long where) {
+  using Where = std::conditional_t<PAGES, Rows, long>;
+  auto locate = [&](int i) -> Where {
+    if constexpr (PAGES) {
+      if (i && (i & 31) == 0) {
+        page = page_of(i + lane, 0);
+        page2 = cut < 16 ? page_of(i + lane, cut) : page;
+      }
+      const int at = base + i * stride, its = __shfl_sync(0xffffffffu, page, i & 31), its2 = __shfl_sync(0xffffffffu, page2, i & 31);
+      auto in_page = [&](int x) { return p.page_shift >= 0 ? x & (p.page_tokens - 1) : x % p.page_tokens; };
+      Rows r{its < 0 ? NOWHERE : its * p.page_tokens + in_page(at), NOWHERE};
+      if (cut == 16) r.b = r.a;
+      else if (its2 >= 0) r.b = its2 * p.page_tokens + in_page(at + cut) - cut;
+      return r;
+    } else {
+      const int k = first + i * stride + (lane & 15);
+      if (k >= k_end) return -1;
+      bool pooled;
+      const long r = key_row(p, seen, k, slot, &pooled);
+      if (r < 0) {
+        if (lane < 16 && p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
+        return -1;
+      }
+      return 2 * r + pooled;
+    }
+  };
+  auto live_key = [&](const Where& where, int i, int key) {
+    if constexpr (PAGES) return (key < cut ? where.a : where.b) != NOWHERE && there(i, key);
+    else return __shfl_sync(0xffffffffu, where, key) >= 0;
+  };
+  auto whole_tile = [&](const Where& where, int i) {
+    if constexpr (PAGES) return where.a != NOWHERE && where.b != NOWHERE && there(i, S::KEYS - 1);
+    else return false;
+  };
+  auto load = [&](int stage, int i, const Where& where) {
     const uint32_t dst0 = ring + stage * S::STAGE;
     const int ch = lane % S::CH;
-    if (PAGES) {
+    if constexpr (PAGES) {
       constexpr int STEP = 32 / S::CH;
       const int key0 = lane / S::CH;
-      const long at = (where < 0 ? 0 : where + key0) * kv_elems + (long)kvh * HD + ch * 8;
-      const bool whole = where >= 0 && there(i, 0) && there(i, S::KEYS - 1);
+      const int column = kvh * HD + ch * 8;
+      const bool whole = whole_tile(where, i);
 #pragma unroll
       for (int j = 0; j < S::KEYS / STEP; ++j) {
         const int key = key0 + j * STEP;
         const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
-        const bool live = whole || (where >= 0 && there(i, key));
-        const long off = live ? at + (long)j * STEP * kv_elems : 0;
+        const bool live = whole || live_key(where, i, key);
+        const long off = live ? (long)((key < cut ? where.a : where.b) + key) * kv_elems + column : 0;
         copy16(dst, p.k_cache + off, live);
         copy16(dst + S::KEYS * S::ROW, p.v_cache + off, live);
       }
-      return;
     }
     if constexpr (!PAGES) {
 #pragma unroll
@@ -408,9 +432,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
       }
     }
   };
-  long at[S::STAGES];          // of the tiles in the ring, by stage
-#pragma unroll
-  for (int i = 0; i < S::STAGES; ++i) at[i] = -1;
+  Where at[S::STAGES] = {};          // of the tiles in the ring, by stage
 #pragma unroll
   for (int i = 0; i < S::STAGES - 1; ++i) {
     if (i < tiles) {
@@ -432,7 +454,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
         q[i][j] = gh >= G ? 0u : pairs ? *reinterpret_cast<const uint32_t*>(e) : (uint32_t)__bfloat16_as_ushort(e[0]) | (uint32_t)__bfloat16_as_ushort(e[1]) << 16;
       }
   }
-  long next = S::STAGES - 1 < tiles ? locate(S::STAGES - 1) : -1;
+  Where next = locate(S::STAGES - 1);
   for (int i0 = 0; i0 < tiles; i0 += S::STAGES) {
 #pragma unroll
     for (int st = 0; st < S::STAGES; ++st) {
@@ -445,7 +467,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
         load(to, i + AHEAD, next);
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
-      next = i + AHEAD + 1 < tiles ? locate(i + AHEAD + 1) : -1;
+      if (i + AHEAD + 1 < tiles) next = locate(i + AHEAD + 1);
       asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
       __syncwarp();
       const uint32_t kb = ring + st * S::STAGE, vb = kb + S::KEYS * S::ROW;
@@ -474,18 +496,13 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
       // this lane: keys c2, c2 + 1, c2 + 8, c2 + 9 of the tile against head gh
       float w[4];
       float mn = m;
-      const bool whole = PAGES && at[st] >= 0 && there(i, 0) && there(i, S::KEYS - 1);
+      const bool whole = whole_tile(at[st], i);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = c2 + (j >> 1) * 8 + (j & 1);
         w[j] = (s[j >> 1][j & 1] + s[j >> 1][2 + (j & 1)]) * p.scale;
-        if (PAGES) {
-          if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, pos - (base + i * stride + key));
-          if (!whole && (at[st] < 0 || !there(i, key))) w[j] = -INFINITY;
-        } else {
-          if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
-          if (__shfl_sync(0xffffffffu, at[st], key) < 0) w[j] = -INFINITY;
-        }
+        if (ruled) w[j] = ruled_score<true>(w[j], p.rule, slope, n - 1 - (first + i * stride + key));
+        if (!whole && !live_key(at[st], i, key)) w[j] = -INFINITY;
         mn = fmaxf(mn, w[j]);
       }
       mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
@@ -623,7 +640,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
 
 // grid (Hq, T), HD threads
 template <int HD>
-__global__ void gqa_merge_kernel(GqaParams p, int pages, bf16* out, long ldo) {
+__global__ void gqa_merge_kernel(GqaParams p, bf16* out, long ldo) {
   __shared__ float wgt[64];
   __shared__ float Ls;
   grid_dep_launch();
@@ -631,7 +648,7 @@ __global__ void gqa_merge_kernel(GqaParams p, int pages, bf16* out, long ldo) {
   const int h = blockIdx.x, t = blockIdx.y;
   const int pos = p.positions[t];
   if (pos < 0) return;
-  const int n = Seen(p, pos, pages != 0).n;
+  const int n = Seen(p, pos).n;
   const int per = p.per_split(n), ns = (n + per - 1) / per;
   const float* base = p.scratch + ((long)t * p.Hq + h) * p.max_splits * (HD + 2);
   if (threadIdx.x < 32) {      // up to 64 splits: two per lane
@@ -658,8 +675,8 @@ __global__ void gqa_merge_kernel(GqaParams p, int pages, bf16* out, long ldo) {
 }
 
 template <int HD>
-int launch_merge(const GqaParams& p, int pages, bf16* out, long ldo, cudaStream_t s) {
-  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, pages, out, ldo);
+int launch_merge(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
+  return launch_chain(gqa_merge_kernel<HD>, dim3(p.Hq, p.T), dim3(HD < 128 ? 64 : 128), 0, s, p, out, ldo);
 }
 template <int HD, int G>
 int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
@@ -668,7 +685,7 @@ int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   if (int rc = opt_in_smem(k, smem)) return rc;
   dim3 grid(p.max_splits, p.Hkv, p.T);
   if (int rc = launch_chain(k, grid, dim3(256), smem, s, p)) return rc;
-  return launch_merge<HD>(p, 0, out, ldo, s);
+  return launch_merge<HD>(p, out, ldo, s);
 }
 template <int HD, bool CLUSTER, bool WIDE, bool PAGES, int W>
 int launch_split(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
@@ -682,7 +699,7 @@ template <int HD, bool WIDE, bool PAGES>
 int launch_mma(const GqaParams& p, bool cluster, int warps, bf16* out, long ldo, cudaStream_t s) {
   if (cluster) return warps == 8 ? launch_split<HD, true, WIDE, PAGES, 8>(p, out, ldo, s) : launch_split<HD, true, WIDE, PAGES, 4>(p, out, ldo, s);
   if (int rc = launch_split<HD, false, WIDE, PAGES, 4>(p, out, ldo, s)) return rc;
-  return launch_merge<HD>(p, PAGES, out, ldo, s);
+  return launch_merge<HD>(p, out, ldo, s);
 }
 
 template <int HD>

@@ -218,3 +218,26 @@ def test_pages_windows_and_order(page, kv, group, hd, contexts, window, splits):
         # a rounding to bf16 (at most 2^-8 of the value); f32 scores, weights and sums (2^-18 of values up to 5 is ample)
         torch.testing.assert_close(out[t].double(), ref, rtol=2 ** -8, atol=2e-5)
     assert int(status) == 0
+
+
+def test_windows_take_the_parts_of_their_keys():
+    """A row that sees a window of keys is shared as so many keys, wherever among sixteen positions its first one is: 33 parts of 128 keys, no 34th for keys ahead of the window."""
+    from ironpangu_b200.ops.window_attn import gqa_window
+
+    window, hd, group, splits, page = 33 * 128, 64, 4, 64, 16
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(BF16)
+    for last in (6000, 6007, 6015):
+        pages = last // page + 1
+        kc, vc, q = rand(pages, page, 1, hd), rand(pages, page, 1, hd), rand(1, group * hd)
+        table = torch.randperm(pages, generator=g, device="cuda").int()[None]
+        pos, slots = torch.tensor([last], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        scratch = torch.full((group, splits, hd + 2), float("nan"), device="cuda")
+        out = torch.empty(1, group * hd, dtype=BF16, device="cuda")
+        gqa_window(q, kc, vc, pos, slots, table, heads=group, window=window, scale=hd ** -0.5, splits=splits, scratch=scratch, out=out)
+        assert int(scratch.isfinite().all(-1)[0].sum()) == 33
+        at = torch.arange(last + 1 - window, last + 1, device="cuda")
+        rows = table[0].long()[at // page] * page + at % page
+        ref = _reference(q.view(group, hd), kc.view(-1, 1, hd)[rows], vc.view(-1, 1, hd)[rows], hd ** -0.5).reshape(-1)
+        # a rounding to bf16; f32 scores, weights and sums
+        torch.testing.assert_close(out[0].double(), ref, rtol=2 ** -8, atol=2e-5)
