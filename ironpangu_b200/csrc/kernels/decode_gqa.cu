@@ -408,12 +408,23 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
       const int key0 = lane / S::CH;
       const int column = kvh * HD + ch * 8;
       const bool whole = whole_tile(where, i);
+      if (whole && where.a == where.b) {
+        const long at = (long)(where.a + key0) * kv_elems + column;
+#pragma unroll
+        for (int j = 0; j < S::KEYS / STEP; ++j) {
+          const int key = key0 + j * STEP;
+          const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
+          copy16(dst, p.k_cache + at + j * STEP * kv_elems, true);
+          copy16(dst + S::KEYS * S::ROW, p.v_cache + at + j * STEP * kv_elems, true);
+        }
+        return;
+      }
 #pragma unroll
       for (int j = 0; j < S::KEYS / STEP; ++j) {
         const int key = key0 + j * STEP;
         const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
         const bool live = whole || live_key(where, i, key);
-        const long off = live ? (long)((key < cut ? where.a : where.b) + key) * kv_elems + column : 0;
+        const long off = (long)(live ? (key < cut ? where.a : where.b) + key : 0) * kv_elems + column;
         copy16(dst, p.k_cache + off, live);
         copy16(dst + S::KEYS * S::ROW, p.v_cache + off, live);
       }
@@ -719,10 +730,14 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
       if (cluster) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
+        // 32 clusters of eight begin to get in one another's way (33 are all that run at once), 33 of four CTAs of eight warps do not: 32 rows of 1000 keys 9.0 us and 8.2,
+        // windows of 512 8.1 and 6.9, 33 rows of 2000 keys 13.0 and 11.5; from there on it is even, at 4000 keys 17.0 and 17.7.
+        if (p.max_splits == 8 && rows > 31 && rows <= 33 && (long)p.kps * asked <= 2048) p.max_splits = 4;
       }
-      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). Sixteen
-      // clusters of eight such CTAs do not fit the GPCs at once (4 rows of 1000 keys, four kv heads of two: 11.6 us by eight, 7.9 by four).
-      const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : 148) ? 8 : 4;
+      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). The clusters have to
+      // fit the GPCs at once, 15 of eight such CTAs and 33 of four (4 rows of 1000 keys, four kv heads of two, in sixteen of eight: 11.6 us by eight, 7.9 by four; 34 rows
+      // of 300 keys in 34 of four: 10.4 and 7.3).
+      const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : p.max_splits == 4 ? 132 : 148) ? 8 : 4;
       p.split_shift = log2_of(p.max_splits);
       // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
       // less than their order (60 rows of 100 keys 11.7 and 13.5)

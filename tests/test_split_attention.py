@@ -241,3 +241,28 @@ def test_windows_take_the_parts_of_their_keys():
         ref = _reference(q.view(group, hd), kc.view(-1, 1, hd)[rows], vc.view(-1, 1, hd)[rows], hd ** -0.5).reshape(-1)
         # a rounding to bf16; f32 scores, weights and sums
         torch.testing.assert_close(out[0].double(), ref, rtol=2 ** -8, atol=2e-5)
+
+
+@pytest.mark.parametrize("T,group,hd,window", [(31, 4, 128, 0), (32, 4, 128, 0), (33, 8, 64, 0), (33, 2, 128, 100), (34, 4, 128, 300), (37, 8, 128, 300)])
+def test_about_as_many_clusters_as_run_at_once(T, group, hd, window):
+    """Clusters of eight CTAs and of four, of eight warps and of four, over rows of one kv head (contexts to 600 keys)."""
+    from ironpangu_b200.ops.window_attn import gqa_window
+
+    g = torch.Generator(device="cuda").manual_seed(T + group)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(BF16)
+    contexts = [1 + (37 * t) % 600 for t in range(T)]
+    most = 38
+    kc, vc, q = rand(T * most, 16, 1, hd), rand(T * most, 16, 1, hd), rand(T, group * hd)
+    table = torch.randperm(T * most, generator=g, device="cuda").int().view(T, most)
+    pos, slots = torch.tensor([c - 1 for c in contexts], dtype=torch.int32, device="cuda"), torch.arange(T, dtype=torch.int32, device="cuda")
+    out = torch.empty(T, group * hd, dtype=BF16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    gqa_window(q, kc, vc, pos, slots, table, heads=group, window=window or 600, scale=hd ** -0.5, splits=((window or 600) + 63) // 64,
+               scratch=torch.empty(T * group * 16 * (hd + 2), device="cuda"), out=out, status_ptr=status.data_ptr())
+    for t, c in enumerate(contexts):
+        at = torch.arange(max(0, c - window) if window else 0, c, device="cuda")
+        rows = table[t].long()[at // 16] * 16 + at % 16
+        ref = _reference(q[t].view(group, hd), kc.view(-1, 1, hd)[rows], vc.view(-1, 1, hd)[rows], hd ** -0.5).reshape(-1)
+        # a rounding to bf16; f32 scores, weights and sums
+        torch.testing.assert_close(out[t].double(), ref, rtol=2 ** -8, atol=2e-5)
+    assert int(status) == 0
