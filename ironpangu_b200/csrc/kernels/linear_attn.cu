@@ -36,7 +36,7 @@ __device__ __forceinline__ float qk_value(const LaParams& p, const A* head, int 
 // HELD: heads of up to 128 columns, a multiple of four. A state stays in registers over the rows of a run and is requested ahead of everything that the rows need: its bytes
 // are what the launch is bound by (27 rows of 16 heads of 128: 57 MB, 17.2 -> 15.3 us).
 template <typename A, bool HELD>
-__global__ void __launch_bounds__(256, HELD ? 4 : 1) la_step_kernel(LaParams p, float* o, long ldo) {
+__global__ void __launch_bounds__(256, HELD ? 4 : 3) la_step_kernel(LaParams p, float* o, long ldo) {
   extern __shared__ float sm[];        // q [d], k [d]
   grid_dep_launch();
   grid_dep_wait();
