@@ -17,6 +17,7 @@
 // decay^n comes from a table [H, 129] made in double on the host. Chunk table: int32 [n, 4] = first row, rows, slot, 2 * chunks of
 // the run + 1 at the first chunk of a run and 0 at the others; the position of a run's first row from `positions`.
 #include "linear_attn.cuh"
+#include "tc_common.cuh"
 #include "ifab_kernels.h"
 
 using namespace ifab;
@@ -298,7 +299,9 @@ extern "C" int ifab_la_step(const void* proj, long ldp, int f32, int q_off, int 
   LaParams p{proj, ldp, q_off, k_off, v_off, H, d, e, {(const float2*)rope, rot, interleaved}, act, k_scale, powers, state, positions, slots, T};
   const dim3 grid(H, T, (e + 31) / 32);
   const size_t smem = (size_t)2 * d * sizeof(float);
-  const bool held = p.d % 4 == 0 && p.d <= 128;
+  // Four CTAs an SM hold a state, three do not: from a second wave of those on. us of rows of 16 heads of 128 (64 CTAs each), states from HBM, not held and held: 2 rows 3.8
+  // and 4.2, 6 rows 4.8 and 5.3, 7 rows 5.9 and 5.3, 16 rows 10.3 and 9.1
+  const bool held = p.d % 4 == 0 && p.d <= 128 && (long)H * T * ((e + 31) / 32) > 3l * tc::device_sms();
   if (f32) return held ? launch_chain(la_step_kernel<float, true>, grid, dim3(256), smem, (cudaStream_t)stream, p, o, ldo)
                        : launch_chain(la_step_kernel<float, false>, grid, dim3(256), smem, (cudaStream_t)stream, p, o, ldo);
   return held ? launch_chain(la_step_kernel<bf16, true>, grid, dim3(256), smem, (cudaStream_t)stream, p, o, ldo)

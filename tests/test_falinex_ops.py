@@ -108,6 +108,41 @@ def test_recurrence_forms_match_the_restatement(kind, H, d, e, T, rot):
                 compare(o.view(T, H, e), st, max(act_round, 1e-4 if tiles else 2e-5))
 
 
+@pytest.mark.parametrize("kind,H,d,e", [("rotated", 4, 128, 128), ("activated", 5, 96, 40), ("rotated", 2, 20, 9)])
+def test_steps_of_many_sequences_are_those_of_few(kind, H, d, e):
+    """Steps of more rows than a wave of CTAs hold a state in registers over a run, those of few do not: the same sums in the same order, so the same bits. Fresh rows, runs
+    of one to three rows, rows that are not there, states that are infinite where a row is fresh."""
+    from ironpangu_b200.ops import linear_attn as LA
+
+    T = 3 * 148 // (H * ((e + 31) // 32)) // 6 * 6 + 12
+    opts, proj, _, rot = _recurrence_case(kind, H, d, e, T)
+    mx = LA.DecayedMixer(device="cuda", **opts)
+    length = [1, 2, 3]
+    slots, positions = [], []
+    while len(slots) < T:
+        n = length[len(set(slots)) % 3]
+        slots += [len(set(slots))] * n
+        positions += list(range(len(slots) % 4, len(slots) % 4 + n))
+    slots, positions = slots[:T], positions[:T]
+    positions = [-1 if s % 7 == 5 else x for s, x in zip(slots, positions)]
+    tabs = LA.RotaryTables([(rot, 1e4)], T, "cuda")
+    pos, slot, p = _i32(positions), _i32(slots), proj.cuda()
+    tabs.fill(pos.clamp(min=0))
+    rope = tabs.get(rot, 1e4)
+    first = mx.state(max(slots) + 1, "cuda").normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+    fresh = [s for s, x in zip(slots, positions) if x == 0]
+    first[fresh] = float("inf")
+    many, few = first.clone(), first.clone()
+    o = [torch.full((T, H * e), 7.0, device="cuda") for _ in range(2)]
+    mx.step(p, many, pos, slot, rope, o[0])
+    r = 0
+    while r < T:
+        n = slots.count(slots[r])
+        mx.step(p[r:r + n], few, pos[r:r + n], slot[r:r + n], None if rope is None else rope[r:r + n], o[1][r:r + n])
+        r += n
+    assert fresh and -1 in positions and torch.equal(*o) and torch.equal(many, few) and bool(many[fresh].isfinite().all())
+
+
 def test_tiles_with_head_norm_and_gate_and_many_sequences():
     """Several sequences in one launch, normed and gated in the epilogue, equal each sequence alone."""
     from ironpangu_b200.ops import linear_attn as LA
