@@ -119,8 +119,11 @@ __device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int
   if (p.residual) {
     const bf16* r = p.residual + (long)row * p.ldr + col;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
+      uint4 u[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) add_residual8(v + 8 * i, reinterpret_cast<const uint4*>(r)[i]);
+      for (int i = 0; i < 4; ++i) u[i] = reinterpret_cast<const uint4*>(r)[i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add_residual8(v + 8 * i, u[i]);
     } else {
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = bf16_round(v[i]) + __bfloat162float(r[i]);
