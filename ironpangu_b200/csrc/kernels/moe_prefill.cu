@@ -63,6 +63,14 @@ __global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) 
   const int ranks = p.ranks, rank = blockIdx.x % ranks, t0 = blockIdx.x / ranks * T;
   const int share = p.E / ranks, e0 = rank * share;      // ranks divides E
   stage_x<T>(xs, p.x, p.ldx, t0, p.M, p.D, p.norm_w, p.eps, false, red);
+  auto store_xn = [&]() {            // the normalised rows are reused by the expert GEMMs
+    if (!p.xn) return;
+    for (int i = threadIdx.x; i < T * (p.D >> 3); i += blockDim.x) {
+      const int t = i / (p.D >> 3), c = i % (p.D >> 3);
+      if (t % ranks == rank && t0 + t < p.M) *reinterpret_cast<uint4*>(p.xn + (long)(t0 + t) * p.ldxn + c * 8) = *reinterpret_cast<const uint4*>(xs + (size_t)t * p.D + c * 8);
+    }
+  };
+  if (ranks == 1) store_xn();
   const int quads = p.D >> 2;
   for (int first = warp * EG; first < share; first += 16 * EG) {
     const float4* wr[EG];
@@ -108,12 +116,11 @@ __global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) 
       }
     }
   }
-  router_cluster_sync();             // the logits of every share, and all CTAs' rows of x read (xn may be x)
-  if (p.xn) {   // the normalised rows are reused by the expert GEMMs
-    for (int i = threadIdx.x; i < T * (p.D >> 3); i += blockDim.x) {
-      const int t = i / (p.D >> 3), c = i % (p.D >> 3);
-      if (t % ranks == rank && t0 + t < p.M) *reinterpret_cast<uint4*>(p.xn + (long)(t0 + t) * p.ldxn + c * 8) = *reinterpret_cast<const uint4*>(xs + (size_t)t * p.D + c * 8);
-    }
+  if (ranks > 1) {
+    router_cluster_sync();           // the logits of every share, and all CTAs' rows of x read (xn may be x)
+    store_xn();
+  } else {
+    __syncthreads();
   }
   const int t = warp * ranks + rank;
   constexpr int PER = 8;
@@ -122,10 +129,10 @@ __global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) 
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int ei = lane + 32 * i;
-    score[i] = (t < T && ei < p.E) ? ld_of_rank(lg + t * share + ei % share, ei / share) : -INFINITY;
+    score[i] = (t < T && ei < p.E) ? (ranks > 1 ? ld_of_rank(lg + t * share + ei % share, ei / share) : lg[t * share + ei]) : -INFINITY;
     mx = fmaxf(mx, score[i]);
   }
-  router_cluster_sync();             // no CTA leaves while another reads its share
+  if (ranks > 1) router_cluster_sync();             // no CTA leaves while another reads its share
   if (t >= T || t0 + t >= p.M) return;
   mx = warp_max(mx);
   float denom = 0.f;
@@ -360,15 +367,20 @@ template <int T, int EG>
 int launch_router_of(const RouterBlockParams& p, size_t smem, cudaStream_t s) {
   // opened for all experts in a CTA, whatever this chunk's share: by the share, a thread with another chunk would close it for this launch
   if (int rc = opt_in_smem(router_block_kernel<T, EG>, (size_t)T * (p.D * sizeof(bf16) + p.E * sizeof(float)))) return rc;
-  return launch_chain_cluster(router_block_kernel<T, EG>, dim3((p.M + T - 1) / T * p.ranks), dim3(512), (unsigned)p.ranks, smem, s, p);
+  const dim3 grid((p.M + T - 1) / T * p.ranks);
+  return p.ranks > 1 ? launch_chain_cluster(router_block_kernel<T, EG>, grid, dim3(512), (unsigned)p.ranks, smem, s, p) : launch_chain(router_block_kernel<T, EG>, grid, dim3(512), smem, s, p);
 }
 // As many CTAs (a power of two that divides the experts, up to 8) share a block's experts as leave every CTA an SM of its own (a CTA costs 16 us beside its
-// experts' 38 us at 96 x 4096, so a second wave of smaller shares gains nothing: 1200 tokens by 1 105 us, by 2 three waves of 36); a warp's experts in as few
-// passes of up to four as they take, all as wide.
+// experts' 38 us at 96 x 4096, so a second wave of smaller shares gains nothing: 1200 tokens by 1 105 us, by 2 three waves of 36).
+int router_ranks(int M, int E, int T) {
+  int ranks = 1;
+  while (ranks < 8 && (long)((M + T - 1) / T) * 2 * ranks <= 148 && E % (2 * ranks) == 0) ranks *= 2;
+  return ranks;
+}
+// a warp's experts in as few passes of up to four as they take, all as wide
 template <int T>
-int launch_router(RouterBlockParams p, cudaStream_t s) {
-  p.ranks = 1;
-  while (p.ranks < 8 && (long)((p.M + T - 1) / T) * 2 * p.ranks <= 148 && p.E % (2 * p.ranks) == 0) p.ranks *= 2;
+int launch_router(RouterBlockParams p, int ranks, cudaStream_t s) {
+  p.ranks = ranks;
   const int share = p.E / p.ranks, a_warp = (share + 15) / 16, passes = (a_warp + 3) / 4, width = (a_warp + passes - 1) / passes;
   const size_t smem = (size_t)T * p.D * sizeof(bf16) + (size_t)T * share * sizeof(float);
   return width == 1 ? launch_router_of<T, 1>(p, smem, s) : width == 2 ? launch_router_of<T, 2>(p, smem, s) : width == 3 ? launch_router_of<T, 3>(p, smem, s)
@@ -383,9 +395,14 @@ extern "C" int ifab_router_block(const void* x, long ldx, const void* norm_w, fl
   if (M < 1 || E > 256 || topk > MAX_TOPK || topk > E || D % 8) return -1;
   const RouterBlockParams p{(const bf16*)x, ldx, (const bf16*)norm_w, eps, w_router, bias, logits, ids, wts, (bf16*)xn, ldxn,
                             M, D, E, topk, scoring, renorm, scale, 1};
-  // Rows of eight tokens up to 14000 columns; wider ones run four tokens per CTA, up to ~1200 tokens
-  if ((M + 7) / 8 >= 148 || (size_t)8 * (D * sizeof(bf16) + E * sizeof(float)) <= 224 * 1024) return launch_router<8>(p, (cudaStream_t)stream);
-  return launch_router<4>(p, (cudaStream_t)stream);
+  // From ~1200 tokens on eight a CTA; below, four where that takes no more waves, and where rows of eight do not fit. A warp multiplies its experts with all tokens of
+  // its CTA, so what has at most one expert a warp gains nothing by sharing them (8 experts x 4096, 200 tokens: eight tokens in shares of two 24.9 us, four tokens by all
+  // eight 14.6). From a second pass of a warp on, twice as many shares for eight tokens are better (96 x 4096: 200 tokens 26.3 and 24.0, 300 tokens, where
+  // four leave no CTA for a share, 33.9 and 37.6; 64 x 4096 29.3 and 27.1).
+  const int ranks8 = router_ranks(M, E, 8), ranks4 = E <= 16 ? 1 : router_ranks(M, E, 4), a_warp = (E / ranks4 + 15) / 16;
+  const bool once = (M + 3) / 4 <= 148, wide = (size_t)8 * (D * sizeof(bf16) + E * sizeof(float)) > 224 * 1024;
+  if ((M + 7) / 8 < 148 && (wide || E <= 16 || (once && !(ranks8 > ranks4 && a_warp > 4)))) return launch_router<4>(p, ranks4, (cudaStream_t)stream);
+  return launch_router<8>(p, ranks8, (cudaStream_t)stream);
 }
 
 extern "C" int ifab_moe_dispatch(const int32_t* ids, int M, int topk, int e0, int e_local, int32_t* counts, int32_t* route_row,

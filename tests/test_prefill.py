@@ -231,3 +231,9 @@ def test_forward_rows_matches_the_decode_kernels_on_independent_sequences():
         torch.testing.assert_close(a.caches[l].float(), b.caches[l].float(), rtol=2e-2, atol=2e-2)
     assert fab.status() == 0
     fab.close()
+
+
+@pytest.mark.parametrize("M,E,D,topk", [(1, 8, 256, 2), (1100, 16, 264, 4), (1190, 8, 256, 2), (200, 64, 512, 6), (200, 256, 264, 8), (590, 97, 256, 6), (593, 97, 256, 6), (330, 60, 264, 4)])
+def test_router_tokens_of_a_block(M, E, D, topk):
+    """Blocks of four tokens and of eight, on both sides of where one takes over: at most one expert a warp, shares, a second pass of a warp, more blocks than SMs."""
+    test_router_block_shares(M, E, D, topk, False)
