@@ -4,10 +4,11 @@
 // (scales[row][ceil(K / 128)]); the represented value is fp8(w[row][k]) * scale[row][k / 128]. Decode linears are bound
 // by the HBM stream of the weights, so halving the bytes of the expert matrices - 3/4 of the bytes a token touches in a
 // mixture-of-experts layer - is what this buys. Two forms:
-//   expert_gate_up_kernel, expert_down_kernel   one rank: every listed expert is streamed through rings in shared memory once for all
+//   expert_gate_up_kernel, expert_down_kernel (one rank)   every listed expert is streamed through rings in shared memory once for all
 //                       tokens that chose it, its weights widened once, and multiplied on the tensor cores
-//   the kernels that mirror the bf16 ones of decode_moe.cu (same grids, same routing inputs, same fused all-reduce)   several ranks, and
-//                       sizes whose rows don't fit beside the rings: every lane converts its 16-byte chunk (16 weights), forms the
+//   the kernels that mirror the bf16 ones of decode_moe.cu (same grids, same routing inputs, same fused all-reduce)   token by token: gate / up
+//                       where the caller says so (small experts, from four ranks on), for more than 1024 experts a rank and where a row doesn't fit
+//                       beside the rings; down on several ranks. Every lane converts its 16-byte chunk (16 weights), forms the
 //                       chunk's dot product with the activations staged in shared memory, and scales it once
 // Reference: W8A8 expert matrices of the 92B program (dequantising grouped matmul, native/src/token_executor.h:640-700).
 #include <cuda_fp8.h>
@@ -811,9 +812,9 @@ extern "C" int ifab_dequantize_fp8_block(const void* q, const float* scales, lon
   return launch_chain(dequantize_fp8_block_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (const uint8_t*)q, scales, rows, K, (bf16*)out);
 }
 
-extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F,
-                                           int topk, int e0, int e_local, const void* w_gu, const float* s_gu, const void* w_shared_gu,
-                                           const float* s_shared_gu, int Fs, void* act, void* stream) {
+namespace {
+int run_gate_up8(bool streamed, const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F, int topk, int e0, int e_local,
+                 const void* w_gu, const float* s_gu, const void* w_shared_gu, const float* s_shared_gu, int Fs, void* act, void* stream) {
   if (D % 16 != 0 || F % 16 != 0 || Fs % 16 != 0 || Fs > F) return -1;
   GateUp8Params p{(const bf16*)x, ldx, (const bf16*)norm_w, eps, ids, T, D, F, topk, e0, e_local,
                   (const uint8_t*)w_gu, s_gu, (const uint8_t*)w_shared_gu, s_shared_gu, Fs, (bf16*)act};
@@ -821,7 +822,7 @@ extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* 
   const uintptr_t bits = (uintptr_t)x | (uintptr_t)w_gu | (uintptr_t)w_shared_gu | (uintptr_t)norm_w;
   const size_t room = 232448 - 8192 - XP_RING - XP_RED, row = (size_t)((D * 2 + 127) / 128 * 128 + 16);
   const int at_once = (int)std::min<size_t>(RL_TOKENS, room / row);
-  if (T >= 1 && at_once >= 1 && topk >= 1 && topk <= MAX_TOPK8 && e_local >= 1 && e_local <= RL_EXPERTS && bits % 16 == 0 && ldx % 8 == 0) {
+  if (streamed && T >= 1 && at_once >= 1 && topk >= 1 && topk <= MAX_TOPK8 && e_local >= 1 && e_local <= RL_EXPERTS && bits % 16 == 0 && ldx % 8 == 0) {
     for (int t0 = 0; t0 < T; t0 += at_once) {
       GateUp8Params q = p;
       q.T = std::min(at_once, T - t0);
@@ -840,6 +841,19 @@ extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* 
   const size_t smem = (size_t)D * sizeof(bf16);
   if (int rc = opt_in_smem(moe_gate_up_fp8_kernel, smem)) return rc;
   return launch_chain(moe_gate_up_fp8_kernel, grid, dim3(256), smem, (cudaStream_t)stream, p);
+}
+}  // namespace
+
+extern "C" int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F,
+                                           int topk, int e0, int e_local, const void* w_gu, const float* s_gu, const void* w_shared_gu,
+                                           const float* s_shared_gu, int Fs, void* act, void* stream) {
+  return run_gate_up8(true, x, ldx, norm_w, eps, ids, T, D, F, topk, e0, e_local, w_gu, s_gu, w_shared_gu, s_shared_gu, Fs, act, stream);
+}
+// The same token by token: for small experts, and for steps whose other kernels stream through L1
+extern "C" int ifab_moe_gate_up_tokens_fp8(const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F,
+                                           int topk, int e0, int e_local, const void* w_gu, const float* s_gu, const void* w_shared_gu,
+                                           const float* s_shared_gu, int Fs, void* act, void* stream) {
+  return run_gate_up8(false, x, ldx, norm_w, eps, ids, T, D, F, topk, e0, e_local, w_gu, s_gu, w_shared_gu, s_shared_gu, Fs, act, stream);
 }
 
 extern "C" int ifab_moe_down_allreduce_decode_fp8(const void* act, const int32_t* ids, const float* wts, int T, int D, int F, int topk,

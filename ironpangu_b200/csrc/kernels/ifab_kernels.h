@@ -71,6 +71,10 @@ int ifab_dequantize_fp8_block(const void* q, const float* scales, long rows, int
 int ifab_moe_gate_up_decode_fp8(const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F, int topk, int e0,
                                 int e_local, const void* w_gu, const float* s_gu, const void* w_shared_gu, const float* s_shared_gu, int Fs, void* act,
                                 void* stream);
+/* token by token instead of every chosen expert once: for small experts, and for steps whose other kernels stream through L1 */
+int ifab_moe_gate_up_tokens_fp8(const void* x, long ldx, const void* norm_w, float eps, const int32_t* ids, int T, int D, int F, int topk, int e0,
+                                int e_local, const void* w_gu, const float* s_gu, const void* w_shared_gu, const float* s_shared_gu, int Fs, void* act,
+                                void* stream);
 int ifab_moe_down_allreduce_decode_fp8(const void* act, const int32_t* ids, const float* wts, int T, int D, int F, int topk, int e0, int e_local,
                                        const void* w_down, const float* s_down, const void* w_shared_down, const float* s_shared_down, int Fs,
                                        const void* residual, long ldr, void* y, long ldy, const IfabFabric* fab, void* stream);

@@ -230,6 +230,9 @@ class MlaMoeDecoder:
         assert c.shared_ffn % (8 * self.world) == 0
         # linears as streams through shared memory beside expert kernels that stream so themselves; bf16 experts stream through L1
         self.rings = expert_fp8 and fabric.world == 1
+        # Gate / up between linears that stream through L1, a rank's experts of 96 (4096 x 1536, top 8), us of the three in a row for 1 / 2 / 4 / 8 tokens, rings and token by
+        # token: two ranks 34 / 52 / 77 / 130 and 32 / 51 / 86 / 154, four 32 / 43 / 61 / 108 and 30 / 39 / 62 / 115, eight 28 / 38 / 54 / 84 and 24 / 33 / 53 / 84
+        self.expert_rings = None if fabric.world <= 2 else False
         self.hl, self.el, self.vl = c.heads // self.world, c.experts // self.world, c.vocab // self.world
         self.T = max_tokens
         self.max_context = max_context
@@ -310,7 +313,7 @@ class MlaMoeDecoder:
         if self.expert_fp8:
             w8 = self.w8
             K.moe_gate_up_fp8(xn, self.route_ids[:T], w8[p + "gate_up"], self.rank * self.el,
-                              w_shared_gu=w8[p + "shared_gate_up"], act=self.act[:T])
+                              w_shared_gu=w8[p + "shared_gate_up"], act=self.act[:T], rings=self.expert_rings)
             K.moe_down_allreduce_fp8(self.act[:T], self.route_ids[:T], self.route_w[:T], w8[p + "down"], self.rank * self.el,
                                      fab, w_shared_down=w8[p + "shared_down"], residual=x, out=x)
             return

@@ -251,8 +251,12 @@ def dequantize_fp8_block(qs, out: Optional[torch.Tensor] = None) -> torch.Tensor
 
 
 def moe_gate_up_fp8(x: torch.Tensor, ids: torch.Tensor, w_gu, e0: int, *, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-5,
-                    w_shared_gu=None, act: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``moe_gate_up`` over block-scaled fp8 weights: ``w_gu`` and ``w_shared_gu`` are ``(q, scales)`` pairs."""
+                    w_shared_gu=None, act: Optional[torch.Tensor] = None, rings: Optional[bool] = None) -> torch.Tensor:
+    """``moe_gate_up`` over block-scaled fp8 weights: ``w_gu`` and ``w_shared_gu`` are ``(q, scales)`` pairs. ``rings``: every chosen expert streams through shared
+    memory once, or token by token; ``None``: by what a token's experts have, whatever the number of tokens, so that a token's bits do not depend on it. Token by token
+    starts 2 us earlier, rings read shared experts once. us, rings and token by token, of 1 / 2 / 4 / 8 tokens (D x F, top-k and shared): 512 x 256, 2 + 1 (0.8 MB) 5.4 / 5.7 / 6.3 /
+    7.4 and 3.2 / 3.5 / 3.7 / 5.7; 1024 x 512, 2 + 1 (3.1 MB) 5.8 / 6.6 / 8.1 / 9.9 and 4.1 / 4.4 / 7.2 / 11.5, 4 + 1 (5.2 MB) 6.6 / 8.1 / 9.9 / 11.3 and 4.2 / 6.4 / 11.2 / 17.8;
+    4096 x 1536, 8 + 1 27.9 / 41.9 / 67.9 / 107 and 29.6 / 52.9 / 100 / 192."""
     T, D = x.shape
     topk = ids.shape[1]
     q, sc = w_gu
@@ -262,7 +266,10 @@ def moe_gate_up_fp8(x: torch.Tensor, ids: torch.Tensor, w_gu, e0: int, *, norm_w
     Fs = 0 if sq is None else sq.shape[0] // 2
     if act is None:
         act = torch.zeros(T, topk + 1, F, dtype=BF16, device=x.device)
-    check(_lib.load().ifab_moe_gate_up_decode_fp8(x.data_ptr(), _rows(x), _ptr(norm_w), eps, ids.data_ptr(), T, D, F, topk, e0, e_local,
+    if rings is None:
+        rings = 2 * D * (topk * F + Fs) > 4 << 20
+    fn = _lib.load().ifab_moe_gate_up_decode_fp8 if rings else _lib.load().ifab_moe_gate_up_tokens_fp8
+    check(fn(x.data_ptr(), _rows(x), _ptr(norm_w), eps, ids.data_ptr(), T, D, F, topk, e0, e_local,
                                                   q.data_ptr(), sc.data_ptr(), _ptr(sq), _ptr(ss), Fs, act.data_ptr(), _stream()),
           "moe_gate_up_fp8")
     return act

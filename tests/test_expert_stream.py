@@ -88,3 +88,50 @@ def test_threads_with_steps_of_different_widths():
     for t in threads:
         t.join()
     assert codes == {0}
+
+
+def test_rows_too_wide_for_one_launch():
+    """A launch has room for five rows of 9472 columns beside its rings: eight tokens take two, and each has what it has alone."""
+    from ironpangu_b200.ops import decode as K
+
+    test_lists_and_shares(8, 3, 2, 9472, 128, 128, True)
+    g = torch.Generator(device="cuda").manual_seed(9472)
+    rand = lambda *s: (torch.randn(*s, generator=g, device="cuda") * 0.05).to(BF16)
+    T, E, topk, D, F = 8, 3, 2, 9472, 128
+    x, gu, sgu, gain = rand(T, D) * 20, K.quantize_fp8_block(rand(E, 2 * F, D)), K.quantize_fp8_block(rand(2 * F, D)), rand(D) + 1
+    ids = torch.randint(0, E, (T, topk), generator=g, device="cuda").int()
+    act = K.moe_gate_up_fp8(x, ids, gu, 0, norm_w=gain, w_shared_gu=sgu)
+    for t in range(T):
+        assert torch.equal(act[t:t + 1], K.moe_gate_up_fp8(x[t:t + 1].clone(), ids[t:t + 1].clone(), gu, 0, norm_w=gain, w_shared_gu=sgu))
+
+
+@pytest.mark.parametrize("E,rings", [(1024, True), (1030, True), (1030, None), (1024, False)])
+def test_as_many_experts_as_a_list_has_and_more(E, rings):
+    """1024 experts are what a list of routes has room for; more take the form that goes token by token, as small ones do. Small whole numbers, so that every sum is exact
+    in either."""
+    from ironpangu_b200.ops import decode as K
+    from ironpangu_b200.parallel.fabric import Fabric
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    whole = lambda *s, top: torch.randint(-top, top + 1, s, generator=g, device="cuda").float()
+    T, topk, D, F = 3, 4, 64, 16
+    x, act_in = whole(T, D, top=1).to(BF16), whole(T, topk + 1, F, top=1).to(BF16)
+    ids = torch.stack([torch.randperm(1020, generator=g, device="cuda")[:topk] for _ in range(T)]).int()
+    ids[0] = torch.tensor([E - 1, E - 2, 0, 1023], device="cuda")
+    wts = 2.0 ** -torch.randint(0, 3, (T, topk), generator=g, device="cuda").float()
+    gu, dn = whole(E, 2 * F, D, top=4), whole(E, D, F, top=4)
+    fp8 = lambda w: (w.to(torch.float8_e4m3fn).view(torch.uint8), torch.full((*w.shape[:-1], 1), 0.25, device="cuda"))
+    fab = Fabric(0, 1)
+    act = K.moe_gate_up_fp8(x, ids, fp8(gu), 0, rings=rings)
+    y = K.moe_down_allreduce_fp8(act_in, ids, wts, fp8(dn), 0, fab)
+    for t in range(T):
+        total = torch.zeros(D, dtype=torch.float64, device="cuda")
+        for k in range(topk):
+            e = int(ids[t, k])
+            got = (gu[e].double() @ x[t].double() * 0.25).to(BF16).double()
+            a = torch.nn.functional.silu(got[:F]) * got[F:]
+            assert bool(((act[t, k].double() - a).abs() <= a.abs() * (2.0 ** -8 + 2.0 ** -18)).all())          # one rounding, and silu in f32
+            total += float(wts[t, k]) * (dn[e].double() @ act_in[t, k].double() * 0.25)
+        assert torch.equal(y[t].double(), total.to(BF16).double())
+    assert fab.status() == 0
+    fab.close()
