@@ -205,7 +205,7 @@ class DensePrefill:
                 K.gemv(self.act[:m], w[p + "down"], residual=x, out=x, rings=True)
             else:
                 G.gemm(self.act[:m], w[p + "down"], residual=x, out=x, status_ptr=st, fixed=True)
-        self.launches = 1 + c.layers * (8 + 2 * ((m + self.QC - 1) // self.QC))
+        self.launches = 1 + c.layers * ((4 if self._few(m, w["layers.0.qkv"]) else 7) + 2 * ((m + self.QC - 1) // self.QC))
         return x
 
     # -- sequence parallel ------------------------------------------------------------------------------------------------

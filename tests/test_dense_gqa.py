@@ -210,6 +210,35 @@ def test_tensor_core_prefill_matches_the_decode_path_and_the_oracle():
 
 
 @pytest.mark.gpu
+def test_launches_of_few_rows_are_counted_as_their_own(monkeypatch):
+    """Up to eight rows: projection (with norm, rotation and pages), output, gate / up (with norm) and down; more: seven launches. Attention counts as two."""
+    from ironpangu_b200.models import dense_prefill as D
+
+    cfg, _, fab, dec = _setup()
+    pre = D.DensePrefill(dec, max_rows=64, attn_rows=32)
+    calls = []
+
+    class Counted:
+        def __init__(self, module):
+            self.module = module
+
+        def __getattr__(self, name):
+            fn = getattr(self.module, name)
+            if not callable(fn):
+                return fn
+            return lambda *a, **k: (calls.append(name), fn(*a, **k))[1]
+
+    for module in ("K", "G", "N"):
+        monkeypatch.setattr(D, module, Counted(getattr(D, module)))
+    for m in (1, 8, 9, 40):
+        calls.clear()
+        pre._layers(m)
+        assert pre.launches == len(calls) + calls.count("gqa_decode_attention")
+    assert fab.status() == 0
+    fab.close()
+
+
+@pytest.mark.gpu
 def test_prompt_attention_on_the_tensor_cores_for_128_wide_heads():
     """Heads of 128 columns: prompt chunks gather the context (values transposed) and run the tcgen05 attention kernel in its
     grouped-query form. Same last-row logits as the oracle and the decode kernels, same caches; decode continues from it."""
