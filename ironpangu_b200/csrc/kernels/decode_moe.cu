@@ -575,7 +575,8 @@ __global__ void __launch_bounds__(256) argmax_rows_kernel(HeadParams p) {
   finish_argmax<8>(p, &is_last);
 }
 
-// What either form of the head asks of its sizes and of the room for the partial maxima: a place a token for every `rows` rows of the matrix
+// What the head takes, whichever form: rows of up to 226 KB together (neither form needs the limit, but what is taken does not depend on the form), and room for
+// the partial maxima: a place a token for every `rows` rows of the matrix
 int head_fits(const HeadParams& p, int T, int rows, uint64_t partial_bytes) {
   if ((size_t)T * (p.K * sizeof(bf16) + 33 * 4 + 64) > 232448) return (int)cudaErrorInvalidValue;
   return (uint64_t)((p.V + rows - 1) / rows) * T * sizeof(float2) > partial_bytes ? -5 : 0;
