@@ -12,7 +12,6 @@
 // Query rows carry their own position and sequence slot (continuous batching: rows of different
 // sequences and prefill chunks share one launch). Reference counterparts: attention_qk_prepare /
 // paged_attention_prepare composites (native/src/inferfabric_acl.cpp:1236-1433).
-#include <atomic>
 #include <climits>
 #include <type_traits>
 
@@ -265,7 +264,7 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
   }
 }
 
-// The same on the tensor cores, for heads of 64 or 128 columns and groups of up to eight query heads. A CTA of four or eight warps works on one split of
+// The same on the tensor cores, for heads of 64 or 128 columns and groups of up to eight query heads. A CTA of four warps works on one split of
 // one (row, kv head); every warp streams 16 keys and values at a time through a ring of its own in shared memory (cp.async, 16 bytes, no barrier
 // among the warps) and keeps a running maximum, sum and output, merged at the end.
 //
@@ -557,7 +556,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();             // the rings become the warps' results: [WARPS][8][HD], maxima and sums
+  __syncthreads();             // the rings become the warps' results: [4][8][HD], maxima and sums
   float* sm_acc = reinterpret_cast<float*>(smem_raw);
   __shared__ float sm_m[S::WARPS * 8], sm_l[S::WARPS * 8];
   if ((lane & 3) == 0) {
@@ -714,32 +713,6 @@ int launch_mma(const GqaParams& p, bool cluster, int warps, bf16* out, long ldo,
   return launch_merge<HD>(p, out, ldo, s);
 }
 
-// Clusters of `splits` CTAs (a power of two up to eight) of W warps that the current device runs at once: its GPCs, which differ, hold whole ones
-template <int HD, int W>
-int clusters_at_once(int splits) {
-  static std::atomic<int> known[16][4];        // by device; 0: not asked yet
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev)) return 0;
-  std::atomic<int>* place = dev < 16 ? &known[dev][log2_of(splits)] : nullptr;
-  if (place && (n = place->load(std::memory_order_relaxed))) return n;
-  constexpr int smem = MmaSplit<HD, W>::SMEM;
-  auto k = gqa_split_mma_kernel<HD, true, false, true, W>;
-  if (opt_in_smem(k, smem)) return 0;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits);
-  cfg.blockDim = dim3(32 * W);
-  cfg.dynamicSmemBytes = smem;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg)) return 0;
-  if (place) place->store(n, std::memory_order_relaxed);
-  return n;
-}
-
 template <int HD>
 int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
   const int G = p.Hq / p.Hkv;
@@ -753,40 +726,22 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
     if (bits % 16 == 0) {
       // A cluster of up to eight splits merges by itself, which saves the merge's launch. A few rows with long contexts take more splits than that: from
       // about 512 keys in each of eight on, more CTAs are worth the second launch (one row, four kv heads).
-      const long capacity = (long)p.kps * asked, most = p.window > 0 && p.window < capacity ? p.window : capacity;      // keys that a row sees at most
-      const bool cluster = rows >= 16 || capacity <= 4096;
-      int warps = 4;
+      const bool cluster = rows >= 16 || (long)p.kps * asked <= 4096;
       if (cluster) {
-        // As many warps a row as run at once, eight a CTA: clusters of CTAs of four, two an SM, get in one another's way before they stop fitting (31 and more of eight CTAs
-        // where 33 fit, 66 and more of four where 71 do); up to there eight of four are a little better than four of eight. us behind a small launch, heads of 128, rows
-        // of 500 and of 4000 keys:
-        //   16 rows  8 x 8 warps 13.0 23.4, 4 x 8 8.4 19.1, 8 x 4 8.5 18.7      33 rows  8 x 4 13.9 33.9, 4 x 8 9.0 19.7, 4 x 4 9.9 29.8
-        //   37 rows  4 x 8 14.0 35.2, 4 x 4 10.0 30.1, 2 x 8 10.0 31.0          71 rows  4 x 4 16.3 52.6, 2 x 8 12.0 33.4, 2 x 4 13.1 50.8
-        //   100 rows 2 x 8 17.7 59.4, 2 x 4 13.7 52.0, 1 x 8 13.9 54.5          15 rows  8 x 8 8.2 13.5, 8 x 4 8.3 18.0
-        // Two CTAs of eight warps share an SM with heads of 64, so that the same holds for the last tenth of what fits.
-        int splits = 1;
-        while (splits < 8 && 2 * splits <= asked) splits *= 2;
-        auto fits = [&](int n) {
-          const int at_once = clusters_at_once<HD, 8>(n);
-          return rows <= (HD == 64 ? at_once - at_once / 10 : at_once);
-        };
-        const int eight = HD == 128 && splits == 8 && !fits(8) ? clusters_at_once<HD, 4>(8) : 0;
-        while (splits > 1 && !fits(splits)) splits /= 2;
-        if (rows <= eight - eight / 10) {
-          splits = 8;
-        } else if (splits > 1 || (most > 64 && asked == 1 && fits(1))) {
-          warps = 8;
-        } else if (asked > 1 && (rows <= clusters_at_once<HD, 4>(2) || (rows < 296 && most > 1024))) {
-          // beyond what runs at once, two splits in the rows' order where rows may be long: 64 rows of four kv heads of 50 to 200 keys 18.4 us so and 14.5 by one
-          // split, of 250 to 1000 30.0 and 29.8, of 500 to 2000 42.9 and 50.5
-          splits = 2;
-        }
-        p.max_splits = splits;
-        // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; short rows cost less than their order (60 rows
-        // of 100 keys 11.7 and 13.5)
-        p.order = p.T <= 32 * warps && most > 512 && rows > (warps == 8 ? clusters_at_once<HD, 8>(splits) : clusters_at_once<HD, 4>(splits));
+        p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
+        while (p.max_splits > asked) p.max_splits /= 2;
+        // 32 clusters of eight begin to get in one another's way (33 are all that run at once), 33 of four CTAs of eight warps do not: 32 rows of 1000 keys 9.0 us and 8.2,
+        // windows of 512 8.1 and 6.9, 33 rows of 2000 keys 13.0 and 11.5; from there on it is even, at 4000 keys 17.0 and 17.7.
+        if (p.max_splits == 8 && rows > 31 && rows <= 33 && (long)p.kps * asked <= 2048) p.max_splits = 4;
       }
+      // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). The clusters have to
+      // fit the GPCs at once, 15 of eight such CTAs and 33 of four (4 rows of 1000 keys, four kv heads of two, in sixteen of eight: 11.6 us by eight, 7.9 by four; 34 rows
+      // of 300 keys in 34 of four: 10.4 and 7.3).
+      const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : p.max_splits == 4 ? 132 : 148) ? 8 : 4;
       p.split_shift = log2_of(p.max_splits);
+      // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
+      // less than their order (60 rows of 100 keys 11.7 and 13.5)
+      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > 296 && (long)p.kps * asked > 512;
       if (p.page_tokens % 16 == 0 && !p.ahead.any())
         return G == 8 ? launch_mma<HD, true, true>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, true>(p, cluster, warps, out, ldo, s);
       return G == 8 ? launch_mma<HD, true, false>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, false>(p, cluster, warps, out, ldo, s);
