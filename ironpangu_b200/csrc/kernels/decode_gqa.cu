@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
   }
 }
 
-// The same on the tensor cores, for heads of 64 or 128 columns and groups of up to eight query heads. A CTA of four warps works on one split of
+// The same on the tensor cores, for heads of 64 or 128 columns and groups of up to eight query heads. A CTA of four or eight warps works on one split of
 // one (row, kv head); every warp streams 16 keys and values at a time through a ring of its own in shared memory (cp.async, 16 bytes, no barrier
 // among the warps) and keeps a running maximum, sum and output, merged at the end.
 //
@@ -279,12 +279,15 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 // requested behind them) and the merge (a warp a head; parts pushed to the CTA that adds them up, one cluster barrier). 16 query heads over 4: 64 rows of 2560
 // keys (335 MB) 376 us on the CUDA cores, 96 before these, 75 now (4.5 TB/s); 64 rows of 1250, 32 heads 65 -> 49; one row of 2000 keys 10.8 -> 8.0, of
 // 4000 16.2 -> 11.0; 8 rows of 1900 15.7 -> 15.5. A third stage of keys or a third CTA an SM gave nothing.
-// PAGES: where pages hold a multiple of 16 positions a tile is rows that lie one behind the other in one page, with no masks inside; behind a window that begins inside
-// sixteen positions, the last of one page's and the first of the next one's. (Tiles from a multiple of sixteen on counted up to 15 keys more than the window has, a tile
+// WITHIN, TWO: where pages hold a multiple of 16 positions a tile is rows that lie one behind the other in one page, with no masks inside; behind a window that begins
+// inside sixteen positions, the last of one page's and the first of the next one's (a form of its own: the choice of a page cost the others 0.3 us, one row of
+// 1000 keys 8.6 us and 8.3, 28 of 4000 keys 19.1 and 18.7). (Tiles from a multiple of sixteen on counted up to 15 keys more than the window has, a tile
 // more and, in whole rounds of a CTA, up to twice the share: windows of 512, eight splits, four rows of four kv heads 7.7 us so, 6.9 now, six 8.2 and 7.0.)
 // Every product of sixteen is added to its f32 sum outside the tensor core, scores in two sums each: the tensor core cuts off what it adds up, and chains of its
 // products left results 0.6e-6 to 1.9e-6 off, where these are 2.5e-7 to 4.2e-7 and FMAs 2.4e-7 to 4.4e-7. Against two terms of a weight and chains: 64 rows of up
 // to 4096 keys 91.2 -> 92.8 us; groups of eight (over one kv head) 32.9 -> 35.0 us.
+// Where a tile's sixteen keys lie: ANY one of its own; WITHIN a page, one behind the other; in a page or the last of one and the first of another (TWO)
+enum class Tiles { ANY, WITHIN, TWO };
 template <int HD, int W>
 struct MmaSplit {
   static constexpr int KEYS = 16, WARPS = W, STAGES = 2, CH = HD / 8;      // CH: 16-byte chunks of a row
@@ -309,10 +312,11 @@ __device__ __forceinline__ void st_peer2(float* mine, uint32_t rank, float a, fl
 
 // CLUSTER: the splits of a (row, kv head) are one cluster (at most eight) and merge their parts over distributed shared memory into `out`; otherwise
 // the parts go to the scratch and gqa_merge_kernel follows.
-template <int HD, bool CLUSTER, bool WIDE, bool PAGES, int W>
+template <int HD, bool CLUSTER, bool WIDE, Tiles TILES, int W>
 __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_mma_kernel(GqaParams p, bf16* res, long ldo) {
   using S = MmaSplit<HD, W>;
   constexpr int NT = 32 * W;
+  constexpr bool PAGES = TILES != Tiles::ANY, WITHIN = TILES == Tiles::WITHIN;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   grid_dep_launch();
   grid_dep_wait();
@@ -347,8 +351,8 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   const uint32_t ring = smem_addr(smem_raw) + warp * S::STAGES * S::STAGE;
   const int kv_elems = p.Hkv * HD;
   const int first = k_begin + warp * S::KEYS, stride = S::WARPS * S::KEYS;
-  // PAGES: a tile's positions are base + i * stride on; its keys before `cut` lie in the page of the first of them, the others in that of the last. Behind `pos` is nothing
-  const int base = PAGES ? seen.first + first : 0, cut = 16 - (base & 15);
+  // PAGES (WITHIN and TWO): a tile's positions are base + i * stride on; its keys before `cut` lie in the page of the first of them, the others in that of the last. Behind `pos` is nothing
+  const int base = PAGES ? seen.first + first : 0, cut = WITHIN ? 16 : 16 - (base & 15);
   auto there = [&](int i, int key) { return base + i * stride + key <= pos; };
   const int tiles = first < k_end ? (k_end - first + stride - 1) / stride : 0;
   // pages of 32 tiles, one a lane: one trip to memory for all of them
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
     if (p.status) atomicOr(p.status, IFAB_STATUS_BAD_INDEX);
     return -1;
   };
-  int page = PAGES ? page_of(lane, 0) : 0, page2 = PAGES && cut < 16 ? page_of(lane, cut) : page;
+  int page = PAGES ? page_of(lane, 0) : 0, page2 = PAGES && !WITHIN && cut < 16 ? page_of(lane, cut) : page;
   // Where a tile lies. PAGES: its key 0 by the page of the first keys and by that of the others (rows; NOWHERE: no such page). Otherwise key `first + i * stride +
   // (lane & 15)`: 2 * row + (1: among the blocks); -1: nowhere
   constexpr int NOWHERE = INT_MIN;
@@ -372,12 +376,12 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
     if constexpr (PAGES) {
       if (i && (i & 31) == 0) {
         page = page_of(i + lane, 0);
-        page2 = cut < 16 ? page_of(i + lane, cut) : page;
+        page2 = !WITHIN && cut < 16 ? page_of(i + lane, cut) : page;
       }
       const int at = base + i * stride, its = __shfl_sync(0xffffffffu, page, i & 31), its2 = __shfl_sync(0xffffffffu, page2, i & 31);
       auto in_page = [&](int x) { return p.page_shift >= 0 ? x & (p.page_tokens - 1) : x % p.page_tokens; };
       Rows r{its < 0 ? NOWHERE : its * p.page_tokens + in_page(at), NOWHERE};
-      if (cut == 16) r.b = r.a;
+      if (WITHIN || cut == 16) r.b = r.a;
       else if (its2 >= 0) r.b = its2 * p.page_tokens + in_page(at + cut) - cut;
       return r;
     } else {
@@ -393,11 +397,11 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
     }
   };
   auto live_key = [&](const Where& where, int i, int key) {
-    if constexpr (PAGES) return (key < cut ? where.a : where.b) != NOWHERE && there(i, key);
+    if constexpr (PAGES) return (WITHIN || key < cut ? where.a : where.b) != NOWHERE && there(i, key);
     else return __shfl_sync(0xffffffffu, where, key) >= 0;
   };
   auto whole_tile = [&](const Where& where, int i) {
-    if constexpr (PAGES) return where.a != NOWHERE && where.b != NOWHERE && there(i, S::KEYS - 1);
+    if constexpr (PAGES) return where.a != NOWHERE && (WITHIN || where.b != NOWHERE) && there(i, S::KEYS - 1);
     else return false;
   };
   auto load = [&](int stage, int i, const Where& where) {
@@ -408,7 +412,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
       const int key0 = lane / S::CH;
       const int column = kvh * HD + ch * 8;
       const bool whole = whole_tile(where, i);
-      if (whole && where.a == where.b) {
+      if (whole && (WITHIN || where.a == where.b)) {
         const long at = (long)(where.a + key0) * kv_elems + column;
 #pragma unroll
         for (int j = 0; j < S::KEYS / STEP; ++j) {
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
         const int key = key0 + j * STEP;
         const uint32_t dst = dst0 + key * S::ROW + ((ch ^ (key & 7)) << 4);
         const bool live = whole || live_key(where, i, key);
-        const long off = (long)(live ? (key < cut ? where.a : where.b) + key : 0) * kv_elems + column;
+        const long off = (long)(live ? (WITHIN || key < cut ? where.a : where.b) + key : 0) * kv_elems + column;
         copy16(dst, p.k_cache + off, live);
         copy16(dst + S::KEYS * S::ROW, p.v_cache + off, live);
       }
@@ -556,7 +560,7 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();             // the rings become the warps' results: [4][8][HD], maxima and sums
+  __syncthreads();             // the rings become the warps' results: [WARPS][8][HD], maxima and sums
   float* sm_acc = reinterpret_cast<float*>(smem_raw);
   __shared__ float sm_m[S::WARPS * 8], sm_l[S::WARPS * 8];
   if ((lane & 3) == 0) {
@@ -698,7 +702,7 @@ int launch_gqa(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   if (int rc = launch_chain(k, grid, dim3(256), smem, s, p)) return rc;
   return launch_merge<HD>(p, out, ldo, s);
 }
-template <int HD, bool CLUSTER, bool WIDE, bool PAGES, int W>
+template <int HD, bool CLUSTER, bool WIDE, Tiles PAGES, int W>
 int launch_split(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   constexpr int smem = MmaSplit<HD, W>::SMEM;
   const dim3 grid(p.max_splits, p.Hkv, p.T);
@@ -706,7 +710,7 @@ int launch_split(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   if (int rc = opt_in_smem(k, smem)) return rc;
   return CLUSTER ? launch_chain_cluster(k, grid, dim3(32 * W), (unsigned)p.max_splits, smem, s, p, out, ldo) : launch_chain(k, grid, dim3(32 * W), smem, s, p, out, ldo);
 }
-template <int HD, bool WIDE, bool PAGES>
+template <int HD, bool WIDE, Tiles PAGES>
 int launch_mma(const GqaParams& p, bool cluster, int warps, bf16* out, long ldo, cudaStream_t s) {
   if (cluster) return warps == 8 ? launch_split<HD, true, WIDE, PAGES, 8>(p, out, ldo, s) : launch_split<HD, true, WIDE, PAGES, 4>(p, out, ldo, s);
   if (int rc = launch_split<HD, false, WIDE, PAGES, 4>(p, out, ldo, s)) return rc;
@@ -730,21 +734,26 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
       if (cluster) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
-        // 32 clusters of eight begin to get in one another's way (33 are all that run at once), 33 of four CTAs of eight warps do not: 32 rows of 1000 keys 9.0 us and 8.2,
-        // windows of 512 8.1 and 6.9, 33 rows of 2000 keys 13.0 and 11.5; from there on it is even, at 4000 keys 17.0 and 17.7.
-        if (p.max_splits == 8 && rows > 31 && rows <= 33 && (long)p.kps * asked <= 2048) p.max_splits = 4;
+        // 32 clusters of eight begin to get in one another's way (33 are all that run at once), 33 of four CTAs of eight warps do not: windows of 512, 32 rows
+        // 8.1 us and 6.9. Rows without a window keep their eight parts, and so their bits, although four are as good or better here and beyond (32 rows of 1000 keys 9.0 and 8.2)
+        if (p.max_splits == 8 && rows > 31 && rows <= 33 && p.window > 0 && (long)p.kps * asked <= 2048) p.max_splits = 4;
       }
       // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). The clusters have to
       // fit the GPCs at once, 15 of eight such CTAs and 33 of four (4 rows of 1000 keys, four kv heads of two, in sixteen of eight: 11.6 us by eight, 7.9 by four; 34 rows
       // of 300 keys in 34 of four: 10.4 and 7.3).
       const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : p.max_splits == 4 ? 132 : 148) ? 8 : 4;
       p.split_shift = log2_of(p.max_splits);
-      // more CTAs than run at once: 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
+      // more CTAs than run at once (two an SM, heads of 64 four): 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
       // less than their order (60 rows of 100 keys 11.7 and 13.5)
-      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > 296 && (long)p.kps * asked > 512;
-      if (p.page_tokens % 16 == 0 && !p.ahead.any())
-        return G == 8 ? launch_mma<HD, true, true>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, true>(p, cluster, warps, out, ldo, s);
-      return G == 8 ? launch_mma<HD, true, false>(p, cluster, warps, out, ldo, s) : launch_mma<HD, false, false>(p, cluster, warps, out, ldo, s);
+      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > (HD == 64 ? 592 : 296) && (long)p.kps * asked > 512;
+      const Tiles tiles = p.page_tokens % 16 || p.ahead.any() ? Tiles::ANY : p.window > 0 ? Tiles::TWO : Tiles::WITHIN;
+      if (G == 8)
+        return tiles == Tiles::ANY      ? launch_mma<HD, true, Tiles::ANY>(p, cluster, warps, out, ldo, s)
+               : tiles == Tiles::WITHIN ? launch_mma<HD, true, Tiles::WITHIN>(p, cluster, warps, out, ldo, s)
+                                        : launch_mma<HD, true, Tiles::TWO>(p, cluster, warps, out, ldo, s);
+      return tiles == Tiles::ANY      ? launch_mma<HD, false, Tiles::ANY>(p, cluster, warps, out, ldo, s)
+             : tiles == Tiles::WITHIN ? launch_mma<HD, false, Tiles::WITHIN>(p, cluster, warps, out, ldo, s)
+                                      : launch_mma<HD, false, Tiles::TWO>(p, cluster, warps, out, ldo, s);
     }
   }
   switch (G) {

@@ -266,3 +266,11 @@ def test_about_as_many_clusters_as_run_at_once(T, group, hd, window):
         # a rounding to bf16; f32 scores, weights and sums
         torch.testing.assert_close(out[t].double(), ref, rtol=2 ** -8, atol=2e-5)
     assert int(status) == 0
+
+
+@pytest.mark.parametrize("T,kv,hd,longest", [(15, 1, 128, 300), (16, 1, 128, 300), (29, 1, 128, 300), (30, 1, 128, 300), (67, 1, 128, 300), (37, 2, 128, 300), (75, 1, 128, 300),
+                                             (37, 4, 128, 300), (149, 1, 128, 300), (75, 2, 128, 1100), (74, 4, 128, 100), (99, 3, 128, 100), (31, 1, 64, 300), (65, 1, 64, 300),
+                                             (67, 2, 64, 300), (149, 2, 64, 300)])
+def test_splits_and_warps_by_rows(T, kv, hd, longest):
+    """Both sides of where eight, four, two and one split of eight or four warps are taken, short and long rows of more than run at once."""
+    test_pages_windows_and_order(16, kv, 4, hd, [1 + (37 * t) % longest for t in range(T - 1)] + [longest], 0, 64 if longest > 1024 else 8)
