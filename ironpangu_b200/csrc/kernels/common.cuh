@@ -88,25 +88,36 @@ inline int launch_chain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// Same, with thread-block clusters of `cluster_x` CTAs along x (grid.x must be a multiple of it).
+// Same, with thread-block clusters of `cluster_x` CTAs along x (grid.x must be a multiple of it). `balanced`: clusters go where SMs are free, rather than where the
+// device's own preference puts them.
 template <typename... KArgs, typename... Args>
-inline int launch_chain_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster_x, size_t smem, cudaStream_t s,
-                                Args&&... args) {
+inline int launch_clusters(bool balanced, void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster_x, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cluster_x;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[3];
+  int n = 0;
+  attr[n].id = cudaLaunchAttributeClusterDimension;
+  attr[n].val.clusterDim.x = cluster_x;
+  attr[n].val.clusterDim.y = 1;
+  attr[n++].val.clusterDim.z = 1;
+  if (balanced) {
+    attr[n].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
+    attr[n++].val.clusterSchedulingPolicyPreference = cudaClusterSchedulingPolicyLoadBalancing;
+  }
+  if (pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = n;
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline int launch_chain_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, unsigned cluster_x, size_t smem, cudaStream_t s, Args&&... args) {
+  return launch_clusters(false, kernel, grid, block, cluster_x, smem, s, static_cast<Args&&>(args)...);
 }
 
 template <typename KernelT>

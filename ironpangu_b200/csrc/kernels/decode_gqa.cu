@@ -708,7 +708,9 @@ int launch_split(const GqaParams& p, bf16* out, long ldo, cudaStream_t s) {
   const dim3 grid(p.max_splits, p.Hkv, p.T);
   auto k = gqa_split_mma_kernel<HD, CLUSTER, WIDE, PAGES, W>;
   if (int rc = opt_in_smem(k, smem)) return rc;
-  return CLUSTER ? launch_chain_cluster(k, grid, dim3(32 * W), (unsigned)p.max_splits, smem, s, p, out, ldo) : launch_chain(k, grid, dim3(32 * W), smem, s, p, out, ldo);
+  // Balanced: by the device's preference about 30 clusters of eight CTAs ran at once where 33 fit, and the others waited for them. us behind a small launch, 4000 keys: 30 rows 21.5
+  // and 18.9, 33 rows 33.0 and 18.9, 8 rows of four kv heads 24.0 and 18.7
+  return CLUSTER ? launch_clusters(true, k, grid, dim3(32 * W), (unsigned)p.max_splits, smem, s, p, out, ldo) : launch_chain(k, grid, dim3(32 * W), smem, s, p, out, ldo);
 }
 template <int HD, bool WIDE, Tiles PAGES>
 int launch_mma(const GqaParams& p, bool cluster, int warps, bf16* out, long ldo, cudaStream_t s) {
@@ -734,9 +736,6 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
       if (cluster) {
         p.max_splits = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
         while (p.max_splits > asked) p.max_splits /= 2;
-        // 32 clusters of eight begin to get in one another's way (33 are all that run at once), 33 of four CTAs of eight warps do not: windows of 512, 32 rows
-        // 8.1 us and 6.9. Rows without a window keep their eight parts, and so their bits, although four are as good or better here and beyond (32 rows of 1000 keys 9.0 and 8.2)
-        if (p.max_splits == 8 && rows > 31 && rows <= 33 && p.window > 0 && (long)p.kps * asked <= 2048) p.max_splits = 4;
       }
       // Eight warps a CTA where all CTAs have an SM each: half as many tiles one after the other (one row of 4000 keys 16.1 us by four, 11.0 by eight). The clusters have to
       // fit the GPCs at once, 15 of eight such CTAs and 33 of four (4 rows of 1000 keys, four kv heads of two, in sixteen of eight: 11.6 us by eight, 7.9 by four; 34 rows
