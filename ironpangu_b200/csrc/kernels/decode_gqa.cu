@@ -321,20 +321,32 @@ __global__ void __launch_bounds__(32 * W, HD == 64 ? 16 / W : 8 / W) gqa_split_m
   grid_dep_launch();
   grid_dep_wait();
   const int split = blockIdx.x, kvh = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int t = blockIdx.z;
+  int t = blockIdx.z, pos, slot;
   if (p.order) {                   // the rows that see most first: a long one that starts last is what a launch waits for
-    __shared__ int s_n[NT], s_t;
-    const int mine = threadIdx.x < p.T ? p.positions[threadIdx.x] : -1;
-    const int seen_n = mine < 0 ? 0 : Seen(p, mine).n;
-    s_n[threadIdx.x] = seen_n;
+    __shared__ __align__(16) uint32_t s_key[NT];
+    __shared__ int s_row[3];
+    const int mine = threadIdx.x < p.T ? p.positions[threadIdx.x] : -1, its = threadIdx.x < p.T ? p.slots[threadIdx.x] : 0;
+    const uint32_t key = (uint32_t)(mine < 0 ? 0 : Seen(p, mine).n) << 8 | (255u - threadIdx.x);      // no two alike; at most 256 threads, fewer than 2^23 keys
+    s_key[threadIdx.x] = threadIdx.x < p.T ? key : 0;
     __syncthreads();
     int before = 0;
-    for (int i = 0; i < p.T; ++i) before += s_n[i] > seen_n || (s_n[i] == seen_n && i < (int)threadIdx.x);
-    if (threadIdx.x < p.T && before == t) s_t = threadIdx.x;
+    for (int i = 0; i < (p.T + 3) / 4; ++i) {
+      const uint4 k = reinterpret_cast<const uint4*>(s_key)[i];
+      before += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+    }
+    if (threadIdx.x < p.T && before == t) {
+      s_row[0] = threadIdx.x;
+      s_row[1] = mine;
+      s_row[2] = its;
+    }
     __syncthreads();
-    t = s_t;
+    t = s_row[0];
+    pos = s_row[1];
+    slot = s_row[2];
+  } else {
+    pos = p.positions[t];
+    slot = p.slots[t];
   }
-  const int pos = p.positions[t], slot = p.slots[t];
   if (pos < 0) return;
   if (CLUSTER) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const Seen seen(p, pos);
@@ -744,7 +756,7 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
       p.split_shift = log2_of(p.max_splits);
       // more CTAs than run at once (two an SM, heads of 64 four): 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
       // less than their order (60 rows of 100 keys 11.7 and 13.5)
-      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > (HD == 64 ? 592 : 296) && (long)p.kps * asked > 512;
+      p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > (HD == 64 ? 592 : 296) && (long)p.kps * asked > 512 && (long)p.kps * asked < 1 << 23;
       const Tiles tiles = p.page_tokens % 16 || p.ahead.any() ? Tiles::ANY : p.window > 0 ? Tiles::TWO : Tiles::WITHIN;
       if (G == 8)
         return tiles == Tiles::ANY      ? launch_mma<HD, true, Tiles::ANY>(p, cluster, warps, out, ldo, s)
