@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256) gqa_split_kernel(GqaParams p) {
 // Every product of sixteen is added to its f32 sum outside the tensor core, scores in two sums each: the tensor core cuts off what it adds up, and chains of its
 // products left results 0.6e-6 to 1.9e-6 off, where these are 2.5e-7 to 4.2e-7 and FMAs 2.4e-7 to 4.4e-7. Against two terms of a weight and chains: 64 rows of up
 // to 4096 keys 91.2 -> 92.8 us; groups of eight (over one kv head) 32.9 -> 35.0 us.
-// Where a tile's sixteen keys lie: ANY one of its own; WITHIN a page, one behind the other; in a page or the last of one and the first of another (TWO)
+// Where a tile's sixteen keys lie: each by itself (ANY), one behind the other in a page (WITHIN), or the first ones at the end of a page and the others in another (TWO)
 enum class Tiles { ANY, WITHIN, TWO };
 template <int HD, int W>
 struct MmaSplit {
@@ -755,7 +755,7 @@ int dispatch_g(GqaParams p, bf16* out, long ldo, cudaStream_t s) {
       const int warps = cluster && rows * p.max_splits <= (p.max_splits == 8 ? 120 : p.max_splits == 4 ? 132 : 148) ? 8 : 4;
       p.split_shift = log2_of(p.max_splits);
       // more CTAs than run at once (two an SM, heads of 64 four): 64 rows of 1000 to 4000 keys, two splits, 94 us in the rows' order, 82 so; 250 to 1000 keys 30.1 and 28.8; short rows cost
-      // less than their order (60 rows of 100 keys 11.7 and 13.5)
+      // less than their order (64 rows of four kv heads of 100 keys 15.1 and 16.2)
       p.order = cluster && p.T <= 32 * warps && rows * p.max_splits > (HD == 64 ? 592 : 296) && (long)p.kps * asked > 512 && (long)p.kps * asked < 1 << 23;
       const Tiles tiles = p.page_tokens % 16 || p.ahead.any() ? Tiles::ANY : p.window > 0 ? Tiles::TWO : Tiles::WITHIN;
       if (G == 8)

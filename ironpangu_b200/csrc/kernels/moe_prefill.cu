@@ -45,12 +45,12 @@ __device__ __forceinline__ void router_cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// A cluster per T tokens (8; 4 where the rows of 8 don't fit), each of its CTAs a share of the experts; a warp takes EG experts at a time through all
+// A cluster per T tokens (4 or 8), each of its CTAs a share of the experts; a warp takes EG experts at a time through all
 // columns, and after a cluster barrier warp t selects for a token from the shares' logits. Bound by the issue of its multiply-adds and by the router's rows
 // from L2. One CTA for all experts of 4 tokens read every row of the router in each of 128 CTAs (201 MB of L2 reads for 512 tokens) and unpacked the tokens'
 // bf16 columns anew for every expert; a share of the experts halves the reads, and EG experts at a time share the unpacked columns.
-// us before -> after, 96 experts x 4096: 16 tokens 49.3 -> 24.2, 256 67.6 -> 28.6, 512 82.5 -> 35.7, 1100 86.2 -> 55.1, 4096 280 -> 216; 512 tokens with 128 x 2048
-// 61.6 -> 29.7, 256 x 7168 334 -> 101. A sum's order is that of one expert and token alone, so shares and widths don't show in the results.
+// us before -> after, 96 experts x 4096: 16 tokens 49.3 -> 18.2, 256 67.6 -> 25.7, 512 82.5 -> 35.3, 1100 86.2 -> 52.9, 4096 280 -> 206; 512 tokens with 128 x 2048
+// 61.6 -> 27.4, 256 x 7168 334 -> 100. A sum's order is that of one expert and token alone, so shares and widths don't show in the results.
 template <int T, int EG>
 __global__ void __launch_bounds__(512) router_block_kernel(RouterBlockParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];

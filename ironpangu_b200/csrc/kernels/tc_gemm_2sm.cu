@@ -119,7 +119,7 @@ __device__ __forceinline__ void store_row32_2(const Gemm2Params& p, int row, int
   if (p.residual) {
     const bf16* r = p.residual + (long)row * p.ldr + col;
     if ((reinterpret_cast<uintptr_t>(r) & 15) == 0) {
-      uint4 u[4];
+      uint4 u[4];          // together: one after the other, four trips to L2 for 32 columns (2048 x 2048, K 64, f32 result: 18.3 us, 11.8 so)
 #pragma unroll
       for (int i = 0; i < 4; ++i) u[i] = reinterpret_cast<const uint4*>(r)[i];
 #pragma unroll
