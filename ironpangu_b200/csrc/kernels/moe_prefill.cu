@@ -1,6 +1,6 @@
 // Prefill-side MoE plumbing around the grouped tcgen05 GEMM (tc_grouped.cu), for chunks of hundreds of tokens:
 //
-//   router_block_kernel   f32 router projection + top-k for blocks of 8 tokens, the experts shared by a cluster (the decode router handles <= 8 rows
+//   router_block_kernel   f32 router projection + top-k for blocks of 4 or 8 tokens, the experts shared by a cluster (the decode router handles <= 8 rows
 //                         per launch; a prefill chunk would need 64 launches)
 //   moe_dispatch_kernel   routes of this rank's experts -> rows sorted by expert (stable: token-major inside an
 //                         expert), per-expert counts, the 128-row tile table of the grouped GEMM and, for every
